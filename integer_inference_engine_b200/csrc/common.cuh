@@ -133,6 +133,9 @@ __host__ __device__ __forceinline__ uint64_t balanced_digits8(int64_t x, bool &o
     return ((uint64_t)x + C) ^ C;
 }
 
+// Number of balanced digits in use in a packed digit word (highest non-zero digit + 1).
+__device__ __forceinline__ int digits_used(uint64_t d) { return d == 0 ? 1 : 8 - (__clzll((long long)d) >> 3); }
+
 // ---- warp-level integer MMA (legacy tensor path; the decode kernels are HBM-bound) ---------------------
 // D(16x8,s32) += A(16x32,u8,row) * B(32x8,s8,col)
 __device__ __forceinline__ void mma_u8s8_k32(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,

@@ -9,6 +9,14 @@ namespace iie {
 extern unsigned long long g_launches;
 inline void note_launch(unsigned long long n = 1) { __atomic_fetch_add(&g_launches, n, __ATOMIC_RELAXED); }
 
+// What a kernel that writes digit planes does beside them for the product behind it (Q1_0)
+struct PlaneDuties {
+    int *nl = nullptr;             // receives the digits in use (raised, never lowered)
+    int *nl_clear = nullptr;       // set to zero
+    int64_t *zero = nullptr;       // zero_n values set to zero
+    long long zero_n = 0;
+};
+
 enum SkinnyMode { MODE_LINEAR = 0, MODE_GATEUP = 1, MODE_DOWN = 2, MODE_FRONT = 3 };
 
 // Arguments of the streamed ("skinny") fused-dequant product.  Work is organised in groups: group g
@@ -215,9 +223,10 @@ cudaError_t launch_topk(const int64_t *logits, long long rows, int n_experts, in
 cudaError_t launch_rmsnorm(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
                            unsigned long long eps, int64_t *out, int *flags, cudaStream_t s);
 // the same with the normalised rows also (out may be NULL: only) written as Q1_0 activation operands: digit planes
-// [row][8][width] and 128-element block sums [row][width/128]; width must be a multiple of 128
+// [row][8][width] and 128-element block sums [row][width/128]; width must be a multiple of 128 (duties: see launch_q1_prep)
 cudaError_t launch_rmsnorm_planes(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
-                                  unsigned long long eps, int64_t *out, int8_t *planes, int64_t *totals, int *flags, cudaStream_t s);
+                                  unsigned long long eps, int64_t *out, int8_t *planes, int64_t *totals, int *flags, const PlaneDuties &duties,
+                                  cudaStream_t s);
 
 // Counting-sort dispatch of (token, slot) pairs by expert (single CTA, n_experts <= 1024).
 //   ids [T*k], gates [T*k] -> grp_off [E+1], pair_tok [T*k] (token of each sorted pair),
@@ -321,14 +330,30 @@ cudaError_t launch_decode(const DecodeArgs &a, int n_ctas, cudaStream_t s);
 // Q1_0 linear (q1.cu).  Units: 16-row tiles x 128-weight blocks, 256 B of sign bits in MMA order + 16 scales.
 size_t q1_unit_bytes(bool sc32);
 cudaError_t launch_q1_repack(const uint8_t *bits, const void *scale, int src_bits, bool sc32, long long out_f, long long nb,
-                             uint8_t *units, cudaStream_t s);
-cudaError_t launch_q1_prep(const int64_t *x, long long T, long long nb, int8_t *planes, int64_t *totals, int *nl_out,
+                             uint8_t *units, unsigned long long *max_scale, cudaStream_t s);
+// Digit planes [T][8][K] and block sums [T][nb] of T rows (with the wrapping SwiGLU of gate and up in front of them in the
+// second form).
+cudaError_t launch_q1_prep(const int64_t *x, long long T, long long nb, int8_t *planes, int64_t *totals, const PlaneDuties &duties,
                            cudaStream_t s);
-cudaError_t launch_q1_apply(const uint8_t *units, bool sc32, long long out_f, long long nb, const int8_t *planes,
-                            const int64_t *totals, long long T, long long frac, int64_t *out, cudaStream_t s,
-                            const int64_t *add = nullptr);
 cudaError_t launch_q1_prep_swiglu(const int64_t *gate, const int64_t *up, long long ld, int frac, long long T, long long nb,
-                                  int8_t *planes, int64_t *totals, cudaStream_t s);
+                                  int8_t *planes, int64_t *totals, const PlaneDuties &duties, cudaStream_t s);
+// Products of the same rows with up to three matrices of one width; out[T][out_f] = x W^T (+ add, which may be out itself).
+constexpr int Q1_MAX_PARTS = 3;
+struct Q1Part {
+    const uint8_t *units;
+    long long out_f;
+    int64_t *out;
+    const int64_t *add;
+    unsigned long long max_scale;  // largest |scale| of the matrix
+};
+constexpr int Q1_TC_CTAS = 148;    // one CTA per SM
+// Whether the products of T rows with matrices of `row_tiles` 128-row tiles in all add shares of a tile atomically: `out` then has
+// to hold zeros (or be `add`) when launch_q1_apply runs.
+bool q1_tc_split(long long row_tiles, long long T);
+cudaError_t launch_q1_apply(const Q1Part *parts, int n_parts, bool sc32, long long nb, const int8_t *planes, const int64_t *totals,
+                            long long T, long long frac, const int *nl, cudaStream_t s);
+cudaError_t launch_q1_tc(const Q1Part *parts, int n_parts, bool sc32, long long nb, const int8_t *planes, long long T, int sh,
+                         const int *nl_dev, cudaStream_t s);
 cudaError_t launch_rmsnorm_pair(const int64_t *x, long long rows_a, long long rows_b, long long width, const int64_t *gain_a,
                                 const int64_t *gain_b, int fa, unsigned long long eps, int64_t *out, int *flags, cudaStream_t s);
 bool attn_shape_ok(int n_heads, int n_kv, int head_dim);      // shapes launch_attn_decode accepts

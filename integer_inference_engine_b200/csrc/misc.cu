@@ -338,12 +338,15 @@ __device__ __forceinline__ int64_t norm_value(int64_t xv, unsigned long long rms
 __global__ void __launch_bounds__(1024) rmsnorm_kernel(const int64_t *x, long long rows, long long width, const int64_t *gain_a,
                                                        int fa, unsigned long long eps, int64_t *out, int *flags,
                                                        int8_t *planes, int64_t *totals, const int64_t *gain_b, long long rows_a,
-                                                       int split) {
+                                                       int split, const PlaneDuties duties) {
     // `split` CTAs share a row: each sums the squares of the whole row (cheap, the row sits in L2) and normalises its own
     // slice, so that the divisions of a long row are spread over several SMs
     __shared__ unsigned long long s_lo[32], s_hi[32], s_max[32], s_gmax[32];
     __shared__ unsigned long long s_rms, s_gm, s_inv;
     __shared__ int s_bad;
+    int *nl_out = duties.nl;
+    if (duties.nl_clear && blockIdx.x == 0 && threadIdx.x == 0) *duties.nl_clear = 0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < duties.zero_n; i += (long long)gridDim.x * blockDim.x) duties.zero[i] = 0;
     const long long row = blockIdx.x / split;
     const int part = blockIdx.x - (int)row * split;
     const int64_t *gain = row < rows_a ? gain_a : gain_b;
@@ -403,6 +406,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const int64_t *x, long lo
         // digit planes [row][8][width] and 128-element block sums of the normalised row, for the Q1_0 product
         const long long nb = width >> 7, per = (nb + split - 1) / split;
         const long long b_end = min(nb, (part + 1) * per);
+        int nl = 0;
         for (long long b = part * per + warp; b < b_end; b += nwarps) {
             const long long i0 = b * 128 + lane * 4;
             uint32_t pl[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -413,6 +417,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const int64_t *x, long lo
                 if (out) yr[i0 + j] = y;
                 bool ok;
                 const uint64_t d = balanced_digits8(y, ok);
+                nl = max(nl, ok ? digits_used(d) : 9);
                 sum += (unsigned long long)y;
 #pragma unroll
                 for (int l = 0; l < 8; l++) pl[l] |= (uint32_t)((d >> (8 * l)) & 0xFF) << (8 * j);
@@ -423,6 +428,8 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const int64_t *x, long lo
             for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
             if (lane == 0) totals[row * nb + b] = (int64_t)sum;
         }
+        nl = __reduce_max_sync(0xffffffffu, nl);
+        if (lane == 0 && nl_out && nl > *(volatile int *)nl_out) atomicMax(nl_out, nl);
     } else {
         const long long per = (width + split - 1) / split, i_end = min(width, (part + 1) * per);
         for (long long i = part * per + tid; i < i_end; i += blockDim.x)
@@ -545,7 +552,7 @@ cudaError_t launch_rmsnorm(const int64_t *x, long long rows, long long width, co
     const int split = (rows <= 16 && width >= 1024) ? (int)((width + 511) / 512) : 1;      // few long rows: 512 values per CTA
     const int threads = split > 1 ? 128 : (width >= 2048 ? 1024 : width > 128 ? 256 : 128);
     rmsnorm_kernel<<<(unsigned)(rows * split), threads, 0, s>>>(x, rows, width, gain, fa, eps, out, flags, nullptr, nullptr, nullptr, rows,
-                                                                 split);
+                                                                 split, PlaneDuties());
     note_launch();
     return cudaGetLastError();
 }
@@ -554,20 +561,20 @@ cudaError_t launch_rmsnorm_pair(const int64_t *x, long long rows_a, long long ro
                                 const int64_t *gain_b, int fa, unsigned long long eps, int64_t *out, int *flags, cudaStream_t s) {
     const int threads = width >= 2048 ? 1024 : width > 128 ? 256 : 128;
     rmsnorm_kernel<<<(unsigned)(rows_a + rows_b), threads, 0, s>>>(x, rows_a + rows_b, width, gain_a, fa, eps, out, flags, nullptr, nullptr,
-                                                                  gain_b, rows_a, 1);
+                                                                  gain_b, rows_a, 1, PlaneDuties());
     note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_rmsnorm_planes(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
-                                  unsigned long long eps, int64_t *out, int8_t *planes, int64_t *totals, int *flags, cudaStream_t s) {
+                                  unsigned long long eps, int64_t *out, int8_t *planes, int64_t *totals, int *flags, const PlaneDuties &duties, cudaStream_t s) {
     if (width <= 0 || (width & 127) || !planes || !totals) return cudaErrorInvalidValue;
     // one warp per 128-element block; few rows of a long row: four blocks per CTA, several CTAs per row
     const long long nb = width >> 7;
     const int split = (rows <= 16 && nb >= 8) ? (int)((nb + 3) / 4) : 1;
     const int threads = split > 1 ? 128 : (width >= 4096 ? 1024 : width >= 1024 ? (int)(width >> 2) : 256);
     rmsnorm_kernel<<<(unsigned)(rows * split), threads, 0, s>>>(x, rows, width, gain, fa, eps, out, flags, planes, totals, nullptr, rows,
-                                                                 split);
+                                                                 split, duties);
     note_launch();
     return cudaGetLastError();
 }

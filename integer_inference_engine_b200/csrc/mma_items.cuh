@@ -197,7 +197,4 @@ __device__ __forceinline__ int64_t recombine_cols(const unsigned long long *cols
     return (int64_t)(v >> fw);
 }
 
-// Number of balanced digits in use in a packed digit word (highest non-zero digit + 1).
-__device__ __forceinline__ int digits_used(uint64_t d) { return d == 0 ? 1 : 8 - (__clzll((long long)d) >> 3); }
-
 }  // namespace iie

@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <mutex>
 #include <vector>
 
@@ -21,6 +22,7 @@ namespace {
 struct Q1Weight {
     uint8_t *units = nullptr;
     long long out_f = 0, nb = 0;
+    unsigned long long max_scale = 0;
     bool sc32 = false;
     bool live = false;
 };
@@ -29,7 +31,7 @@ std::recursive_mutex q_mu;
 std::vector<Q1Weight> q_w;
 unsigned long long q_weight_bytes = 0;
 cudaStream_t q_stream = nullptr;
-int *q_cells = nullptr;                 // device ints: [0] digits in use, [1] rmsnorm flags
+int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [8..15] digits in use (a ring, see next_digits)
 int q_ready = -1;
 
 enum QRole { QR_X, QR_PLANES, QR_TOTALS, QR_OUT, QR_GAIN, QR_COUNT };
@@ -73,6 +75,46 @@ void *q_ensure(int role, size_t bytes) {
     return b.p;
 }
 
+// The cell that receives the digits in use of the next digit planes, and the one to clear for later: a ring of eight, each
+// cleared four planes ahead of its use by the kernel that writes the planes (a cell that was not, as in a short replayed
+// graph, is only too large, which costs time and changes no result).
+PlaneDuties next_digits() {
+    static unsigned turn = 0;
+    turn++;
+    PlaneDuties d;
+    d.nl = q_cells + 8 + (turn & 7); d.nl_clear = q_cells + 8 + ((turn + 4) & 7);
+    return d;
+}
+
+// Products of rows whose digit planes a kernel `write(duties)` is about to leave in `planes` / `totals`.  Where the products add
+// shares of a tile to their outputs, that kernel clears them, unless they lie over something it reads ([in, in + in_n) or
+// [in2, in2 + in_n)): then they are cleared behind it.
+template <typename Write>
+bool planes_and_products(Write write, const Q1Part *parts, int n, bool sc32, long long nb, const int8_t *planes, const int64_t *totals, long long T,
+                         long long frac, const int64_t *in, const int64_t *in2, long long in_n, cudaStream_t s) {
+    PlaneDuties d;
+    bool clear = false, fused = true;
+    if (T > 1 || nb > 128) {                           // a single row takes every digit as it comes
+        d = next_digits();
+        long long row_tiles = 0;
+        for (int i = 0; i < n; i++) row_tiles += (parts[i].out_f + 127) / 128;
+        clear = q1_tc_split(row_tiles, T);
+    }
+    for (int i = 0; clear && i < n; i++) {
+        const Q1Part &p = parts[i];
+        const int64_t *end = p.out + T * p.out_f;
+        fused = fused && p.add != p.out && (i == 0 || p.out == d.zero + d.zero_n) && (end <= in || in + in_n <= p.out) &&
+                (!in2 || end <= in2 || in2 + in_n <= p.out);
+        if (i == 0) d.zero = p.out;
+        d.zero_n += T * p.out_f;
+    }
+    if (!clear || !fused) { d.zero = nullptr; d.zero_n = 0; }
+    if (write(d) != cudaSuccess) return false;
+    for (int i = 0; clear && !fused && i < n; i++)
+        if (parts[i].add != parts[i].out && cudaMemsetAsync(parts[i].out, 0, (size_t)T * parts[i].out_f * 8, s) != cudaSuccess) return false;
+    return launch_q1_apply(parts, n, sc32, nb, planes, totals, T, frac, d.nl, s) == cudaSuccess;
+}
+
 bool valid(long long h) { return h >= 0 && (size_t)h < q_w.size() && q_w[(size_t)h].live; }
 
 // upload + re-order; scale_bits is the width of the caller's scale array
@@ -96,13 +138,16 @@ long long register_any(const unsigned char *bits, const void *scale, int scale_b
               cudaMalloc(&units, usz) == cudaSuccess;
     ok = ok && cudaMemcpyAsync(dbits, bits, bsz, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
     ok = ok && cudaMemcpyAsync(dscale, scale, ssz, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
-    ok = ok && launch_q1_repack(dbits, dscale, scale_bits, sc32, out_f, nb, units, q_stream) == cudaSuccess;
+    unsigned long long *max_cell = (unsigned long long *)(q_cells + 2), max_scale = 0;
+    ok = ok && cudaMemsetAsync(max_cell, 0, 8, q_stream) == cudaSuccess &&
+         launch_q1_repack(dbits, dscale, scale_bits, sc32, out_f, nb, units, max_cell, q_stream) == cudaSuccess &&
+         cudaMemcpyAsync(&max_scale, max_cell, 8, cudaMemcpyDeviceToHost, q_stream) == cudaSuccess;
     ok = ok && cudaStreamSynchronize(q_stream) == cudaSuccess;
     if (dbits) cudaFree(dbits);
     if (dscale) cudaFree(dscale);
     if (!ok) { if (units) cudaFree(units); fail(2, "q1 register: CUDA failure"); return -1; }
     Q1Weight w;
-    w.units = units; w.out_f = out_f; w.nb = nb; w.sc32 = sc32; w.live = true;
+    w.units = units; w.out_f = out_f; w.nb = nb; w.max_scale = max_scale; w.sc32 = sc32; w.live = true;
     q_w.push_back(w);
     if (keep) q_weight_bytes += bsz + ssz;
     return (long long)q_w.size() - 1;
@@ -115,20 +160,19 @@ int apply_device(const Q1Weight &w, const int64_t *xd, long long T, long long fr
     int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * K);
     int64_t *totals = (int64_t *)q_ensure(QR_TOTALS, (size_t)T * w.nb * 8);
     if (!planes || !totals) return 2;
-    int *nl = nullptr;
-    if (max_digits < 8) {
-        nl = q_cells;
-        if (cudaMemsetAsync(nl, 0, sizeof(int), s) != cudaSuccess) return 2;
-    }
-    if (launch_q1_prep(xd, T, w.nb, planes, totals, nl, s) != cudaSuccess) return 2;
-    if (nl) {
-        int used = 0;
-        if (cudaMemcpyAsync(&used, nl, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess) return 2;
-        if (used > max_digits) return 4;
-    }
-    if (launch_q1_apply(w.units, w.sc32, w.out_f, w.nb, planes, totals, T, frac, outd, s) != cudaSuccess) return 2;
-    return 0;
+    const Q1Part part = {w.units, w.out_f, outd, nullptr, w.max_scale};
+    int used = 0;
+    auto write = [&](const PlaneDuties &d) {
+        PlaneDuties dd = d;
+        if (max_digits < 8 && !dd.nl) dd.nl = q_cells;
+        cudaError_t e = max_digits < 8 ? cudaMemsetAsync(dd.nl, 0, sizeof(int), s) : cudaSuccess;
+        if (e == cudaSuccess) e = launch_q1_prep(xd, T, w.nb, planes, totals, dd, s);
+        if (e == cudaSuccess && max_digits < 8) e = cudaMemcpyAsync(&used, dd.nl, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess && max_digits < 8) e = cudaStreamSynchronize(s);
+        return e == cudaSuccess && used > max_digits ? cudaErrorInvalidValue : e;
+    };
+    if (planes_and_products(write, &part, 1, w.sc32, w.nb, planes, totals, T, frac, xd, nullptr, T * K, s)) return 0;
+    return used > max_digits ? 4 : 2;
 }
 
 int apply_host(const Q1Weight &w, const long long *x, long long T, long long frac, long long *out, int max_digits) {
@@ -280,19 +324,17 @@ extern "C" int iie_q1_apply_fused_dev(long long handle, int mode, const int64_t 
     int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * K);
     int64_t *totals = (int64_t *)q_ensure(QR_TOTALS, (size_t)T * w.nb * 8);
     if (!planes || !totals) return 2;
-    cudaError_t e;
-    if (mode == 1) {
-        int *flags = iie::shared_flag_word();
-        if (!flags) return 2;
-        e = iie::launch_rmsnorm_planes(x_dev, T, K, gain_dev, (int)frac, 1ULL, nullptr, planes, totals, flags, s);
-    } else if (mode == 2) {
-        if (!x2_dev || ld < K) return 1;
-        e = iie::launch_q1_prep_swiglu(x_dev, x2_dev, ld, (int)frac, T, w.nb, planes, totals, s);
-    } else {
-        e = iie::launch_q1_prep(x_dev, T, w.nb, planes, totals, nullptr, s);
-    }
-    if (e != cudaSuccess) return 2;
-    return iie::launch_q1_apply(w.units, w.sc32, w.out_f, w.nb, planes, totals, T, frac, out_dev, s, add_dev) == cudaSuccess ? 0 : 2;
+    if (mode == 2 && (!x2_dev || ld < K)) return 1;
+    int *flags = iie::shared_flag_word();
+    if (!flags) return 2;
+    auto write = [&](const PlaneDuties &d) {
+        if (mode == 1) return iie::launch_rmsnorm_planes(x_dev, T, K, gain_dev, (int)frac, 1ULL, nullptr, planes, totals, flags, d, s);
+        if (mode == 2) return iie::launch_q1_prep_swiglu(x_dev, x2_dev, ld, (int)frac, T, w.nb, planes, totals, d, s);
+        return iie::launch_q1_prep(x_dev, T, w.nb, planes, totals, d, s);
+    };
+    const Q1Part part = {w.units, w.out_f, out_dev, add_dev, w.max_scale};
+    return planes_and_products(write, &part, 1, w.sc32, w.nb, planes, totals, T, frac, x_dev, mode == 2 ? x2_dev : gain_dev,
+                               mode == 2 ? (T - 1) * ld + K : T * K, s) ? 0 : 2;
 }
 
 extern "C" int iie_q1_head_norm_dev(const int64_t *x_dev, long long rows_a, long long rows_b, long long width, const int64_t *gain_a_dev,
@@ -394,39 +436,58 @@ bool alloc_work(Work &w, const Q1Stack &m, long long rows) {
     const size_t n = T * ((size_t)m.d + 3 * qd + 3 * kd + 2 * (size_t)m.dff);
     if (cudaMalloc(&w.base, n * 8) != cudaSuccess) { cudaGetLastError(); w.base = nullptr; return false; }
     int64_t *p = (int64_t *)w.base;
-    w.x = p; p += T * m.d; w.q = p; p += T * qd; w.qn = p; p += T * qd; w.att = p; p += T * qd;
-    w.k = p; p += T * kd; w.kn = p; p += T * kd; w.v = p; p += T * kd; w.g = p; p += T * m.dff; w.u = p;
+    // q, k, v and g, u side by side: one range each for the kernel that clears them
+    w.x = p; p += T * m.d; w.q = p; p += T * qd; w.k = p; p += T * kd; w.v = p; p += T * kd; w.g = p; p += T * m.dff; w.u = p; p += T * m.dff;
+    w.qn = p; p += T * qd; w.att = p; p += T * qd; w.kn = p;
     return true;
 }
 void free_work(Work &w) { if (w.base) cudaFree(w.base); w = Work(); }
 
-bool product(long long h, const int8_t *planes, const int64_t *totals, long long T, long long frac, int64_t *out, const int64_t *add = nullptr) {
-    const Q1Weight &w = q_w[(size_t)h];
-    return launch_q1_apply(w.units, w.sc32, w.out_f, w.nb, planes, totals, T, frac, out, q_stream, add) == cudaSuccess;
+// products of the same rows with up to three matrices behind the kernel that writes their planes; one launch where their scales
+// have one width
+struct Product { long long h; int64_t *out; const int64_t *add = nullptr; };
+template <typename Write>
+bool products(Write write, std::initializer_list<Product> list, const int8_t *planes, const int64_t *totals, long long T, long long frac,
+              const int64_t *in, long long in_n) {
+    Q1Part parts[Q1_MAX_PARTS];
+    int n = 0;
+    bool sc32 = true, same = true;
+    for (const Product &p : list) {
+        const Q1Weight &w = q_w[(size_t)p.h];
+        same = same && (n == 0 || w.sc32 == sc32);
+        sc32 = w.sc32;
+        parts[n++] = {w.units, w.out_f, p.out, p.add, w.max_scale};
+    }
+    const long long nb = q_w[(size_t)list.begin()->h].nb;
+    if (same) return planes_and_products(write, parts, n, sc32, nb, planes, totals, T, frac, in, nullptr, in_n, q_stream);
+    for (int i = 0; i < n; i++)
+        if (!planes_and_products(write, parts + i, 1, q_w[(size_t)list.begin()[i].h].sc32, nb, planes, totals, T, frac, in, nullptr, in_n, q_stream)) return false;
+    return true;
 }
 
 // One layer on T rows of w.x.  attend(q normalised, k normalised, v) runs rotation, cache append and attention into w.att.
 template <typename Attend>
 bool layer_rows(const Q1Stack &m, long long li, Work &w, long long T, int *flags, Attend attend) {
     const size_t i = (size_t)li;
-    const long long qd = m.H * m.hd, kd = m.Hkv * m.hd, widest = std::max({m.d, qd, m.dff});
+    const long long qd = m.H * m.hd, widest = std::max({m.d, qd, m.dff});
     int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * (size_t)widest);
     int64_t *totals = (int64_t *)q_ensure(QR_TOTALS, (size_t)T * (size_t)(widest / 128) * 8);
     if (!planes || !totals) return false;
     const int f = (int)m.frac;
-    bool ok = launch_rmsnorm_planes(w.x, T, m.d, q_bufs[(size_t)m.n1g[i]].p, f, m.eps, nullptr, planes, totals, flags, q_stream) == cudaSuccess &&
-              product(m.wq[i], planes, totals, T, m.frac, w.q) && product(m.wk[i], planes, totals, T, m.frac, w.k) &&
-              product(m.wv[i], planes, totals, T, m.frac, w.v) &&
+    auto norm = [&](long long gain) {
+        return [&, gain](const PlaneDuties &d) {
+            return launch_rmsnorm_planes(w.x, T, m.d, q_bufs[(size_t)gain].p, f, m.eps, nullptr, planes, totals, flags, d, q_stream);
+        };
+    };
+    bool ok = products(norm(m.n1g[i]), {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, planes, totals, T, m.frac, w.x, T * m.d) &&
               launch_rmsnorm(w.q, T * m.H, m.hd, q_bufs[(size_t)m.qng[i]].p, f, m.eps, w.qn, flags, q_stream) == cudaSuccess &&
               launch_rmsnorm(w.k, T * m.Hkv, m.hd, q_bufs[(size_t)m.kng[i]].p, f, m.eps, w.kn, flags, q_stream) == cudaSuccess;
     ok = ok && attend(w.qn, w.kn, w.v, w.att);
-    ok = ok && launch_q1_prep(w.att, T, qd / 128, planes, totals, nullptr, q_stream) == cudaSuccess &&
-         product(m.wo[i], planes, totals, T, m.frac, w.x, w.x) &&
-         launch_rmsnorm_planes(w.x, T, m.d, q_bufs[(size_t)m.n2g[i]].p, f, m.eps, nullptr, planes, totals, flags, q_stream) == cudaSuccess &&
-         product(m.w1[i], planes, totals, T, m.frac, w.g) && product(m.wu[i], planes, totals, T, m.frac, w.u) &&
-         launch_q1_prep_swiglu(w.g, w.u, m.dff, f, T, m.dff / 128, planes, totals, q_stream) == cudaSuccess &&
-         product(m.w2[i], planes, totals, T, m.frac, w.x, w.x);
-    (void)kd;
+    ok = ok && products([&](const PlaneDuties &d) { return launch_q1_prep(w.att, T, qd / 128, planes, totals, d, q_stream); },
+                        {{m.wo[i], w.x, w.x}}, planes, totals, T, m.frac, w.att, T * qd) &&
+         products(norm(m.n2g[i]), {{m.w1[i], w.g}, {m.wu[i], w.u}}, planes, totals, T, m.frac, w.x, T * m.d) &&
+         products([&](const PlaneDuties &d) { return launch_q1_prep_swiglu(w.g, w.u, m.dff, f, T, m.dff / 128, planes, totals, d, q_stream); },
+                  {{m.w2[i], w.x, w.x}}, planes, totals, T, m.frac, w.g, 2 * T * m.dff);
     return ok;
 }
 
@@ -434,9 +495,10 @@ bool layer_rows(const Q1Stack &m, long long li, Work &w, long long T, int *flags
 bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logits, int *flags) {
     int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)rows * 8 * (size_t)m.d);
     int64_t *totals = (int64_t *)q_ensure(QR_TOTALS, (size_t)rows * (size_t)(m.d / 128) * 8);
-    return planes && totals &&
-           launch_rmsnorm_planes(x, rows, m.d, q_bufs[(size_t)m.finalg].p, (int)m.frac, m.eps, nullptr, planes, totals, flags, q_stream) == cudaSuccess &&
-           product(m.out_head, planes, totals, rows, m.frac, logits);
+    if (!planes || !totals) return false;
+    return products([&](const PlaneDuties &d) {
+        return launch_rmsnorm_planes(x, rows, m.d, q_bufs[(size_t)m.finalg].p, (int)m.frac, m.eps, nullptr, planes, totals, flags, d, q_stream);
+    }, {{m.out_head, logits}}, planes, totals, rows, m.frac, x, rows * m.d);
 }
 
 // int64 host rows -> int32; false when a value does not fit

@@ -1,0 +1,43 @@
+"""Q1_0 products of several tokens on the tensor-core tiles against the CPU oracle, where the tiles can go wrong: token counts
+around the tile widths, rows around 128, few and many blocks, one to eight digit planes, scales beyond the three-plane
+read-out, shared tiles (added atomically, in place or over cleared outputs) and whole ones."""
+import numpy as np
+import pytest
+
+from oracle import native as onat
+from oracle import qk_oracle as o
+
+pytestmark = pytest.mark.gpu
+FRAC = 16
+
+
+@pytest.mark.parametrize("out_f,nb,T,magbits,scale_bits", [
+    (1, 1, 2, 20, 12), (127, 9, 16, 22, 12), (129, 8, 17, 22, 12), (640, 33, 32, 22, 14), (300, 7, 33, 30, 12), (4096, 3, 64, 22, 12),
+    (200, 130, 65, 38, 12), (384, 16, 130, 47, 20), (150, 5, 19, 62, 40), (96, 12, 6, 22, 31), (2400, 1, 2047, 22, 12)])
+def test_tiles_match_the_oracle(out_f, nb, T, magbits, scale_bits):
+    import torch
+
+    from integer_inference_engine_b200 import device, q1_gpu
+    rng = np.random.default_rng(out_f * 7 + nb * 3 + T)
+    bits, scale = o.synth_q1(rng, out_f, nb)
+    lim = 1 << scale_bits
+    scale = rng.integers(-lim, lim, size=scale.shape, dtype=np.int64)
+    x = rng.integers(-(1 << magbits), 1 << magbits, size=(T, nb * 128), dtype=np.int64)
+    if magbits == 22:
+        x[0, :3] = [8355711, -8421504, 8355711]                      # the ends of three balanced digits
+    device.read_flags()
+    h = q1_gpu.q1_register_weight(bits, scale.astype(np.int32) if scale_bits < 31 else scale)
+    want = onat.q1_linear(x, bits, scale, FRAC)
+    xd = torch.from_numpy(x).cuda()
+    assert np.array_equal(q1_gpu.apply_dev(h, xd, FRAC).cpu().numpy(), want)
+    other = rng.integers(-(1 << 40), 1 << 40, size=want.shape, dtype=np.int64)
+    res = torch.from_numpy(other).cuda()
+    q1_gpu.apply_fused_dev(h, xd, FRAC, res, add=res)                 # the residual row in place
+    assert np.array_equal(res.cpu().numpy(), want + other)
+    out = torch.full(want.shape, 7, dtype=torch.int64, device="cuda")
+    q1_gpu.apply_fused_dev(h, xd, FRAC, out, add=torch.from_numpy(other).cuda())
+    assert np.array_equal(out.cpu().numpy(), want + other)
+    if out_f * T <= xd.numel():                                      # the output over the input
+        q1_gpu.apply_dev(h, xd, FRAC, out=xd.view(-1)[:out_f * T].view(T, out_f))
+        assert np.array_equal(xd.view(-1)[:out_f * T].view(T, out_f).cpu().numpy(), want)
+    assert device.read_flags() == 0
