@@ -61,7 +61,7 @@ int g_pdl = 1;                        // programmatic dependent launch between t
 long long g_hl_d = 0;                 // width of the digit planes the last single-token routing left in the R_XL scratch
 int64_t *g_pow2 = nullptr;            // device: 2^i for i = 0..31 (unit gates at any activation scale)
 int g_attn_parity = 0;                // which of the two attention digit-count cells the next block call uses
-long long g_tc_min_tokens = 192;      // from this many tokens on, the MoE block runs on the tcgen05 grouped GEMMs
+long long g_tc_min_tokens = 2;        // from this many rows on, products run on the tcgen05 tiles
 int g_ready = -1;                     // -1 unknown, 0 usable, 1 unusable
 int g_stage_mask = 0;                 // profiling: when non-zero, iie_moe_forward_dev runs only these stages
 enum Stage { ST_LIMBS = 1, ST_ROUTER = 2, ST_TOPK = 4, ST_GATEUP = 8, ST_DOWN = 16 };
@@ -69,7 +69,7 @@ inline bool stage_on(int st) { return g_stage_mask == 0 || (g_stage_mask & st); 
 
 // Persistent device scratch by role, grown on demand (never shrunk until released).
 enum Role { R_X, R_XL, R_OUT, R_RAW, R_GU, R_GUL, R_TMP0, R_TMP1, R_TMP2, R_TABS, R_META, R_LOGITS, R_IDS, R_GATES,
-            R_GRPOFF, R_PAIRTOK, R_PAIRGATE, R_HNORM, R_ZERO, R_ASCORES, R_AEXP, R_ASTAT, R_APART, R_PSCORES, R_PEXP, R_PSTAT, R_BSCORES, R_BEXP, R_BSTAT, R_BPART, R_XG, R_COUNT };
+            R_GRPOFF, R_PAIRTOK, R_PAIRGATE, R_HNORM, R_ZERO, R_ASCORES, R_AEXP, R_ASTAT, R_APART, R_PSCORES, R_PEXP, R_PSTAT, R_BSCORES, R_BEXP, R_BSTAT, R_BPART, R_XG, R_XS, R_COUNT };
 struct Buf { void *p = nullptr; size_t cap = 0; };
 Buf g_buf[R_COUNT];
 long long g_ws_allocs = 0;
@@ -187,19 +187,31 @@ long long register_quant(const void *raw, bool raw_on_device, long long out_f, l
     return h;
 }
 
+// Block scales the tiles' read-out carries: d * 256 and 16 * dmin in 32 bits.
+bool tile_scales(int qtype, long long nb, unsigned maxd, unsigned maxdmin, int fw) {
+    return small_scales(maxd, maxdmin, fw) && nb <= 64 && half_to_fixed(maxd, fw) < ((int64_t)1 << 23) &&
+           (qtype != QT_Q4K || half_to_fixed(maxdmin, fw) < ((int64_t)1 << 26));
+}
+
+// A product on the tcgen05 tiles, its scratch included; false when there is no tile for it (the caller takes other kernels).
+bool tiles(int qtype, int mode, TileArgs a, cudaStream_t s) {
+    if (a.xidx && !(a.xg = (int8_t *)ensure(R_XG, (size_t)a.n_rows * 8 * a.nb * 256))) return false;
+    if (qtype == QT_Q4K && !(a.xs = (int8_t *)ensure(R_XS, tile_sums_bytes(a.n_rows, a.nb)))) return false;
+    a.flags = g_flags;
+    const cudaError_t e = launch_tiles(qtype, mode, a, s);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+}
+
 // y[T,out_f] on device from x[T,K] on device.  check_flags: synchronise and re-run the exact kernel
 // if an activation left the limb envelope (host-pointer entries); otherwise flags stay raised.
-// Dense product of a prefill-sized batch on the tensor-core tiles; returns false when the shape, the weights or the stream
-// (a capture cannot read the digit count back) rule them out, and the caller then takes the batched kernels.
-bool linear_tc(const Weight &w, const int8_t *xl, const int *x_nl, long long T, int fw, int64_t *out, cudaStream_t s);
-
 bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t *out, bool check_flags, cudaStream_t s,
-                const int8_t *xl_ready = nullptr) {
+                const int8_t *xl_ready = nullptr, const int *nl_ready = nullptr) {
     const long long K = w.nb * 256;
     if (!fast_envelope(w.qtype, w.nb, w.maxd, w.maxdmin, fw))
         return launch_exact_linear((const uint8_t *)w.d, w.qtype, w.out_f, w.nb, x, T, fw, out, s) == cudaSuccess;
     const int8_t *xl = xl_ready;
-    const int *x_nl = nullptr;                             // digits in use by the rows, where the planes are made here
+    const int *x_nl = nl_ready;                            // digits in use by the rows, where they are known
     if (!xl) {
         int8_t *buf = (int8_t *)ensure(R_XL, (size_t)T * 8 * K);
         if (!buf) return false;
@@ -210,8 +222,16 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
         if (launch_limbs(x, T, K, buf, g_flags, s, const_cast<int *>(x_nl)) != cudaSuccess) return false;
         xl = buf;
     }
-    if (T >= g_tc_min_tokens && x_nl && g_stage_mask == 0 && linear_tc(w, xl, x_nl, T, fw, out, s)) {
-        // done on the tcgen05 tiles
+    bool done = false;
+    if (T >= 2 && T >= g_tc_min_tokens && T < (1 << 24) && g_stage_mask == 0 && tile_scales(w.qtype, w.nb, w.maxd, w.maxdmin, fw)) {
+        int *off = (int *)ensure(R_META, 64);
+        if (!off || launch_set2(off, 0, (int)T, s) != cudaSuccess) return false;
+        TileArgs ta = {};
+        ta.wa = w.cell; ta.wb = w.cell; ta.grp_off = off; ta.n_groups = 1; ta.nb = (int)w.nb; ta.n_rows = T; ta.out_f = w.out_f; ta.fw = fw;
+        ta.fa = 16; ta.xl = xl; ta.x_nl = x_nl; ta.out = out;
+        done = tiles(w.qtype, MODE_LINEAR, ta, s);
+    }
+    if (done) {
     } else if (T == 1 && w.out_f >= 256 && g_stage_mask == 0) {
         // one row: the bulk-copy streaming kernel (every CTA requests its run of 16-row tiles up front)
         StreamArgs sa = {};
@@ -250,24 +270,47 @@ struct MoePlan {                      // everything the fused MoE kernels need o
 // Fused path: limbs(h) -> gate/up (+SiLU*up, limbs of gu) -> down (+gate-weighted accumulate).
 // Groups: n_groups experts; grp_expert / grp_off / pair arrays as in SkinnyArgs.  n_pairs activation
 // rows of gu are produced.  out [T,d_model] must be initialised by the caller.
-bool moe_fused(const MoePlan &p, const int8_t *hl, bool x_bcast_zero, const int *xidx, const int *grp_expert,
+bool moe_fused(const MoePlan &p, const int8_t *hl, long long rows, const int *xidx, const int *grp_expert,
                const int *grp_off, int n_groups, long long n_pairs, int max_pairs, const int64_t *pair_gate,
                const int *pair_tok, int fa, int fw, int64_t *out, cudaStream_t s, const int *h_nl = nullptr,
                unsigned maxd_gate = 0x7C00, unsigned maxdmin_gate = 0x7C00, unsigned maxd_down = 0x7C00, unsigned maxdmin_down = 0x7C00) {
     int8_t *gul = (int8_t *)ensure(R_GUL, (size_t)n_pairs * 8 * p.e_ffn);
     if (!gul) return false;
-    (void)x_bcast_zero;
-    if (!grp_expert && grp_off && g_stage_mask == 0) {
-        // groups are the experts themselves: stream every touched expert tile once for all of its rows
-        if (cudaMemsetAsync(g_cells + 1, 0, sizeof(int), s) != cudaSuccess) return false;
+    auto gateup_batch = [&] {
         BatchArgs ga = {};
         ga.wa = p.gate; ga.wb = p.up; ga.grp_off = grp_off; ga.n_groups = n_groups; ga.out_f = p.e_ffn; ga.n_blocks = p.d_model / 256;
         ga.fw = fw; ga.fa = fa; ga.fast = small_scales(maxd_gate, maxdmin_gate, fw); ga.xl = hl; ga.xidx = xidx; ga.x_nl = h_nl;
         ga.out = nullptr; ga.out_limbs = gul; ga.out_nl = g_cells + 1; ga.flags = g_flags;
+        return ga;
+    };
+    auto down_batch = [&] {
         BatchArgs da = {};
         da.wa = p.down; da.wb = p.down; da.grp_off = grp_off; da.n_groups = n_groups; da.out_f = p.d_model; da.n_blocks = p.e_ffn / 256;
         da.fw = fw; da.fa = fa; da.fast = small_scales(maxd_down, maxdmin_down, fw); da.xl = gul; da.xidx = nullptr; da.x_nl = g_cells + 1;
         da.out = out; da.gates = pair_gate; da.pair_tok = pair_tok; da.flags = g_flags;
+        return da;
+    };
+    if (!grp_expert && grp_off && g_stage_mask == 0) {
+        // groups are the experts themselves: stream every touched expert tile once for all of its rows
+        if (cudaMemsetAsync(g_cells + 1, 0, sizeof(int), s) != cudaSuccess) return false;
+        if (n_pairs >= 2 && rows >= g_tc_min_tokens && tile_scales(p.gate_q, p.d_model / 256, maxd_gate, maxdmin_gate, fw) &&
+            tile_scales(p.down_q, p.e_ffn / 256, maxd_down, maxdmin_down, fw)) {
+            TileArgs tg = {};
+            tg.wa = p.gate; tg.wb = p.up; tg.grp_off = grp_off; tg.n_groups = n_groups; tg.nb = (int)(p.d_model / 256); tg.n_rows = n_pairs;
+            tg.out_f = p.e_ffn; tg.fw = fw; tg.fa = fa; tg.xl = hl; tg.xidx = xidx; tg.x_nl = h_nl; tg.out_limbs = gul; tg.out_nl = g_cells + 1;
+            TileArgs td = {};
+            td.wa = p.down; td.wb = p.down; td.grp_off = grp_off; td.n_groups = n_groups; td.nb = (int)(p.e_ffn / 256); td.n_rows = n_pairs;
+            td.out_f = p.d_model; td.fw = fw; td.fa = fa; td.xl = gul; td.x_nl = g_cells + 1; td.out = out; td.gates = pair_gate; td.pair_tok = pair_tok;
+            // gate / up below three rows per expert on average: the warp-level kernel, which multiplies one row at a time without a
+            // tile's padding, is the faster one (16 tokens over 128 experts 81 against 88 us, 45 tokens 139 / 141, 64 tokens 163 / 135);
+            // down takes the tiles from two rows on (16 tokens 55 against 78 us)
+            const bool first = n_pairs >= 3LL * n_groups && tiles(p.gate_q, MODE_GATEUP, tg, s);
+            if (first || launch_batch(p.gate_q, MODE_GATEUP, gateup_batch(), s) == cudaSuccess)
+                return tiles(p.down_q, MODE_DOWN, td, s) || launch_batch(p.down_q, MODE_DOWN, down_batch(), s) == cudaSuccess;
+            cudaGetLastError();
+        }
+        const BatchArgs ga = gateup_batch();
+        const BatchArgs da = down_batch();
         const cudaError_t e1 = launch_batch(p.gate_q, MODE_GATEUP, ga, s);
         if (e1 == cudaSuccess) return launch_batch(p.down_q, MODE_DOWN, da, s) == cudaSuccess;
         cudaGetLastError();
@@ -306,132 +349,6 @@ bool moe_exact_pairs(const std::vector<const Weight *> &gw, const std::vector<co
         if (launch_exact_linear((const uint8_t *)dw[i]->d, dw[i]->qtype, d_model, dw[i]->nb, g + i * e_ffn, 1, fw,
                                 dn + i * d_model, g_stream) != cudaSuccess) return false;
     return launch_combine(dn, gates_dev, T, k, d_model, fa, out_dev, g_stream) == cudaSuccess;
-}
-
-// Largest dequantised |weight| of a tensor family at this fw (from the largest block scales).
-unsigned __int128 max_weight(int qtype, unsigned maxd, unsigned maxdmin, int fw) {
-    const unsigned __int128 dq = (unsigned __int128)half_to_fixed(maxd, fw), dm = (unsigned __int128)half_to_fixed(maxdmin, fw);
-    return qtype == QT_Q4K ? dq * 945 + dm * 63 : dq * 128 * 32;
-}
-const unsigned __int128 CAP4 = 2139062143ULL;                              // 127 * (256^4 - 1) / 255
-
-int read_cell(int idx, cudaStream_t s) {
-    int v = -1;
-    if (cudaMemcpyAsync(&v, g_cells + idx, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) return -1;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-    return v;
-}
-
-bool linear_tc(const Weight &w, const int8_t *xl, const int *x_nl, long long T, int fw, int64_t *out, cudaStream_t s) {
-    if (w.qtype != QT_Q4K || w.nb * 256 > 8192 || fw > 32 || !small_scales(w.maxd, w.maxdmin, fw) ||
-        max_weight(QT_Q4K, w.maxd, w.maxdmin, fw) > CAP4) return false;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { cudaGetLastError(); return false; }
-    int nl = -1;
-    if (cudaMemcpyAsync(&nl, x_nl, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return false;
-    if (nl < 1 || nl > 5) return false;
-    int *one_off = (int *)ensure(R_META, 64);
-    if (!one_off || launch_set2(one_off, 0, (int)T, s) != cudaSuccess) return false;
-    PrefillArgs ra = {};
-    ra.wa = w.cell; ra.wb = w.cell; ra.grp_off = one_off; ra.n_experts = 1; ra.n_pairs = T; ra.out_f = w.out_f;
-    ra.n_blocks = w.nb; ra.fw = fw; ra.fa = 16; ra.xl = xl; ra.out = out; ra.flags = g_flags;
-    if (launch_prefill(QT_Q4K, MODE_LINEAR, nl, ra, s) != cudaSuccess) { cudaGetLastError(); return false; }
-    return true;
-}
-
-// Expert stage on the tensor-core (tcgen05) tiles for pairs already sorted by group: group x uses the weights
-// gate[x] / up[x] / down[x] and owns pairs [off[x], off[x+1]); xidx maps a pair to its row of digit planes, ptok to its
-// output row, pg holds its gate weight.  gate/up (+SiLU*up, digit planes of the product) -> down (+gate-weighted combine).
-// Returns -1 when the weights or the activation are outside what the tiles carry (the caller then streams), 0 ok, 1 failure.
-struct GroupedWeights {
-    const uint8_t *const *gate, *const *up, *const *down;
-    int gate_q, down_q;
-    long long d_model, e_ffn;
-    unsigned maxd_gate, maxdmin_gate, maxd_down, maxdmin_down;
-};
-
-int grouped_tc(const GroupedWeights &w, int n_groups, const int *off, const int *xidx, const int *ptok, const int64_t *pg,
-               const int8_t *hl, int nl_h, long long T, long long P, int fa, int fw, int accumulate, int64_t *out_dev,
-               cudaStream_t s) {
-    if (w.gate_q != QT_Q4K || w.d_model > 8192 || w.e_ffn > 8192 || nl_h < 1 || nl_h > 4 || fw > 32) return -1;
-    if (!small_scales(w.maxd_gate, w.maxdmin_gate, fw) || !small_scales(w.maxd_down, w.maxdmin_down, fw)) return -1;
-    if (max_weight(QT_Q4K, w.maxd_gate, w.maxdmin_gate, fw) > CAP4) return -1;
-    if (max_weight(w.down_q, w.maxd_down, w.maxdmin_down, fw) > (w.down_q == QT_Q4K ? CAP4 : (unsigned __int128)0x7FFFFFFFULL * 32)) return -1;   // Q6_K: d_q * 128 stays in int32
-    int8_t *gul = (int8_t *)ensure(R_GUL, (size_t)P * 8 * w.e_ffn);
-    int8_t *xg = xidx ? (int8_t *)ensure(R_XG, (size_t)P * 4 * w.d_model) : nullptr;
-    if (!gul || (xidx && !xg)) return 1;
-    if (cudaMemsetAsync(g_cells + 1, 0, sizeof(int), s) != cudaSuccess) return 1;
-    PrefillArgs ga = {};
-    ga.wa = w.gate; ga.wb = w.up; ga.grp_off = off; ga.n_experts = n_groups; ga.n_pairs = P; ga.out_f = w.e_ffn;
-    ga.n_blocks = w.d_model / 256; ga.fw = fw; ga.fa = fa; ga.xl = hl; ga.xidx = xidx; ga.xg = xg; ga.out = nullptr; ga.out_limbs = gul;
-    ga.out_nl = g_cells + 1; ga.flags = g_flags;
-    if (launch_prefill(QT_Q4K, MODE_GATEUP, nl_h, ga, s) != cudaSuccess) { cudaGetLastError(); return 1; }
-    const int nl_gu = read_cell(1, s);
-    if (nl_gu < 0) return 1;
-    if (!accumulate && cudaMemsetAsync(out_dev, 0, (size_t)T * w.d_model * 8, s) != cudaSuccess) return 1;
-    PrefillArgs da = {};
-    da.wa = w.down; da.wb = w.down; da.grp_off = off; da.n_experts = n_groups; da.n_pairs = P; da.out_f = w.d_model;
-    da.n_blocks = w.e_ffn / 256; da.fw = fw; da.fa = fa; da.xl = gul; da.xidx = nullptr; da.out = out_dev; da.gates = pg;
-    da.pair_tok = ptok; da.flags = g_flags;
-    const cudaError_t de = launch_prefill(w.down_q, MODE_DOWN, nl_gu < 1 ? 1 : nl_gu, da, s);
-    if (de == cudaSuccess) return 0;
-    cudaGetLastError();
-    // the activation needs more digits than the tensor-core tiles carry: streamed kernels for the down stage
-    SkinnyArgs d = {};
-    d.wa = w.down; d.wb = w.down; d.grp_off = off; d.pairs_per_group = 1; d.out_f = w.d_model; d.n_blocks = w.e_ffn / 256;
-    d.fw = fw; d.fa = fa; d.xl = gul; d.out = out_dev; d.gates = pg; d.pair_tok = ptok; d.flags = g_flags;
-    return launch_skinny(w.down_q, MODE_DOWN, d, n_groups, 4, s) == cudaSuccess ? 0 : 1;
-}
-
-// The same for a registered layer: hl = digit planes of the T hidden rows (nl_h digits in use), ids/gates = routing of
-// every row; experts of this layer are ids expert_base .. expert_base + n_experts - 1, other slots are skipped.
-int moe_experts_tc(const MoeLayer &L, const int8_t *hl, int nl_h, long long T, const int *ids, const int64_t *gates,
-                   int expert_base, int fa, int fw, int accumulate, int64_t *out_dev, cudaStream_t s) {
-    const int E = L.n_experts, k = L.top_k;
-    const long long P = T * k;
-    int *off = (int *)ensure(R_GRPOFF, (size_t)(E + 2) * sizeof(int));
-    int *ptok = (int *)ensure(R_PAIRTOK, (size_t)P * sizeof(int));
-    int64_t *pg = (int64_t *)ensure(R_PAIRGATE, (size_t)P * 8);
-    if (!off || !ptok || !pg) return 1;
-    if (launch_dispatch(ids, gates, T, k, E, off, ptok, pg, s, expert_base) != cudaSuccess) return 1;
-    const GroupedWeights w = {L.tabs, L.tabs + E, L.tabs + 2 * E, L.gate_q, L.down_q, L.d_model, L.e_ffn,
-                              L.maxd_gate, L.maxdmin_gate, L.maxd_down, L.maxdmin_down};
-    return grouped_tc(w, E, off, ptok, ptok, pg, hl, nl_h, T, P, fa, fw, accumulate, out_dev, s);
-}
-
-// Whole block (router GEMM, top-k, expert stage) on the tensor-core tiles.  Same return codes.
-int moe_prefill_tc(const MoeLayer &L, const int64_t *h_dev, long long T, int fa, int fw, int accumulate, int64_t *out_dev,
-                   int *ids, int64_t *gates, cudaStream_t s) {
-    const Weight &r = g_w[L.router];
-    const int E = L.n_experts, k = L.top_k;
-    if (r.qtype != QT_Q4K || L.gate_q != QT_Q4K || L.d_model > 8192 || L.e_ffn > 8192) return -1;
-    if (!small_scales(r.maxd, r.maxdmin, fw) || max_weight(QT_Q4K, r.maxd, r.maxdmin, fw) > CAP4) return -1;
-    int8_t *hl = (int8_t *)ensure(R_XL, (size_t)T * 8 * L.d_model);
-    int64_t *lg = (int64_t *)ensure(R_LOGITS, (size_t)T * E * 8);
-    int *one_off = (int *)ensure(R_META, 64);
-    if (!hl || !lg || !one_off) return 1;
-    if (cudaMemsetAsync(g_cells, 0, 2 * sizeof(int), s) != cudaSuccess) return 1;
-    if (launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, g_cells) != cudaSuccess) return 1;
-    const int nl_h = read_cell(0, s);
-    if (nl_h < 1 || nl_h > 4) return nl_h < 1 ? 1 : -1;
-    // router: one "expert" that owns all T rows
-    if (launch_set2(one_off, 0, (int)T, s) != cudaSuccess) return 1;
-    PrefillArgs ra = {};
-    ra.wa = r.cell; ra.wb = r.cell; ra.grp_off = one_off; ra.n_experts = 1; ra.n_pairs = T; ra.out_f = E;
-    ra.n_blocks = L.d_model / 256; ra.fw = fw; ra.fa = fa; ra.xl = hl; ra.out = lg; ra.flags = g_flags;
-    if (launch_prefill(QT_Q4K, MODE_LINEAR, nl_h, ra, s) != cudaSuccess) { cudaGetLastError(); return -1; }
-    if (launch_topk(lg, T, E, k, fa, ids, gates, s) != cudaSuccess) return 1;
-    const int rc = moe_experts_tc(L, hl, nl_h, T, ids, gates, 0, fa, fw, accumulate, out_dev, s);
-    if (rc != -1) return rc;
-    // routing is done; stream the expert stage
-    int *off = (int *)ensure(R_GRPOFF, (size_t)(E + 2) * sizeof(int));
-    int *ptok = (int *)ensure(R_PAIRTOK, (size_t)T * k * sizeof(int));
-    int64_t *pg = (int64_t *)ensure(R_PAIRGATE, (size_t)T * k * 8);
-    if (!off || !ptok || !pg || launch_dispatch(ids, gates, T, k, E, off, ptok, pg, s) != cudaSuccess) return 1;
-    if (!accumulate && cudaMemsetAsync(out_dev, 0, (size_t)T * L.d_model * 8, s) != cudaSuccess) return 1;
-    MoePlan plan = {L.tabs, L.tabs + E, L.tabs + 2 * E, L.gate_q, L.down_q, L.d_model, L.e_ffn};
-    return moe_fused(plan, hl, false, ptok, nullptr, off, E, T * k, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, g_cells,
-                     L.maxd_gate, L.maxdmin_gate, L.maxd_down, L.maxdmin_down) ? 0 : 1;
 }
 
 // Single-token fused path: route (optional RMSNorm, limbs, router, top-k) -> gate/up -> down.
@@ -555,17 +472,8 @@ int moe_host_entry(const long long *gate_h, const long long *up_h, const long lo
                   cudaMemsetAsync(out_dev, 0, (size_t)m * d_model * 8, g_stream) == cudaSuccess &&
                   cudaMemsetAsync(g_cells, 0, sizeof(int), g_stream) == cudaSuccess &&
                   launch_limbs(h_dev, m, d_model, hl, g_flags, g_stream, g_cells) == cudaSuccess;
-        int tc = -1;
-        if (ok && m >= g_tc_min_tokens && g_stage_mask == 0) {
-            // prefill-sized call (Engine._moe's batched entry, engine.py:389-411): the grouped tensor-core tiles
-            const int nl_h = read_cell(0, g_stream);
-            const GroupedWeights w = {tabs_dev, tabs_dev + G, tabs_dev + 2 * G, gw[0]->qtype, dw[0]->qtype, d_model, e_ffn, mg, mgm, md, mdm};
-            tc = nl_h < 1 ? 1 : grouped_tc(w, G, off_dev, tok_dev, tok_dev, pg_dev, hl, nl_h, m, (long long)P, fa, fw, 1, out_dev, g_stream);
-            ok = tc != 1;
-        }
-        if (ok && tc < 0)
-            ok = moe_fused(plan, hl, false, tok_dev, nullptr, off_dev, G, (long long)P, maxp, pg_dev, tok_dev, fa, fw, out_dev, g_stream,
-                           g_cells, mg, mgm, md, mdm);
+        ok = ok && moe_fused(plan, hl, m, tok_dev, nullptr, off_dev, G, (long long)P, maxp, pg_dev, tok_dev, fa, fw, out_dev, g_stream,
+                             g_cells, mg, mgm, md, mdm);
         if (!ok) { cudaGetLastError(); return 1; }
         const int f = read_flags_clear();
         if (f < 0) return 1;
@@ -725,8 +633,8 @@ extern "C" int qk_apply_resident_grouped(const long long *handles, const int *ph
     const long long K = nb * 256;
     int64_t *xd = (int64_t *)ensure(R_X, (size_t)T * K * 8), *od = (int64_t *)ensure(R_OUT, (size_t)total * 8);
     int8_t *xl = (int8_t *)ensure(R_XL, (size_t)T * 8 * K);
-    if (!xd || !od || !xl || !h2d(xd, x, (size_t)T * K * 8) ||
-        launch_limbs(xd, T, K, xl, g_flags, g_stream) != cudaSuccess) { cudaGetLastError(); return 1; }
+    if (!xd || !od || !xl || !h2d(xd, x, (size_t)T * K * 8) || cudaMemsetAsync(g_cells + 4, 0, sizeof(int), g_stream) != cudaSuccess ||
+        launch_limbs(xd, T, K, xl, g_flags, g_stream, g_cells + 4) != cudaSuccess) { cudaGetLastError(); return 1; }
     const int f0 = read_flags_clear();
     if (f0 < 0) return 1;
     long long off = 0;
@@ -737,7 +645,7 @@ extern "C" int qk_apply_resident_grouped(const long long *handles, const int *ph
         prof(calls[phase >= 0 && phase <= 4 ? phase : 0]);
         bool ok;
         if (f0 & 1) ok = launch_exact_linear((const uint8_t *)w.d, w.qtype, w.out_f, w.nb, xd, T, fw, od + off, g_stream) == cudaSuccess;
-        else ok = linear_dev(w, xd, T, fw, od + off, false, g_stream, xl);
+        else ok = linear_dev(w, xd, T, fw, od + off, false, g_stream, xl, T > 1 ? g_cells + 4 : nullptr);
         if (!ok) { cudaGetLastError(); return 1; }
         off += T * w.out_f;
     }
@@ -890,10 +798,6 @@ extern "C" int iie_moe_forward_dev(long long layer, const int64_t *h_dev, long l
     int *ids = ids_dev ? ids_dev : (int *)ensure(R_IDS, (size_t)P * sizeof(int));
     int64_t *gates = gates_dev ? gates_dev : (int64_t *)ensure(R_GATES, (size_t)P * 8);
     if (!ids || !gates) return 1;
-    if (T >= g_tc_min_tokens && g_stage_mask == 0) {
-        const int rc = moe_prefill_tc(L, h_dev, T, fa, fw, accumulate, out_dev, ids, gates, s);
-        if (rc >= 0) { if (rc) cudaGetLastError(); return rc; }
-    }
     int8_t *hl = (int8_t *)ensure(R_XL, (size_t)T * 8 * L.d_model);
     int64_t *lg = (int64_t *)ensure(R_LOGITS, (size_t)T * E * 8);
     if (!hl || !lg) return 1;
@@ -902,7 +806,7 @@ extern "C" int iie_moe_forward_dev(long long layer, const int64_t *h_dev, long l
     if (stage_on(ST_ROUTER)) {
         if (r.qtype == QT_I64) {
             if (launch_exact_dense((const int64_t *)r.d, E, L.d_model, h_dev, T, fw, lg, g_flags, s) != cudaSuccess) return 1;
-        } else if (!linear_dev(r, h_dev, T, fw, lg, false, s, hl)) return 1;
+        } else if (!linear_dev(r, h_dev, T, fw, lg, false, s, hl, g_cells)) return 1;
     }
     if (stage_on(ST_TOPK) && launch_topk(lg, T, E, k, fa, ids, gates, s) != cudaSuccess) return 1;
     if (!accumulate && cudaMemsetAsync(out_dev, 0, (size_t)T * L.d_model * 8, s) != cudaSuccess) return 1;
@@ -914,13 +818,13 @@ extern "C" int iie_moe_forward_dev(long long layer, const int64_t *h_dev, long l
         int *zero = (int *)ensure(R_ZERO, 4096 * sizeof(int));          // all-zero index table, written once
         if (!zero || P > 4096) return 1;
         if (fresh && (cudaMemsetAsync(zero, 0, 4096 * sizeof(int), g_stream) != cudaSuccess || !sync())) return 1;
-        ok = moe_fused(plan, hl, true, zero, ids, nullptr, k, P, 1, gates, zero, fa, fw, out_dev, s);
+        ok = moe_fused(plan, hl, 1, zero, ids, nullptr, k, P, 1, gates, zero, fa, fw, out_dev, s);
     } else {
         int *off = (int *)ensure(R_GRPOFF, (size_t)(E + 1) * sizeof(int));
         int *ptok = (int *)ensure(R_PAIRTOK, (size_t)P * sizeof(int));
         int64_t *pg = (int64_t *)ensure(R_PAIRGATE, (size_t)P * 8);
         if (!off || !ptok || !pg || launch_dispatch(ids, gates, T, k, E, off, ptok, pg, s) != cudaSuccess) return 1;
-        ok = moe_fused(plan, hl, false, ptok, nullptr, off, E, P, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, g_cells,
+        ok = moe_fused(plan, hl, T, ptok, nullptr, off, E, P, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, g_cells,
                        L.maxd_gate, L.maxdmin_gate, L.maxd_down, L.maxdmin_down);
     }
     if (!ok) { cudaGetLastError(); return 1; }
@@ -962,19 +866,13 @@ extern "C" int iie_moe_experts_dev(long long layer, const int64_t *h_dev, long l
     if (!hl) return 1;
     if (cudaMemsetAsync(g_cells, 0, sizeof(int), s) != cudaSuccess) return 1;
     if (launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, g_cells) != cudaSuccess) return 1;
-    if (T >= g_tc_min_tokens) {
-        const int nl_h = read_cell(0, s);
-        if (nl_h < 1) return 1;
-        const int rc = moe_experts_tc(L, hl, nl_h, T, ids_dev, gates_dev, expert_base, fa, fw, accumulate, out_dev, s);
-        if (rc >= 0) { if (rc) cudaGetLastError(); return rc; }
-    }
     int *off = (int *)ensure(R_GRPOFF, (size_t)(E + 2) * sizeof(int));
     int *ptok = (int *)ensure(R_PAIRTOK, (size_t)P * sizeof(int));
     int64_t *pg = (int64_t *)ensure(R_PAIRGATE, (size_t)P * 8);
     if (!off || !ptok || !pg || launch_dispatch(ids_dev, gates_dev, T, slots, E, off, ptok, pg, s, expert_base) != cudaSuccess) return 1;
     if (!accumulate && cudaMemsetAsync(out_dev, 0, (size_t)T * L.d_model * 8, s) != cudaSuccess) return 1;
     MoePlan plan = {L.tabs, L.tabs + E, L.tabs + 2 * E, L.gate_q, L.down_q, L.d_model, L.e_ffn};
-    if (!moe_fused(plan, hl, false, ptok, nullptr, off, E, P, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, g_cells,
+    if (!moe_fused(plan, hl, T, ptok, nullptr, off, E, P, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, g_cells,
                    L.maxd_gate, L.maxdmin_gate, L.maxd_down, L.maxdmin_down)) {
         cudaGetLastError(); return 1;
     }
@@ -1742,9 +1640,9 @@ extern "C" unsigned long long iie_workspace_generation(void) {
 }
 
 extern "C" int iie_prefill_launch_counts(unsigned long long *out, int capacity) {
-    if (!out || capacity < iie::PF_SHAPES) return -1;
-    for (int i = 0; i < iie::PF_SHAPES; i++) out[i] = __atomic_load_n(&iie::g_prefill_launches[i], __ATOMIC_RELAXED);
-    return iie::PF_SHAPES;
+    if (!out || capacity < iie::TILE_SHAPES) return -1;
+    iie::tile_launch_counts(out);
+    return iie::TILE_SHAPES;
 }
 
 extern "C" unsigned long long iie_launch_count(void) { return __atomic_load_n(&iie::g_launches, __ATOMIC_RELAXED); }

@@ -121,6 +121,47 @@ __host__ __device__ __forceinline__ int64_t mul_shift(int64_t a, int64_t b, int 
 
 __host__ __device__ __forceinline__ int64_t silu_fixed(int64_t x, int fa) { return mul_shift(x, sigmoid_fixed(x, fa), fa); }
 
+// ((g * sigmoid(g)) >> fa) * u >> fa, the gated product of an expert.  For 1 <= fa <= 24 every operand of the sigmoid fits 32 bits:
+// 32 x 32 -> 64 products, single funnel shifts, a division without a loop; no branch, so that several evaluations interleave in one
+// thread (the general form's 64- and 128-bit shifts by a run-time amount and its fix-up loops took 3100 clocks each in the epilogue
+// of the tiles, where a warp has no other work to hide them under).  The same values.
+__host__ __device__ __forceinline__ int64_t silu_up_fixed(int64_t g, int64_t u, int fa, int64_t log2e, int64_t clip) {
+    if (fa > 24 || fa < 1) return mul_shift(mul_shift(g, sigmoid_fixed_c(g, fa, log2e, clip), fa), u, fa);
+    const bool neg = g < 0;
+    const uint64_t mag = neg ? 0ULL - (uint64_t)g : (uint64_t)g;
+    const uint32_t d = mag > (uint64_t)clip ? (uint32_t)clip : (uint32_t)mag;                   // clip < 2^(fa + 5)
+    const uint32_t e = (uint32_t)(((uint64_t)d * (uint32_t)log2e) >> fa);                       // < 2^(fa + 5)
+    const uint32_t one = 1u << fa, f = e & (one - 1), k = e >> fa;
+    const int s = 16 - fa;
+    const uint32_t c0 = s >= 0 ? 65536u >> s : 65536u << -s, c1 = s >= 0 ? 45426u >> s : 45426u << -s, c2 = s >= 0 ? 15743u >> s : 15743u << -s,
+                   c3 = s >= 0 ? 3638u >> s : 3638u << -s;
+    const uint32_t f2 = (uint32_t)(((uint64_t)f * f) >> fa), f3 = (uint32_t)(((uint64_t)f2 * f) >> fa);
+    int p = (int)c0 - (int)(uint32_t)(((uint64_t)c1 * f) >> fa) + (int)(uint32_t)(((uint64_t)c2 * f2) >> fa) - (int)(uint32_t)(((uint64_t)c3 * f3) >> fa);
+    p = p < 0 ? 0 : p;
+    const uint32_t es = (uint32_t)p >> (k < 31 ? k : 31), num = neg ? es : one, z = es + one;
+    // sg = floor(num 2^fa / z) <= 2^fa: a single-precision estimate within 5 (num is exact, z and the products round to 2^-24), then its
+    // remainder, which fits 32 bits, divided the same way: within one, the sign of what is left decides
+#ifdef __CUDA_ARCH__
+    const float rz = __frcp_rn((float)z);
+    uint32_t sg = __float2uint_rz((float)num * (float)one * rz);
+    int r = (int)((num << fa) - sg * z);
+    const int q2 = __float2int_rn((float)r * rz);
+    r -= q2 * (int)z;
+    sg += (uint32_t)q2 - (r < 0 ? 1u : 0u);
+#else
+    const uint32_t sg = (uint32_t)(((uint64_t)num << fa) / z);
+#endif
+    // g * sg = (high word) * sg * 2^32 + (low word) * sg: only the second part is floored
+    const uint64_t lo = (uint64_t)(uint32_t)g * sg;
+    const int64_t hi = (int64_t)(int32_t)(g >> 32) * (int64_t)sg;
+    const int64_t silu = (int64_t)(((uint64_t)hi << (32 - fa)) + (lo >> fa));
+#ifdef __CUDA_ARCH__
+    return (int64_t)(((uint64_t)__mul64hi(silu, u) << (64 - fa)) | (((uint64_t)silu * (uint64_t)u) >> fa));
+#else
+    return mul_shift(silu, u, fa);
+#endif
+}
+
 // ---- balanced base-256 digits: x = sum_l d_l * 256^l, d_l in [-128,127] --------------------------------
 // Eight digits cover |x| <= 127*(2^64-1)/255; `ok` is cleared when a ninth digit would be needed
 // (capacity rule of north-mini-code/src/nmc/qk_cuda.py:973-992).

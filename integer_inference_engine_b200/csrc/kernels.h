@@ -154,33 +154,36 @@ struct BatchArgs {
 };
 cudaError_t launch_batch(int qtype, int mode, const BatchArgs &a, cudaStream_t s);
 
-// Prefill-regime grouped products on tcgen05 (prefill.cu).  Pairs are sorted by expert: expert x owns
-// pairs [grp_off[x], grp_off[x+1]).
-struct PrefillArgs {
-    const uint8_t *const *wa;      // per expert: repacked weight (down / linear weight, or gate)
-    const uint8_t *const *wb;      // per expert: up weight (MODE_GATEUP)
-    const int *grp_off;            // [n_experts + 1]
-    int n_experts;
-    long long n_pairs;             // total pairs (bounds the grid)
-    long long out_f, n_blocks;
+// Products of two rows and more on tcgen05 (tiles.cu): group g (an expert, or the one matrix of a dense product) owns the rows
+// ("pairs") [grp_off[g], grp_off[g+1]).  cudaErrorNotSupported: no tile for this format, mode or shape.
+struct TileArgs {
+    const uint8_t *const *wa;      // per group: linear / down weight, or gate
+    const uint8_t *const *wb;      // per group: up weight (MODE_GATEUP)
+    const int *grp_off;            // device [n_groups + 1]
+    int n_groups, nb;              // nb: 256-column super-blocks
+    long long n_rows;              // upper bound of grp_off[n_groups]
+    long long out_f;
     int fw, fa;
-    int n_ntiles;                  // filled in by the launcher
-    long long sig_log2e, sig_clip;
-    const int8_t *xl;              // activation limb planes [x_row][8][K]
+    const int8_t *xl;              // digit planes [x_row][8][K]
     const int *xidx;               // pair -> x_row, or nullptr (identity)
-    int8_t *xg;                    // with xidx: scratch for the planes gathered into pair order, n_pairs * 4 * K bytes
-    int64_t *out;                  // GATEUP: gu [pair][out_f] (nullable); DOWN: [token][out_f] accumulated; LINEAR [pair][out_f]
-    int8_t *out_limbs;             // GATEUP: limb planes of gu [pair][8][out_f]
-    int *out_nl;                   // GATEUP: atomicMax of the limbs gu needs
+    int8_t *xg;                    // with xidx: scratch for the planes in pair order, n_rows * 8 * K bytes
+    int8_t *xs;                    // Q4_K: scratch for the sub-block sums, tile_sums_bytes(n_rows, nb)
+    const int *x_nl;               // device: digits in use by x, or nullptr (eight)
+    int64_t *out;                  // LINEAR [pair][out_f]; GATEUP gu [pair][out_f] (nullable); DOWN [token][out_f] accumulated
+    int8_t *out_limbs;             // GATEUP: digit planes of gu [pair][8][out_f]
+    int *out_nl;                   // GATEUP: atomicMax of the digits gu needs
     const int64_t *gates;          // DOWN: per pair
-    const int *pair_tok;           // DOWN: pair -> token row
-    int *flags;
+    const int *pair_tok;           // DOWN: pair -> token row, or nullptr (identity)
+    int *flags;                    // bit 0 digit envelope, bit 3 a wait gave up
+    int wide;                      // filled in by the launcher
+    long long sig_log2e, sig_clip;
 };
-cudaError_t launch_prefill(int qtype, int mode, int nl, const PrefillArgs &a, cudaStream_t s);
-// launches of each tensor-core tile shape since the library was loaded, in the order: Q4_K gate/up with 3 / 4 activation
-// digits, Q6_K down with 5 / 6, Q4_K down with 5, Q4_K linear with 3 / 5
-constexpr int PF_SHAPES = 7;
-extern unsigned long long g_prefill_launches[PF_SHAPES];
+cudaError_t launch_tiles(int qtype, int mode, const TileArgs &a, cudaStream_t s);
+size_t tile_sums_bytes(long long rows, long long n_blocks);
+// launches by tile shape since the library was loaded: Q4_K gate/up with 3 / 4 activation digits, Q6_K down with up to 5 / 6,
+// Q4_K down with up to 5, Q4_K linear with 3 / up to 5, all others (counted on the device, where the digits are known)
+constexpr int TILE_SHAPES = 8;
+void tile_launch_counts(unsigned long long *out);
 
 // Re-order raw GGUF blocks into the half-tile layout; also reduces max |d| and max |dmin| half bit
 // patterns (sign stripped) into maxbits[0..1] (device memory, caller zeroes).

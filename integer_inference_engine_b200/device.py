@@ -328,8 +328,8 @@ def workspace_generation() -> int:
 
 
 def prefill_launch_counts() -> list:
-    """Launches of each tensor-core tile shape since load: [gate/up 3 digits, gate/up 4, Q6_K down 5, Q6_K down 6,
-    Q4_K down 5, linear 3, linear 5]."""
+    """Launches of each tensor-core tile shape since load: [gate/up 3 digits, gate/up 4, Q6_K down up to 5, Q6_K down 6,
+    Q4_K down up to 5, Q4_K linear 3, Q4_K linear up to 5, all others].  Counted on the device: synchronises."""
     buf = (ctypes.c_uint64 * 8)()
     n = qk_cuda.load_library().iie_prefill_launch_counts(buf, 8)
     return [int(buf[i]) for i in range(n)]

@@ -1,0 +1,69 @@
+"""Products of two rows and more on the tensor-core tiles against the CPU oracle, where the tiles can go wrong: row counts around
+the tile widths, matrix rows around 128, one to many super-blocks (the sub-block sums are padded to four), three to eight
+activation digits, both block formats, extreme scale patterns, uneven expert groups with experts that get no row."""
+import numpy as np
+import pytest
+
+from oracle import native as onat
+from oracle import qk_oracle as o
+
+pytestmark = pytest.mark.gpu
+FA, FW = 16, 24
+
+
+@pytest.fixture(autouse=True)
+def _from_two_rows():
+    from integer_inference_engine_b200 import qk_cuda
+    assert qk_cuda.available(), "CUDA library or GPU missing"
+    qk_cuda.load_library().iie_set_tc_min_tokens(2)
+    yield
+    qk_cuda.free_all()
+
+
+@pytest.mark.parametrize("qtype", [o.Q4_K, o.Q6_K])
+@pytest.mark.parametrize("out_f,nb,T,xbits", [(8, 1, 2, 20), (128, 1, 16, 22), (129, 2, 17, 22), (120, 3, 32, 22), (200, 5, 33, 29), (264, 8, 31, 38),
+                                              (130, 4, 65, 46), (72, 9, 5, 62), (2056, 1, 300, 22)])
+def test_dense_tiles_match_the_oracle(qtype, out_f, nb, T, xbits):
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(out_f + nb * 5 + T)
+    raw = np.frombuffer((o.synth_q4k if qtype == o.Q4_K else o.synth_q6k)(rng, out_f, nb), np.uint8).copy().reshape(out_f * nb, -1)
+    fill = slice(4, 144) if qtype == o.Q4_K else slice(0, 208)                 # every scale, minimum and code at its largest in some blocks
+    raw[::3, fill] = 0xFF
+    if qtype == o.Q6_K:
+        raw[1::3, 192:208] = 0x80                                             # scales of -128
+    raw = raw.tobytes()
+    x = rng.integers(-(1 << xbits), 1 << xbits, size=(T, nb * 256), dtype=np.int64)
+    if xbits == 22:
+        x[0], x[-1] = 8355711, -8421504                                        # the ends of three balanced digits
+    device.read_flags()
+    h = qk_cuda.register_weight(raw, out_f, nb, qtype)
+    before = device.prefill_launch_counts()
+    got = device.apply(h, torch.from_numpy(x).cuda(), out_f, FW).cpu().numpy()
+    assert sum(device.prefill_launch_counts()) == sum(before) + 1, "the product did not run on the tiles"
+    assert device.read_flags() == 0
+    assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, qtype))
+
+
+@pytest.mark.parametrize("down_q", [o.Q4_K, o.Q6_K])
+@pytest.mark.parametrize("d,eff,E,k,T,mult", [(256, 256, 5, 2, 3, 1), (512, 256, 40, 1, 2, 1), (768, 512, 6, 3, 70, 1), (256, 768, 3, 3, 33, 200)])
+def test_expert_tiles_match_the_oracle(down_q, d, eff, E, k, T, mult):
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(d + eff + T)
+    q4 = lambda r, c: o.synth_q4k(rng, r, c // 256)
+    router, gate, up = q4(E, d), [q4(eff, d) for _ in range(E)], [q4(eff, d) for _ in range(E)]
+    down = [(o.synth_q4k if down_q == o.Q4_K else o.synth_q6k)(rng, d, eff // 256) for _ in range(E)]
+    h = o.to_fixed(rng.standard_normal((T, d)), FA) * mult
+    reg = lambda w, r, c, q=o.Q4_K: qk_cuda.register_weight(w, r, c // 256, q)
+    layer = device.MoELayer(reg(router, E, d), [reg(w, eff, d) for w in gate], [reg(w, eff, d) for w in up], [reg(w, d, eff, down_q) for w in down], k, d, eff)
+    device.read_flags()
+    out, ids, gates = layer.forward(torch.from_numpy(h).cuda(), FA, FW)
+    torch.cuda.synchronize()
+    assert device.read_flags() == 0
+    ids_ref, gates_ref, out_ref = onat.moe_block(router, o.Q4_K, gate, up, down, o.Q4_K, down_q, k, h, d, eff, FA, FW)
+    assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
+    assert np.array_equal(out.cpu().numpy(), out_ref)
+    layer.close()
