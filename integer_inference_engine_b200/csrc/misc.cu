@@ -3,6 +3,9 @@
 // element-wise steps used by the fallback composition.
 #include "kernels.h"
 #include "layout.cuh"
+#include "norm.cuh"
+
+#include <algorithm>
 
 namespace iie {
 
@@ -284,30 +287,6 @@ __global__ void dispatch_kernel(const int *ids, const int64_t *gates, long long 
 // ---------------------------------------------------------------------------------------------------
 // integer RMSNorm (north-mini-code/src/nmc/_bonsai/fixedpoint.py:32-72), one CTA per row
 // ---------------------------------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long uabs64(int64_t v) { return v < 0 ? (0ULL - (unsigned long long)v) : (unsigned long long)v; }
-
-__device__ u128 isqrt_u128(u128 v) {
-    u128 res = 0, bit = (u128)1 << 126;
-    while (bit > v) bit >>= 2;
-    while (bit != 0) {
-        if (v >= res + bit) { v -= res + bit; res = (res >> 1) + bit; } else res >>= 1;
-        bit >>= 2;
-    }
-    return res;
-}
-
-// floor(sqrt(v)): a double estimate fixed up with exact 128-bit products while v < 2^104, else the bitwise root
-__device__ u128 isqrt_fast(u128 v) {
-    if (v < ((u128)1 << 104)) {
-        const double dv = (double)(unsigned long long)(v >> 64) * 18446744073709551616.0 + (double)(unsigned long long)v;
-        unsigned long long r = (unsigned long long)sqrt(dv);
-        for (int it = 0; it < 8 && (u128)r * r > v; it++) r--;
-        for (int it = 0; it < 8 && (u128)(r + 1) * (r + 1) <= v; it++) r++;
-        if ((u128)r * r <= v && (u128)(r + 1) * (r + 1) > v) return r;
-    }
-    return isqrt_u128(v);
-}
-
 // one element of the normalised row: floor((x << fa) / rms), then (y * gain) >> fa; `bad` is set (and 0 returned)
 // where the oracle's envelope checks would refuse the value
 __device__ __forceinline__ int64_t norm_value(int64_t xv, unsigned long long rms, unsigned long long inv, unsigned long long gm,
@@ -334,108 +313,227 @@ __device__ __forceinline__ int64_t norm_value(int64_t xv, unsigned long long rms
     return y;
 }
 
-// rows from `rows_a` on use gain_b (per-head norms of queries and keys in one launch)
-__global__ void __launch_bounds__(1024) rmsnorm_kernel(const int64_t *x, long long rows, long long width, const int64_t *gain_a,
-                                                       int fa, unsigned long long eps, int64_t *out, int *flags,
-                                                       int8_t *planes, int64_t *totals, const int64_t *gain_b, long long rows_a,
-                                                       int split, const PlaneDuties duties) {
-    // `split` CTAs share a row: each sums the squares of the whole row (cheap, the row sits in L2) and normalises its own
-    // slice, so that the divisions of a long row are spread over several SMs
-    __shared__ unsigned long long s_lo[32], s_hi[32], s_max[32], s_gmax[32];
-    __shared__ unsigned long long s_rms, s_gm, s_inv;
-    __shared__ int s_bad;
-    int *nl_out = duties.nl;
-    if (duties.nl_clear && blockIdx.x == 0 && threadIdx.x == 0) *duties.nl_clear = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < duties.zero_n; i += (long long)gridDim.x * blockDim.x) duties.zero[i] = 0;
-    const long long row = blockIdx.x / split;
-    const int part = blockIdx.x - (int)row * split;
-    const int64_t *gain = row < rows_a ? gain_a : gain_b;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int64_t *xr = x + row * width;
-    int64_t *yr = out + row * width;
-    u128 ssq = 0; unsigned long long mx = 0, gmx = 0;
-    for (long long i0 = tid; i0 < width; i0 += (long long)blockDim.x * 8) {      // eight loads in flight per thread
-        int64_t xv[8], gv[8];
+// sum over the warp of 128-bit (64-bit) values: pieces of 22 bits, one warp reduction each
+__device__ __forceinline__ u128 warp_sum128(u128 v) {
+    u128 sum = 0;
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const long long i = i0 + (long long)u * blockDim.x;
-            xv[u] = i < width ? xr[i] : 0;
-            gv[u] = (gain && i < width) ? gain[i] : 0;
+    for (int k = 0; k < 6; k++) sum += (u128)__reduce_add_sync(0xffffffffu, (uint32_t)(v >> (22 * k)) & 0x3FFFFFu) << (22 * k);
+    return sum;
+}
+__device__ __forceinline__ uint64_t warp_sum64(uint64_t v) {
+    uint64_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) sum += (uint64_t)__reduce_add_sync(0xffffffffu, (uint32_t)(v >> (22 * k)) & 0x3FFFFFu) << (22 * k);
+    return sum;
+}
+
+struct NormArgs {
+    const int64_t *x;
+    long long rows, rows_a;        // rows from rows_a on take gain_b (per-head norms of queries and keys in one launch)
+    int width, wpr;                // warps of a row
+    bool wide;                     // every row and the gains start on 16 bytes
+    const int64_t *gain_a, *gain_b;
+    int fa;
+    unsigned long long eps;
+    int64_t *out;                  // nullable
+    int8_t *planes;                // nullable: digit planes [row][8][width]
+    int64_t *totals;               // nullable: 128-element block sums [row][width / 128]
+    int *flags;
+    PlaneDuties duties;
+};
+
+// The row stays in registers: a thread holds G groups of four consecutive values, a warp 128 values per group, `wpr` warps a row
+// (several short rows share a CTA).  One barrier: every warp adds up the warps' sums and takes the root itself.  What bounds it for
+// one row is that chain (row load, two rounds of warp reductions, root and reciprocal, quotients: about 4.5 us with the launch; the
+// row read twice, a thread taking the root alone and 64-bit quotients for all: 7), for many rows the eight bytes per value in and
+// out and the quotients (2048 x 2048: 103 us before).
+template <int G>
+__global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormArgs a) {
+    __shared__ uint64_t s_lo[32], s_hi[32];
+    __shared__ uint32_t s_bits[32];
+    if (a.duties.nl_clear && blockIdx.x == 0 && threadIdx.x == 0) *a.duties.nl_clear = 0;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.duties.zero_n; i += (long long)gridDim.x * blockDim.x) a.duties.zero[i] = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpr = a.wpr, in_row = warp % wpr;      // wpr is 1 or the CTA's warps
+    const long long row = wpr == 1 ? (long long)blockIdx.x * (blockDim.x >> 5) + warp : blockIdx.x;
+    const bool live = row < a.rows;
+    const int64_t *gain = row < a.rows_a ? a.gain_a : a.gain_b;
+    const int step = wpr * 128, i0 = in_row * 128 + lane * 4;
+    int64_t x[G][4], g[G][4];
+    u128 ssq = 0;
+    uint64_t mx = 0, gmx = 0;
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+        const bool in = live && i0 + k * step < a.width;
+        const int64_t *src = a.x + row * a.width + i0 + k * step, *gs = gain + i0 + k * step;
+        longlong2 v0 = make_longlong2(0, 0), v1 = v0, g0 = make_longlong2(1, 1), g1 = g0;
+        if (in && a.wide) {
+            v0 = *reinterpret_cast<const longlong2 *>(src); v1 = *reinterpret_cast<const longlong2 *>(src + 2);
+            if (gain) { g0 = *reinterpret_cast<const longlong2 *>(gs); g1 = *reinterpret_cast<const longlong2 *>(gs + 2); }
+        } else if (in) {
+            v0 = make_longlong2(src[0], src[1]); v1 = make_longlong2(src[2], src[3]);
+            if (gain) { g0 = make_longlong2(gs[0], gs[1]); g1 = make_longlong2(gs[2], gs[3]); }
         }
+        x[k][0] = v0.x; x[k][1] = v0.y; x[k][2] = v1.x; x[k][3] = v1.y;
+        g[k][0] = g0.x; g[k][1] = g0.y; g[k][2] = g1.x; g[k][3] = g1.y;
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const unsigned long long a = uabs64(xv[u]), ga = uabs64(gv[u]);
-            ssq += (u128)a * a;
-            mx = a > mx ? a : mx;
-            gmx = ga > gmx ? ga : gmx;
+        for (int e = 0; e < 4; e++) {
+            const uint64_t m = uabs64(x[k][e]), gm = uabs64(g[k][e]);
+            ssq += (u128)m * m;
+            mx = m > mx ? m : mx; gmx = gm > gmx ? gm : gmx;
         }
     }
-    auto fold = [&]() {
-#pragma unroll
-        for (int off = 16; off; off >>= 1) {
-            const unsigned long long lo = __shfl_down_sync(0xffffffffu, (unsigned long long)ssq, off);
-            const unsigned long long hi = __shfl_down_sync(0xffffffffu, (unsigned long long)(ssq >> 64), off);
-            const unsigned long long m2 = __shfl_down_sync(0xffffffffu, mx, off), g2 = __shfl_down_sync(0xffffffffu, gmx, off);
-            ssq += ((u128)hi << 64) | lo;
-            mx = m2 > mx ? m2 : mx; gmx = g2 > gmx ? g2 : gmx;
-        }
-    };
-    fold();
-    if (lane == 0) { s_lo[warp] = (unsigned long long)ssq; s_hi[warp] = (unsigned long long)(ssq >> 64); s_max[warp] = mx; s_gmax[warp] = gmx; }
-    __syncthreads();
-    if (warp == 0) {
-        ssq = lane < nwarps ? (((u128)s_hi[lane] << 64) | s_lo[lane]) : (u128)0;
-        mx = lane < nwarps ? s_max[lane] : 0; gmx = lane < nwarps ? s_gmax[lane] : 0;
-        fold();
-        if (lane == 0) {
-            // |x| <= 2^57 keeps the 128-bit sum of squares exact for any width <= 2^13
-            int bad = (mx > (1ULL << 57) || width > 8192) ? 1 : 0;
-            const u128 mean = ((width & (width - 1)) == 0 ? ssq >> (63 - __clzll(width)) : ssq / (u128)(unsigned long long)width) + eps;
-            const u128 rms = isqrt_fast(mean);
-            if (rms == 0 || rms > (u128)0xFFFFFFFFFFFFFFFFULL) bad = 1;
-            s_rms = (unsigned long long)rms; s_gm = gmx; s_bad = bad;
-            s_inv = (rms != 0 && rms < ((u128)1 << 62)) ? 0xFFFFFFFFFFFFFFFFULL / (unsigned long long)rms : 0ULL;
-        }
+    // bit lengths of the largest |x| and |gain|; beyond 2^57 in |x| the sum of squares may wrap and the row is refused
+    uint32_t bits = (uint32_t)(64 - __clzll((long long)mx)) | (uint32_t)(64 - __clzll((long long)gmx)) << 8;
+    bool beyond = mx > (1ULL << 57);
+    uint32_t xb = __reduce_max_sync(0xffffffffu, (bits & 0xFF) | (beyond ? 128u : 0u)), gb = __reduce_max_sync(0xffffffffu, bits >> 8);
+    ssq = warp_sum128(ssq);
+    if (wpr > 1) {
+        if (lane == 0) { s_lo[warp] = (uint64_t)ssq; s_hi[warp] = (uint64_t)(ssq >> 64); s_bits[warp] = xb | gb << 8; }
+        __syncthreads();
+        ssq = lane < wpr ? ((u128)s_hi[lane] << 64) | s_lo[lane] : (u128)0;
+        bits = lane < wpr ? s_bits[lane] : 0;
+        ssq = warp_sum128(ssq);
+        xb = __reduce_max_sync(0xffffffffu, bits & 0xFF); gb = __reduce_max_sync(0xffffffffu, bits >> 8);
     }
-    __syncthreads();
-    if (s_bad) { if (tid == 0 && part == 0) atomicOr(flags, 2); return; }
-    const unsigned long long rms = s_rms, inv = s_inv;
-    const unsigned long long gm = s_gm;
+    beyond = (xb & 128u) != 0; xb &= 127u;
+    const u128 mean = ((a.width & (a.width - 1)) == 0 ? ssq >> (31 - __clz(a.width)) : ssq / (u128)(unsigned)a.width) + a.eps;
+    const u128 root = isqrt128(mean);
+    const uint64_t rms = (uint64_t)root;
+    if (beyond || root == 0 || (root >> 64) != 0) {                // refused: nothing is written
+        if (live && lane == 0 && in_row == 0) atomicOr(a.flags, 2);
+        return;
+    }
+    const int fa = a.fa;
+    // Every |x| < 2^xb and |gain| < 2^gb: with n = 2^(xb + fa) the quotients stay below 2^31 when n < rms 2^31, and the gain products inside
+    // four balanced digits when n 2^gb <= rms (0x7F7F7F7D 2^sh - 2^gb)
+    bool fast = false;
+    const int sh = gain ? fa : 0;                                  // without a gain: a factor of one
+    if ((int)xb + fa <= 62 && gb <= 31 && rms < (1ULL << 62)) {
+        const u128 n = (u128)1 << (xb + fa), lim = (u128)2139062141ULL << sh, g1 = (u128)1 << gb;
+        fast = n < (u128)rms * 2147483646ULL && lim > g1 && (n << gb) <= (u128)rms * (lim - g1);
+    }
+    const uint64_t inv = rms < (1ULL << 62) ? recip_below(rms) : 0;
+    uint64_t gm = 0;
+    if (!fast && gain) {                                           // the general form refuses against the row's largest |gain|
+        for (int k = 0; k < a.width; k += 32) { const int i = k + lane; const uint64_t v = i < a.width ? uabs64(gain[i]) : 0; gm = v > gm ? v : gm; }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) { const uint64_t o = __shfl_xor_sync(0xffffffffu, gm, off); gm = o > gm ? o : gm; }
+    }
     bool bad = false;
-    if (planes) {
-        // digit planes [row][8][width] and 128-element block sums of the normalised row, for the Q1_0 product
-        const long long nb = width >> 7, per = (nb + split - 1) / split;
-        const long long b_end = min(nb, (part + 1) * per);
-        int nl = 0;
-        for (long long b = part * per + warp; b < b_end; b += nwarps) {
-            const long long i0 = b * 128 + lane * 4;
-            uint32_t pl[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            unsigned long long sum = 0;
+    int nl = 0;
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int64_t y = norm_value(xr[i0 + j], rms, inv, gm, gain ? gain[i0 + j] : 0, gain != nullptr, fa, bad);
-                if (out) yr[i0 + j] = y;
-                bool ok;
-                const uint64_t d = balanced_digits8(y, ok);
-                nl = max(nl, ok ? digits_used(d) : 9);
-                sum += (unsigned long long)y;
+    for (int k = 0; k < G; k++) {
+        const int i = i0 + k * step;
+        const bool in = live && i < a.width;
+        int64_t y[4];
+        if (fast) {
 #pragma unroll
-                for (int l = 0; l < 8; l++) pl[l] |= (uint32_t)((d >> (8 * l)) & 0xFF) << (8 * j);
+            for (int e = 0; e < 4; e++) {
+                const uint64_t n = uabs64(x[k][e]) << fa;
+                uint64_t q = __umul64hi(n, inv), r = n - q * rms;
+#pragma unroll
+                for (int fix = 0; fix < 2; fix++) { const bool up = r >= rms; q += up; r -= up ? rms : 0; }      // at most two below: n < 2^62
+                const int yq = x[k][e] >= 0 ? (int)q : -(int)q - (r != 0);                // floor of the signed quotient
+                y[e] = ((int64_t)yq * (int)g[k][e]) >> sh;
             }
+        } else {
 #pragma unroll
-            for (int l = 0; l < 8; l++) *reinterpret_cast<uint32_t *>(planes + (row * 8 + l) * width + i0) = pl[l];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-            if (lane == 0) totals[row * nb + b] = (int64_t)sum;
+            for (int e = 0; e < 4; e++) y[e] = in ? norm_value(x[k][e], rms, inv, gm, g[k][e], gain != nullptr, fa, bad) : 0;
         }
-        nl = __reduce_max_sync(0xffffffffu, nl);
-        if (lane == 0 && nl_out && nl > *(volatile int *)nl_out) atomicMax(nl_out, nl);
-    } else {
-        const long long per = (width + split - 1) / split, i_end = min(width, (part + 1) * per);
-        for (long long i = part * per + tid; i < i_end; i += blockDim.x)
-            yr[i] = norm_value(xr[i], rms, inv, gm, gain ? gain[i] : 0, gain != nullptr, fa, bad);
+        if (in && a.out) {
+            int64_t *to = a.out + row * a.width + i;
+            if (a.wide) {
+                *reinterpret_cast<longlong2 *>(to) = make_longlong2(y[0], y[1]); *reinterpret_cast<longlong2 *>(to + 2) = make_longlong2(y[2], y[3]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) to[e] = y[e];
+            }
+        }
+        if (a.planes) {
+            uint32_t pl[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            if (fast) {                                            // byte l of (y + 0x80808080) ^ 0x80808080 is the balanced digit l
+                uint32_t d[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) d[e] = ((uint32_t)(int)y[e] + 0x80808080u) ^ 0x80808080u;
+                const uint32_t any = d[0] | d[1] | d[2] | d[3];
+                nl = max(nl, any == 0 ? 1 : 4 - (__clz((int)any) >> 3));
+                const uint32_t t0 = __byte_perm(d[0], d[1], 0x5140), t1 = __byte_perm(d[2], d[3], 0x5140);
+                const uint32_t t2 = __byte_perm(d[0], d[1], 0x7362), t3 = __byte_perm(d[2], d[3], 0x7362);
+                pl[0] = __byte_perm(t0, t1, 0x5410); pl[1] = __byte_perm(t0, t1, 0x7632); pl[2] = __byte_perm(t2, t3, 0x5410); pl[3] = __byte_perm(t2, t3, 0x7632);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    bool ok;
+                    const uint64_t d = balanced_digits8(y[e], ok);
+                    nl = max(nl, ok ? digits_used(d) : 9);
+#pragma unroll
+                    for (int l = 0; l < 8; l++) pl[l] |= (uint32_t)((d >> (8 * l)) & 0xFF) << (8 * e);
+                }
+            }
+            if (in) {
+#pragma unroll
+                for (int l = 0; l < 8; l++) *reinterpret_cast<uint32_t *>(a.planes + (row * 8 + l) * a.width + i) = pl[l];
+            }
+            if (a.totals) {
+                const uint64_t sum = warp_sum64((uint64_t)y[0] + (uint64_t)y[1] + (uint64_t)y[2] + (uint64_t)y[3]);
+                if (in && lane == 0) a.totals[row * (a.width >> 7) + (i >> 7)] = (int64_t)sum;
+            }
+        }
     }
-    if (bad) atomicOr(flags, 2);
+    if (a.planes && a.duties.nl) {
+        nl = __reduce_max_sync(0xffffffffu, live ? nl : 0);
+        if (lane == 0 && nl > *(volatile int *)a.duties.nl) atomicMax(a.duties.nl, nl);
+    }
+    if (live && bad) atomicOr(a.flags, 2);
+}
+
+// any width: one CTA per row, values read again for the quotients
+__global__ void __launch_bounds__(256) rmsnorm_any_kernel(const NormArgs a) {
+    __shared__ uint64_t s_lo[8], s_hi[8], s_max[8], s_gmax[8];
+    const long long row = blockIdx.x;
+    const int64_t *gain = row < a.rows_a ? a.gain_a : a.gain_b, *xr = a.x + row * a.width;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    u128 ssq = 0;
+    uint64_t mx = 0, gm = 0;
+    for (int i = tid; i < a.width; i += 256) {
+        const uint64_t m = uabs64(xr[i]), gv = gain ? uabs64(gain[i]) : 0;
+        ssq += (u128)m * m;
+        mx = m > mx ? m : mx; gm = gv > gm ? gv : gm;
+    }
+    auto top = [&](uint64_t v) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) { const uint64_t o = __shfl_xor_sync(0xffffffffu, v, off); v = o > v ? o : v; }
+        return v;
+    };
+    ssq = warp_sum128(ssq); mx = top(mx); gm = top(gm);
+    if (lane == 0) { s_lo[warp] = (uint64_t)ssq; s_hi[warp] = (uint64_t)(ssq >> 64); s_max[warp] = mx; s_gmax[warp] = gm; }
+    __syncthreads();
+    ssq = warp_sum128(lane < 8 ? ((u128)s_hi[lane] << 64) | s_lo[lane] : (u128)0);
+    mx = top(lane < 8 ? s_max[lane] : 0); gm = top(lane < 8 ? s_gmax[lane] : 0);
+    const u128 root = isqrt128(ssq / (u128)(unsigned)a.width + a.eps);
+    if (mx > (1ULL << 57) || a.width > 8192 || root == 0 || (root >> 64) != 0) { if (tid == 0) atomicOr(a.flags, 2); return; }
+    const uint64_t rms = (uint64_t)root, inv = rms < (1ULL << 62) ? recip_below(rms) : 0;
+    bool bad = false;
+    for (int i = tid; i < a.width; i += 256) a.out[row * a.width + i] = norm_value(xr[i], rms, inv, gm, gain ? gain[i] : 0, gain != nullptr, a.fa, bad);
+    if (bad) atomicOr(a.flags, 2);
+}
+
+cudaError_t launch_norm(NormArgs a, cudaStream_t s) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.gain_a) | reinterpret_cast<uintptr_t>(a.gain_b) | reinterpret_cast<uintptr_t>(a.out);
+    a.wide = (at & 15) == 0;
+    if (a.width > 8192 || a.width % 4) {                           // (beyond 8192 every row is refused)
+        rmsnorm_any_kernel<<<(unsigned)a.rows, 256, 0, s>>>(a);
+    } else {
+        const int groups = (a.width + 127) / 128;                  // of 128 values
+        a.wpr = groups <= 2 ? 1 : groups <= 32 ? groups : (groups + 1) / 2;          // one or two groups: a warp per row, eight rows per CTA
+        const int threads = a.wpr == 1 ? 256 : a.wpr * 32;
+        long long grid = a.wpr == 1 ? (a.rows + 7) / 8 : a.rows;
+        grid = std::max(grid, std::min(148LL, a.duties.zero_n / (threads * 8)));     // few rows: more CTAs for the words to clear
+        if (groups == 1 || (groups > 2 && groups <= 32)) rmsnorm_kernel<1><<<(unsigned)grid, threads, 0, s>>>(a);
+        else rmsnorm_kernel<2><<<(unsigned)grid, threads, 0, s>>>(a);
+    }
+    note_launch();
+    return cudaGetLastError();
 }
 
 inline unsigned grid_for(long long n, int tpb, long long cap = 148LL * 64) {
@@ -549,34 +647,20 @@ cudaError_t launch_topk(const int64_t *logits, long long rows, int n_experts, in
 
 cudaError_t launch_rmsnorm(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
                            unsigned long long eps, int64_t *out, int *flags, cudaStream_t s) {
-    const int split = (rows <= 16 && width >= 1024) ? (int)((width + 511) / 512) : 1;      // few long rows: 512 values per CTA
-    const int threads = split > 1 ? 128 : (width >= 2048 ? 1024 : width > 128 ? 256 : 128);
-    rmsnorm_kernel<<<(unsigned)(rows * split), threads, 0, s>>>(x, rows, width, gain, fa, eps, out, flags, nullptr, nullptr, nullptr, rows,
-                                                                 split, PlaneDuties());
-    note_launch();
-    return cudaGetLastError();
+    if (rows <= 0 || width <= 0 || width > (1 << 30)) return cudaErrorInvalidValue;
+    return launch_norm({x, rows, rows, (int)width, 0, false, gain, nullptr, fa, eps, out, nullptr, nullptr, flags, PlaneDuties()}, s);
 }
 
 cudaError_t launch_rmsnorm_pair(const int64_t *x, long long rows_a, long long rows_b, long long width, const int64_t *gain_a,
                                 const int64_t *gain_b, int fa, unsigned long long eps, int64_t *out, int *flags, cudaStream_t s) {
-    const int threads = width >= 2048 ? 1024 : width > 128 ? 256 : 128;
-    rmsnorm_kernel<<<(unsigned)(rows_a + rows_b), threads, 0, s>>>(x, rows_a + rows_b, width, gain_a, fa, eps, out, flags, nullptr, nullptr,
-                                                                  gain_b, rows_a, 1, PlaneDuties());
-    note_launch();
-    return cudaGetLastError();
+    if (rows_a + rows_b <= 0 || width <= 0 || width > (1 << 30)) return cudaErrorInvalidValue;
+    return launch_norm({x, rows_a + rows_b, rows_a, (int)width, 0, false, gain_a, gain_b, fa, eps, out, nullptr, nullptr, flags, PlaneDuties()}, s);
 }
 
 cudaError_t launch_rmsnorm_planes(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
                                   unsigned long long eps, int64_t *out, int8_t *planes, int64_t *totals, int *flags, const PlaneDuties &duties, cudaStream_t s) {
-    if (width <= 0 || (width & 127) || !planes || !totals) return cudaErrorInvalidValue;
-    // one warp per 128-element block; few rows of a long row: four blocks per CTA, several CTAs per row
-    const long long nb = width >> 7;
-    const int split = (rows <= 16 && nb >= 8) ? (int)((nb + 3) / 4) : 1;
-    const int threads = split > 1 ? 128 : (width >= 4096 ? 1024 : width >= 1024 ? (int)(width >> 2) : 256);
-    rmsnorm_kernel<<<(unsigned)(rows * split), threads, 0, s>>>(x, rows, width, gain, fa, eps, out, flags, planes, totals, nullptr, rows,
-                                                                 split, duties);
-    note_launch();
-    return cudaGetLastError();
+    if (rows <= 0 || width <= 0 || (width & 127) || width > (1 << 30) || !planes) return cudaErrorInvalidValue;
+    return launch_norm({x, rows, rows, (int)width, 0, false, gain, nullptr, fa, eps, out, planes, totals, flags, duties}, s);
 }
 
 cudaError_t launch_dispatch(const int *ids, const int64_t *gates, long long T, int k, int n_experts, int *grp_off,
