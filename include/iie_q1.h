@@ -116,7 +116,7 @@ void bonsai_decode_ctx_free(long long ctx_h);
  * stream).  Scratch for the digit planes is process-global and grows on demand: one caller at a time. */
 int iie_q1_apply_dev(long long handle, const int64_t *x_dev, long long tokens, long long frac, int64_t *out_dev,
                      void *stream);
-/* Product with the activation step before it and the residual after it in the same two launches:
+/* Product with the activation step before it and the residual after it in two launches (one row: one; mode 2: two):
  *   mode 0: a = x;   mode 1: a = rmsnorm(x, gain_dev, eps 1) (gain_dev NULL = no gain; an envelope violation sets
  *   bit 1 of the flag word iie_flags_read_clear reports);   mode 2: a = ((x * sigmoid(x)) >> frac) * x2 >> frac with
  *   wrapping products, x and x2 rows `ld` apart (reference_bonsai.py:603-615 _ffn_ref).
@@ -134,11 +134,19 @@ int iie_q1_head_norm_dev(const int64_t *x_dev, long long rows_a, long long rows_
  * bonsai/src/trinote/infer_int/reference_bonsai.py:246-262 and 611-614.  0 ok, 1 bad argument, 2 CUDA failure. */
 int iie_q1_silu_mul_dev(const int64_t *gate_dev, const int64_t *up_dev, long long n, long long frac, int64_t *out_dev,
                         void *stream);
+/* One decoder layer of a decode token (reference_bonsai.py:941-966 _run_layers, 656-720 _attention_with_cache_bonsai) in five
+ * launches on device buffers: x [d] (updated in place); weights wqkv (Wq, Wk, Wv rows stacked), wo, w1u (gate rows, then up
+ * rows), w2; gains n1, n2 [d], qn, kn [head_dim]; scratch qkv [(n_heads + 2 n_kv) head_dim], qkvn [(n_heads + n_kv) head_dim],
+ * att [n_heads head_dim], h [2 ffn]; caches [n_kv][cache_rows][head_dim] int32, row `position` of which is written.  pos_dev /
+ * pos as in iie_attn_decode_dev; cos, sin [cache_rows][head_dim / 2] (rotate-half).  0 ok, 1 bad argument, 2 CUDA failure. */
+int iie_q1_decode_layer_dev(long long wqkv, long long wo, long long w1u, long long w2, const int64_t *n1, const int64_t *n2,
+                            const int64_t *qn, const int64_t *kn, int64_t *x, int64_t *qkv, int64_t *qkvn, int64_t *att, int64_t *h,
+                            int32_t *kcache, int32_t *vcache, long long pos, const int *pos_dev, const int64_t *cos, const int64_t *sin,
+                            int n_heads, int n_kv, int head_dim, long long cache_rows, long long frac, long long inv_sqrt, void *stream);
 /* One row of a registered weight as int64 (sign * block scale, reference_bonsai.py:138-146 q1_rows_fp): the row index
  * is read from the device cell `row_dev` when that is not NULL, else `row`. */
 int iie_q1_embed_dev(long long handle, const int *row_dev, long long row, int64_t *out_dev, void *stream);
-/* Launch form of the single-token product: 1 = the run of tiles of a CTA is requested with bulk copies into shared
- * memory up front, 0 (default) = per-lane loads with one tile of look-ahead.  Same results, same speed within 3 %. */
+/* Kept for its callers: the single-token product has one launch form, whose weights come by bulk copies. */
 void iie_q1_set_stream(int on);
 /* Changes whenever a scratch buffer of the Q1_0 entries is freed (to grow, or by bonsai_q1_free_weights): a CUDA graph
  * captured over iie_q1_*_dev calls holds the old addresses and must be captured again. */

@@ -928,6 +928,26 @@ extern "C" int iie_attn_decode_dev(const int64_t *q_dev, const int64_t *k_dev, c
     return 0;
 }
 
+// Decode attention that applies the per-head norms itself, launched behind a kernel that starts its dependents early: 0, 1 on
+// failure, 3 where the launch form at hand does not carry the norms (nothing was launched).
+int iie::attn_decode_normed(const int64_t *q, const int64_t *k, const int64_t *v, int32_t *kcache, int32_t *vcache, long long pos,
+                            const int *pos_dev, const int64_t *cos, const int64_t *sin, int rope, int H, int Hkv, int hd, long long cache_rows,
+                            int fa, long long inv_sqrt, const int64_t *qgain, const int64_t *kgain, unsigned long long eps, int64_t *out, cudaStream_t s) {
+    std::lock_guard<std::recursive_mutex> lk(g_mu);
+    if (!init()) return 1;
+    AttnArgs a = {};
+    a.q = q; a.k = k; a.v = v; a.kcache = kcache; a.vcache = vcache; a.pos = pos; a.pos_dev = pos_dev; a.Lmax = cache_rows;
+    a.cos = cos; a.sin = sin; a.rope = rope; a.H = H; a.Hkv = Hkv; a.hd = hd;
+    attn_consts(a, fa, inv_sqrt);
+    if (!attn_scratch(a, s)) return 1;
+    a.qgain = qgain; a.kgain = kgain; a.eps = eps; a.pdl = 1;
+    a.out = out; a.flags = g_flags;
+    const cudaError_t e = launch_attn_decode(a, s);
+    if (e == cudaErrorNotSupported) return 3;
+    if (e != cudaSuccess) { cudaGetLastError(); return 1; }
+    return 0;
+}
+
 extern "C" int iie_attn_prefill_dev(const int64_t *q_dev, const int64_t *k_dev, const int64_t *v_dev, int32_t *kcache_dev,
                                     int32_t *vcache_dev, long long start, long long tokens, long long window,
                                     const int64_t *cos_dev, const int64_t *sin_dev, int rope, int n_heads, int n_kv, int head_dim,

@@ -723,6 +723,41 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
     for (int r = 8 * tid; r < nk_old; r += 8 * AF_THREADS)
         af_copy(sk + koff(r), a.kcache + ((long long)kv * a.Lmax + l0 + r) * hd, (uint32_t)(min(8, nk_old - r) * hd * 4), &bars[0]);
     if (a.pdl) { asm volatile("griddepcontrol.wait;" ::: "memory"); asm volatile("griddepcontrol.launch_dependents;"); }
+    // ---- per-head norms, where the caller wants them here: a warp per head, the new key row (by the CTA that appends it) into the
+    //      partial sums' space, which pass 1 does not use before the rotation is done
+    int64_t *knew = reinterpret_cast<int64_t *>(red);
+    if (a.qgain) {
+        if (warp < rep + (own ? 1 : 0)) {
+            const bool is_k = warp == rep;
+            const int64_t *src = is_k ? a.k + kv * hd : a.q + (long long)(kv * rep + warp) * hd, *gain = is_k ? a.kgain : a.qgain;
+            int64_t *dst = is_k ? knew : reinterpret_cast<int64_t *>(q64) + warp * hd;
+            int64_t x[8], gv[8];                                            // hd <= 256
+            u128 ssq = 0;
+            uint64_t mx = 0, gm = 0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) { const int i = lane + 32 * k; x[k] = i < hd ? src[i] : 0; gv[k] = i < hd ? gain[i] : 0; }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const uint64_t m = uabs64(x[k]), ga = uabs64(gv[k]);
+                if ((m >> 32) == 0) ssq += (uint64_t)(uint32_t)m * (uint32_t)m; else ssq += (u128)m * m;
+                mx = m > mx ? m : mx; gm = ga > gm ? ga : gm;
+            }
+            const uint32_t xb = __reduce_max_sync(0xffffffffu, (uint32_t)(64 - __clzll((long long)mx)) | (mx > (1ULL << 57) ? 128u : 0u));
+            const uint32_t gb = __reduce_max_sync(0xffffffffu, (uint32_t)(64 - __clzll((long long)gm)));
+            const NormRow n(warp_sum128(ssq), (int)(xb & 127u), (int)gb, (xb & 128u) != 0, hd, a.eps, a.fa, true);
+            bool bad = n.refused;
+            if (n.fast || n.refused) {
+#pragma unroll
+                for (int k = 0; k < 8; k++) if (lane + 32 * k < hd) dst[lane + 32 * k] = n.refused ? 0 : n.fast_value((int)x[k], (int)gv[k]);
+            } else {
+                const uint64_t inv = n.rms < (1ULL << 62) ? recip_below(n.rms) : 0, gmax = warp_gain_max(gain, hd);
+#pragma unroll 1
+                for (int i = lane; i < hd; i += 32) dst[i] = norm_value(src[i], n.rms, inv, gmax, gain[i], true, a.fa, bad);
+            }
+            if (bad) atomicOr(a.flags, 2);
+        }
+        __syncthreads();
+    }
     // ---- rotated queries ------------------------------------------------------------------------------------------------
     bool wide = false;
     for (int idx = tid; idx < AF_HEADS * half; idx += AF_THREADS) {
@@ -730,7 +765,7 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
         const int i0 = a.rope == 2 ? i : 2 * i, i1 = a.rope == 2 ? i + half : 2 * i + 1;
         int64_t x0 = 0, x1 = 0;
         if (r < rep) {
-            const int64_t *src = a.q + (long long)(kv * rep + r) * hd;
+            const int64_t *src = a.qgain ? reinterpret_cast<const int64_t *>(q64) + r * hd : a.q + (long long)(kv * rep + r) * hd;      // in place: a pair is one thread's
             x0 = src[i0]; x1 = src[i1];
             at_rotate(a, a.pos, i, x0, x1);
         }
@@ -752,7 +787,8 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
         bool bad = false;
         for (int i = tid; i < half; i += AF_THREADS) {
             const int i0 = a.rope == 2 ? i : 2 * i, i1 = a.rope == 2 ? i + half : 2 * i + 1;
-            int64_t x0 = a.k[kv * hd + i0], x1 = a.k[kv * hd + i1];
+            const int64_t *src = a.qgain ? knew : a.k + kv * hd;
+            int64_t x0 = src[i0], x1 = src[i1];
             at_rotate(a, a.pos, i, x0, x1);
             bad |= x0 != (int32_t)x0 || x1 != (int32_t)x1;
             int32_t *dst = a.kcache + ((long long)kv * a.Lmax + a.pos) * hd;
@@ -1354,6 +1390,7 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s) {
         }
         cudaGetLastError();
     }
+    if (a.qgain) return cudaErrorNotSupported;             // nothing was launched: the caller norms the heads itself
     bool fused = g_attn_fused && a.partial && n_sms > 0 && rep4 <= 256 / AT_CH && fused_smem <= 200 * 1024;
     if (fused) {
         int per_sm = 0;

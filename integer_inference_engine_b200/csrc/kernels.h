@@ -226,9 +226,9 @@ cudaError_t launch_topk(const int64_t *logits, long long rows, int n_experts, in
 cudaError_t launch_rmsnorm(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
                            unsigned long long eps, int64_t *out, int *flags, cudaStream_t s);
 // the same with the normalised rows also (out may be NULL: only) written as Q1_0 activation operands: digit planes
-// [row][8][width] and 128-element block sums [row][width/128]; width must be a multiple of 128 (duties: see launch_q1_prep)
+// [row][8][width]; width must be a multiple of 128 (duties: see launch_q1_prep)
 cudaError_t launch_rmsnorm_planes(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
-                                  unsigned long long eps, int64_t *out, int8_t *planes, int64_t *totals, int *flags, const PlaneDuties &duties,
+                                  unsigned long long eps, int64_t *out, int8_t *planes, int *flags, const PlaneDuties &duties,
                                   cudaStream_t s);
 
 // Counting-sort dispatch of (token, slot) pairs by expert (single CTA, n_experts <= 1024).
@@ -260,6 +260,8 @@ struct AttnArgs {
     int64_t *out;                  // [H*hd], nullable
     int8_t *out_limbs;             // nullable: digit planes [8][H*hd] of the result
     int *out_nl;                   // nullable: digits in use by the result (the one-CTA-per-SM decode form leaves one count per KV head: out_nl[kv])
+    const int64_t *qgain, *kgain;  // nullable: per-head RMSNorm gains [hd] of queries and key, applied before the rotation (only the
+    unsigned long long eps;        // one-CTA-per-SM decode form takes them; others answer cudaErrorNotSupported)
     int pdl;                       // 1: the one-launch form is launched with programmatic stream serialization
     int *flags;                    // bit 0 digit envelope, bit 2 a key / value does not fit the int32 cache
     int batch;                     // > 0: that many consecutive new tokens (prefill); q, k, v, out then hold one row per token,
@@ -272,6 +274,9 @@ struct AttnArgs {
     long long *pv_part;            // scratch [batch][pv_splits][H][hd] for their raw sums
 };
 cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s);
+int attn_decode_normed(const int64_t *q, const int64_t *k, const int64_t *v, int32_t *kcache, int32_t *vcache, long long pos,
+                       const int *pos_dev, const int64_t *cos, const int64_t *sin, int rope, int H, int Hkv, int hd, long long cache_rows,
+                       int fa, long long inv_sqrt, const int64_t *qgain, const int64_t *kgain, unsigned long long eps, int64_t *out, cudaStream_t s);
 // `batch` new tokens at positions pos .. pos + batch - 1 against the cache rows before them and each other (causal):
 // all K/V rows are appended first, then scores, exponentials and the probability-value sums run per token
 cudaError_t launch_attn_prefill(const AttnArgs &a, cudaStream_t s);
@@ -334,13 +339,13 @@ cudaError_t launch_decode(const DecodeArgs &a, int n_ctas, cudaStream_t s);
 size_t q1_unit_bytes(bool sc32);
 cudaError_t launch_q1_repack(const uint8_t *bits, const void *scale, int src_bits, bool sc32, long long out_f, long long nb,
                              uint8_t *units, unsigned long long *max_scale, cudaStream_t s);
-// Digit planes [T][8][K] and block sums [T][nb] of T rows (with the wrapping SwiGLU of gate and up in front of them in the
+// Digit planes [T][8][K] of T rows (with the wrapping SwiGLU of gate and up in front of them in the
 // second form).
-cudaError_t launch_q1_prep(const int64_t *x, long long T, long long nb, int8_t *planes, int64_t *totals, const PlaneDuties &duties,
+cudaError_t launch_q1_prep(const int64_t *x, long long T, long long nb, int8_t *planes, const PlaneDuties &duties,
                            cudaStream_t s);
 cudaError_t launch_q1_prep_swiglu(const int64_t *gate, const int64_t *up, long long ld, int frac, long long T, long long nb,
-                                  int8_t *planes, int64_t *totals, const PlaneDuties &duties, cudaStream_t s);
-// Products of the same rows with up to three matrices of one width; out[T][out_f] = x W^T (+ add, which may be out itself).
+                                  int8_t *planes, const PlaneDuties &duties, cudaStream_t s);
+// Products of the same rows (two and more; a single row: launch_q1_row) with up to three matrices of one width; out[T][out_f] = x W^T (+ add, which may be out itself).
 constexpr int Q1_MAX_PARTS = 3;
 struct Q1Part {
     const uint8_t *units;
@@ -349,18 +354,26 @@ struct Q1Part {
     const int64_t *add;
     unsigned long long max_scale;  // largest |scale| of the matrix
 };
+// Products of one row (int64, 16-byte aligned, outside every `out`) with matrices of the same row length in one launch (q1_row.cu).
+// swiglu: two matrices, out of the first = (silu(product 0) * product 1) >> frac (wrapping); rows of up to 32 blocks.
+struct Q1RowInput {
+    const int64_t *x;
+    bool norm;                     // RMS-normalise the row first, with an optional gain
+    const int64_t *gain;
+    unsigned long long eps;
+};
+cudaError_t launch_q1_row(const Q1Part *mats, int n, bool sc32, long long nb, const Q1RowInput &in, bool swiglu, long long frac, cudaStream_t s);
 constexpr int Q1_TC_CTAS = 148;    // one CTA per SM
 // Whether the products of T rows with matrices of `row_tiles` 128-row tiles in all add shares of a tile atomically: `out` then has
 // to hold zeros (or be `add`) when launch_q1_apply runs.
 bool q1_tc_split(long long row_tiles, long long T);
-cudaError_t launch_q1_apply(const Q1Part *parts, int n_parts, bool sc32, long long nb, const int8_t *planes, const int64_t *totals,
+cudaError_t launch_q1_apply(const Q1Part *parts, int n_parts, bool sc32, long long nb, const int8_t *planes,
                             long long T, long long frac, const int *nl, cudaStream_t s);
 cudaError_t launch_q1_tc(const Q1Part *parts, int n_parts, bool sc32, long long nb, const int8_t *planes, long long T, int sh,
                          const int *nl_dev, cudaStream_t s);
 cudaError_t launch_rmsnorm_pair(const int64_t *x, long long rows_a, long long rows_b, long long width, const int64_t *gain_a,
                                 const int64_t *gain_b, int fa, unsigned long long eps, int64_t *out, int *flags, cudaStream_t s);
 bool attn_shape_ok(int n_heads, int n_kv, int head_dim);      // shapes launch_attn_decode accepts
-void set_q1_stream(int on);        // 1: single-token Q1_0 products through the bulk-copy kernel, 0 (default): per-lane loads
 int *shared_flag_word();           // the library's device flag word (bit 1: RMSNorm envelope), NULL without a device
 void restore_flag_bits(int bits);  // OR bits back into the flag word (flags an entry set aside while it ran)
 cudaError_t launch_q1_silu_mul(const int64_t *gate, const int64_t *up, long long n, int frac, int64_t *out, cudaStream_t s);

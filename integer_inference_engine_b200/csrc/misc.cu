@@ -287,46 +287,6 @@ __global__ void dispatch_kernel(const int *ids, const int64_t *gates, long long 
 // ---------------------------------------------------------------------------------------------------
 // integer RMSNorm (north-mini-code/src/nmc/_bonsai/fixedpoint.py:32-72), one CTA per row
 // ---------------------------------------------------------------------------------------------------
-// one element of the normalised row: floor((x << fa) / rms), then (y * gain) >> fa; `bad` is set (and 0 returned)
-// where the oracle's envelope checks would refuse the value
-__device__ __forceinline__ int64_t norm_value(int64_t xv, unsigned long long rms, unsigned long long inv, unsigned long long gm,
-                                              int64_t g, bool has_gain, int fa, bool &bad) {
-    int64_t y;
-    if (inv != 0 && uabs64(xv) < (1ULL << (62 - fa))) {
-        // |x << fa| < 2^62 and rms < 2^62: quotient from the reciprocal inv = floor((2^64 - 1) / rms), at most 2 low
-        const unsigned long long n = uabs64(xv) << fa;
-        unsigned long long q = __umul64hi(n, inv), r = n - q * rms;
-        while (r >= rms) { q++; r -= rms; }
-        y = xv >= 0 ? (int64_t)q : -(int64_t)q - (r != 0);      // floor toward -inf
-    } else {
-        const i128 num = (i128)xv << fa;
-        i128 q = num / (i128)rms;
-        if (num < 0 && q * (i128)rms != num) q -= 1;
-        if (q > (i128)INT64_MAX || q < (i128)INT64_MIN) { bad = true; return 0; }
-        y = (int64_t)q;
-    }
-    if (has_gain) {
-        // the oracle refuses a gain product that could leave int64
-        if ((u128)uabs64(y) * gm > (u128)INT64_MAX) { bad = true; return 0; }
-        y = (int64_t)(((i128)y * g) >> fa);
-    }
-    return y;
-}
-
-// sum over the warp of 128-bit (64-bit) values: pieces of 22 bits, one warp reduction each
-__device__ __forceinline__ u128 warp_sum128(u128 v) {
-    u128 sum = 0;
-#pragma unroll
-    for (int k = 0; k < 6; k++) sum += (u128)__reduce_add_sync(0xffffffffu, (uint32_t)(v >> (22 * k)) & 0x3FFFFFu) << (22 * k);
-    return sum;
-}
-__device__ __forceinline__ uint64_t warp_sum64(uint64_t v) {
-    uint64_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < 3; k++) sum += (uint64_t)__reduce_add_sync(0xffffffffu, (uint32_t)(v >> (22 * k)) & 0x3FFFFFu) << (22 * k);
-    return sum;
-}
-
 struct NormArgs {
     const int64_t *x;
     long long rows, rows_a;        // rows from rows_a on take gain_b (per-head norms of queries and keys in one launch)
@@ -337,7 +297,6 @@ struct NormArgs {
     unsigned long long eps;
     int64_t *out;                  // nullable
     int8_t *planes;                // nullable: digit planes [row][8][width]
-    int64_t *totals;               // nullable: 128-element block sums [row][width / 128]
     int *flags;
     PlaneDuties duties;
 };
@@ -378,7 +337,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const uint64_t m = uabs64(x[k][e]), gm = uabs64(g[k][e]);
-            ssq += (u128)m * m;
+            if ((m >> 32) == 0) ssq += (uint64_t)(uint32_t)m * (uint32_t)m; else ssq += (u128)m * m;
             mx = m > mx ? m : mx; gmx = gm > gmx ? gm : gmx;
         }
     }
@@ -396,29 +355,14 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormArgs a) {
         xb = __reduce_max_sync(0xffffffffu, bits & 0xFF); gb = __reduce_max_sync(0xffffffffu, bits >> 8);
     }
     beyond = (xb & 128u) != 0; xb &= 127u;
-    const u128 mean = ((a.width & (a.width - 1)) == 0 ? ssq >> (31 - __clz(a.width)) : ssq / (u128)(unsigned)a.width) + a.eps;
-    const u128 root = isqrt128(mean);
-    const uint64_t rms = (uint64_t)root;
-    if (beyond || root == 0 || (root >> 64) != 0) {                // refused: nothing is written
+    const NormRow nr(ssq, (int)xb, (int)gb, beyond, a.width, a.eps, a.fa, gain != nullptr);
+    if (nr.refused) {                                              // nothing is written
         if (live && lane == 0 && in_row == 0) atomicOr(a.flags, 2);
         return;
     }
-    const int fa = a.fa;
-    // Every |x| < 2^xb and |gain| < 2^gb: with n = 2^(xb + fa) the quotients stay below 2^31 when n < rms 2^31, and the gain products inside
-    // four balanced digits when n 2^gb <= rms (0x7F7F7F7D 2^sh - 2^gb)
-    bool fast = false;
-    const int sh = gain ? fa : 0;                                  // without a gain: a factor of one
-    if ((int)xb + fa <= 62 && gb <= 31 && rms < (1ULL << 62)) {
-        const u128 n = (u128)1 << (xb + fa), lim = (u128)2139062141ULL << sh, g1 = (u128)1 << gb;
-        fast = n < (u128)rms * 2147483646ULL && lim > g1 && (n << gb) <= (u128)rms * (lim - g1);
-    }
-    const uint64_t inv = rms < (1ULL << 62) ? recip_below(rms) : 0;
-    uint64_t gm = 0;
-    if (!fast && gain) {                                           // the general form refuses against the row's largest |gain|
-        for (int k = 0; k < a.width; k += 32) { const int i = k + lane; const uint64_t v = i < a.width ? uabs64(gain[i]) : 0; gm = v > gm ? v : gm; }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) { const uint64_t o = __shfl_xor_sync(0xffffffffu, gm, off); gm = o > gm ? o : gm; }
-    }
+    const bool fast = nr.fast;
+    const uint64_t inv = !fast && nr.rms < (1ULL << 62) ? recip_below(nr.rms) : 0;
+    const uint64_t gm = !fast && gain ? warp_gain_max(gain, a.width) : 0;      // the general form refuses against the row's largest |gain|
     bool bad = false;
     int nl = 0;
 #pragma unroll
@@ -428,17 +372,10 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormArgs a) {
         int64_t y[4];
         if (fast) {
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const uint64_t n = uabs64(x[k][e]) << fa;
-                uint64_t q = __umul64hi(n, inv), r = n - q * rms;
-#pragma unroll
-                for (int fix = 0; fix < 2; fix++) { const bool up = r >= rms; q += up; r -= up ? rms : 0; }      // at most two below: n < 2^62
-                const int yq = x[k][e] >= 0 ? (int)q : -(int)q - (r != 0);                // floor of the signed quotient
-                y[e] = ((int64_t)yq * (int)g[k][e]) >> sh;
-            }
+            for (int e = 0; e < 4; e++) y[e] = nr.fast_value((int)x[k][e], (int)g[k][e]);
         } else {
 #pragma unroll
-            for (int e = 0; e < 4; e++) y[e] = in ? norm_value(x[k][e], rms, inv, gm, g[k][e], gain != nullptr, fa, bad) : 0;
+            for (int e = 0; e < 4; e++) y[e] = in ? norm_value(x[k][e], nr.rms, inv, gm, g[k][e], gain != nullptr, a.fa, bad) : 0;
         }
         if (in && a.out) {
             int64_t *to = a.out + row * a.width + i;
@@ -473,10 +410,6 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormArgs a) {
             if (in) {
 #pragma unroll
                 for (int l = 0; l < 8; l++) *reinterpret_cast<uint32_t *>(a.planes + (row * 8 + l) * a.width + i) = pl[l];
-            }
-            if (a.totals) {
-                const uint64_t sum = warp_sum64((uint64_t)y[0] + (uint64_t)y[1] + (uint64_t)y[2] + (uint64_t)y[3]);
-                if (in && lane == 0) a.totals[row * (a.width >> 7) + (i >> 7)] = (int64_t)sum;
             }
         }
     }
@@ -648,19 +581,19 @@ cudaError_t launch_topk(const int64_t *logits, long long rows, int n_experts, in
 cudaError_t launch_rmsnorm(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
                            unsigned long long eps, int64_t *out, int *flags, cudaStream_t s) {
     if (rows <= 0 || width <= 0 || width > (1 << 30)) return cudaErrorInvalidValue;
-    return launch_norm({x, rows, rows, (int)width, 0, false, gain, nullptr, fa, eps, out, nullptr, nullptr, flags, PlaneDuties()}, s);
+    return launch_norm({x, rows, rows, (int)width, 0, false, gain, nullptr, fa, eps, out, nullptr, flags, PlaneDuties()}, s);
 }
 
 cudaError_t launch_rmsnorm_pair(const int64_t *x, long long rows_a, long long rows_b, long long width, const int64_t *gain_a,
                                 const int64_t *gain_b, int fa, unsigned long long eps, int64_t *out, int *flags, cudaStream_t s) {
     if (rows_a + rows_b <= 0 || width <= 0 || width > (1 << 30)) return cudaErrorInvalidValue;
-    return launch_norm({x, rows_a + rows_b, rows_a, (int)width, 0, false, gain_a, gain_b, fa, eps, out, nullptr, nullptr, flags, PlaneDuties()}, s);
+    return launch_norm({x, rows_a + rows_b, rows_a, (int)width, 0, false, gain_a, gain_b, fa, eps, out, nullptr, flags, PlaneDuties()}, s);
 }
 
 cudaError_t launch_rmsnorm_planes(const int64_t *x, long long rows, long long width, const int64_t *gain, int fa,
-                                  unsigned long long eps, int64_t *out, int8_t *planes, int64_t *totals, int *flags, const PlaneDuties &duties, cudaStream_t s) {
+                                  unsigned long long eps, int64_t *out, int8_t *planes, int *flags, const PlaneDuties &duties, cudaStream_t s) {
     if (rows <= 0 || width <= 0 || (width & 127) || width > (1 << 30) || !planes) return cudaErrorInvalidValue;
-    return launch_norm({x, rows, rows, (int)width, 0, false, gain, nullptr, fa, eps, out, planes, totals, flags, duties}, s);
+    return launch_norm({x, rows, rows, (int)width, 0, false, gain, nullptr, fa, eps, out, planes, flags, duties}, s);
 }
 
 cudaError_t launch_dispatch(const int *ids, const int64_t *gates, long long T, int k, int n_experts, int *grp_off,

@@ -34,7 +34,7 @@ cudaStream_t q_stream = nullptr;
 int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [8..15] digits in use (a ring, see next_digits)
 int q_ready = -1;
 
-enum QRole { QR_X, QR_PLANES, QR_TOTALS, QR_OUT, QR_GAIN, QR_COUNT };
+enum QRole { QR_X, QR_PLANES, QR_OUT, QR_GAIN, QR_COUNT };
 struct QBuf { void *p = nullptr; size_t cap = 0; };
 unsigned long long q_generation = 0;   // changes whenever a scratch buffer is freed: captured graphs hold the old addresses
 QBuf q_buf[QR_COUNT];
@@ -86,20 +86,17 @@ PlaneDuties next_digits() {
     return d;
 }
 
-// Products of rows whose digit planes a kernel `write(duties)` is about to leave in `planes` / `totals`.  Where the products add
+// Products of rows whose digit planes a kernel `write(duties)` is about to leave in `planes`.  Where the products add
 // shares of a tile to their outputs, that kernel clears them, unless they lie over something it reads ([in, in + in_n) or
 // [in2, in2 + in_n)): then they are cleared behind it.
 template <typename Write>
-bool planes_and_products(Write write, const Q1Part *parts, int n, bool sc32, long long nb, const int8_t *planes, const int64_t *totals, long long T,
-                         long long frac, const int64_t *in, const int64_t *in2, long long in_n, cudaStream_t s) {
-    PlaneDuties d;
-    bool clear = false, fused = true;
-    if (T > 1 || nb > 128) {                           // a single row takes every digit as it comes
-        d = next_digits();
-        long long row_tiles = 0;
-        for (int i = 0; i < n; i++) row_tiles += (parts[i].out_f + 127) / 128;
-        clear = q1_tc_split(row_tiles, T);
-    }
+bool planes_and_products(Write write, const Q1Part *parts, int n, bool sc32, long long nb, const int8_t *planes, long long T, long long frac,
+                         const int64_t *in, const int64_t *in2, long long in_n, cudaStream_t s) {
+    PlaneDuties d = next_digits();
+    bool fused = true;
+    long long row_tiles = 0;
+    for (int i = 0; i < n; i++) row_tiles += (parts[i].out_f + 127) / 128;
+    const bool clear = q1_tc_split(row_tiles, T);
     for (int i = 0; clear && i < n; i++) {
         const Q1Part &p = parts[i];
         const int64_t *end = p.out + T * p.out_f;
@@ -112,7 +109,20 @@ bool planes_and_products(Write write, const Q1Part *parts, int n, bool sc32, lon
     if (write(d) != cudaSuccess) return false;
     for (int i = 0; clear && !fused && i < n; i++)
         if (parts[i].add != parts[i].out && cudaMemsetAsync(parts[i].out, 0, (size_t)T * parts[i].out_f * 8, s) != cudaSuccess) return false;
-    return launch_q1_apply(parts, n, sc32, nb, planes, totals, T, frac, d.nl, s) == cudaSuccess;
+    return launch_q1_apply(parts, n, sc32, nb, planes, T, frac, d.nl, s) == cudaSuccess;
+}
+
+// Products of a single row.  A row that the kernel cannot read in place (misaligned, or under one of the outputs) is copied first.
+bool row_products(const Q1Part *parts, int n, bool sc32, long long nb, Q1RowInput in, bool swiglu, long long frac, cudaStream_t s) {
+    const long long K = nb * 128;
+    bool copy = (reinterpret_cast<uintptr_t>(in.x) & 15) != 0;
+    for (int i = 0; i < n; i++) copy = copy || (parts[i].out < in.x + K && in.x < parts[i].out + parts[i].out_f);
+    if (copy) {
+        int64_t *own = (int64_t *)q_ensure(QR_PLANES, (size_t)K * 8);
+        if (!own || cudaMemcpyAsync(own, in.x, (size_t)K * 8, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return false;
+        in.x = own;
+    }
+    return launch_q1_row(parts, n, sc32, nb, in, swiglu, frac, s) == cudaSuccess;
 }
 
 bool valid(long long h) { return h >= 0 && (size_t)h < q_w.size() && q_w[(size_t)h].live; }
@@ -157,21 +167,23 @@ long long register_any(const unsigned char *bits, const void *scale, int scale_b
 int apply_device(const Q1Weight &w, const int64_t *xd, long long T, long long frac, int64_t *outd, int max_digits,
                  cudaStream_t s) {
     const long long K = w.nb * 128;
-    int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * K);
-    int64_t *totals = (int64_t *)q_ensure(QR_TOTALS, (size_t)T * w.nb * 8);
-    if (!planes || !totals) return 2;
+    int8_t *planes = T > 1 || max_digits < 8 ? (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * K) : nullptr;
+    if (!planes && (T > 1 || max_digits < 8)) return 2;
     const Q1Part part = {w.units, w.out_f, outd, nullptr, w.max_scale};
     int used = 0;
     auto write = [&](const PlaneDuties &d) {
         PlaneDuties dd = d;
         if (max_digits < 8 && !dd.nl) dd.nl = q_cells;
         cudaError_t e = max_digits < 8 ? cudaMemsetAsync(dd.nl, 0, sizeof(int), s) : cudaSuccess;
-        if (e == cudaSuccess) e = launch_q1_prep(xd, T, w.nb, planes, totals, dd, s);
+        if (e == cudaSuccess) e = launch_q1_prep(xd, T, w.nb, planes, dd, s);
         if (e == cudaSuccess && max_digits < 8) e = cudaMemcpyAsync(&used, dd.nl, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess && max_digits < 8) e = cudaStreamSynchronize(s);
         return e == cudaSuccess && used > max_digits ? cudaErrorInvalidValue : e;
     };
-    if (planes_and_products(write, &part, 1, w.sc32, w.nb, planes, totals, T, frac, xd, nullptr, T * K, s)) return 0;
+    bool ok;
+    if (T > 1) ok = planes_and_products(write, &part, 1, w.sc32, w.nb, planes, T, frac, xd, nullptr, T * K, s);
+    else ok = (max_digits >= 8 || write(PlaneDuties()) == cudaSuccess) && row_products(&part, 1, w.sc32, w.nb, {xd, false, nullptr, 0}, false, frac, s);
+    if (ok) return 0;
     return used > max_digits ? 4 : 2;
 }
 
@@ -321,20 +333,66 @@ extern "C" int iie_q1_apply_fused_dev(long long handle, int mode, const int64_t 
     const Q1Weight &w = q_w[(size_t)handle];
     const long long K = w.nb * 128, T = tokens;
     cudaStream_t s = (cudaStream_t)stream;
-    int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * K);
-    int64_t *totals = (int64_t *)q_ensure(QR_TOTALS, (size_t)T * w.nb * 8);
-    if (!planes || !totals) return 2;
     if (mode == 2 && (!x2_dev || ld < K)) return 1;
+    int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * K);
+    if (!planes) return 2;
     int *flags = iie::shared_flag_word();
     if (!flags) return 2;
-    auto write = [&](const PlaneDuties &d) {
-        if (mode == 1) return iie::launch_rmsnorm_planes(x_dev, T, K, gain_dev, (int)frac, 1ULL, nullptr, planes, totals, flags, d, s);
-        if (mode == 2) return iie::launch_q1_prep_swiglu(x_dev, x2_dev, ld, (int)frac, T, w.nb, planes, totals, d, s);
-        return iie::launch_q1_prep(x_dev, T, w.nb, planes, totals, d, s);
-    };
     const Q1Part part = {w.units, w.out_f, out_dev, add_dev, w.max_scale};
-    return planes_and_products(write, &part, 1, w.sc32, w.nb, planes, totals, T, frac, x_dev, mode == 2 ? x2_dev : gain_dev,
+    if (T == 1) {
+        const int64_t *x = x_dev;
+        if (mode == 2) {
+            x = (const int64_t *)planes;                               // 8 K bytes: the row itself in place of its digit planes
+            if (launch_q1_silu_mul(x_dev, x2_dev, K, (int)frac, (int64_t *)planes, s) != cudaSuccess) return 2;
+        }
+        return row_products(&part, 1, w.sc32, w.nb, {x, mode == 1, mode == 1 ? gain_dev : nullptr, 1ULL}, false, frac, s) ? 0 : 2;
+    }
+    auto write = [&](const PlaneDuties &d) {
+        if (mode == 1) return iie::launch_rmsnorm_planes(x_dev, T, K, gain_dev, (int)frac, 1ULL, nullptr, planes, flags, d, s);
+        if (mode == 2) return iie::launch_q1_prep_swiglu(x_dev, x2_dev, ld, (int)frac, T, w.nb, planes, d, s);
+        return iie::launch_q1_prep(x_dev, T, w.nb, planes, d, s);
+    };
+    return planes_and_products(write, &part, 1, w.sc32, w.nb, planes, T, frac, x_dev, mode == 2 ? x2_dev : gain_dev,
                                mode == 2 ? (T - 1) * ld + K : T * K, s) ? 0 : 2;
+}
+
+// One layer of a decode token: norm + Q/K/V product; attention with the per-head norms; O product with the residual; norm + gate/up
+// products + SwiGLU; down product with the residual.  Five launches, each started while the one before it runs and waiting for it
+// behind the requests for its weights.
+extern "C" int iie_q1_decode_layer_dev(long long wqkv, long long wo, long long w1u, long long w2, const int64_t *n1, const int64_t *n2,
+                                       const int64_t *qn, const int64_t *kn, int64_t *x, int64_t *qkv, int64_t *qkvn, int64_t *att, int64_t *h,
+                                       int32_t *kcache, int32_t *vcache, long long pos, const int *pos_dev, const int64_t *cos, const int64_t *sin,
+                                       int n_heads, int n_kv, int head_dim, long long cache_rows, long long frac, long long inv_sqrt, void *stream) {
+    std::lock_guard<std::recursive_mutex> lk(q_mu);
+    if (!valid(wqkv) || !valid(wo) || !valid(w1u) || !valid(w2) || !n1 || !n2 || !qn || !kn || !x || !qkv || !qkvn || !att || !h || !kcache ||
+        !vcache || !cos || !sin || n_heads <= 0 || n_kv <= 0 || head_dim <= 0 || n_heads % n_kv || cache_rows <= 0 || pos < 0 || frac < 1 || frac > 29) return 1;
+    const Q1Weight &a = q_w[(size_t)wqkv], &o = q_w[(size_t)wo], &g = q_w[(size_t)w1u], &dn = q_w[(size_t)w2];
+    const long long qd = (long long)n_heads * head_dim, kd = (long long)n_kv * head_dim, ffn = dn.nb * 128;
+    if (a.out_f != qd + 2 * kd || o.nb * 128 != qd || o.out_f != a.nb * 128 || g.nb != a.nb || g.out_f != 2 * ffn || dn.out_f != o.out_f) return 1;
+    cudaStream_t s = (cudaStream_t)stream;
+    const int f = (int)frac;
+    int *flags = iie::shared_flag_word();
+    if (!flags) return 2;
+    const Q1Part pa = {a.units, a.out_f, qkv, nullptr, a.max_scale}, po = {o.units, o.out_f, x, x, o.max_scale}, pd = {dn.units, dn.out_f, x, x, dn.max_scale};
+    if (!row_products(&pa, 1, a.sc32, a.nb, {x, true, n1, 1ULL}, false, frac, s)) return 2;
+    int rc = attn_decode_normed(qkv, qkv + qd, qkv + qd + kd, kcache, vcache, pos, pos_dev, cos, sin, 2, n_heads, n_kv, head_dim, cache_rows, f,
+                                inv_sqrt, qn, kn, 1ULL, att, s);
+    if (rc == 3)                                       // contexts and head shapes beyond the one-launch form
+        rc = launch_rmsnorm_pair(qkv, n_heads, n_kv, head_dim, qn, kn, f, 1ULL, qkvn, flags, s) == cudaSuccess
+                 ? iie_attn_decode_dev(qkvn, qkvn + qd, qkv + qd + kd, kcache, vcache, pos, pos_dev, 0, cos, sin, 2, n_heads, n_kv, head_dim,
+                                       cache_rows, f, inv_sqrt, att, stream) : 2;
+    if (rc != 0) return rc;
+    if (!row_products(&po, 1, o.sc32, o.nb, {att, false, nullptr, 0}, false, frac, s)) return 2;
+    const size_t up_at = (size_t)(ffn / 16) * g.nb * q1_unit_bytes(g.sc32);          // the rows of the up matrix follow the gate's
+    const Q1Part gu[2] = {{g.units, ffn, h, nullptr, g.max_scale}, {g.units + up_at, ffn, h, nullptr, g.max_scale}};
+    if (g.nb <= 32) {
+        if (!row_products(gu, 2, g.sc32, g.nb, {x, true, n2, 1ULL}, true, frac, s)) return 2;
+    } else {
+        const Q1Part both = {g.units, g.out_f, h, nullptr, g.max_scale};
+        if (!row_products(&both, 1, g.sc32, g.nb, {x, true, n2, 1ULL}, false, frac, s) ||
+            launch_q1_silu_mul(h, h + ffn, ffn, f, h, s) != cudaSuccess) return 2;
+    }
+    return row_products(&pd, 1, dn.sc32, dn.nb, {h, false, nullptr, 0}, false, frac, s) ? 0 : 2;
 }
 
 extern "C" int iie_q1_head_norm_dev(const int64_t *x_dev, long long rows_a, long long rows_b, long long width, const int64_t *gain_a_dev,
@@ -347,7 +405,7 @@ extern "C" int iie_q1_head_norm_dev(const int64_t *x_dev, long long rows_a, long
 }
 
 extern "C" unsigned long long iie_q1_workspace_generation(void) { return q_generation; }
-extern "C" void iie_q1_set_stream(int on) { iie::set_q1_stream(on); }
+extern "C" void iie_q1_set_stream(int) {}             // single-row products have one form: the weights always come by bulk copies
 
 extern "C" int iie_q1_silu_mul_dev(const int64_t *gate_dev, const int64_t *up_dev, long long n, long long frac, int64_t *out_dev,
                                    void *stream) {
@@ -447,8 +505,7 @@ void free_work(Work &w) { if (w.base) cudaFree(w.base); w = Work(); }
 // have one width
 struct Product { long long h; int64_t *out; const int64_t *add = nullptr; };
 template <typename Write>
-bool products(Write write, std::initializer_list<Product> list, const int8_t *planes, const int64_t *totals, long long T, long long frac,
-              const int64_t *in, long long in_n) {
+bool products(Write write, std::initializer_list<Product> list, const int8_t *planes, long long T, long long frac, const int64_t *in, long long in_n) {
     Q1Part parts[Q1_MAX_PARTS];
     int n = 0;
     bool sc32 = true, same = true;
@@ -459,10 +516,29 @@ bool products(Write write, std::initializer_list<Product> list, const int8_t *pl
         parts[n++] = {w.units, w.out_f, p.out, p.add, w.max_scale};
     }
     const long long nb = q_w[(size_t)list.begin()->h].nb;
-    if (same) return planes_and_products(write, parts, n, sc32, nb, planes, totals, T, frac, in, nullptr, in_n, q_stream);
+    if (same) return planes_and_products(write, parts, n, sc32, nb, planes, T, frac, in, nullptr, in_n, q_stream);
     for (int i = 0; i < n; i++)
-        if (!planes_and_products(write, parts + i, 1, q_w[(size_t)list.begin()[i].h].sc32, nb, planes, totals, T, frac, in, nullptr, in_n, q_stream)) return false;
+        if (!planes_and_products(write, parts + i, 1, q_w[(size_t)list.begin()[i].h].sc32, nb, planes, T, frac, in, nullptr, in_n, q_stream)) return false;
     return true;
+}
+// the same for one row
+bool products_of_row(const Q1RowInput &in, std::initializer_list<Product> list, bool swiglu, long long frac) {
+    Q1Part parts[Q1_MAX_PARTS];
+    int n = 0;
+    bool sc32 = true, same = true;
+    for (const Product &p : list) {
+        const Q1Weight &w = q_w[(size_t)p.h];
+        same = same && (n == 0 || w.sc32 == sc32);
+        sc32 = w.sc32;
+        parts[n++] = {w.units, w.out_f, p.out, p.add, w.max_scale};
+    }
+    const long long nb = q_w[(size_t)list.begin()->h].nb;
+    if (swiglu && same && nb <= 32) return row_products(parts, n, sc32, nb, in, true, frac, q_stream);
+    if (same) { if (!row_products(parts, n, sc32, nb, in, false, frac, q_stream)) return false; }
+    else
+        for (int i = 0; i < n; i++)
+            if (!row_products(parts + i, 1, q_w[(size_t)list.begin()[i].h].sc32, nb, in, false, frac, q_stream)) return false;
+    return !swiglu || launch_q1_silu_mul(parts[0].out, parts[1].out, parts[0].out_f, (int)frac, parts[0].out, q_stream) == cudaSuccess;
 }
 
 // One layer on T rows of w.x.  attend(q normalised, k normalised, v) runs rotation, cache append and attention into w.att.
@@ -470,35 +546,37 @@ template <typename Attend>
 bool layer_rows(const Q1Stack &m, long long li, Work &w, long long T, int *flags, Attend attend) {
     const size_t i = (size_t)li;
     const long long qd = m.H * m.hd, widest = std::max({m.d, qd, m.dff});
-    int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * (size_t)widest);
-    int64_t *totals = (int64_t *)q_ensure(QR_TOTALS, (size_t)T * (size_t)(widest / 128) * 8);
-    if (!planes || !totals) return false;
     const int f = (int)m.frac;
-    auto norm = [&](long long gain) {
-        return [&, gain](const PlaneDuties &d) {
-            return launch_rmsnorm_planes(w.x, T, m.d, q_bufs[(size_t)gain].p, f, m.eps, nullptr, planes, totals, flags, d, q_stream);
-        };
+    int8_t *planes = T > 1 ? (int8_t *)q_ensure(QR_PLANES, (size_t)T * 8 * (size_t)widest) : nullptr;
+    if (T > 1 && !planes) return false;
+    auto gain = [&](long long h) { return q_bufs[(size_t)h].p; };
+    auto norm = [&](long long h) {
+        return [&, h](const PlaneDuties &d) { return launch_rmsnorm_planes(w.x, T, m.d, gain(h), f, m.eps, nullptr, planes, flags, d, q_stream); };
     };
-    bool ok = products(norm(m.n1g[i]), {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, planes, totals, T, m.frac, w.x, T * m.d) &&
-              launch_rmsnorm(w.q, T * m.H, m.hd, q_bufs[(size_t)m.qng[i]].p, f, m.eps, w.qn, flags, q_stream) == cudaSuccess &&
-              launch_rmsnorm(w.k, T * m.Hkv, m.hd, q_bufs[(size_t)m.kng[i]].p, f, m.eps, w.kn, flags, q_stream) == cudaSuccess;
+    bool ok = (T == 1 ? products_of_row({w.x, true, gain(m.n1g[i]), m.eps}, {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, false, m.frac)
+                      : products(norm(m.n1g[i]), {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, planes, T, m.frac, w.x, T * m.d)) &&
+              launch_rmsnorm(w.q, T * m.H, m.hd, gain(m.qng[i]), f, m.eps, w.qn, flags, q_stream) == cudaSuccess &&
+              launch_rmsnorm(w.k, T * m.Hkv, m.hd, gain(m.kng[i]), f, m.eps, w.kn, flags, q_stream) == cudaSuccess;
     ok = ok && attend(w.qn, w.kn, w.v, w.att);
-    ok = ok && products([&](const PlaneDuties &d) { return launch_q1_prep(w.att, T, qd / 128, planes, totals, d, q_stream); },
-                        {{m.wo[i], w.x, w.x}}, planes, totals, T, m.frac, w.att, T * qd) &&
-         products(norm(m.n2g[i]), {{m.w1[i], w.g}, {m.wu[i], w.u}}, planes, totals, T, m.frac, w.x, T * m.d) &&
-         products([&](const PlaneDuties &d) { return launch_q1_prep_swiglu(w.g, w.u, m.dff, f, T, m.dff / 128, planes, totals, d, q_stream); },
-                  {{m.w2[i], w.x, w.x}}, planes, totals, T, m.frac, w.g, 2 * T * m.dff);
-    return ok;
+    if (T == 1)
+        return ok && products_of_row({w.att, false, nullptr, 0}, {{m.wo[i], w.x, w.x}}, false, m.frac) &&
+               products_of_row({w.x, true, gain(m.n2g[i]), m.eps}, {{m.w1[i], w.g}, {m.wu[i], w.u}}, true, m.frac) &&
+               products_of_row({w.g, false, nullptr, 0}, {{m.w2[i], w.x, w.x}}, false, m.frac);
+    return ok && products([&](const PlaneDuties &d) { return launch_q1_prep(w.att, T, qd / 128, planes, d, q_stream); },
+                          {{m.wo[i], w.x, w.x}}, planes, T, m.frac, w.att, T * qd) &&
+           products(norm(m.n2g[i]), {{m.w1[i], w.g}, {m.wu[i], w.u}}, planes, T, m.frac, w.x, T * m.d) &&
+           products([&](const PlaneDuties &d) { return launch_q1_prep_swiglu(w.g, w.u, m.dff, f, T, m.dff / 128, planes, d, q_stream); },
+                    {{m.w2[i], w.x, w.x}}, planes, T, m.frac, w.g, 2 * T * m.dff);
 }
 
 // logits of `rows` rows starting at x: final norm, output matrix
 bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logits, int *flags) {
+    const int64_t *gain = q_bufs[(size_t)m.finalg].p;
+    if (rows == 1) return products_of_row({x, true, gain, m.eps}, {{m.out_head, logits}}, false, m.frac);
     int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)rows * 8 * (size_t)m.d);
-    int64_t *totals = (int64_t *)q_ensure(QR_TOTALS, (size_t)rows * (size_t)(m.d / 128) * 8);
-    if (!planes || !totals) return false;
-    return products([&](const PlaneDuties &d) {
-        return launch_rmsnorm_planes(x, rows, m.d, q_bufs[(size_t)m.finalg].p, (int)m.frac, m.eps, nullptr, planes, totals, flags, d, q_stream);
-    }, {{m.out_head, logits}}, planes, totals, rows, m.frac, x, rows * m.d);
+    if (!planes) return false;
+    return products([&](const PlaneDuties &d) { return launch_rmsnorm_planes(x, rows, m.d, gain, (int)m.frac, m.eps, nullptr, planes, flags, d, q_stream); },
+                    {{m.out_head, logits}}, planes, rows, m.frac, x, rows * m.d);
 }
 
 // int64 host rows -> int32; false when a value does not fit

@@ -84,19 +84,13 @@ class Q1Decoder:
 
     def _launch_step(self, pos_bound: int) -> None:
         """One token: reads ``self.token`` / ``self.pos`` on the device, leaves the next id in ``self.token`` and advances
-        ``self.pos``.  Per layer ten launches: norm + digit planes, QKV product, both head norms, attention, planes,
-        O product with the residual, norm + planes, gate/up product, SwiGLU + planes, down product with the residual."""
-        f, qd, kd = self.frac, self.H * self.hd, self.Hkv * self.hd
+        ``self.pos``.  Five launches per layer: norm + QKV product, head norms + attention, O product with the residual, norm +
+        gate/up product + SwiGLU, down product with the residual."""
         q1_gpu.embed_dev(self.embed, self.token, self.x)
         for L in self.layers:
-            q1_gpu.apply_fused_dev(L["wqkv"], self.x, f, self.qkv, norm=True, gain=L["n1"])
-            q1_gpu.head_norm_dev(self.qkv, self.H, self.Hkv, self.hd, L["qn"], L["kn"], f, self.qkvn)
-            device.attention_decode(self.qkvn[0, :qd], self.qkvn[0, qd:], self.qkv[0, qd + kd:], L["k"], L["v"], pos_bound,
-                                    self.H, self.Hkv, self.hd, f, 0, self.cos, self.sin, 2, out=self.att.view(-1), pos_dev=self.pos)
-            q1_gpu.apply_fused_dev(L["wo"], self.att, f, self.x, add=self.x)
-            q1_gpu.apply_fused_dev(L["w1u"], self.x, f, self.gu, norm=True, gain=L["n2"])
-            q1_gpu.apply_fused_dev(L["w2"], self.gu[:, :self.ffn], f, self.x, up=self.gu[:, self.ffn:], add=self.x)
-        q1_gpu.apply_fused_dev(self.head, self.x, f, self.logits, norm=True, gain=self.out_gain)
+            q1_gpu.decode_layer_dev(L, self.x, self.qkv, self.qkvn, self.att, self.gu, pos_bound, self.pos, self.cos, self.sin,
+                                    self.H, self.Hkv, self.hd, self.frac)
+        q1_gpu.apply_fused_dev(self.head, self.x, self.frac, self.logits, norm=True, gain=self.out_gain)
         device.argmax(self.logits.view(-1), out=self.token)
         self.pos += 1
 
