@@ -1363,7 +1363,8 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s) {
         a.fa <= 23 && a.Hkv <= 120) {                                       // probabilities (at most 2^fa) as three bytes
         static bool fat_configured = false;
         if (!fat_configured) {
-            if (cudaFuncSetAttribute(attn_fat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess) return cudaGetLastError();
+            if (cudaFuncSetAttribute(attn_fat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess ||
+                cudaFuncSetAttribute(attn_fat_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) return cudaGetLastError();
             fat_configured = true;
         }
         const int per_head = std::max(1, std::min(n_sms, 192) / a.Hkv);      // the partial-sum scratch holds 192 chunks

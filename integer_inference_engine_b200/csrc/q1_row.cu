@@ -39,7 +39,7 @@ struct Q1RowArgs {
     int tile_end[Q1_MAX_PARTS];                   // tiles up to and with that matrix
     int n_mats, tiles;                            // tiles of all matrices
     int nb, parts, part_blocks, per_part;         // blocks of the row, its parts, blocks of a part, CTAs of a part
-    int depth, sh;
+    int depth, sh, small_scales;
     const int64_t *x, *gain;                      // the row; gain (nullable) where it is normalised
     int norm, frac;
     unsigned long long eps;
@@ -64,10 +64,12 @@ __device__ __forceinline__ void rw_mma_first(int (&c)[4], uint32_t a0, uint32_t 
                  : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
 
-// Twice the sums over the 128 values of a block of the set bits' values, for two units at once: a lane ends with that of row
-// g + 8 (t & 1) of unit t >> 1.  The columns of the MMA are the digits.  A register of weight bits is one AND: bits 0 and 1 of every
-// byte stand for the two rows as they lie, which doubles the rows g + 8 (the digits' weights double the others).  Two exchanges
-// bring the digits of a lane's row and unit together; with four digits in use (NARROW) every second column is zero and stays out.
+// Sums over the 128 values of a block of the set bits' values, for two units at once, times a factor of two: a lane ends with that
+// of row g + 8 (t & 1) of unit t >> 1.  The columns of the MMA are the digits.  A register of weight bits is one AND behind a left
+// shift (a multiplication, so that the logic unit, which bounds the walk over the tiles, has the ANDs alone): bits 6 and 7 of every
+// byte stand for the rows g and g + 8, which doubles the latter (the digits' weights double the others).  Two exchanges bring the
+// digits of a lane's row and unit together; with four digits in use (NARROW) every second column is zero and stays out.
+// NARROW: 128 times the sums; otherwise, where the factor could carry into the wrapped product, twice them.
 struct RowFold {
     int f[4];                                     // weights of the digits that this lane, lane xor 1, xor 2 and xor 3 hold
     bool second, odd;
@@ -90,11 +92,15 @@ __device__ __forceinline__ uint64_t rw_unit_sums(const uint2 (&w)[2], const uint
     for (int m = 0; m < 4; m++)
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            const uint32_t raw = (m >> 1) ? w[u].y : w[u].x, low = (m & 1) ? raw >> 4 : raw, high = raw >> (4 * (m & 1) + 2);
-            const uint32_t a0 = low & 0x01010101u, a1 = low & 0x02020202u, a2 = high & 0x01010101u, a3 = high & 0x02020202u;
+            const uint32_t raw = (m >> 1) ? w[u].y : w[u].x, high = raw * ((m & 1) ? 1u : 16u), low = raw * ((m & 1) ? 4u : 64u);
+            const uint32_t a0 = low & 0x40404040u, a1 = low & 0x80808080u, a2 = high & 0x40404040u, a3 = high & 0x80808080u;
             if (m == 0) rw_mma_first(c[u], a0, a1, a2, a3, bf[u][0], bf[u][1]);
             else mma_u8s8_k32(c[u], a0, a1, a2, a3, bf[u][2 * m], bf[u][2 * m + 1]);
         }
+    if (!NARROW) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) { c[u][0] >>= 6; c[u][1] >>= 6; c[u][2] >>= 6; c[u][3] >>= 6; }
+    }
     uint64_t v = (uint64_t)fold(c[0][0], c[0][2], c[1][0], c[1][2]);
     if (!NARROW) v += (uint64_t)fold(c[0][1], c[0][3], c[1][1], c[1][3]) << 32;      // columns 2t + 1: digits four further up
     return v;
@@ -315,7 +321,8 @@ __global__ void __launch_bounds__(RW_THREADS, 2) q1_row_kernel(const Q1RowArgs a
         const int column = (2 * warp + (t >> 1)) * RW_COL + g + 8 * (t & 1);
         // blocks beyond the part have no digits, so whatever units stand in for theirs add nothing
         const int first = min(2 * warp, ((a.part_blocks + 1) & ~1) - 2);
-        const uint64_t total = s_total[2 * warp + (t >> 1)];
+        const uint64_t total = s_total[2 * warp + (t >> 1)] * (NARROW ? 64 : 1);
+        const int sh = a.sh + (NARROW ? 6 : 0);
         int s = 0, asked = min(a.depth, groups);                          // behind a failure nothing more is asked for, and only that awaited
         uint32_t parity = 0;
         for (int q = 0; q < groups; q++) {
@@ -328,7 +335,7 @@ __global__ void __launch_bounds__(RW_THREADS, 2) q1_row_kernel(const Q1RowArgs a
             for (int i = 0; i < n; i++) {
                 const uint2 w[2] = {*reinterpret_cast<const uint2 *>(unit + lane * 8), *reinterpret_cast<const uint2 *>(unit + US + lane * 8)};
                 const int64_t sc = (int64_t)*(reinterpret_cast<const DT *>(unit + (t >> 1) * US + 256) + g + 8 * (t & 1));
-                *to = (uint64_t)((int64_t)((rw_unit_sums<NARROW>(w, bf, fold) - total) * (uint64_t)sc) >> a.sh);
+                *to = (uint64_t)((int64_t)((rw_unit_sums<NARROW>(w, bf, fold) - total) * (uint64_t)sc) >> sh);
                 unit += tile_stride; to += 32 * RW_COL;
             }
             __syncthreads();                                              // the group has been read; the other half of the sums is free
@@ -346,7 +353,8 @@ __global__ void __launch_bounds__(RW_THREADS, 2) q1_row_kernel(const Q1RowArgs a
             if ((q & 7) == 7 || q + 1 == groups) finish(q & ~7, (q & 7) + 1);
         }
     };
-    if (narrow) walk(std::true_type()); else walk(std::false_type());
+    // (products of narrow values with scales below 2^20 keep the factor of 64 within 64 bits)
+    if (narrow && a.small_scales) walk(std::true_type()); else walk(std::false_type());
     if (dead && lane == 0) atomicOr(a.flags, 8);
     if (bad) atomicOr(a.flags, 2);
 }
@@ -367,8 +375,10 @@ cudaError_t launch_row(const Q1RowArgs &a, cudaStream_t s) {
     const size_t slots = groups <= b.depth ? (size_t)(b.depth - 1) * RW_GROUP + (SWIGLU ? std::min(run, RW_GROUP) : run - (groups - 1) * RW_GROUP) : (size_t)b.depth * RW_GROUP;
     static bool configured = false;
     if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(q1_row_kernel<DT, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)(RW_HEAD_BYTES + (size_t)RW_RING * RW_GROUP * RW_BLOCKS * (256 + 16 * sizeof(DT))));
+        cudaError_t e = cudaFuncSetAttribute(q1_row_kernel<DT, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(RW_HEAD_BYTES + (size_t)RW_RING * RW_GROUP * RW_BLOCKS * (256 + 16 * sizeof(DT))));
+        // all of the SM's memory as shared memory: otherwise the next kernel's CTAs do not fit beside these and start behind them, two to an SM
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(q1_row_kernel<DT, SWIGLU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
         configured = true;
     }
@@ -397,6 +407,8 @@ cudaError_t launch_q1_row(const Q1Part *mats, int n, bool sc32, long long nb, co
         if (tiles > (1 << 28)) return cudaErrorInvalidValue;
         a.tiles = (int)tiles; a.tile_end[i] = a.tiles;
     }
+    a.small_scales = frac <= 57;
+    for (int i = 0; i < n; i++) if (mats[i].max_scale >= (1u << 20)) a.small_scales = 0;
     a.n_mats = n; a.nb = (int)nb;
     a.parts = (int)((nb + RW_BLOCKS - 1) / RW_BLOCKS);
     a.part_blocks = (int)((nb + a.parts - 1) / a.parts);
