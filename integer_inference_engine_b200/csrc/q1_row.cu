@@ -75,7 +75,10 @@ struct RowFold {
     bool second, odd;
     __device__ __forceinline__ explicit RowFold(int t) : second(t >= 2), odd(t & 1) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) f[k] = (odd ? 1 : 2) << (8 * (t ^ k));
+        for (int k = 0; k < 4; k++) {
+            f[k] = (odd ? 1 : 2) << (8 * (t ^ k));
+            asm volatile("" : "+r"(f[k]));        // a factor, one wide multiply-add each: known as a power of two it would be a 64-bit shift
+        }
     }
     __device__ __forceinline__ int64_t operator()(int a0, int a1, int b0, int b1) const {      // units a, b; rows g, g + 8
         const int k0 = second ? b0 : a0, k1 = second ? b1 : a1;
