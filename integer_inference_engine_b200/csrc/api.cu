@@ -948,6 +948,26 @@ int iie::attn_decode_normed(const int64_t *q, const int64_t *k, const int64_t *v
     return 0;
 }
 
+// The new tokens of n_seqs sequences, each at its own position (pos_each on the device, pos_max their largest), with the per-head norms:
+// 0, 1 on failure, 3 where the cluster form does not carry the shape (nothing was launched).
+int iie::attn_decode_each(const int64_t *q, const int64_t *k, const int64_t *v, int32_t *kcache, int32_t *vcache, const int *pos_each, long long pos_max,
+                          long long n_seqs, long long seq_stride, const int64_t *cos, const int64_t *sin, int rope, int H, int Hkv, int hd,
+                          long long cache_rows, int fa, long long inv_sqrt, const int64_t *qgain, const int64_t *kgain, unsigned long long eps,
+                          int64_t *out, cudaStream_t s) {
+    std::lock_guard<std::recursive_mutex> lk(g_mu);
+    if (!init()) return 1;
+    AttnArgs a = {};
+    a.batch = (int)n_seqs; a.seq_stride = seq_stride; a.pos_each = pos_each;
+    a.q = q; a.k = k; a.v = v; a.kcache = kcache; a.vcache = vcache; a.pos = pos_max; a.Lmax = cache_rows;
+    a.cos = cos; a.sin = sin; a.rope = rope; a.H = H; a.Hkv = Hkv; a.hd = hd;
+    attn_consts(a, fa, inv_sqrt);
+    a.qgain = qgain; a.kgain = kgain; a.eps = eps; a.out = out; a.flags = g_flags;
+    int n_c = 0, tiles = 0;
+    if (g_attn_fused != 1 || n_seqs > 65535 || pos_max >= cache_rows || !attn_shape_ok(H, Hkv, hd) || !attn_cluster_plan(a, n_c, tiles)) return 3;
+    if (launch_attn_cluster(a, n_c, tiles, s) != cudaSuccess) { cudaGetLastError(); return 1; }
+    return 0;
+}
+
 extern "C" int iie_attn_prefill_dev(const int64_t *q_dev, const int64_t *k_dev, const int64_t *v_dev, int32_t *kcache_dev,
                                     int32_t *vcache_dev, long long start, long long tokens, long long window,
                                     const int64_t *cos_dev, const int64_t *sin_dev, int rope, int n_heads, int n_kv, int head_dim,
@@ -989,18 +1009,23 @@ extern "C" int iie_attn_decode_batch_dev(const int64_t *q_dev, const int64_t *k_
         seq_stride < (long long)n_kv * cache_rows * head_dim) return 1;
     cudaStream_t s = (cudaStream_t)stream;
     const long long Ls = (pos + 1 + 63) / 64 * 64;
-    // scratch roles of their own (a captured single-token step keeps the addresses of the single-token buffers)
-    int64_t *scores = (int64_t *)ensure(R_BSCORES, (size_t)n_seqs * n_heads * Ls * 8);
-    int32_t *e = (int32_t *)ensure(R_BEXP, (size_t)n_seqs * n_heads * Ls * 4);
-    uint8_t *st = (uint8_t *)ensure(R_BSTAT, (size_t)n_seqs * n_heads * 16);
-    if (!scores || !e || !st) return 1;
     AttnArgs a = {};
     a.batch = (int)n_seqs; a.seq_stride = seq_stride;
     a.q = q_dev; a.k = k_dev; a.v = v_dev; a.kcache = kcache_dev; a.vcache = vcache_dev; a.pos = pos; a.window = window;
     a.Lmax = cache_rows; a.Ls = Ls; a.cos = cos_dev; a.sin = sin_dev; a.rope = rope; a.H = n_heads; a.Hkv = n_kv; a.hd = head_dim;
     attn_consts(a, fa, inv_sqrt);
-    a.scores = scores; a.e = e; a.hmax = (long long *)st; a.Z = (unsigned long long *)(st + (size_t)n_seqs * n_heads * 8);
     a.out = out_dev; a.flags = g_flags;
+    int n_c = 0, tiles = 0;
+    if (g_attn_fused == 1 && attn_shape_ok(a.H, a.Hkv, a.hd) && attn_cluster_plan(a, n_c, tiles)) {      // needs no scratch
+        if (launch_attn_prefill(a, s) != cudaSuccess) { cudaGetLastError(); return 1; }
+        return 0;
+    }
+    // scratch roles of their own (a captured single-token step keeps the addresses of the single-token buffers)
+    int64_t *scores = (int64_t *)ensure(R_BSCORES, (size_t)n_seqs * n_heads * Ls * 8);
+    int32_t *e = (int32_t *)ensure(R_BEXP, (size_t)n_seqs * n_heads * Ls * 4);
+    uint8_t *st = (uint8_t *)ensure(R_BSTAT, (size_t)n_seqs * n_heads * 16);
+    if (!scores || !e || !st) return 1;
+    a.scores = scores; a.e = e; a.hmax = (long long *)st; a.Z = (unsigned long long *)(st + (size_t)n_seqs * n_heads * 8);
     // few sequences leave most SMs idle in the probability x value pass: share each pair's chunks over up to eight CTAs
     const long long pairs = n_seqs * n_kv;
     int splits = (int)std::min<long long>(8, std::min<long long>(Ls / 64, (2368 + pairs - 1) / pairs));   // about two CTAs per SM, four waves

@@ -676,6 +676,8 @@ __device__ __forceinline__ bool af_group_barrier(unsigned *counter, unsigned tar
     return s_open != 0;
 }
 
+// NORM: the per-head norms of queries and key first (a form of its own: their code costs the others about 1 us a launch)
+template <bool NORM>
 __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs a_in) {
     AttnArgs a = a_in;
     if (!at_span(a_in, a.pos, a.lo)) { at_refuse(a_in); return; }          // uniform over the grid
@@ -726,7 +728,7 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
     // ---- per-head norms, where the caller wants them here: a warp per head, the new key row (by the CTA that appends it) into the
     //      partial sums' space, which pass 1 does not use before the rotation is done
     int64_t *knew = reinterpret_cast<int64_t *>(red);
-    if (a.qgain) {
+    if (NORM) {
         if (warp < rep + (own ? 1 : 0)) {
             const bool is_k = warp == rep;
             const int64_t *src = is_k ? a.k + kv * hd : a.q + (long long)(kv * rep + warp) * hd, *gain = is_k ? a.kgain : a.qgain;
@@ -765,7 +767,7 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
         const int i0 = a.rope == 2 ? i : 2 * i, i1 = a.rope == 2 ? i + half : 2 * i + 1;
         int64_t x0 = 0, x1 = 0;
         if (r < rep) {
-            const int64_t *src = a.qgain ? reinterpret_cast<const int64_t *>(q64) + r * hd : a.q + (long long)(kv * rep + r) * hd;      // in place: a pair is one thread's
+            const int64_t *src = NORM ? reinterpret_cast<const int64_t *>(q64) + r * hd : a.q + (long long)(kv * rep + r) * hd;      // in place: a pair is one thread's
             x0 = src[i0]; x1 = src[i1];
             at_rotate(a, a.pos, i, x0, x1);
         }
@@ -787,7 +789,7 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
         bool bad = false;
         for (int i = tid; i < half; i += AF_THREADS) {
             const int i0 = a.rope == 2 ? i : 2 * i, i1 = a.rope == 2 ? i + half : 2 * i + 1;
-            const int64_t *src = a.qgain ? knew : a.k + kv * hd;
+            const int64_t *src = NORM ? knew : a.k + kv * hd;
             int64_t x0 = src[i0], x1 = src[i1];
             at_rotate(a, a.pos, i, x0, x1);
             bad |= x0 != (int32_t)x0 || x1 != (int32_t)x1;
@@ -1363,8 +1365,9 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s) {
         a.fa <= 23 && a.Hkv <= 120) {                                       // probabilities (at most 2^fa) as three bytes
         static bool fat_configured = false;
         if (!fat_configured) {
-            if (cudaFuncSetAttribute(attn_fat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess ||
-                cudaFuncSetAttribute(attn_fat_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) return cudaGetLastError();
+            if (cudaFuncSetAttribute(attn_fat_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess ||
+                cudaFuncSetAttribute(attn_fat_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess ||
+                cudaFuncSetAttribute(attn_fat_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) return cudaGetLastError();
             fat_configured = true;
         }
         const int per_head = std::max(1, std::min(n_sms, 192) / a.Hkv);      // the partial-sum scratch holds 192 chunks
@@ -1375,7 +1378,7 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s) {
                                 (size_t)AF_THREADS / a.hd * AF_HEADS * a.hd * 8 + (size_t)4 * AF_HEADS * (a.hd + 16) + (size_t)3 * AF_HEADS * (C + 16);
         int per_sm = 0;
         if (C <= 2 * 8 * (AF_THREADS / 32) && fat_smem <= 208 * 1024 &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_fat_kernel, AF_THREADS, fat_smem) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, a.qgain ? attn_fat_kernel<true> : attn_fat_kernel<false>, AF_THREADS, fat_smem) == cudaSuccess &&
             (long long)fat_chunks * a.Hkv <= (long long)per_sm * n_sms) {
             AttnArgs f = a;
             f.chunk = C;
@@ -1385,7 +1388,7 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s) {
             attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1;
             attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr; cfg.numAttrs = a.pdl ? 2 : 1;
-            const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_fat_kernel, f);
+            const cudaError_t e = cudaLaunchKernelEx(&cfg, a.qgain ? attn_fat_kernel<true> : attn_fat_kernel<false>, f);
             note_launch(1);
             return e != cudaSuccess ? e : cudaGetLastError();
         }
@@ -1419,8 +1422,12 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s) {
 cudaError_t launch_attn_prefill(const AttnArgs &a, cudaStream_t s) {
     const long long last_pos = a.seq_stride > 0 ? a.pos : a.pos + a.batch - 1;
     if (!attn_shape_ok(a.H, a.Hkv, a.hd) || a.batch <= 0 || a.batch > 65535 || a.pos < 0 || last_pos >= a.Lmax || a.seq_stride < 0 || a.fa < 1 ||
-        a.fa > 29 || (a.rope && (!a.cos || !a.sin)) || a.pos_dev || !a.out || !a.scores || !a.e || !a.hmax || !a.Z)
+        a.fa > 29 || (a.rope && (!a.cos || !a.sin)) || a.pos_dev || !a.out)
         return cudaErrorInvalidValue;
+    // independent sequences: a cluster per (sequence, KV head) reads keys and values once and keeps the scores on the chip
+    int n_c = 0, tiles = 0;
+    if (a.seq_stride > 0 && g_attn_fused == 1 && attn_cluster_plan(a, n_c, tiles)) return launch_attn_cluster(a, n_c, tiles, s);
+    if (a.pos_each || !a.scores || !a.e || !a.hmax || !a.Z) return cudaErrorInvalidValue;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(attn_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||

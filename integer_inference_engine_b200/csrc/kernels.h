@@ -245,6 +245,7 @@ struct AttnArgs {
     long long pos, lo, Lmax;       // position of the new token (an upper bound when pos_dev is set), first visible key
                                    // (computed on the device), cache rows
     const int *pos_dev;            // optional: the position in device memory (for replayed graphs)
+    const int *pos_each;           // optional, batched decode of the cluster form: a position per sequence in device memory (pos: their bound)
     long long window;              // > 0: only the last `window` keys are visible
     const int64_t *cos, *sin;      // [>= pos+1][hd/2] at 2^fa, or nullptr when rope == 0
     int rope;                      // 0 none, 1 interleaved pairs (2i, 2i+1), 2 rotate-half pairs (i, i + hd/2)
@@ -274,9 +275,17 @@ struct AttnArgs {
     long long *pv_part;            // scratch [batch][pv_splits][H][hd] for their raw sums
 };
 cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s);
+// one cluster per (sequence, KV head): the new tokens of independent sequences (attn_cluster.cu); the plan says
+// whether the shape is carried, with how many CTAs per cluster and tiles per CTA
+bool attn_cluster_plan(const AttnArgs &a, int &n_c, int &tiles);
+cudaError_t launch_attn_cluster(const AttnArgs &a, int n_c, int tiles, cudaStream_t s);
 int attn_decode_normed(const int64_t *q, const int64_t *k, const int64_t *v, int32_t *kcache, int32_t *vcache, long long pos,
                        const int *pos_dev, const int64_t *cos, const int64_t *sin, int rope, int H, int Hkv, int hd, long long cache_rows,
                        int fa, long long inv_sqrt, const int64_t *qgain, const int64_t *kgain, unsigned long long eps, int64_t *out, cudaStream_t s);
+int attn_decode_each(const int64_t *q, const int64_t *k, const int64_t *v, int32_t *kcache, int32_t *vcache, const int *pos_each, long long pos_max,
+                     long long n_seqs, long long seq_stride, const int64_t *cos, const int64_t *sin, int rope, int H, int Hkv, int hd,
+                     long long cache_rows, int fa, long long inv_sqrt, const int64_t *qgain, const int64_t *kgain, unsigned long long eps,
+                     int64_t *out, cudaStream_t s);
 // `batch` new tokens at positions pos .. pos + batch - 1 against the cache rows before them and each other (causal):
 // all K/V rows are appended first, then scores, exponentials and the probability-value sums run per token
 cudaError_t launch_attn_prefill(const AttnArgs &a, cudaStream_t s);

@@ -541,7 +541,14 @@ bool products_of_row(const Q1RowInput &in, std::initializer_list<Product> list, 
     return !swiglu || launch_q1_silu_mul(parts[0].out, parts[1].out, parts[0].out_f, (int)frac, parts[0].out, q_stream) == cudaSuccess;
 }
 
-// One layer on T rows of w.x.  attend(q normalised, k normalised, v) runs rotation, cache append and attention into w.att.
+// the per-head norms: w.q, w.k -> w.qn, w.kn
+bool head_norms(const Q1Stack &m, size_t layer, Work &w, long long T, int *flags) {
+    const int f = (int)m.frac;
+    return launch_rmsnorm(w.q, T * m.H, m.hd, q_bufs[(size_t)m.qng[layer]].p, f, m.eps, w.qn, flags, q_stream) == cudaSuccess &&
+           launch_rmsnorm(w.k, T * m.Hkv, m.hd, q_bufs[(size_t)m.kng[layer]].p, f, m.eps, w.kn, flags, q_stream) == cudaSuccess;
+}
+
+// One layer on T rows of w.x.  attend(layer) runs the per-head norms of w.q and w.k, rotation, cache append and attention into w.att.
 template <typename Attend>
 bool layer_rows(const Q1Stack &m, long long li, Work &w, long long T, int *flags, Attend attend) {
     const size_t i = (size_t)li;
@@ -555,9 +562,7 @@ bool layer_rows(const Q1Stack &m, long long li, Work &w, long long T, int *flags
     };
     bool ok = (T == 1 ? products_of_row({w.x, true, gain(m.n1g[i]), m.eps}, {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, false, m.frac)
                       : products(norm(m.n1g[i]), {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, planes, T, m.frac, w.x, T * m.d)) &&
-              launch_rmsnorm(w.q, T * m.H, m.hd, gain(m.qng[i]), f, m.eps, w.qn, flags, q_stream) == cudaSuccess &&
-              launch_rmsnorm(w.k, T * m.Hkv, m.hd, gain(m.kng[i]), f, m.eps, w.kn, flags, q_stream) == cudaSuccess;
-    ok = ok && attend(w.qn, w.kn, w.v, w.att);
+              attend(i);
     if (T == 1)
         return ok && products_of_row({w.att, false, nullptr, 0}, {{m.wo[i], w.x, w.x}}, false, m.frac) &&
                products_of_row({w.x, true, gain(m.n2g[i]), m.eps}, {{m.w1[i], w.g}, {m.wu[i], w.u}}, true, m.frac) &&
@@ -623,6 +628,7 @@ struct DecodeCtx {
     long long B = 0, cap = 0, vocab = 0;
     int32_t *K = nullptr, *V = nullptr;            // [n_layers][B][Hkv][cap][hd]
     int64_t *logits = nullptr;
+    int *pos = nullptr;                            // [B]: where the sequences stand in the step under way
     Work w;
     std::vector<char> wide;                        // per sequence: a seeded value did not fit the int32 rows
 };
@@ -632,6 +638,7 @@ void free_ctx(DecodeCtx &c) {
     if (c.K) cudaFree(c.K);
     if (c.V) cudaFree(c.V);
     if (c.logits) cudaFree(c.logits);
+    if (c.pos) cudaFree(c.pos);
     free_work(c.w);
     c = DecodeCtx();
 }
@@ -795,8 +802,9 @@ extern "C" int bonsai_prefill_forward_gpu(const long long *x_embed, long long T,
         ok = ok && fw;
         const int64_t *cosd = q_bufs[(size_t)cos_h].p, *sind = q_bufs[(size_t)sin_h].p;
         for (long long li = 0; ok && li < n_layers; li++) {
-            ok = layer_rows(m, li, w, T, fw, [&](const int64_t *qn, const int64_t *kn, const int64_t *v, int64_t *att) {
-                return iie_attn_prefill_dev(qn, kn, v, kc, vc, 0, T, 0, cosd, sind, 2, (int)H, (int)Hkv, (int)hd, T, (int)frac, inv_sqrt_fp, att,
+            ok = layer_rows(m, li, w, T, fw, [&](size_t layer) {
+                return head_norms(m, layer, w, T, fw) &&
+                       iie_attn_prefill_dev(w.qn, w.kn, w.v, kc, vc, 0, T, 0, cosd, sind, 2, (int)H, (int)Hkv, (int)hd, T, (int)frac, inv_sqrt_fp, w.att,
                                             q_stream) == 0;
             });
             if (ok && (out_k || out_v)) {
@@ -842,7 +850,7 @@ extern "C" long long bonsai_decode_ctx_create(long long B, long long n_layers, l
     c.B = B; c.cap = cap; c.vocab = vocab; c.wide.assign((size_t)B, 0);
     const size_t kv = (size_t)n_layers * B * Hkv * cap * hd * 4;
     if (cudaMalloc(&c.K, kv) != cudaSuccess || cudaMalloc(&c.V, kv) != cudaSuccess || cudaMemset(c.K, 0, kv) != cudaSuccess ||
-        cudaMemset(c.V, 0, kv) != cudaSuccess || cudaMalloc(&c.logits, (size_t)B * vocab * 8) != cudaSuccess || !alloc_work(c.w, m, B)) {
+        cudaMemset(c.V, 0, kv) != cudaSuccess || cudaMalloc(&c.logits, (size_t)B * vocab * 8) != cudaSuccess || cudaMalloc(&c.pos, (size_t)B * 4) != cudaSuccess || !alloc_work(c.w, m, B)) {
         cudaGetLastError(); free_ctx(c); fail(2, "decode context: out of device memory"); return -1;
     }
     c.alive = true;
@@ -885,7 +893,10 @@ extern "C" int bonsai_decode_step(long long ctx_h, const long long *x_in, const 
     for (char wide : c.wide) if (wide) return fail(4, "decode step: a seeded K/V value is beyond int32");
     const long long qd = m.H * m.hd, kd = m.Hkv * m.hd;
     const size_t per_seq = (size_t)m.Hkv * c.cap * m.hd;
-    bool ok = cudaMemcpyAsync(c.w.x, x_in, (size_t)c.B * m.d * 8, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
+    std::vector<int> at(pos, pos + c.B);
+    const long long longest = *std::max_element(pos, pos + c.B);
+    bool ok = cudaMemcpyAsync(c.w.x, x_in, (size_t)c.B * m.d * 8, cudaMemcpyHostToDevice, q_stream) == cudaSuccess &&
+              cudaMemcpyAsync(c.pos, at.data(), (size_t)c.B * 4, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
     int flags = -1;
     {
         FlagScope scope;
@@ -895,12 +906,19 @@ extern "C" int bonsai_decode_step(long long ctx_h, const long long *x_in, const 
         const int64_t *cosd = q_bufs[(size_t)m.cos_h].p, *sind = q_bufs[(size_t)m.sin_h].p;
         for (long long li = 0; ok && li < m.n_layers; li++) {
             int32_t *Kl = c.K + (size_t)li * c.B * per_seq, *Vl = c.V + (size_t)li * c.B * per_seq;
-            ok = layer_rows(m, li, c.w, c.B, fw, [&](const int64_t *qn, const int64_t *kn, const int64_t *v, int64_t *att) {
-                // sequences sit at their own positions: one single-token attention per sequence
+            ok = layer_rows(m, li, c.w, c.B, fw, [&](size_t layer) {
+                // sequences sit at their own positions: one launch for all of them, else one single-token attention per sequence
+                const int64_t *qg = q_bufs[(size_t)m.qng[layer]].p, *kg = q_bufs[(size_t)m.kng[layer]].p;
+                const int rc = c.B == 1 ? attn_decode_normed(c.w.q, c.w.k, c.w.v, Kl, Vl, pos[0], nullptr, cosd, sind, 2, (int)m.H, (int)m.Hkv, (int)m.hd,
+                                                             c.cap, (int)m.frac, m.inv_sqrt, qg, kg, m.eps, c.w.att, q_stream)
+                                        : attn_decode_each(c.w.q, c.w.k, c.w.v, Kl, Vl, c.pos, longest, c.B, (long long)per_seq, cosd, sind, 2, (int)m.H,
+                                                           (int)m.Hkv, (int)m.hd, c.cap, (int)m.frac, m.inv_sqrt, qg, kg, m.eps, c.w.att, q_stream);
+                if (rc != 3) return rc == 0;
+                if (!head_norms(m, layer, c.w, c.B, fw)) return false;
                 for (long long b = 0; b < c.B; b++)
-                    if (iie_attn_decode_dev(qn + (size_t)b * qd, kn + (size_t)b * kd, v + (size_t)b * kd, Kl + (size_t)b * per_seq,
+                    if (iie_attn_decode_dev(c.w.qn + (size_t)b * qd, c.w.kn + (size_t)b * kd, c.w.v + (size_t)b * kd, Kl + (size_t)b * per_seq,
                                             Vl + (size_t)b * per_seq, pos[b], nullptr, 0, cosd, sind, 2, (int)m.H, (int)m.Hkv, (int)m.hd, c.cap,
-                                            (int)m.frac, m.inv_sqrt, att + (size_t)b * qd, q_stream) != 0) return false;
+                                            (int)m.frac, m.inv_sqrt, c.w.att + (size_t)b * qd, q_stream) != 0) return false;
                 return true;
             });
         }
