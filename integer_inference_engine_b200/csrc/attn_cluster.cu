@@ -10,6 +10,10 @@
 // Scores: 16 keys x 8 heads x 32 dimensions per step.  Values: probabilities are bytes too; the low bytes of the eight heads are rows
 // 0..7 of the operand, the second bytes rows 8..15, and columns are taken so that one 16-byte load of a value row feeds four steps.
 //
+// What bounds it: 64 sequences of 4096 keys, 4 KV heads of 128 (1.07 GB): 258 us; the copies alone take 164, the rest is the latency of
+// eight warps per SM (their registers hold the loads under way: with twelve warps and less of it 330), about 1800 instructions per
+// tile.  Three kernels with the scores in memory took 540.  One sequence does not come here: its chain of one warp per tile is longer
+// than that of attn_fat_kernel (16 against 12 us at 513 keys).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -28,7 +32,8 @@ constexpr int AC_WARPS = 4, AC_THREADS = 32 * AC_WARPS;
 constexpr int AC_TILE = 32;                    // keys of a tile
 constexpr int AC_HEADS = 8;                    // query heads of a KV head at most
 constexpr int AC_MAX_CLUSTER = 8;
-constexpr int AC_MAX_TILES = 48;               // tiles of a CTA: three CTAs then fit an SM
+constexpr int AC_AHEAD = 1;                    // tiles of a warp that are on their way to the cache ahead of the one at hand
+constexpr int AC_MAX_TILES = 64;               // tiles of a CTA: two CTAs then fit an SM
 
 template <int HD>
 __host__ __device__ constexpr size_t ac_smem(int tiles) {          // scores [8][32 tiles + 4] and queries as int64, later the warps' sums [4][8][HD]; queries as bytes; the new key
@@ -36,6 +41,10 @@ __host__ __device__ constexpr size_t ac_smem(int tiles) {          // scores [8]
     return (a > b ? a : b) + (size_t)4 * AC_HEADS * (HD + 16) + (size_t)HD * 8;
 }
 
+// rows that a later tile reads, on their way from memory to the cache: one request per tile
+__device__ __forceinline__ void ac_ahead(const int32_t *rows, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rows), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ int4 ac_load(const int32_t *p) { return __ldcg(reinterpret_cast<const int4 *>(p)); }
 
 // the four bytes of four consecutive values, transposed: d[b] = byte b of (x, y, z, w)
@@ -43,22 +52,41 @@ __device__ __forceinline__ void ac_bytes(uint32_t x, uint32_t y, uint32_t z, uin
     const uint32_t t0 = __byte_perm(x, y, 0x5140), t1 = __byte_perm(x, y, 0x7362), t2 = __byte_perm(z, w, 0x5140), t3 = __byte_perm(z, w, 0x7362);
     d[0] = __byte_perm(t0, t2, 0x5410); d[1] = __byte_perm(t0, t2, 0x7632); d[2] = __byte_perm(t1, t3, 0x5410); d[3] = __byte_perm(t1, t3, 0x7632);
 }
-// D(16x8,s32) += A(16x32, 8-bit, row) * B(32x8, 8-bit, col), each operand signed or not
-template <bool AS, bool BS>
+// D(16x8,s32) = A(16x32, 8-bit, row) * B(32x8, 8-bit, col) (+ D), the operands signed or not.  (An unsigned B costs two instructions.)
+template <bool AS>
 __device__ __forceinline__ void ac_mma(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    if (AS && BS)
+    if (AS)
         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else if (AS)
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else if (BS)
+    else
         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-    else
-        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                     : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+template <bool BS>
+__device__ __forceinline__ void ac_mma_first(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if (BS)
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                     : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+    else
+        asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                     : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+
+// exp2_neg_fixed of (d log2e) >> fa for 0 <= d <= clip and fa <= 23: every operand fits 32 bits
+struct AcExp {
+    uint32_t c0 = 65536, c1 = 45426, c2 = 15743, c3 = 3638, log2e;
+    int fa;
+    __device__ __forceinline__ AcExp(int fa_, long long log2e_) : log2e((uint32_t)log2e_), fa(fa_) {
+        const int s = 16 - fa;
+        if (s >= 0) { c0 >>= s; c1 >>= s; c2 >>= s; c3 >>= s; } else { c0 <<= -s; c1 <<= -s; c2 <<= -s; c3 <<= -s; }
+    }
+    __device__ __forceinline__ uint32_t mul(uint32_t x, uint32_t y) const { return (uint32_t)(((uint64_t)x * y) >> fa); }
+    __device__ __forceinline__ int operator()(uint32_t d) const {
+        const uint32_t u = mul(d, log2e), f = u & ((1u << fa) - 1), f2 = mul(f, f), f3 = mul(f2, f);
+        const int p = (int)(c0 - mul(c1, f) + mul(c2, f2) - mul(c3, f3));
+        return max(p, 0) >> (u >> fa);
+    }
+};
 
 __device__ __forceinline__ void ac_rotate(const AttnArgs &a, long long pos, int i, int64_t &x0, int64_t &x1) {
     if (!a.rope) return;
@@ -69,12 +97,12 @@ __device__ __forceinline__ void ac_rotate(const AttnArgs &a, long long pos, int 
 }
 
 template <int HD>
-__global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnArgs a) {
+__global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnArgs a) {
     constexpr int QLD = HD + 16, HALF = HD / 2;
     extern __shared__ __align__(128) unsigned char ac_sm[];
     __shared__ long long s_max[AC_WARPS][AC_HEADS], s_base[AC_WARPS][AC_HEADS];
     __shared__ unsigned long long s_z[AC_WARPS][AC_HEADS];
-    __shared__ int s_wide, s_q24;
+    __shared__ int s_wide;
     cg::cluster_group cluster = cg::this_cluster();
     const int n_c = (int)gridDim.x, rank = (int)blockIdx.x, kv = blockIdx.y, seq = blockIdx.z, rep = a.H / a.Hkv;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -89,11 +117,20 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
     const bool own = first < end && end == n_tiles;                         // this CTA appends the new row
     int32_t *off = reinterpret_cast<int32_t *>(ac_sm);                      // [8][stride]: scores, then exponentials
     int64_t *q64 = reinterpret_cast<int64_t *>(off + AC_HEADS * stride);   // rotated queries [8][HD] (rows beyond rep are zero)
-    int8_t *qd = reinterpret_cast<int8_t *>(ac_sm + ac_smem<HD>(a.chunk) - HD * 8 - 4 * AC_HEADS * QLD);      // their bytes [4][8][HD + 16]
+    int8_t *qd = reinterpret_cast<int8_t *>(ac_sm + ac_smem<HD>(a.chunk) - HD * 8 - 4 * AC_HEADS * QLD);      // their balanced digits [4][8][HD + 16]
     int64_t *knew = reinterpret_cast<int64_t *>(qd + 4 * AC_HEADS * QLD);   // the new key, normed
     const int32_t *kc = a.kcache + (long long)seq * a.seq_stride + ((long long)kv * a.Lmax + lo) * HD;
     const int32_t *vc = a.vcache + (long long)seq * a.seq_stride + ((long long)kv * a.Lmax + lo) * HD;
-    if (tid == 0) { s_wide = 0; s_q24 = 0; }
+    // tile `tile` of the keys, or of the values behind the warp's last key tile; rows that the cache held before this token
+    const int mine = first + warp < end ? (end - first - warp + AC_WARPS - 1) / AC_WARPS : 0;      // tiles of this warp
+    auto ahead = [&](int i) {
+        const int32_t *cache = i < mine ? kc : vc;
+        const int tile = first + warp + AC_WARPS * (i < mine ? i : i - mine), rows = min(AC_TILE, n_keys - 1 - tile * AC_TILE);
+        if (lane == 0 && i < 2 * mine && rows > 0) ac_ahead(cache + (long long)tile * AC_TILE * HD, (uint32_t)(rows * HD * 4));
+    };
+#pragma unroll
+    for (int i = 0; i < AC_AHEAD; i++) ahead(i);
+    if (tid == 0) s_wide = 0;
     if (lane < AC_HEADS) s_base[warp][lane] = 0;                            // (no tile: never used)
     // ---- per-head norms where the caller wants them here, rotation, bytes of the queries; the new row into the cache ----------------
     const int64_t *q_in = a.q + (long long)seq * a.H * HD + (long long)kv * rep * HD, *k_in = a.k + ((long long)seq * a.Hkv + kv) * HD;
@@ -129,7 +166,7 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
         }
     }
     __syncthreads();                                                        // norms and the words set above
-    bool wide = false, wide24 = false;
+    bool wide = false;                                                      // a query beyond four balanced digits
     for (int idx = tid; idx < AC_HEADS * HALF; idx += AC_THREADS) {
         const int r = idx / HALF, i = idx - r * HALF;
         const int i0 = a.rope == 2 ? i : 2 * i, i1 = a.rope == 2 ? i + HALF : 2 * i + 1;
@@ -140,16 +177,15 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
             ac_rotate(a, pos, i, x0, x1);
         }
         q64[r * HD + i0] = x0; q64[r * HD + i1] = x1;
+        const uint32_t d0 = ((uint32_t)x0 + 0x80808080u) ^ 0x80808080u, d1 = ((uint32_t)x1 + 0x80808080u) ^ 0x80808080u;
 #pragma unroll
         for (int b = 0; b < 4; b++) {
-            qd[(b * AC_HEADS + r) * QLD + i0] = (int8_t)((uint32_t)(int32_t)x0 >> (8 * b));
-            qd[(b * AC_HEADS + r) * QLD + i1] = (int8_t)((uint32_t)(int32_t)x1 >> (8 * b));
+            qd[(b * AC_HEADS + r) * QLD + i0] = (int8_t)(d0 >> (8 * b));
+            qd[(b * AC_HEADS + r) * QLD + i1] = (int8_t)(d1 >> (8 * b));
         }
-        wide |= x0 != (int32_t)x0 || x1 != (int32_t)x1;
-        wide24 |= x0 < -(1 << 23) || x0 >= (1 << 23) || x1 < -(1 << 23) || x1 >= (1 << 23);
+        wide |= x0 < -0x80808080LL || x0 > 0x7F7F7F7FLL || x1 < -0x80808080LL || x1 > 0x7F7F7F7FLL;
     }
     if (wide) s_wide = 1;
-    if (wide24) s_q24 = 1;
     if (own) {                                                              // a 128-thread CTA: one value and at most one pair each
         bool bad = false;
         int32_t *kd = a.kcache + (long long)seq * a.seq_stride + ((long long)kv * a.Lmax + pos) * HD;
@@ -166,7 +202,7 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
         if (bad) atomicOr(a.flags, 4);
     }
     __syncthreads();
-    const bool use_wide = s_wide != 0, q_narrow = s_q24 == 0;
+    const bool use_wide = s_wide != 0;
 
     // ---- pass 1: scores of this warp's tiles, as 32-bit distances from a base per head: the first tile's maximum; a score more than 2^31
     //      above moves it and the distances so far, one more than 2^31 below is beyond every exponential's reach and stays at the edge ---
@@ -184,10 +220,25 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
         __syncwarp();
     };
     auto put = [&](int h, int local, long long score) {                    // local: key of the CTA
-        off[h * stride + local] = (int32_t)max(min(score - s_base[warp][h], (long long)INT32_MAX), (long long)INT32_MIN);
+        off[h * stride + local] = (int32_t)max(score - s_base[warp][h], (long long)INT32_MIN);      // (rows past the last hold anything)
     };
     int j = 0;
+    // key rows g and g + 8 of group i of sixteen (two per tile), dimensions 4t .. and 16 + 4t .. of every 32
+    auto key_rows = [&](int i, const int32_t *&ra, const int32_t *&rb) {
+        const int key = (first + warp + AC_WARPS * (i >> 1)) * AC_TILE + 16 * (i & 1) + g;
+        ra = kc + (long long)min(key, last) * HD + 4 * t; rb = kc + (long long)min(key + 8, last) * HD + 4 * t;
+    };
+    int4 k[HD / 32][4];                                                     // the group at hand; every step's place takes the next group's load
+    if (!use_wide && mine > 0) {
+        const int32_t *ra, *rb;
+        key_rows(0, ra, rb);
+#pragma unroll
+        for (int st = 0; st < HD / 32; st++) {
+            k[st][0] = ac_load(ra + 32 * st); k[st][1] = ac_load(rb + 32 * st); k[st][2] = ac_load(ra + 32 * st + 16); k[st][3] = ac_load(rb + 32 * st + 16);
+        }
+    }
     for (int tile = first + warp; tile < end; tile += AC_WARPS, j++) {
+        ahead(j + AC_AHEAD);
         const int left = n_keys - tile * AC_TILE, local0 = (tile - first) * AC_TILE;      // visible keys of the tile
         if (!use_wide) {
             long long sc[2][4];
@@ -196,48 +247,23 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
                 int acc[7][4];
 #pragma unroll
                 for (int i = 0; i < 7; i++) { acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0; }
-                const int key = tile * AC_TILE + 16 * mt + g;               // fragment rows g and g + 8
-                const int32_t *ra = kc + (long long)min(key, last) * HD + 4 * t, *rb = kc + (long long)min(key + 8, last) * HD + 4 * t;
-                int4 n0 = ac_load(ra), n1 = ac_load(rb), n2 = ac_load(ra + 16), n3 = ac_load(rb + 16);
-#pragma unroll 1
+                const int32_t *ra, *rb;
+                key_rows(min(2 * j + mt + 1, 2 * mine - 1), ra, rb);
+#pragma unroll
                 for (int st = 0; st < HD / 32; st++) {
-                    const int4 k0 = n0, k1 = n1, k2 = n2, k3 = n3;
-                    const int nx = min(st + 1, HD / 32 - 1) * 32;
-                    n0 = ac_load(ra + nx); n1 = ac_load(rb + nx); n2 = ac_load(ra + nx + 16); n3 = ac_load(rb + nx + 16);
+                    const int4 k0 = k[st][0], k1 = k[st][1], k2 = k[st][2], k3 = k[st][3];
+                    k[st][0] = ac_load(ra + 32 * st); k[st][1] = ac_load(rb + 32 * st); k[st][2] = ac_load(ra + 32 * st + 16); k[st][3] = ac_load(rb + 32 * st + 16);
                     uint32_t A0[4], A1[4], A2[4], A3[4];
                     ac_bytes(k0.x, k0.y, k0.z, k0.w, A0); ac_bytes(k1.x, k1.y, k1.z, k1.w, A1);
                     ac_bytes(k2.x, k2.y, k2.z, k2.w, A2); ac_bytes(k3.x, k3.y, k3.z, k3.w, A3);
-                    // keys and queries within [-2^23, 2^23): three byte planes each, the third signed (9 products instead of 16)
-                    auto fits = [](const int4 v) {
-                        return ((unsigned)(v.x + (1 << 23)) | (unsigned)(v.y + (1 << 23)) | (unsigned)(v.z + (1 << 23)) | (unsigned)(v.w + (1 << 23))) < (1u << 24);
-                    };
-                    const bool narrow = q_narrow && __all_sync(0xffffffffu, fits(k0) && fits(k1) && fits(k2) && fits(k3));
 #pragma unroll
                     for (int b = 0; b < 4; b++) {
-                        if (b == 3 && narrow) break;
                         const int8_t *qb = qd + (b * AC_HEADS + g) * QLD + 32 * st + 4 * t;
                         const uint32_t b0 = *reinterpret_cast<const uint32_t *>(qb), b1 = *reinterpret_cast<const uint32_t *>(qb + 16);
-                        if (narrow) {
-                            if (b < 2) {
-                                ac_mma<false, false>(acc[b], A0[0], A1[0], A2[0], A3[0], b0, b1);
-                                ac_mma<false, false>(acc[b + 1], A0[1], A1[1], A2[1], A3[1], b0, b1);
-                                ac_mma<true, false>(acc[b + 2], A0[2], A1[2], A2[2], A3[2], b0, b1);
-                            } else {
-                                ac_mma<false, true>(acc[b], A0[0], A1[0], A2[0], A3[0], b0, b1);
-                                ac_mma<false, true>(acc[b + 1], A0[1], A1[1], A2[1], A3[1], b0, b1);
-                                ac_mma<true, true>(acc[b + 2], A0[2], A1[2], A2[2], A3[2], b0, b1);
-                            }
-                        } else if (b < 3) {
-                            ac_mma<false, false>(acc[b], A0[0], A1[0], A2[0], A3[0], b0, b1);
-                            ac_mma<false, false>(acc[b + 1], A0[1], A1[1], A2[1], A3[1], b0, b1);
-                            ac_mma<false, false>(acc[b + 2], A0[2], A1[2], A2[2], A3[2], b0, b1);
-                            ac_mma<true, false>(acc[b + 3], A0[3], A1[3], A2[3], A3[3], b0, b1);
-                        } else {
-                            ac_mma<false, true>(acc[b], A0[0], A1[0], A2[0], A3[0], b0, b1);
-                            ac_mma<false, true>(acc[b + 1], A0[1], A1[1], A2[1], A3[1], b0, b1);
-                            ac_mma<false, true>(acc[b + 2], A0[2], A1[2], A2[2], A3[2], b0, b1);
-                            ac_mma<true, true>(acc[b + 3], A0[3], A1[3], A2[3], A3[3], b0, b1);
-                        }
+                        ac_mma<false>(acc[b], A0[0], A1[0], A2[0], A3[0], b0, b1);
+                        ac_mma<false>(acc[b + 1], A0[1], A1[1], A2[1], A3[1], b0, b1);
+                        ac_mma<false>(acc[b + 2], A0[2], A1[2], A2[2], A3[2], b0, b1);
+                        ac_mma<true>(acc[b + 3], A0[3], A1[3], A2[3], A3[3], b0, b1);
                     }
                 }
 #pragma unroll
@@ -313,6 +339,7 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
     m_all = max(m_all, __shfl_xor_sync(0xffffffffu, m_all, 16));
     const long long above = __shfl_sync(0xffffffffu, m_all, g) - s_base[warp][g];      // from here on a lane has head g, keys 8t .. 8t + 7 of a tile
     // ---- pass 2: exponentials over the scores, their sum --------------------------------------------------------------------------
+    const AcExp exp2(a.fa, a.log2e);
     unsigned long long z = 0;
     for (int tile = first + warp; tile < end; tile += AC_WARPS) {
         int4 *e4 = reinterpret_cast<int4 *>(off + g * stride + (tile - first) * AC_TILE + 8 * t);
@@ -321,8 +348,7 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
         int e[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const long long d = min(above - e[i], a.clip);
-            const int v = (int)exp2_neg_fixed((d * a.log2e) >> a.fa, a.fa);
+            const int v = exp2((uint32_t)min(above - e[i], a.clip));
             e[i] = i < left && g < rep ? v : 0;
             z += (unsigned)e[i];
         }
@@ -337,29 +363,39 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
     z_all += __shfl_xor_sync(0xffffffffu, z_all, 8);
     z_all += __shfl_xor_sync(0xffffffffu, z_all, 16);
     z = __shfl_sync(0xffffffffu, z_all, g);
-    const unsigned long long inv = recip_below(z);
+    // floor((e << fa) / z) = e M >> s with s = 61 + l - fa for z of l + 1 bits and M up to 2^11 above 2^(fa + s) / z: e 2^11 z < 2^s as fa <= 23
+    const int l = 63 - __clzll((long long)z), post = 30 + l - a.fa;
+    const uint64_t mul = (uint64_t)(21267647932558653966460912964485513216.0 / (double)(z << (63 - l))) + 1024;      // 2^124
+    const uint32_t mh = g < rep ? (uint32_t)(mul >> 31) : 0u, ml = g < rep ? (uint32_t)(mul & 0x7FFFFFFF) : 0u;
     // ---- pass 3: probabilities floor(e 2^fa / z) as bytes, times the values --------------------------------------------------------
     long long sum[HD / 8][2];
 #pragma unroll
     for (int i = 0; i < HD / 8; i++) sum[i][0] = sum[i][1] = 0;
     int f8 = 1 << 8, f16 = 1 << 16, f24 = 1 << 24;                          // weights of the value bytes: factors of wide multiply-adds
     asm volatile("" : "+r"(f8), "+r"(f16), "+r"(f24));
-    for (int tile = first + warp; tile < end; tile += AC_WARPS) {
-        int4 v[8];                                                          // keys 8t .. 8t + 7 (steps 4t + i and 16 + 4t + i), dimensions 4g ..
-        const int32_t *vt = vc + 4 * g;
-        int vrow[8];
+    int4 v[8];                                                              // keys 8t .. 8t + 7 (steps 4t + i and 16 + 4t + i), dimensions 4g .. of 32
+    auto value_rows = [&](int tile, int ch) {
+        const int row = tile * AC_TILE + 8 * t;
+        const int32_t *at = vc + (long long)row * HD + 4 * g + 32 * ch;
+        if (tile + 1 < n_tiles) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) { vrow[i] = min(tile * AC_TILE + 8 * t + i, last) * HD; v[i] = ac_load(vt + vrow[i]); }
+            for (int i = 0; i < 8; i++) v[i] = ac_load(at + i * HD);
+        } else {                                                            // rows past the last read as it
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = ac_load(at + (long long)(min(row + i, last) - row) * HD);
+        }
+    };
+    if (mine > 0) value_rows(first + warp, 0);
+    j = 0;
+    for (int tile = first + warp; tile < end; tile += AC_WARPS, j++) {
+        ahead(mine + j + AC_AHEAD);
         const int4 *e4 = reinterpret_cast<const int4 *>(off + g * stride + (tile - first) * AC_TILE + 8 * t);
         const int4 lo4 = e4[0], hi4 = e4[1];
         uint32_t p[8] = {(uint32_t)lo4.x, (uint32_t)lo4.y, (uint32_t)lo4.z, (uint32_t)lo4.w, (uint32_t)hi4.x, (uint32_t)hi4.y, (uint32_t)hi4.z, (uint32_t)hi4.w};
         uint32_t any = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const unsigned long long n = (unsigned long long)p[i] << a.fa;
-            unsigned long long q = __umul64hi(n, inv), r = n - q * z;
-            if (z) while (r >= z) { q++; r -= z; }
-            p[i] = z ? (uint32_t)q : 0u;
+            p[i] = (uint32_t)(((uint64_t)p[i] * mh + (((uint64_t)p[i] * ml) >> 31)) >> post);
             any |= p[i];
         }
         uint32_t P0[4], P1[4];
@@ -372,18 +408,16 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
             ac_bytes(v[0].y, v[1].y, v[2].y, v[3].y, B0[1]); ac_bytes(v[4].y, v[5].y, v[6].y, v[7].y, B1[1]);
             ac_bytes(v[0].z, v[1].z, v[2].z, v[3].z, B0[2]); ac_bytes(v[4].z, v[5].z, v[6].z, v[7].z, B1[2]);
             ac_bytes(v[0].w, v[1].w, v[2].w, v[3].w, B0[3]); ac_bytes(v[4].w, v[5].w, v[6].w, v[7].w, B1[3]);
-            if (ch + 1 < HD / 32) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = ac_load(vt + vrow[i] + 32 * (ch + 1));
-            }
+            if (ch + 1 < HD / 32) value_rows(tile, ch + 1);
+            else value_rows(min(tile + AC_WARPS, end - 1), 0);
 #pragma unroll
             for (int n = 0; n < 4; n++) {
                 int u[4][2];
 #pragma unroll
                 for (int b = 0; b < 4; b++) {
-                    int c[4] = {0, 0, 0, 0};
-                    if (b < 3) ac_mma<false, false>(c, P0[0], P0[1], P1[0], P1[1], B0[n][b], B1[n][b]);
-                    else ac_mma<false, true>(c, P0[0], P0[1], P1[0], P1[1], B0[n][b], B1[n][b]);
+                    int c[4];
+                    if (b < 3) ac_mma_first<false>(c, P0[0], P0[1], P1[0], P1[1], B0[n][b], B1[n][b]);
+                    else ac_mma_first<true>(c, P0[0], P0[1], P1[0], P1[1], B0[n][b], B1[n][b]);
                     u[b][0] = c[2] * 256 + c[0]; u[b][1] = c[3] * 256 + c[1];
                 }
 #pragma unroll
@@ -392,9 +426,9 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
                 if (third) {                                                // a probability of 2^16 and more (2^fa at most)
 #pragma unroll
                     for (int b = 0; b < 4; b++) {
-                        int c[4] = {0, 0, 0, 0};
-                        if (b < 3) ac_mma<false, false>(c, P0[2], 0u, P1[2], 0u, B0[n][b], B1[n][b]);
-                        else ac_mma<false, true>(c, P0[2], 0u, P1[2], 0u, B0[n][b], B1[n][b]);
+                        int c[4];
+                        if (b < 3) ac_mma_first<false>(c, P0[2], 0u, P1[2], 0u, B0[n][b], B1[n][b]);
+                        else ac_mma_first<true>(c, P0[2], 0u, P1[2], 0u, B0[n][b], B1[n][b]);
                         sum[4 * ch + n][0] += (long long)c[0] << (16 + 8 * b); sum[4 * ch + n][1] += (long long)c[1] << (16 + 8 * b);
                     }
                 }
@@ -403,12 +437,12 @@ __global__ void __launch_bounds__(AC_THREADS, 3) attn_cluster_kernel(const AttnA
     }
     // ---- the warps' sums over scores and queries, then one CTA's, then the cluster's: a CTA reads out its share of the heads ----------
     __syncthreads();
-    unsigned long long *mine = reinterpret_cast<unsigned long long *>(ac_sm) + (size_t)warp * AC_HEADS * HD;           // [8][HD]
+    unsigned long long *warp_sum = reinterpret_cast<unsigned long long *>(ac_sm) + (size_t)warp * AC_HEADS * HD;           // [8][HD]
 #pragma unroll
     for (int ch = 0; ch < HD / 32; ch++)
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            longlong2 *to = reinterpret_cast<longlong2 *>(mine + g * HD + 32 * ch + 8 * t + 4 * i);
+            longlong2 *to = reinterpret_cast<longlong2 *>(warp_sum + g * HD + 32 * ch + 8 * t + 4 * i);
             to[0] = make_longlong2(sum[4 * ch][i], sum[4 * ch + 1][i]); to[1] = make_longlong2(sum[4 * ch + 2][i], sum[4 * ch + 3][i]);
         }
     __syncthreads();
@@ -473,11 +507,11 @@ bool attn_cluster_plan(const AttnArgs &a, int &n_c, int &tiles) {
     const long long nt = (n_keys + AC_TILE - 1) / AC_TILE, pairs = (long long)a.Hkv * std::max(1, a.batch);
     if (nt > (long long)AC_MAX_TILES * AC_MAX_CLUSTER) return false;
     const int least = (int)((nt + AC_MAX_TILES - 1) / AC_MAX_TILES), most = (int)std::min<long long>(AC_MAX_CLUSTER, (nt + AC_WARPS - 1) / AC_WARPS);
-    // as few rounds of a warp per CTA as the cluster allows; with three CTAs per SM and more at hand, the cluster whose rounds are fullest
+    // as few rounds of a warp per CTA as the cluster allows; with two CTAs per SM and more at hand, the cluster whose rounds are fullest
     long long cost = 0;
     n_c = 0;
     for (int c = std::max(1, least); c <= std::max(1, std::max(least, most)); c++) {
-        const long long rounds = ((nt + c - 1) / c + AC_WARPS - 1) / AC_WARPS, waves = (pairs * c + 3 * 148 - 1) / (3 * 148);
+        const long long rounds = ((nt + c - 1) / c + AC_WARPS - 1) / AC_WARPS, waves = (pairs * c + 2 * 148 - 1) / (2 * 148);
         const long long now = waves * (rounds + 3);                        // a CTA's start, exchanges and read-out cost about three rounds
         if (n_c == 0 || now < cost) { n_c = c; cost = now; }
     }
