@@ -27,6 +27,7 @@
 #include "layout.cuh"
 #include "mma_items.cuh"
 #include "norm.cuh"
+#include "softmax.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -889,6 +890,7 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
     if (tid < rep && s_max[tid] != INT64_MIN) atomicMax(a.hmax + kv * rep + tid, s_max[tid]);
     if (!af_group_barrier(a.ticket + 1 + kv, gridDim.x)) s_timeout = 1;
     // ---- pass 2: exponentials into shared memory and their sums ------------------------------------------------------------
+    const SoftmaxExp exp2(a.fa, a.log2e, a.clip);
     unsigned long long zloc = 0ULL;
     const long long hm = head < rep ? __ldcg(a.hmax + kv * rep + head) : 0;
 #pragma unroll
@@ -897,9 +899,7 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
         if (i >= nk * AF_HEADS) continue;
         unsigned e = 0;
         if (head < rep) {
-            long long dlt = hm - sc[u];
-            dlt = dlt < a.clip ? dlt : a.clip;
-            e = (unsigned)exp2_neg_fixed((dlt * a.log2e) >> a.fa, a.fa);
+            e = (unsigned)exp2(hm - sc[u]);
             zloc += e;
         }
         s_e[i] = e;
@@ -914,19 +914,11 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
     //      out[head][dim] = sum over keys p[key][head] v[key][dim]: A = bytes of p (heads x keys; p <= 2^fa has three unsigned
     //      bytes), B = bytes of v gathered from four key rows (keys x dims), a warp owns eight dimensions for all keys
     const int nk32 = (nk + 31) & ~31;
-    // a thread's pairs all belong to head tid % 8: one reciprocal of that head's normaliser, then floor(e 2^fa / z) per pair
-    // as a high product with an exact fix-up instead of a 64-bit division each
-    const unsigned long long z_own = head < rep ? __ldcg(a.Z + kv * rep + head) : 0ULL;
-    const unsigned long long z_inv = recip_below(z_own);
+    // a thread's pairs all belong to head tid % 8: one reciprocal of that head's normaliser
+    const SoftmaxQuotient quotient(head < rep ? __ldcg(a.Z + kv * rep + head) : 0ULL, a.fa);
     for (int idx = tid; idx < nk32 * AF_HEADS; idx += AF_THREADS) {
         const int key = idx >> 3, h = idx & (AF_HEADS - 1);
-        unsigned p = 0;
-        if (key < nk && z_own) {
-            const unsigned long long n = (unsigned long long)s_e[idx] << a.fa;
-            unsigned long long q = __umul64hi(n, z_inv), r = n - q * z_own;
-            while (r >= z_own) { q++; r -= z_own; }
-            p = (unsigned)q;
-        }
+        const unsigned p = key < nk ? quotient(s_e[idx]) : 0u;
         // position of the key inside its 32-key step: keys 8t + 4u + j sit at 16u + 4t + j, so that the four rows a lane
         // gathers for one step come from four different groups of the value rows
         const int kpos = (key & ~31) | ((key & 4) << 2) | ((key & 24) >> 1) | (key & 3);

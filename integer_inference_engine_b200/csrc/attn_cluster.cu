@@ -21,6 +21,7 @@
 #include "kernels.h"
 #include "mma_items.cuh"
 #include "norm.cuh"
+#include "softmax.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -71,22 +72,6 @@ __device__ __forceinline__ void ac_mma_first(int (&c)[4], uint32_t a0, uint32_t 
         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
-
-// exp2_neg_fixed of (d log2e) >> fa for 0 <= d <= clip and fa <= 23: every operand fits 32 bits
-struct AcExp {
-    uint32_t c0 = 65536, c1 = 45426, c2 = 15743, c3 = 3638, log2e;
-    int fa;
-    __device__ __forceinline__ AcExp(int fa_, long long log2e_) : log2e((uint32_t)log2e_), fa(fa_) {
-        const int s = 16 - fa;
-        if (s >= 0) { c0 >>= s; c1 >>= s; c2 >>= s; c3 >>= s; } else { c0 <<= -s; c1 <<= -s; c2 <<= -s; c3 <<= -s; }
-    }
-    __device__ __forceinline__ uint32_t mul(uint32_t x, uint32_t y) const { return (uint32_t)(((uint64_t)x * y) >> fa); }
-    __device__ __forceinline__ int operator()(uint32_t d) const {
-        const uint32_t u = mul(d, log2e), f = u & ((1u << fa) - 1), f2 = mul(f, f), f3 = mul(f2, f);
-        const int p = (int)(c0 - mul(c1, f) + mul(c2, f2) - mul(c3, f3));
-        return max(p, 0) >> (u >> fa);
-    }
-};
 
 __device__ __forceinline__ void ac_rotate(const AttnArgs &a, long long pos, int i, int64_t &x0, int64_t &x1) {
     if (!a.rope) return;
@@ -339,7 +324,7 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
     m_all = max(m_all, __shfl_xor_sync(0xffffffffu, m_all, 16));
     const long long above = __shfl_sync(0xffffffffu, m_all, g) - s_base[warp][g];      // from here on a lane has head g, keys 8t .. 8t + 7 of a tile
     // ---- pass 2: exponentials over the scores, their sum --------------------------------------------------------------------------
-    const AcExp exp2(a.fa, a.log2e);
+    const SoftmaxExp exp2(a.fa, a.log2e, a.clip);
     unsigned long long z = 0;
     for (int tile = first + warp; tile < end; tile += AC_WARPS) {
         int4 *e4 = reinterpret_cast<int4 *>(off + g * stride + (tile - first) * AC_TILE + 8 * t);
@@ -348,7 +333,7 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
         int e[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const int v = exp2((uint32_t)min(above - e[i], a.clip));
+            const int v = exp2(above - e[i]);
             e[i] = i < left && g < rep ? v : 0;
             z += (unsigned)e[i];
         }
@@ -363,10 +348,7 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
     z_all += __shfl_xor_sync(0xffffffffu, z_all, 8);
     z_all += __shfl_xor_sync(0xffffffffu, z_all, 16);
     z = __shfl_sync(0xffffffffu, z_all, g);
-    // floor((e << fa) / z) = e M >> s with s = 61 + l - fa for z of l + 1 bits and M up to 2^11 above 2^(fa + s) / z: e 2^11 z < 2^s as fa <= 23
-    const int l = 63 - __clzll((long long)z), post = 30 + l - a.fa;
-    const uint64_t mul = (uint64_t)(21267647932558653966460912964485513216.0 / (double)(z << (63 - l))) + 1024;      // 2^124
-    const uint32_t mh = g < rep ? (uint32_t)(mul >> 31) : 0u, ml = g < rep ? (uint32_t)(mul & 0x7FFFFFFF) : 0u;
+    const SoftmaxQuotient quotient(g < rep ? z : 0, a.fa);
     // ---- pass 3: probabilities floor(e 2^fa / z) as bytes, times the values --------------------------------------------------------
     long long sum[HD / 8][2];
 #pragma unroll
@@ -395,7 +377,7 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
         uint32_t any = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            p[i] = (uint32_t)(((uint64_t)p[i] * mh + (((uint64_t)p[i] * ml) >> 31)) >> post);
+            p[i] = quotient(p[i]);
             any |= p[i];
         }
         uint32_t P0[4], P1[4];

@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "softmax.cuh"
 #include "kernels.h"
 
 namespace iie {
@@ -78,6 +79,14 @@ __device__ __forceinline__ Tile pt_tile(const AttnArgs &a, long long tile) {
     return t;
 }
 __device__ __forceinline__ long long pt_lo(const AttnArgs &a, long long pos) { return (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0; }
+
+// Scores lie as 32-bit words in the place of the exponentials; one that does not fit leaves INT32_MIN there and stands in the 64-bit
+// scratch instead (half the traffic of 64-bit scores, which nothing in practice needs).
+__device__ __forceinline__ int32_t pt_score(const AttnArgs &a, long long at, long long score) {
+    const bool fits = score > INT32_MIN && score <= INT32_MAX;
+    if (!fits) a.scores[at] = score;
+    return fits ? (int32_t)score : INT32_MIN;
+}
 
 // ---- pass 1: scores[token][head][key] and the row maxima ----------------------------------------------------------------
 // grid (walks, Hkv, tiles): CTA x walks PT_WALK chunks of the tile's key span.  16 warps = 4 key tiles x 4 groups of four
@@ -154,7 +163,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_tile_scores_kernel(const A
                 long long dot = 0;
                 for (int j = 0; j < HD; j++) dot += q64[col * HD + j] * (long long)kk[j];
                 const long long sc = ((dot >> a.fa) * a.inv_sqrt) >> a.fa;
-                a.scores[((T.t0 + qi) * a.H + kv * rep + h) * Ls + l] = sc;
+                { const long long at = ((T.t0 + qi) * a.H + kv * rep + h) * Ls + l; a.e[at] = pt_score(a, at, sc); }
                 atomicMax(&s_max[col], sc);
             }
         }
@@ -246,7 +255,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_tile_scores_kernel(const A
                     const int h = 2 * t + (i & 1);
                     if (qi < T.nq && h < rep && l <= pos_q && l >= lo_q) {
                         const long long sc = ((dot >> a.fa) * a.inv_sqrt) >> a.fa;
-                        a.scores[((T.t0 + qi) * a.H + kv * rep + h) * Ls + l] = sc;
+                        { const long long at = ((T.t0 + qi) * a.H + kv * rep + h) * Ls + l; a.e[at] = pt_score(a, at, sc); }
                         m2[i & 1] = max(m2[i & 1], sc);
                     }
                 }
@@ -266,49 +275,41 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_tile_scores_kernel(const A
 }
 
 // ---- pass 2: exponentials, their sum and the probabilities, one warp per (token, head) row ----------------------------------
-// e_l = 2^-((min(max - score_l, clip) * log2e) >> fa) for the visible keys of the row, two keys per lane and step; the row
-// belongs to this warp, so its normaliser Z needs no atomics and the same lanes turn their e_l into p_l = (e_l << fa) / Z in
-// place (through the reciprocal of Z with an exact fix-up: the estimate is at most 2 low).
+// e_l = 2^-((min(max - score_l, clip) * log2e) >> fa) for the visible keys of the row, in place of the scores, four keys per lane and
+// step; the row belongs to this warp, so its normaliser Z needs no atomics and the same lanes turn their e_l into p_l = (e_l << fa) / Z.
+// Bounded by instructions (about 30 per key) and the eight bytes per key in and out: 2048 tokens x 32 heads 189 us, with 64-bit
+// scores and 64-bit exponentials and quotients 300.
 __global__ void __launch_bounds__(256) attn_tile_exp_kernel(const AttnArgs a) {
     const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5), n_rows = (long long)a.batch * a.H;
     if (row >= n_rows) return;
     const int lane = threadIdx.x & 31;
     const long long tok = row / a.H, pos = a.pos + tok, lo = pt_lo(a, pos), Ls = a.Ls ? a.Ls : a.Lmax;
-    const int64_t *sc = a.scores + row * Ls;
+    const int64_t *far = a.scores + row * Ls;
     int32_t *e = a.e + row * Ls;
     const long long m = a.hmax[row];
+    const SoftmaxExp exp2(a.fa, a.log2e, a.clip);
     unsigned long long sum = 0;
-    for (long long l = (lo & ~1LL) + 2 * lane; l <= pos; l += 64) {
-        const longlong2 s2 = *reinterpret_cast<const longlong2 *>(sc + l);
-        int2 e2 = make_int2(0, 0);
-        if (l >= lo) {
-            long long d = m - s2.x;
-            d = d < a.clip ? d : a.clip;
-            e2.x = (int)exp2_neg_fixed((d * a.log2e) >> a.fa, a.fa);
+    for (long long l = (lo & ~3LL) + 4 * lane; l <= pos; l += 128) {
+        const int4 s4 = *reinterpret_cast<const int4 *>(e + l);
+        int v[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const bool seen = l + k >= lo && l + k <= pos;
+            long long d = m - v[k];
+            if (v[k] == INT32_MIN && seen) d = m - far[l + k];
+            v[k] = seen ? exp2(d) : 0;
+            sum += (unsigned)v[k];
         }
-        if (l + 1 <= pos) {
-            long long d = m - s2.y;
-            d = d < a.clip ? d : a.clip;
-            e2.y = (int)exp2_neg_fixed((d * a.log2e) >> a.fa, a.fa);
-        }
-        sum += (unsigned long long)(unsigned)e2.x + (unsigned long long)(unsigned)e2.y;
-        *reinterpret_cast<int2 *>(e + l) = e2;
+        *reinterpret_cast<int4 *>(e + l) = make_int4(v[0], v[1], v[2], v[3]);
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
     if (lane == 0) a.Z[row] = sum;
-    if (sum == 0) return;                                          // (cannot happen: the row maximum has e = 2^fa)
-    const unsigned long long inv = 0xFFFFFFFFFFFFFFFFULL / sum;
-    auto prob = [&](int ev) {
-        const unsigned long long n = (unsigned long long)(unsigned)ev << a.fa;
-        unsigned long long q = __umul64hi(n, inv), r = n - q * sum;
-        while (r >= sum) { q++; r -= sum; }
-        return (int)q;
-    };
-    for (long long l = (lo & ~1LL) + 2 * lane; l <= pos; l += 64) {
-        int2 e2 = *reinterpret_cast<int2 *>(e + l);               // this lane's own stores
-        e2.x = prob(e2.x); e2.y = prob(e2.y);
-        *reinterpret_cast<int2 *>(e + l) = e2;
+    const SoftmaxQuotient quotient(sum, a.fa);
+    for (long long l = (lo & ~3LL) + 4 * lane; l <= pos; l += 128) {
+        int4 *at = reinterpret_cast<int4 *>(e + l);                // this lane's own stores
+        const int4 v = *at;
+        *at = make_int4((int)quotient((uint32_t)v.x), (int)quotient((uint32_t)v.y), (int)quotient((uint32_t)v.z), (int)quotient((uint32_t)v.w));
     }
 }
 
@@ -648,7 +649,7 @@ __global__ void __launch_bounds__(PC_THREADS, 1) attn_tile_pv_tc_kernel(const At
 // every accumulator of a chunk without accumulation.  The accumulators are single-buffered: the issuer waits until the
 // previous chunk has been read out, the producers are already a chunk ahead.  grid (walks, Hkv, tiles).
 constexpr int SC_WALK = 8, SC_STAGES = 2;
-constexpr int SC_SLD = PT_CH + 2;           // row stride (int64) of the staged scores: 16-byte rows, lanes spread over the banks
+constexpr int SC_SLD = PT_CH + 4;           // row stride (int32) of the staged scores: 16-byte rows, lanes spread over the banks
 
 // every producer thread learns whether all of them got through their waits (a named barrier with an AND reduction): the
 // warps leave the chunk loop together, so none is left waiting at the plain barriers of the write-out
@@ -677,7 +678,7 @@ __global__ void __launch_bounds__(PC_THREADS, 1) attn_tile_scores_tc_kernel(cons
     const int n_chunks = (int)min((long long)SC_WALK, T.pos_last / PT_CH - c_first + 1);
     unsigned char *qd = smem;                                      // query byte planes [4][HD / 16][16 row groups][8 x 16 B]
     unsigned char *kd = qd + 4 * Q_PLANE;                          // key byte planes [2 stages][4][HD / 16][8 key groups][8 x 16 B]
-    long long *sbuf = reinterpret_cast<long long *>(kd + SC_STAGES * K_STAGE);      // a chunk's scores [128 rows][SC_SLD] on their way out
+    int32_t *sbuf = reinterpret_cast<int32_t *>(kd + SC_STAGES * K_STAGE);      // a chunk's scores [128 rows][SC_SLD] on their way out
     if (tid == 0) {
         s_abort = 0; s_wide = 0; s_qwide24 = 0;
         for (int s = 0; s < SC_STAGES; s++) {
@@ -763,7 +764,7 @@ __global__ void __launch_bounds__(PC_THREADS, 1) attn_tile_scores_tc_kernel(cons
                 long long dot = 0;
                 for (int j = 0; j < HD; j++) dot += q64[row * HD + j] * (long long)kk[j];
                 const long long sc = ((dot >> a.fa) * a.inv_sqrt) >> a.fa;
-                a.scores[((T.t0 + qi) * a.H + kv * rep + h) * Ls + l] = sc;
+                { const long long at = ((T.t0 + qi) * a.H + kv * rep + h) * Ls + l; a.e[at] = pt_score(a, at, sc); }
                 atomicMax(&s_max[row], sc);
             }
         }
@@ -828,21 +829,28 @@ __global__ void __launch_bounds__(PC_THREADS, 1) attn_tile_scores_tc_kernel(cons
                     sv[j] = ((dot >> a.fa) * a.inv_sqrt) >> a.fa;
                     if (row_ok && l <= pos_q && l >= lo_q) mloc = max(mloc, sv[j]);
                 }
-                longlong2 *dst = reinterpret_cast<longlong2 *>(sbuf + row * SC_SLD + cg * 16 + half * 8);
+                int32_t s32[8];
+                bool out = false;
 #pragma unroll
-                for (int j = 0; j < 4; j++) dst[j] = make_longlong2(sv[2 * j], sv[2 * j + 1]);
+                for (int j = 0; j < 8; j++) { s32[j] = (int32_t)sv[j]; out = out || sv[j] <= INT32_MIN || sv[j] > INT32_MAX; }
+                if (out && row_ok) {
+#pragma unroll
+                    for (int j = 0; j < 8; j++) s32[j] = pt_score(a, ((T.t0 + qi) * a.H + kv * rep + h) * Ls + l0 + half * 8 + j, sv[j]);
+                }
+                int4 *dst = reinterpret_cast<int4 *>(sbuf + row * SC_SLD + cg * 16 + half * 8);
+                dst[0] = make_int4(s32[0], s32[1], s32[2], s32[3]); dst[1] = make_int4(s32[4], s32[5], s32[6], s32[7]);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(pc_u32(&free_bar)) : "memory");
-            // the chunk's scores leave through shared memory so that a warp writes whole 512-byte rows (entries of keys a token
+            // the chunk's scores leave through shared memory so that a warp writes whole 256-byte rows (entries of keys a token
             // does not see are written too: they lie inside its row of the scratch and are never read)
             asm volatile("bar.sync 1, %0;" ::"r"(PC_PRODUCERS) : "memory");
             for (int rr = warp; rr < PT_COLS; rr += PC_PRODUCERS / 32) {
                 const int q2 = rr >> 3, h2 = rr & 7;
                 if (q2 < T.nq && h2 < rep)
-                    *reinterpret_cast<longlong2 *>(a.scores + ((T.t0 + q2) * a.H + kv * rep + h2) * Ls + lc + 2 * lane) =
-                        *reinterpret_cast<const longlong2 *>(sbuf + rr * SC_SLD + 2 * lane);
+                    *reinterpret_cast<int2 *>(a.e + ((T.t0 + q2) * a.H + kv * rep + h2) * Ls + lc + 2 * lane) =
+                        *reinterpret_cast<const int2 *>(sbuf + rr * SC_SLD + 2 * lane);
             }
             asm volatile("bar.sync 1, %0;" ::"r"(PC_PRODUCERS) : "memory");
         }
@@ -927,7 +935,7 @@ cudaError_t pv_launch(const AttnArgs &a, unsigned tiles, cudaStream_t s) {
 
 template <int HD>
 cudaError_t scores_tc_launch(const AttnArgs &a, unsigned walks, unsigned tiles, cudaStream_t s) {
-    constexpr size_t smem = (size_t)4 * PT_COLS * HD + (size_t)SC_STAGES * 4 * PT_CH * HD + (size_t)PT_COLS * SC_SLD * 8 + 1024;
+    constexpr size_t smem = (size_t)4 * PT_COLS * HD + (size_t)SC_STAGES * 4 * PT_CH * HD + (size_t)PT_COLS * SC_SLD * 4 + 1024;
     static_assert(smem - 1024 >= (size_t)PT_COLS * HD * 8, "the int64 queries of the scalar path overlay the byte planes");
     static bool configured = false;
     if (!configured) {
