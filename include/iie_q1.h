@@ -148,6 +148,10 @@ int iie_q1_decode_layer_dev(long long wqkv, long long wo, long long w1u, long lo
 int iie_q1_embed_dev(long long handle, const int *row_dev, long long row, int64_t *out_dev, void *stream);
 /* Kept for its callers: the single-token product has one launch form, whose weights come by bulk copies. */
 void iie_q1_set_stream(int on);
+/* Page-locked host memory for results, from a pool of at most 64 MB (NULL when that is in use or nothing can be locked: use
+ * pageable memory then); give it back when nobody reads it any more.  Safe with several threads. */
+void *iie_host_take(unsigned long long bytes);
+void iie_host_give(void *p);
 /* Changes whenever a scratch buffer of the Q1_0 entries is freed (to grow, or by bonsai_q1_free_weights): a CUDA graph
  * captured over iie_q1_*_dev calls holds the old addresses and must be captured again. */
 unsigned long long iie_q1_workspace_generation(void);

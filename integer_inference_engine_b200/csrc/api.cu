@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
+#include <initializer_list>
 
 #include <algorithm>
 #include <map>
@@ -120,6 +121,45 @@ bool d2h(void *dst, const void *src, size_t n) {
 }
 bool sync() { return cudaStreamSynchronize(g_stream) == cudaSuccess; }
 
+// Page-locked staging of the host-array entries: a copy from or to pageable memory costs the driver 5 us and more of its own
+// staging and a wait.  One upload and one download per call (the entries hold the lock and end synchronised); larger arrays go direct.
+constexpr size_t PIN_IN = 1 << 20, PIN_OUT = 4 << 20;
+uint8_t *g_pin = nullptr;
+bool pinned() {
+    static bool tried = false;
+    if (!tried) { tried = true; if (cudaHostAlloc(&g_pin, PIN_IN + PIN_OUT, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); g_pin = nullptr; } }
+    return g_pin != nullptr;
+}
+bool upload(void *dst, const void *src, size_t n) {
+    if (n > PIN_IN || !pinned()) return h2d(dst, src, n);
+    memcpy(g_pin, src, n);
+    return h2d(dst, g_pin, n);
+}
+struct Download { void *dst; const void *src; size_t n; };
+// the flag word (cleared where it was set) and the results, behind one wait; -1 on failure
+int download(std::initializer_list<Download> list) {
+    size_t total = 64;
+    for (const Download &d : list) total += (d.n + 63) & ~(size_t)63;
+    int f = 0;
+    const bool staged = total <= PIN_OUT && pinned();
+    int *fp = staged ? (int *)(g_pin + PIN_IN) : &f;
+    if (cudaMemcpyAsync(fp, g_flags, sizeof(int), cudaMemcpyDeviceToHost, g_stream) != cudaSuccess) return -1;
+    size_t at = 64;
+    for (const Download &d : list) {
+        if (d.n && !d2h(staged ? g_pin + PIN_IN + at : d.dst, d.src, d.n)) return -1;
+        at += (d.n + 63) & ~(size_t)63;
+    }
+    if (!sync()) return -1;
+    f = *fp;
+    at = 64;
+    for (const Download &d : list) {
+        if (staged && d.n) memcpy(d.dst, g_pin + PIN_IN + at, d.n);
+        at += (d.n + 63) & ~(size_t)63;
+    }
+    if (f && cudaMemsetAsync(g_flags, 0, sizeof(int), g_stream) != cudaSuccess) return -1;
+    return f;
+}
+
 bool valid_q(long long h) { return h >= 0 && (size_t)h < g_w.size() && g_w[h].live && g_w[h].qtype != QT_I64; }
 bool valid_i64(long long h) { return h >= 0 && (size_t)h < g_w.size() && g_w[h].live && g_w[h].qtype == QT_I64; }
 
@@ -206,7 +246,7 @@ bool tiles(int qtype, int mode, TileArgs a, cudaStream_t s) {
 // y[T,out_f] on device from x[T,K] on device.  check_flags: synchronise and re-run the exact kernel
 // if an activation left the limb envelope (host-pointer entries); otherwise flags stay raised.
 bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t *out, bool check_flags, cudaStream_t s,
-                const int8_t *xl_ready = nullptr, const int *nl_ready = nullptr) {
+                const int8_t *xl_ready = nullptr, const int *nl_ready = nullptr, bool early = false) {
     const long long K = w.nb * 256;
     if (!fast_envelope(w.qtype, w.nb, w.maxd, w.maxdmin, fw))
         return launch_exact_linear((const uint8_t *)w.d, w.qtype, w.out_f, w.nb, x, T, fw, out, s) == cudaSuccess;
@@ -237,7 +277,7 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
         StreamArgs sa = {};
         sa.wa = w.cell; sa.wb = w.cell; sa.n_sel = 1; sa.out_f = w.out_f; sa.n_blocks = w.nb; sa.fw = fw; sa.fa = 16;
         sa.xl = xl; sa.x_per_sel = 0; sa.x_nl = nullptr; sa.out = out; sa.flags = g_flags;
-        sa.fast = small_scales(w.maxd, w.maxdmin, fw); sa.pdl = 0;
+        sa.fast = small_scales(w.maxd, w.maxdmin, fw); sa.pdl = sa.early_weights = early && g_pdl ? 1 : 0;      // early: weights asked for while the kernel before runs
         if (launch_stream(w.qtype, MODE_LINEAR, sa, s) != cudaSuccess) return false;
     } else if (T >= 2 && T < (1 << 20) && g_stage_mask == 0) {
         // a few rows: one group that owns all of them, every tile streamed once
@@ -633,23 +673,26 @@ extern "C" int qk_apply_resident_grouped(const long long *handles, const int *ph
     const long long K = nb * 256;
     int64_t *xd = (int64_t *)ensure(R_X, (size_t)T * K * 8), *od = (int64_t *)ensure(R_OUT, (size_t)total * 8);
     int8_t *xl = (int8_t *)ensure(R_XL, (size_t)T * 8 * K);
-    if (!xd || !od || !xl || !h2d(xd, x, (size_t)T * K * 8) || cudaMemsetAsync(g_cells + 4, 0, sizeof(int), g_stream) != cudaSuccess ||
-        launch_limbs(xd, T, K, xl, g_flags, g_stream, g_cells + 4) != cudaSuccess) { cudaGetLastError(); return 1; }
-    const int f0 = read_flags_clear();
-    if (f0 < 0) return 1;
-    long long off = 0;
-    for (int i = 0; i < count; i++) {
-        const Weight &w = g_w[handles[i]];
-        const int phase = phase_ids ? phase_ids[i] : 0;
-        static const int calls[5] = {PM_OTHER_CALLS, PM_Q_CALLS, PM_K_CALLS, PM_V_CALLS, PM_O_CALLS};
-        prof(calls[phase >= 0 && phase <= 4 ? phase : 0]);
-        bool ok;
-        if (f0 & 1) ok = launch_exact_linear((const uint8_t *)w.d, w.qtype, w.out_f, w.nb, xd, T, fw, od + off, g_stream) == cudaSuccess;
-        else ok = linear_dev(w, xd, T, fw, od + off, false, g_stream, xl, T > 1 ? g_cells + 4 : nullptr);
-        if (!ok) { cudaGetLastError(); return 1; }
-        off += T * w.out_f;
+    int *nl = T > 1 ? g_cells + 4 : nullptr;
+    if (!xd || !od || !xl || !upload(xd, x, (size_t)T * K * 8) || (nl && cudaMemsetAsync(nl, 0, sizeof(int), g_stream) != cudaSuccess) ||
+        launch_limbs(xd, T, K, xl, g_flags, g_stream, nl) != cudaSuccess) { cudaGetLastError(); return 1; }
+    // the products do not wait for the verdict on the digits: an activation beyond them repeats the call with the exact kernel
+    for (int exact = 0; exact < 2; exact++) {
+        long long off = 0;
+        for (int i = 0; i < count; i++) {
+            const Weight &w = g_w[handles[i]];
+            const int phase = phase_ids ? phase_ids[i] : 0;
+            static const int calls[5] = {PM_OTHER_CALLS, PM_Q_CALLS, PM_K_CALLS, PM_V_CALLS, PM_O_CALLS};
+            if (!exact) prof(calls[phase >= 0 && phase <= 4 ? phase : 0]);
+            const bool ok = exact ? launch_exact_linear((const uint8_t *)w.d, w.qtype, w.out_f, w.nb, xd, T, fw, od + off, g_stream) == cudaSuccess
+                                  : linear_dev(w, xd, T, fw, od + off, false, g_stream, xl, nl, true);
+            if (!ok) { cudaGetLastError(); return 1; }
+            off += T * w.out_f;
+        }
+        const int f = download({{out, od, (size_t)total * 8}});
+        if (f < 0) { cudaGetLastError(); return 1; }
+        if (exact || !(f & 1)) break;
     }
-    if (!d2h(out, od, (size_t)total * 8) || !sync()) { cudaGetLastError(); return 1; }
     return 0;
 }
 
@@ -1736,15 +1779,12 @@ extern "C" int iie_moe_block_host(long long layer, long long gain_h, const int64
     int64_t *xd = (int64_t *)ensure(R_X, n * 8), *od = (int64_t *)ensure(R_OUT, n * 8);
     int64_t *gd = (int64_t *)ensure(R_GATES, P * 8);
     int *idd = (int *)ensure(R_IDS, P * sizeof(int));
-    if (!xd || !od || !gd || !idd || !h2d(xd, x, n * 8)) { cudaGetLastError(); return 1; }
+    if (!xd || !od || !gd || !idd || !upload(xd, x, n * 8)) { cudaGetLastError(); return 1; }
     const int rc = iie_moe_block_dev(layer, gain_h, xd, T, fa, fw, eps, od, idd, gd, g_stream);
     if (rc != 0) { cudaGetLastError(); return rc; }
-    const int f = read_flags_clear();
-    if (f < 0) return 1;
-    if (f) return 3;
-    if (!d2h(out, od, n * 8) || (ids_out && !d2h(ids_out, idd, P * sizeof(int))) ||
-        (gates_out && !d2h(gates_out, gd, P * 8)) || !sync()) { cudaGetLastError(); return 1; }
-    return 0;
+    const int f = download({{out, od, n * 8}, {ids_out, idd, ids_out ? P * sizeof(int) : 0}, {gates_out, gd, gates_out ? P * 8 : 0}});
+    if (f < 0) { cudaGetLastError(); return 1; }
+    return f ? 3 : 0;
 }
 
 // ====================================================================================================

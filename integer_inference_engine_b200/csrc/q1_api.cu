@@ -7,8 +7,10 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <initializer_list>
 #include <mutex>
+#include <thread>
 #include <vector>
 
 #include "../../include/iie_q1.h"
@@ -34,7 +36,7 @@ cudaStream_t q_stream = nullptr;
 int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [8..15] digits in use (a ring, see next_digits)
 int q_ready = -1;
 
-enum QRole { QR_X, QR_PLANES, QR_OUT, QR_GAIN, QR_COUNT };
+enum QRole { QR_X, QR_PLANES, QR_WORK, QR_KEYS, QR_VALUES, QR_LOGITS, QR_OUT, QR_GAIN, QR_COUNT };
 struct QBuf { void *p = nullptr; size_t cap = 0; };
 unsigned long long q_generation = 0;   // changes whenever a scratch buffer is freed: captured graphs hold the old addresses
 QBuf q_buf[QR_COUNT];
@@ -68,7 +70,8 @@ bool q_init() {
 void *q_ensure(int role, size_t bytes) {
     QBuf &b = q_buf[role];
     if (b.p && b.cap >= bytes) return b.p;
-    if (b.p) { cudaDeviceSynchronize(); cudaFree(b.p); b.p = nullptr; b.cap = 0; q_generation++; }
+    // (the prefill's buffers are in no captured graph: growing them leaves graphs valid)
+    if (b.p) { cudaDeviceSynchronize(); cudaFree(b.p); b.p = nullptr; b.cap = 0; if (role < QR_WORK || role > QR_LOGITS) q_generation++; }
     const size_t cap = std::max<size_t>(bytes, 256);
     if (cudaMalloc(&b.p, cap) != cudaSuccess) { cudaGetLastError(); b.p = nullptr; return nullptr; }
     b.cap = cap;
@@ -404,6 +407,37 @@ extern "C" int iie_q1_head_norm_dev(const int64_t *x_dev, long long rows_a, long
                                     (cudaStream_t)stream) == cudaSuccess ? 0 : 2;
 }
 
+// Page-locked arrays for results that the caller hands on: a small pool, each array given back when its last user drops it.
+namespace {
+constexpr size_t HOST_POOL = 64 << 20;         // bytes of the pool at most, in use and free
+struct HostArray { void *p; size_t cap; bool used; };
+std::mutex h_mu;
+std::vector<HostArray> h_pool;
+}  // namespace
+extern "C" void *iie_host_take(unsigned long long bytes) {
+    std::lock_guard<std::mutex> lk(h_mu);
+    if (bytes == 0 || bytes > HOST_POOL) return nullptr;
+    size_t total = 0;
+    for (auto &h : h_pool) {
+        if (!h.used && h.cap >= bytes && h.cap <= 2 * bytes) { h.used = true; return h.p; }
+        total += h.cap;
+    }
+    for (size_t i = 0; i < h_pool.size() && total + bytes > HOST_POOL;) {          // free arrays make room
+        if (h_pool[i].used) { i++; continue; }
+        total -= h_pool[i].cap;
+        cudaFreeHost(h_pool[i].p);
+        h_pool.erase(h_pool.begin() + (long)i);
+    }
+    void *p = nullptr;
+    if (total + bytes > HOST_POOL || cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    h_pool.push_back({p, (size_t)bytes, true});
+    return p;
+}
+extern "C" void iie_host_give(void *p) {
+    std::lock_guard<std::mutex> lk(h_mu);
+    for (auto &h : h_pool) if (h.p == p) h.used = false;
+}
+
 extern "C" unsigned long long iie_q1_workspace_generation(void) { return q_generation; }
 extern "C" void iie_q1_set_stream(int) {}             // single-row products have one form: the weights always come by bulk copies
 
@@ -489,11 +523,15 @@ struct Work {
     void *base = nullptr;
     int64_t *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *qn = nullptr, *kn = nullptr, *att = nullptr, *g = nullptr, *u = nullptr;
 };
-bool alloc_work(Work &w, const Q1Stack &m, long long rows) {
+bool alloc_work(Work &w, const Q1Stack &m, long long rows, bool keep) {
     const size_t qd = (size_t)(m.H * m.hd), kd = (size_t)(m.Hkv * m.hd), T = (size_t)rows;
     const size_t n = T * ((size_t)m.d + 3 * qd + 3 * kd + 2 * (size_t)m.dff);
-    if (cudaMalloc(&w.base, n * 8) != cudaSuccess) { cudaGetLastError(); w.base = nullptr; return false; }
-    int64_t *p = (int64_t *)w.base;
+    int64_t *p = keep ? (int64_t *)q_ensure(QR_WORK, n * 8) : nullptr;      // kept between calls, or the caller's
+    if (!keep) {
+        if (cudaMalloc(&w.base, n * 8) != cudaSuccess) { cudaGetLastError(); w.base = nullptr; return false; }
+        p = (int64_t *)w.base;
+    }
+    if (!p) return false;
     // q, k, v and g, u side by side: one range each for the kernel that clears them
     w.x = p; p += T * m.d; w.q = p; p += T * qd; w.k = p; p += T * kd; w.v = p; p += T * kd; w.g = p; p += T * m.dff; w.u = p; p += T * m.dff;
     w.qn = p; p += T * qd; w.att = p; p += T * qd; w.kn = p;
@@ -582,6 +620,47 @@ bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logi
     if (!planes) return false;
     return products([&](const PlaneDuties &d) { return launch_rmsnorm_planes(x, rows, m.d, gain, (int)m.frac, m.eps, nullptr, planes, flags, d, q_stream); },
                     {{m.out_head, logits}}, planes, rows, m.frac, x, rows * m.d);
+}
+
+// Rows from pageable host memory: four threads copy pieces into a page-locked buffer and send each on its way (one thread, or the
+// driver's own staging, copies 11 GB/s: 1.4 ms for 512 rows of 4096).  A single buffer of at most 32 MB, kept.
+bool upload_rows(int64_t *dst, const long long *src, size_t bytes) {
+    constexpr size_t LEAST = 1 << 20, MOST = 32 << 20, PIECE = 512 << 10;
+    constexpr int THREADS = 4;
+    static uint8_t *pin = nullptr;
+    static size_t cap = 0;
+    if (bytes < LEAST) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
+    const size_t want = std::min(bytes, MOST);
+    if (cap < want) {
+        if (pin) { cudaStreamSynchronize(q_stream); cudaFreeHost(pin); pin = nullptr; cap = 0; }
+        if (cudaHostAlloc(&pin, want, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError(); pin = nullptr;
+            return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
+        }
+        cap = want;
+    }
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    for (size_t part = 0; part < bytes; part += cap) {
+        const size_t n = std::min(cap, bytes - part), pieces = (n + PIECE - 1) / PIECE;
+        if (part && cudaStreamSynchronize(q_stream) != cudaSuccess) return false;
+        std::atomic<size_t> next{0};
+        std::atomic<bool> good{true};
+        auto copy = [&]() {
+            if (cudaSetDevice(dev) != cudaSuccess) { good = false; return; }
+            for (size_t i; (i = next.fetch_add(1)) < pieces;) {
+                const size_t at = i * PIECE, len = std::min(PIECE, n - at);
+                memcpy(pin + at, (const uint8_t *)src + part + at, len);
+                if (cudaMemcpyAsync((uint8_t *)dst + part + at, pin + at, len, cudaMemcpyHostToDevice, q_stream) != cudaSuccess) good = false;
+            }
+        };
+        std::thread helpers[THREADS - 1];
+        for (auto &t : helpers) t = std::thread(copy);
+        copy();
+        for (auto &t : helpers) t.join();
+        if (!good) return false;
+    }
+    return true;
 }
 
 // int64 host rows -> int32; false when a value does not fit
@@ -789,10 +868,11 @@ extern "C" int bonsai_prefill_forward_gpu(const long long *x_embed, long long T,
     const long long vocab = q_w[(size_t)out_head].out_f;
     const size_t kv_elems = (size_t)Hkv * T * hd;
     Work w;
-    int32_t *kc = nullptr, *vc = nullptr; int64_t *logits = nullptr;
-    bool ok = alloc_work(w, m, T) && cudaMalloc(&kc, kv_elems * 4) == cudaSuccess && cudaMalloc(&vc, kv_elems * 4) == cudaSuccess &&
-              cudaMalloc(&logits, (size_t)vocab * 8) == cudaSuccess;
-    ok = ok && cudaMemcpyAsync(w.x, x_embed, (size_t)T * d * 8, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
+    // buffers kept between calls: allocating and freeing them took a millisecond of every prompt
+    int32_t *kc = (int32_t *)q_ensure(QR_KEYS, kv_elems * 4), *vc = (int32_t *)q_ensure(QR_VALUES, kv_elems * 4);
+    int64_t *logits = (int64_t *)q_ensure(QR_LOGITS, (size_t)vocab * 8);
+    bool ok = kc && vc && logits && alloc_work(w, m, T, true);
+    ok = ok && upload_rows(w.x, x_embed, (size_t)T * d * 8);
     int flags = -1;
     std::vector<int32_t> rows;
     if (ok) {
@@ -824,9 +904,7 @@ extern "C" int bonsai_prefill_forward_gpu(const long long *x_embed, long long T,
         ok = ok && flags >= 0;
     }
     if (ok && flags == 0) ok = cudaMemcpy(out_logits, logits, (size_t)vocab * 8, cudaMemcpyDeviceToHost) == cudaSuccess;
-    free_work(w);
-    for (void *p : {(void *)kc, (void *)vc, (void *)logits}) if (p) cudaFree(p);
-    if (!ok) return fail(1, "prefill forward: CUDA failure");
+    if (!ok) { cudaStreamSynchronize(q_stream); return fail(1, "prefill forward: CUDA failure"); }
     if (flags) return fail(4, "prefill forward: a value left the exact envelope");
     return 0;
 }
@@ -850,7 +928,7 @@ extern "C" long long bonsai_decode_ctx_create(long long B, long long n_layers, l
     c.B = B; c.cap = cap; c.vocab = vocab; c.wide.assign((size_t)B, 0);
     const size_t kv = (size_t)n_layers * B * Hkv * cap * hd * 4;
     if (cudaMalloc(&c.K, kv) != cudaSuccess || cudaMalloc(&c.V, kv) != cudaSuccess || cudaMemset(c.K, 0, kv) != cudaSuccess ||
-        cudaMemset(c.V, 0, kv) != cudaSuccess || cudaMalloc(&c.logits, (size_t)B * vocab * 8) != cudaSuccess || cudaMalloc(&c.pos, (size_t)B * 4) != cudaSuccess || !alloc_work(c.w, m, B)) {
+        cudaMemset(c.V, 0, kv) != cudaSuccess || cudaMalloc(&c.logits, (size_t)B * vocab * 8) != cudaSuccess || cudaMalloc(&c.pos, (size_t)B * 4) != cudaSuccess || !alloc_work(c.w, m, B, false)) {
         cudaGetLastError(); free_ctx(c); fail(2, "decode context: out of device memory"); return -1;
     }
     c.alive = true;

@@ -148,13 +148,19 @@ def available() -> bool:
         return False
 
 
+_usable_lib = None                                   # the library once a device has answered: it stays usable
+
+
 def _lib():
-    lib = load_library()
-    with _CUDA_LOCK:
-        usable = lib.qk_cuda_available() == 0
-    if not usable:
-        raise CudaUnavailableError("no usable CUDA device; this package has no CPU path")
-    return lib
+    global _usable_lib
+    if _usable_lib is None:
+        lib = load_library()
+        with _CUDA_LOCK:
+            usable = lib.qk_cuda_available() == 0
+        if not usable:
+            raise CudaUnavailableError("no usable CUDA device; this package has no CPU path")
+        _usable_lib = lib
+    return _usable_lib
 
 
 def _native(name: str, *args):
@@ -282,8 +288,11 @@ def apply_resident_grouped(handles, x_int, out_features, fw: int, phase_ids=None
                  packed.size, packed.ctypes.data)
     if rc != 0:
         return None
-    edges = np.cumsum([t * w for w in widths])[:-1]
-    return tuple(part.reshape(t, w) for part, w in zip(np.split(packed, edges), widths))
+    parts, at = [], 0
+    for w in widths:
+        parts.append(packed[at:at + t * w].reshape(t, w))
+        at += t * w
+    return tuple(parts)
 
 
 # ------------------------------------------------------------------------------------------------ limb policy ---
