@@ -307,6 +307,7 @@ __global__ void __launch_bounds__(256) attn_pv_kernel(const AttnArgs a_in) {
 // several tokens, before the passes: rotate the new keys and append keys and values of all `batch` tokens (to one cache at
 // consecutive positions, or each to its own sequence's cache at position pos); grid (batch, Hkv)
 __global__ void __launch_bounds__(128) attn_append_kernel(const AttnArgs a) {
+    pdl_enter();
     const long long i = blockIdx.x, pos = a.seq_stride > 0 ? a.pos : a.pos + i, seq = a.seq_stride > 0 ? i * a.seq_stride : 0;
     const int kv = blockIdx.y, tid = threadIdx.x, half = a.hd / 2;
     const int64_t *ks = a.k + (i * a.Hkv + kv) * a.hd, *vs = a.v + (i * a.Hkv + kv) * a.hd;
@@ -1432,7 +1433,7 @@ cudaError_t launch_attn_prefill(const AttnArgs &a, cudaStream_t s) {
     long long n_keys = last + 1;
     if (a.window > 0 && n_keys > a.window) n_keys = a.window;
     const unsigned chunks = (unsigned)((n_keys + AT_CH - 1) / AT_CH);
-    attn_append_kernel<<<dim3((unsigned)a.batch, a.Hkv), 128, 0, s>>>(a);
+    launch_behind(attn_append_kernel, dim3((unsigned)a.batch, a.Hkv), 128, 0, s, a);
     if (g_attn_fused != 0 && g_attn_tile_tc >= 0 && attn_tiles_ok(a)) {
         // consecutive tokens of one sequence: sixteen tokens per CTA share every staged chunk of keys and values
         note_launch(1);

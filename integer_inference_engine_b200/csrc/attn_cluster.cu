@@ -83,6 +83,7 @@ __device__ __forceinline__ void ac_rotate(const AttnArgs &a, long long pos, int 
 
 template <int HD>
 __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnArgs a) {
+    pdl_enter();
     constexpr int QLD = HD + 16, HALF = HD / 2;
     extern __shared__ __align__(128) unsigned char ac_sm[];
     __shared__ long long s_max[AC_WARPS][AC_HEADS], s_base[AC_WARPS][AC_HEADS];
@@ -468,10 +469,12 @@ cudaError_t launch_cluster(const AttnArgs &a_in, int n_c, int tiles, cudaStream_
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n_c, (unsigned)a.Hkv, (unsigned)std::max(1, a.batch)); cfg.blockDim = dim3(AC_THREADS); cfg.stream = s;
     cfg.dynamicSmemBytes = ac_smem<HD>(tiles);
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // the kernel begins with pdl_enter()
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)n_c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_cluster_kernel<HD>, a);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();

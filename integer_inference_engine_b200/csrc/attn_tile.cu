@@ -93,6 +93,7 @@ __device__ __forceinline__ int32_t pt_score(const AttnArgs &a, long long at, lon
 // tokens; a warp multiplies one key tile with two tokens at a time (56 accumulator registers).
 template <int HD>
 __global__ void __launch_bounds__(PT_THREADS, 1) attn_tile_scores_kernel(const AttnArgs a) {
+    pdl_enter();
     constexpr int QLD = HD + 16, HALF = HD / 2, VPT = HD / 32;     // bytes per plane row; 16-byte vectors of a chunk per thread
     extern __shared__ __align__(16) unsigned char pt_smem[];
     __shared__ long long s_max[PT_COLS];
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_tile_scores_kernel(const A
 // Bounded by instructions (about 30 per key) and the eight bytes per key in and out: 2048 tokens x 32 heads 189 us, with 64-bit
 // scores and 64-bit exponentials and quotients 300.
 __global__ void __launch_bounds__(256) attn_tile_exp_kernel(const AttnArgs a) {
+    pdl_enter();
     const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5), n_rows = (long long)a.batch * a.H;
     if (row >= n_rows) return;
     const int lane = threadIdx.x & 31;
@@ -318,6 +320,7 @@ __global__ void __launch_bounds__(256) attn_tile_exp_kernel(const AttnArgs a) {
 // the two halves of the head dimension; the 64-bit sums of a thread's outputs stay in registers over the whole walk.
 template <int HD>
 __global__ void __launch_bounds__(PT_THREADS, 1) attn_tile_pv_kernel(const AttnArgs a) {
+    pdl_enter();
     constexpr int NT = HD / 16;                                    // 8-wide dimension tiles of a warp
     constexpr int VU = HD / 32;                                    // (dimension, four keys) units of a thread per chunk
     extern __shared__ __align__(16) unsigned char pt_smem[];
@@ -496,6 +499,7 @@ __device__ __forceinline__ void pc_commit(uint64_t *bar) {
 
 template <int HD>
 __global__ void __launch_bounds__(PC_THREADS, 1) attn_tile_pv_tc_kernel(const AttnArgs a) {
+    pdl_enter();
     extern __shared__ __align__(1024) unsigned char pc_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(pc_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t full_bar[PC_STAGES], empty_bar[PC_STAGES], accum_bar;
@@ -662,6 +666,7 @@ __device__ __forceinline__ bool pc_all_ok(bool ok) {
 
 template <int HD>
 __global__ void __launch_bounds__(PC_THREADS, 1) attn_tile_scores_tc_kernel(const AttnArgs a) {
+    pdl_enter();
     constexpr int HALF = HD / 2, Q_PLANE = PT_COLS * HD, K_PLANE = PT_CH * HD, K_STAGE = 4 * K_PLANE;
     extern __shared__ __align__(1024) unsigned char pc_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(pc_raw) + 1023) & ~(uintptr_t)1023);
@@ -916,7 +921,7 @@ cudaError_t scores_launch(const AttnArgs &a, unsigned walks, unsigned tiles, cud
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    attn_tile_scores_kernel<HD><<<dim3(walks, a.Hkv, tiles), PT_THREADS, smem, s>>>(a);
+    launch_behind(attn_tile_scores_kernel<HD>, dim3(walks, a.Hkv, tiles), PT_THREADS, smem, s, a);
     return cudaGetLastError();
 }
 
@@ -929,7 +934,7 @@ cudaError_t pv_launch(const AttnArgs &a, unsigned tiles, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    attn_tile_pv_kernel<HD><<<dim3(1, a.Hkv, tiles), PT_THREADS, smem, s>>>(a);
+    launch_behind(attn_tile_pv_kernel<HD>, dim3(1, a.Hkv, tiles), PT_THREADS, smem, s, a);
     return cudaGetLastError();
 }
 
@@ -943,7 +948,7 @@ cudaError_t scores_tc_launch(const AttnArgs &a, unsigned walks, unsigned tiles, 
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    attn_tile_scores_tc_kernel<HD><<<dim3(walks, a.Hkv, tiles), PC_THREADS, smem, s>>>(a);
+    launch_behind(attn_tile_scores_tc_kernel<HD>, dim3(walks, a.Hkv, tiles), PC_THREADS, smem, s, a);
     return cudaGetLastError();
 }
 
@@ -956,7 +961,7 @@ cudaError_t pv_tc_launch(const AttnArgs &a, unsigned tiles, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    attn_tile_pv_tc_kernel<HD><<<dim3(HD / PC_N, a.Hkv, tiles), PC_THREADS, smem, s>>>(a);
+    launch_behind(attn_tile_pv_tc_kernel<HD>, dim3(HD / PC_N, a.Hkv, tiles), PC_THREADS, smem, s, a);
     return cudaGetLastError();
 }
 
@@ -985,7 +990,7 @@ cudaError_t launch_attn_tile_scores(const AttnArgs &a, cudaStream_t s) {
 cudaError_t launch_attn_tile_exp(const AttnArgs &a, cudaStream_t s) {
     if (!attn_tiles_ok(a)) return cudaErrorInvalidValue;
     const long long rows = (long long)a.batch * a.H;
-    attn_tile_exp_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(a);
+    launch_behind(attn_tile_exp_kernel, (unsigned)((rows + 7) / 8), 256, 0, s, a);
     note_launch();
     return cudaGetLastError();
 }

@@ -39,6 +39,7 @@ __device__ __forceinline__ bool bt_dense(int rows, int digits) { return ((rows +
 
 template <int QT, int MODE, bool FAST>
 __global__ void __launch_bounds__(BT_WARPS * 32, 2) batch_kernel(const BatchArgs a) {
+    pdl_enter();
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int HTB = QT == QT_Q4K ? HTB_Q4K : HTB_Q6K;
     const int nb = (int)a.n_blocks, tile_bytes = 2 * nb * HTB, tpc = a.tiles_per_cta;
@@ -238,7 +239,7 @@ cudaError_t launch_t(const BatchArgs &a_in, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    batch_kernel<QT, MODE, FAST><<<(unsigned)((n_tiles + tpc - 1) / tpc), BT_WARPS * 32, smem, s>>>(a);
+    launch_behind(batch_kernel<QT, MODE, FAST>, (unsigned)((n_tiles + tpc - 1) / tpc), BT_WARPS * 32, smem, s, a);
     note_launch();
     return cudaGetLastError();
 }

@@ -10,6 +10,13 @@
 
 namespace iie {
 
+// First statement of a kernel that launch_behind starts: wait for the kernel before (all its memory operations are visible then), and
+// let the kernel behind start its own launch.  As each waits, everything before the kernel before has finished, too.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 typedef __int128 i128;
 typedef unsigned __int128 u128;
 

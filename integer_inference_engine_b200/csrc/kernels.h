@@ -1,9 +1,24 @@
 // Host-callable launchers of the CUDA kernels (internal interface between the .cu files).
 #pragma once
 #include <cuda_runtime.h>
+
+#include <utility>
 #include <stdint.h>
 
 namespace iie {
+
+// Launch of a kernel that begins with pdl_enter(): its launch overlaps the end of the kernel before it on the stream (a chain of
+// small kernels saves 1 to 2 us each).
+template <typename... P, typename... A>
+cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 // Number of kernels this library has launched since it was loaded (benchmarks report it).
 extern unsigned long long g_launches;

@@ -48,6 +48,7 @@ __global__ void repack_kernel(const uint8_t *src, uint8_t *dst, long long out_f,
 // activation limb planes
 // ---------------------------------------------------------------------------------------------------
 __global__ void limbs_kernel(const int64_t *x, long long n_rows, long long K, int8_t *planes, int *flags, int *nl_out) {
+    pdl_enter();
     const long long total = n_rows * K;
     bool bad = false;
     int nl = 0;
@@ -68,8 +69,9 @@ __global__ void limbs_kernel(const int64_t *x, long long n_rows, long long K, in
 
 // The same for K a multiple of 8: a thread takes eight consecutive columns (64 bytes in), transposes the 8 x 8 digit
 // bytes in registers and writes eight bytes to each plane.
-__global__ void __launch_bounds__(256) limbs8_kernel(const int64_t *__restrict__ x, long long n_rows, long long K, int8_t *__restrict__ planes,
+__global__ void __launch_bounds__(256) limbs8_kernel(const int64_t *x, long long n_rows, long long K, int8_t *planes,
                                                      int *flags, int *nl_out) {
+    pdl_enter();
     const long long per_row = K >> 3, total = n_rows * per_row;
     bool bad = false;
     uint64_t seen = 0;
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(256) limbs8_kernel(const int64_t *__restrict__
         uint32_t lo[8], hi[8];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const ulonglong2 v = __ldg(src + i);
+            const ulonglong2 v = __ldcg(src + i);
             bool ok0, ok1;
             const uint64_t d0 = balanced_digits8((int64_t)v.x, ok0), d1 = balanced_digits8((int64_t)v.y, ok1);
             bad |= !ok0 | !ok1;
@@ -203,6 +205,7 @@ __global__ void combine_kernel(const int64_t *dn, const int64_t *gates, long lon
 // ---------------------------------------------------------------------------------------------------
 __global__ void topk_kernel(const int64_t *logits, long long rows, int n_experts, int k, int fa, int *ids,
                             int64_t *gates) {
+    pdl_enter();
     const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -237,6 +240,7 @@ __global__ void topk_kernel(const int64_t *logits, long long rows, int n_experts
 // ---------------------------------------------------------------------------------------------------
 __global__ void dispatch_kernel(const int *ids, const int64_t *gates, long long T, int k, int n_experts, int expert_base,
                                 int *grp_off, int *pair_tok, int64_t *pair_gate) {
+    pdl_enter();
     extern __shared__ int sm[];                           // cnt[nwarps][E], then start[E + 1]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     int *cnt = sm, *start = sm + nwarps * n_experts;
@@ -308,6 +312,7 @@ struct NormArgs {
 // out and the quotients (2048 x 2048: 103 us before).
 template <int G>
 __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormArgs a) {
+    pdl_enter();
     __shared__ uint64_t s_lo[32], s_hi[32];
     __shared__ uint32_t s_bits[32];
     if (a.duties.nl_clear && blockIdx.x == 0 && threadIdx.x == 0) *a.duties.nl_clear = 0;
@@ -422,6 +427,7 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormArgs a) {
 
 // any width: one CTA per row, values read again for the quotients
 __global__ void __launch_bounds__(256) rmsnorm_any_kernel(const NormArgs a) {
+    pdl_enter();
     __shared__ uint64_t s_lo[8], s_hi[8], s_max[8], s_gmax[8];
     const long long row = blockIdx.x;
     const int64_t *gain = row < a.rows_a ? a.gain_a : a.gain_b, *xr = a.x + row * a.width;
@@ -455,15 +461,15 @@ cudaError_t launch_norm(NormArgs a, cudaStream_t s) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.gain_a) | reinterpret_cast<uintptr_t>(a.gain_b) | reinterpret_cast<uintptr_t>(a.out);
     a.wide = (at & 15) == 0;
     if (a.width > 8192 || a.width % 4) {                           // (beyond 8192 every row is refused)
-        rmsnorm_any_kernel<<<(unsigned)a.rows, 256, 0, s>>>(a);
+        launch_behind(rmsnorm_any_kernel, (unsigned)a.rows, 256, 0, s, a);
     } else {
         const int groups = (a.width + 127) / 128;                  // of 128 values
         a.wpr = groups <= 2 ? 1 : groups <= 32 ? groups : (groups + 1) / 2;          // one or two groups: a warp per row, eight rows per CTA
         const int threads = a.wpr == 1 ? 256 : a.wpr * 32;
         long long grid = a.wpr == 1 ? (a.rows + 7) / 8 : a.rows;
         grid = std::max(grid, std::min(148LL, a.duties.zero_n / (threads * 8)));     // few rows: more CTAs for the words to clear
-        if (groups == 1 || (groups > 2 && groups <= 32)) rmsnorm_kernel<1><<<(unsigned)grid, threads, 0, s>>>(a);
-        else rmsnorm_kernel<2><<<(unsigned)grid, threads, 0, s>>>(a);
+        if (groups == 1 || (groups > 2 && groups <= 32)) launch_behind(rmsnorm_kernel<1>, (unsigned)grid, threads, 0, s, a);
+        else launch_behind(rmsnorm_kernel<2>, (unsigned)grid, threads, 0, s, a);
     }
     note_launch();
     return cudaGetLastError();
@@ -492,10 +498,13 @@ cudaError_t launch_unpack(const uint8_t *src, uint8_t *raw, long long out_f, lon
     return cudaGetLastError();
 }
 
-__global__ void set2_kernel(int *p, int a, int b) { p[0] = a; p[1] = b; }
+__global__ void set2_kernel(int *p, int a, int b) {
+    pdl_enter();
+    p[0] = a; p[1] = b;
+}
 
 cudaError_t launch_set2(int *p, int a, int b, cudaStream_t s) {
-    set2_kernel<<<1, 1, 0, s>>>(p, a, b);
+    launch_behind(set2_kernel, 1, 1, 0, s, p, a, b);
     note_launch();
     return cudaGetLastError();
 }
@@ -532,9 +541,9 @@ cudaError_t launch_add_rows(const int64_t *a, const int64_t *b, int64_t *out, lo
 cudaError_t launch_limbs(const int64_t *x, long long n_rows, long long K, int8_t *planes, int *flags, cudaStream_t s,
                          int *nl_out) {
     if (K % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(planes) & 7) == 0)
-        limbs8_kernel<<<grid_for(n_rows * (K >> 3), 256), 256, 0, s>>>(x, n_rows, K, planes, flags, nl_out);
+        launch_behind(limbs8_kernel, grid_for(n_rows * (K >> 3), 256), 256, 0, s, x, n_rows, K, planes, flags, nl_out);
     else
-        limbs_kernel<<<grid_for(n_rows * K, 256), 256, 0, s>>>(x, n_rows, K, planes, flags, nl_out);
+        launch_behind(limbs_kernel, grid_for(n_rows * K, 256), 256, 0, s, x, n_rows, K, planes, flags, nl_out);
     note_launch();
     return cudaGetLastError();
 }
@@ -573,7 +582,7 @@ cudaError_t launch_topk(const int64_t *logits, long long rows, int n_experts, in
                         cudaStream_t s) {
     if (n_experts > 1024 || n_experts <= 0 || k <= 0) return cudaErrorInvalidValue;
     const long long n = rows * 32;
-    topk_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(logits, rows, n_experts, k, fa, ids, gates);
+    launch_behind(topk_kernel, (unsigned)((n + 127) / 128), 128, 0, s, logits, rows, n_experts, k, fa, ids, gates);
     note_launch();
     return cudaGetLastError();
 }
@@ -601,7 +610,7 @@ cudaError_t launch_dispatch(const int *ids, const int64_t *gates, long long T, i
     if (n_experts > 1024 || n_experts <= 0) return cudaErrorInvalidValue;
     const int warps = n_experts <= 320 ? 32 : 8;                        // cnt[warps][E] + start[E + 1] stays below 48 KB
     const size_t smem = ((size_t)warps * n_experts + n_experts + 1) * sizeof(int);
-    dispatch_kernel<<<1, 32 * warps, smem, s>>>(ids, gates, T, k, n_experts, expert_base, grp_off, pair_tok, pair_gate);
+    launch_behind(dispatch_kernel, 1, 32 * warps, smem, s, ids, gates, T, k, n_experts, expert_base, grp_off, pair_tok, pair_gate);
     note_launch();
     return cudaGetLastError();
 }

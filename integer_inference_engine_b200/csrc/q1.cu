@@ -66,6 +66,7 @@ __global__ void q1_repack_kernel(const uint8_t *bits, const ST *scale, long long
 // x and up then advance by `ld` per token.
 __global__ void q1_prep_kernel(const int64_t *x, const int64_t *up, long long ld, int frac, int64_t log2e, int64_t clip, long long T,
                                long long nb, int8_t *planes, const PlaneDuties duties) {
+    pdl_enter();
     int *nl_out = duties.nl;
     if (duties.nl_clear && blockIdx.x == 0 && threadIdx.x == 0) *duties.nl_clear = 0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < duties.zero_n; i += (long long)gridDim.x * blockDim.x) duties.zero[i] = 0;
@@ -150,7 +151,7 @@ cudaError_t launch_q1_repack(const uint8_t *bits, const void *scale, int src_bit
 cudaError_t launch_q1_prep(const int64_t *x, long long T, long long nb, int8_t *planes, const PlaneDuties &duties,
                            cudaStream_t s) {
     const long long warps = T * nb;
-    q1_prep_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(x, nullptr, 0, 0, 0, 0, T, nb, planes, duties);
+    launch_behind(q1_prep_kernel, (unsigned)((warps * 32 + 255) / 256), 256, 0, s, x, nullptr, 0, 0, 0, 0, T, nb, planes, duties);
     note_launch();
     return cudaGetLastError();
 }
@@ -159,7 +160,7 @@ cudaError_t launch_q1_prep_swiglu(const int64_t *gate, const int64_t *up, long l
                                   int8_t *planes, const PlaneDuties &duties, cudaStream_t s) {
     if (!gate || !up || frac < 1 || frac > 29) return cudaErrorInvalidValue;
     const long long warps = T * nb;
-    q1_prep_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s>>>(gate, up, ld, frac, sigmoid_log2e(frac), sigmoid_clip(frac), T, nb,
+    launch_behind(q1_prep_kernel, (unsigned)((warps * 32 + 255) / 256), 256, 0, s, gate, up, ld, frac, sigmoid_log2e(frac), sigmoid_clip(frac), T, nb,
                                                                         planes, duties);
     note_launch();
     return cudaGetLastError();

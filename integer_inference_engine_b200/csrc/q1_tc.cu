@@ -127,6 +127,7 @@ __device__ __forceinline__ int qc_planes(int nl, bool narrow) { return nl <= 3 &
 
 template <int NT, typename DT>
 __global__ void __launch_bounds__(qc_threads(NT), 1) q1_tc_kernel(const Q1TcArgs a, const __grid_constant__ CUtensorMap xmap) {
+    pdl_enter();
     constexpr int US = 256 + 16 * (int)sizeof(DT);
     constexpr int RAW_BYTES = 8 * QC_CHUNK * US;                   // eight 16-row sub-tiles x eight blocks
     constexpr int QC_READ = qc_read_warps(NT), QC_MMA_WARP = QC_READ + QC_EXPAND, QC_PLANE_WARP = QC_MMA_WARP + 1;
@@ -483,7 +484,7 @@ cudaError_t launch_tc(Q1TcArgs a, const int8_t *planes, cudaStream_t s) {
     a.split = q1_tc_split(a.tile_end[a.n_parts - 1], a.T);
     long long grid = std::min<long long>(Q1_TC_CTAS, a.n_tiles);
     if (a.split) grid = std::min<long long>(Q1_TC_CTAS, std::max<long long>(1, a.n_tiles * a.nb / 4));
-    q1_tc_kernel<NT, DT><<<(unsigned)grid, qc_threads(NT), QC_SMEM, s>>>(a, map);
+    launch_behind(q1_tc_kernel<NT, DT>, (unsigned)grid, qc_threads(NT), QC_SMEM, s, a, map);
     note_launch();
     return cudaGetLastError();
 }

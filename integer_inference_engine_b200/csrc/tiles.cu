@@ -131,6 +131,7 @@ struct TileMaps { CUtensorMap x16, x32, s16, s32; };               // planes and
 
 template <int QT, int MODE>
 __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArgs a, const __grid_constant__ TileMaps maps) {
+    pdl_enter();
     constexpr bool Q4 = QT == QT_Q4K;
     constexpr int HTB = Q4 ? HTB_Q4K : HTB_Q6K, RAW_BYTES = 16 * HTB;
     constexpr int NROW = MODE == MODE_GATEUP ? 64 : 128;           // output rows of a tile
@@ -598,8 +599,9 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
 
 // Sums of the 32 columns of every sub-block as nine balanced digits, xs[row][9][stride] (columns from nb * 8 on are zero), and with
 // `xidx` the digit planes in use copied into pair order.  One thread per (row, sub-block).
-__global__ void __launch_bounds__(256) tile_rows_kernel(const int8_t *__restrict__ xl, const int *__restrict__ xidx, const int *__restrict__ n_live, const int *__restrict__ x_nl,
-                                                        long long n_rows, int nb, int stride, int8_t *__restrict__ xg, int8_t *__restrict__ xs) {
+__global__ void __launch_bounds__(256) tile_rows_kernel(const int8_t *xl, const int *xidx, const int *n_live, const int *x_nl,
+                                                        long long n_rows, int nb, int stride, int8_t *xg, int8_t *xs) {
+    pdl_enter();
     const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
     const int j = (int)(idx % stride);
     const long long row = idx / stride;
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(256) tile_rows_kernel(const int8_t *__restrict
     int carry = 0;
     for (int l = 0; l < 9; l++) {
         if (l < np) {
-            const uint4 u = ldg128(src + l * K), v = ldg128(src + l * K + 16);
+            const uint4 u = __ldcg(reinterpret_cast<const uint4 *>(src + l * K)), v = __ldcg(reinterpret_cast<const uint4 *>(src + l * K + 16));
             if (xidx) {
                 uint4 *dst = reinterpret_cast<uint4 *>(xg + row * 8 * K + l * K + j * 32);
                 dst[0] = u; dst[1] = v;
@@ -663,7 +665,7 @@ cudaError_t launch_tile(const TileArgs &a, const TileMaps &maps, cudaStream_t s)
     // an upper bound on the tiles: every group may end in a partial one
     const long long n_rt = (a.out_f + (MODE == MODE_GATEUP ? 63 : 127)) / (MODE == MODE_GATEUP ? 64 : 128);
     const long long most = (a.n_rows / 16 + std::min<long long>(a.n_groups, a.n_rows)) * n_rt;
-    tile_kernel<QT, MODE><<<(unsigned)std::max<long long>(1, std::min<long long>(148, most)), tl_threads(MODE), TL_SMEM, s>>>(a, maps);
+    launch_behind(tile_kernel<QT, MODE>, (unsigned)std::max<long long>(1, std::min<long long>(148, most)), tl_threads(MODE), TL_SMEM, s, a, maps);
     note_launch();
     return cudaGetLastError();
 }
@@ -685,7 +687,7 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
     const bool q4 = qtype == QT_Q4K;
     if (q4 || a.xidx) {
         const long long n = a.n_rows * stride;
-        tile_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a.xl, a.xidx, a.grp_off + a.n_groups, a.x_nl, a.n_rows, a.nb, stride, a.xg, q4 ? a.xs : nullptr);
+        launch_behind(tile_rows_kernel, (unsigned)((n + 255) / 256), 256, 0, s, a.xl, a.xidx, a.grp_off + a.n_groups, a.x_nl, a.n_rows, a.nb, stride, a.xg, q4 ? a.xs : nullptr);
         note_launch();
     }
     const int8_t *x = a.xidx ? a.xg : a.xl;
