@@ -243,6 +243,15 @@ bool tiles(int qtype, int mode, TileArgs a, cudaStream_t s) {
     return e == cudaSuccess;
 }
 
+// The cell that receives the digits in use of the next rows' planes, and one for that kernel to clear: a ring of eight, each cleared
+// four planes ahead of its use (one that was not, as in a short replayed graph, is only too large, which costs time and changes no result).
+struct DigitCell { int *nl, *clear; };
+DigitCell next_cell() {
+    static unsigned turn = 0;
+    turn++;
+    return {g_cells + 4 + (turn & 7), g_cells + 4 + ((turn + 4) & 7)};
+}
+
 // y[T,out_f] on device from x[T,K] on device.  check_flags: synchronise and re-run the exact kernel
 // if an activation left the limb envelope (host-pointer entries); otherwise flags stay raised.
 bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t *out, bool check_flags, cudaStream_t s,
@@ -256,18 +265,16 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
         int8_t *buf = (int8_t *)ensure(R_XL, (size_t)T * 8 * K);
         if (!buf) return false;
         if (T >= 2) {
-            if (cudaMemsetAsync(g_cells + 4, 0, sizeof(int), s) != cudaSuccess) return false;
-            x_nl = g_cells + 4;
-        }
-        if (launch_limbs(x, T, K, buf, g_flags, s, const_cast<int *>(x_nl)) != cudaSuccess) return false;
+            const DigitCell c = next_cell();
+            if (launch_limbs(x, T, K, buf, g_flags, s, c.nl, c.clear) != cudaSuccess) return false;
+            x_nl = c.nl;
+        } else if (launch_limbs(x, T, K, buf, g_flags, s) != cudaSuccess) return false;
         xl = buf;
     }
     bool done = false;
     if (T >= 2 && T >= g_tc_min_tokens && T < (1 << 24) && g_stage_mask == 0 && tile_scales(w.qtype, w.nb, w.maxd, w.maxdmin, fw)) {
-        int *off = (int *)ensure(R_META, 64);
-        if (!off || launch_set2(off, 0, (int)T, s) != cudaSuccess) return false;
         TileArgs ta = {};
-        ta.wa = w.cell; ta.wb = w.cell; ta.grp_off = off; ta.n_groups = 1; ta.nb = (int)w.nb; ta.n_rows = T; ta.out_f = w.out_f; ta.fw = fw;
+        ta.wa = w.cell; ta.wb = w.cell; ta.grp_off = nullptr; ta.n_groups = 1; ta.nb = (int)w.nb; ta.n_rows = T; ta.out_f = w.out_f; ta.fw = fw;
         ta.fa = 16; ta.xl = xl; ta.x_nl = x_nl; ta.out = out;
         done = tiles(w.qtype, MODE_LINEAR, ta, s);
     }
@@ -313,7 +320,7 @@ struct MoePlan {                      // everything the fused MoE kernels need o
 bool moe_fused(const MoePlan &p, const int8_t *hl, long long rows, const int *xidx, const int *grp_expert,
                const int *grp_off, int n_groups, long long n_pairs, int max_pairs, const int64_t *pair_gate,
                const int *pair_tok, int fa, int fw, int64_t *out, cudaStream_t s, const int *h_nl = nullptr,
-               unsigned maxd_gate = 0x7C00, unsigned maxdmin_gate = 0x7C00, unsigned maxd_down = 0x7C00, unsigned maxdmin_down = 0x7C00) {
+               unsigned maxd_gate = 0x7C00, unsigned maxdmin_gate = 0x7C00, unsigned maxd_down = 0x7C00, unsigned maxdmin_down = 0x7C00, bool gu_cleared = false) {
     int8_t *gul = (int8_t *)ensure(R_GUL, (size_t)n_pairs * 8 * p.e_ffn);
     if (!gul) return false;
     auto gateup_batch = [&] {
@@ -332,7 +339,7 @@ bool moe_fused(const MoePlan &p, const int8_t *hl, long long rows, const int *xi
     };
     if (!grp_expert && grp_off && g_stage_mask == 0) {
         // groups are the experts themselves: stream every touched expert tile once for all of its rows
-        if (cudaMemsetAsync(g_cells + 1, 0, sizeof(int), s) != cudaSuccess) return false;
+        if (!gu_cleared && cudaMemsetAsync(g_cells + 1, 0, sizeof(int), s) != cudaSuccess) return false;
         if (n_pairs >= 2 && rows >= g_tc_min_tokens && tile_scales(p.gate_q, p.d_model / 256, maxd_gate, maxdmin_gate, fw) &&
             tile_scales(p.down_q, p.e_ffn / 256, maxd_down, maxdmin_down, fw)) {
             TileArgs tg = {};
@@ -673,9 +680,10 @@ extern "C" int qk_apply_resident_grouped(const long long *handles, const int *ph
     const long long K = nb * 256;
     int64_t *xd = (int64_t *)ensure(R_X, (size_t)T * K * 8), *od = (int64_t *)ensure(R_OUT, (size_t)total * 8);
     int8_t *xl = (int8_t *)ensure(R_XL, (size_t)T * 8 * K);
-    int *nl = T > 1 ? g_cells + 4 : nullptr;
-    if (!xd || !od || !xl || !upload(xd, x, (size_t)T * K * 8) || (nl && cudaMemsetAsync(nl, 0, sizeof(int), g_stream) != cudaSuccess) ||
-        launch_limbs(xd, T, K, xl, g_flags, g_stream, nl) != cudaSuccess) { cudaGetLastError(); return 1; }
+    const DigitCell cell = T > 1 ? next_cell() : DigitCell{nullptr, nullptr};
+    int *nl = cell.nl;
+    if (!xd || !od || !xl || !upload(xd, x, (size_t)T * K * 8) ||
+        launch_limbs(xd, T, K, xl, g_flags, g_stream, nl, cell.clear) != cudaSuccess) { cudaGetLastError(); return 1; }
     // the products do not wait for the verdict on the digits: an activation beyond them repeats the call with the exact kernel
     for (int exact = 0; exact < 2; exact++) {
         long long off = 0;
@@ -844,15 +852,18 @@ extern "C" int iie_moe_forward_dev(long long layer, const int64_t *h_dev, long l
     int8_t *hl = (int8_t *)ensure(R_XL, (size_t)T * 8 * L.d_model);
     int64_t *lg = (int64_t *)ensure(R_LOGITS, (size_t)T * E * 8);
     if (!hl || !lg) return 1;
-    if (stage_on(ST_LIMBS) && (cudaMemsetAsync(g_cells, 0, sizeof(int), s) != cudaSuccess ||
-                               launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, g_cells) != cudaSuccess)) return 1;
+    // the kernel that splits the rows clears what the experts' kernels add to, too, unless that lies over the rows
+    const DigitCell cell = next_cell();
+    const long long n_out = T * L.d_model;
+    const bool apart = out_dev + n_out <= h_dev || h_dev + n_out <= out_dev, zero_here = !accumulate && stage_on(ST_LIMBS) && apart;
+    if (stage_on(ST_LIMBS) && launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, cell.nl, cell.clear, g_cells + 1, zero_here ? out_dev : nullptr, n_out) != cudaSuccess) return 1;
     if (stage_on(ST_ROUTER)) {
         if (r.qtype == QT_I64) {
             if (launch_exact_dense((const int64_t *)r.d, E, L.d_model, h_dev, T, fw, lg, g_flags, s) != cudaSuccess) return 1;
-        } else if (!linear_dev(r, h_dev, T, fw, lg, false, s, hl, g_cells)) return 1;
+        } else if (!linear_dev(r, h_dev, T, fw, lg, false, s, hl, cell.nl)) return 1;
     }
     if (stage_on(ST_TOPK) && launch_topk(lg, T, E, k, fa, ids, gates, s) != cudaSuccess) return 1;
-    if (!accumulate && cudaMemsetAsync(out_dev, 0, (size_t)T * L.d_model * 8, s) != cudaSuccess) return 1;
+    if (!accumulate && !zero_here && cudaMemsetAsync(out_dev, 0, (size_t)T * L.d_model * 8, s) != cudaSuccess) return 1;
     MoePlan plan = {L.tabs, L.tabs + E, L.tabs + 2 * E, L.gate_q, L.down_q, L.d_model, L.e_ffn};
     bool ok;
     if (T == 1) {
@@ -867,8 +878,8 @@ extern "C" int iie_moe_forward_dev(long long layer, const int64_t *h_dev, long l
         int *ptok = (int *)ensure(R_PAIRTOK, (size_t)P * sizeof(int));
         int64_t *pg = (int64_t *)ensure(R_PAIRGATE, (size_t)P * 8);
         if (!off || !ptok || !pg || launch_dispatch(ids, gates, T, k, E, off, ptok, pg, s) != cudaSuccess) return 1;
-        ok = moe_fused(plan, hl, T, ptok, nullptr, off, E, P, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, g_cells,
-                       L.maxd_gate, L.maxdmin_gate, L.maxd_down, L.maxdmin_down);
+        ok = moe_fused(plan, hl, T, ptok, nullptr, off, E, P, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, cell.nl,
+                       L.maxd_gate, L.maxdmin_gate, L.maxd_down, L.maxdmin_down, stage_on(ST_LIMBS));
     }
     if (!ok) { cudaGetLastError(); return 1; }
     return 0;
@@ -907,16 +918,18 @@ extern "C" int iie_moe_experts_dev(long long layer, const int64_t *h_dev, long l
     const long long P = T * slots;
     int8_t *hl = (int8_t *)ensure(R_XL, (size_t)T * 8 * L.d_model);
     if (!hl) return 1;
-    if (cudaMemsetAsync(g_cells, 0, sizeof(int), s) != cudaSuccess) return 1;
-    if (launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, g_cells) != cudaSuccess) return 1;
+    const DigitCell cell = next_cell();
+    const long long n_out = T * L.d_model;
+    const bool zero_here = !accumulate && (out_dev + n_out <= h_dev || h_dev + n_out <= out_dev);
+    if (launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, cell.nl, cell.clear, g_cells + 1, zero_here ? out_dev : nullptr, n_out) != cudaSuccess) return 1;
     int *off = (int *)ensure(R_GRPOFF, (size_t)(E + 2) * sizeof(int));
     int *ptok = (int *)ensure(R_PAIRTOK, (size_t)P * sizeof(int));
     int64_t *pg = (int64_t *)ensure(R_PAIRGATE, (size_t)P * 8);
     if (!off || !ptok || !pg || launch_dispatch(ids_dev, gates_dev, T, slots, E, off, ptok, pg, s, expert_base) != cudaSuccess) return 1;
-    if (!accumulate && cudaMemsetAsync(out_dev, 0, (size_t)T * L.d_model * 8, s) != cudaSuccess) return 1;
+    if (!accumulate && !zero_here && cudaMemsetAsync(out_dev, 0, (size_t)T * L.d_model * 8, s) != cudaSuccess) return 1;
     MoePlan plan = {L.tabs, L.tabs + E, L.tabs + 2 * E, L.gate_q, L.down_q, L.d_model, L.e_ffn};
-    if (!moe_fused(plan, hl, T, ptok, nullptr, off, E, P, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, g_cells,
-                   L.maxd_gate, L.maxdmin_gate, L.maxd_down, L.maxdmin_down)) {
+    if (!moe_fused(plan, hl, T, ptok, nullptr, off, E, P, (int)std::min<long long>(T, 4), pg, ptok, fa, fw, out_dev, s, cell.nl,
+                   L.maxd_gate, L.maxdmin_gate, L.maxd_down, L.maxdmin_down, true)) {
         cudaGetLastError(); return 1;
     }
     return 0;

@@ -174,7 +174,7 @@ cudaError_t launch_batch(int qtype, int mode, const BatchArgs &a, cudaStream_t s
 struct TileArgs {
     const uint8_t *const *wa;      // per group: linear / down weight, or gate
     const uint8_t *const *wb;      // per group: up weight (MODE_GATEUP)
-    const int *grp_off;            // device [n_groups + 1]
+    const int *grp_off;            // device [n_groups + 1]; nullptr: one group of all n_rows
     int n_groups, nb;              // nb: 256-column super-blocks
     long long n_rows;              // upper bound of grp_off[n_groups]
     long long out_f;
@@ -210,7 +210,8 @@ cudaError_t launch_unpack(const uint8_t *src, uint8_t *raw, long long out_f, lon
 
 // int64 rows -> balanced base-256 limb planes [row][8][K]; sets flags bit 0 on overflow.
 cudaError_t launch_limbs(const int64_t *x, long long n_rows, long long K, int8_t *planes, int *flags, cudaStream_t s,
-                         int *nl_out = nullptr);   // nl_out: atomicMax of the limbs in use (caller zeroes)
+                         int *nl_out = nullptr,    // nl_out: atomicMax of the limbs in use (zero before)
+                         int *clear0 = nullptr, int *clear1 = nullptr, int64_t *zero = nullptr, long long zero_n = 0);   // words that later kernels find zeroed
 
 // p[0] = a, p[1] = b on the stream (kernel arguments travel by value, so a captured launch replays correctly where a
 // copy from a host stack variable would not)

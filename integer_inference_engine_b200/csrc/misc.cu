@@ -47,8 +47,15 @@ __global__ void repack_kernel(const uint8_t *src, uint8_t *dst, long long out_f,
 // ---------------------------------------------------------------------------------------------------
 // activation limb planes
 // ---------------------------------------------------------------------------------------------------
-__global__ void limbs_kernel(const int64_t *x, long long n_rows, long long K, int8_t *planes, int *flags, int *nl_out) {
+struct LimbClears { int *a, *b; int64_t *zero; long long zero_n; };
+__device__ __forceinline__ void limb_clears(const LimbClears &c) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) { if (c.a) *c.a = 0; if (c.b) *c.b = 0; }
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < c.zero_n; i += (long long)gridDim.x * blockDim.x) c.zero[i] = 0;
+}
+
+__global__ void limbs_kernel(const int64_t *x, long long n_rows, long long K, int8_t *planes, int *flags, int *nl_out, const LimbClears clears) {
     pdl_enter();
+    limb_clears(clears);
     const long long total = n_rows * K;
     bool bad = false;
     int nl = 0;
@@ -70,8 +77,9 @@ __global__ void limbs_kernel(const int64_t *x, long long n_rows, long long K, in
 // The same for K a multiple of 8: a thread takes eight consecutive columns (64 bytes in), transposes the 8 x 8 digit
 // bytes in registers and writes eight bytes to each plane.
 __global__ void __launch_bounds__(256) limbs8_kernel(const int64_t *x, long long n_rows, long long K, int8_t *planes,
-                                                     int *flags, int *nl_out) {
+                                                     int *flags, int *nl_out, const LimbClears clears) {
     pdl_enter();
+    limb_clears(clears);
     const long long per_row = K >> 3, total = n_rows * per_row;
     bool bad = false;
     uint64_t seen = 0;
@@ -539,11 +547,12 @@ cudaError_t launch_add_rows(const int64_t *a, const int64_t *b, int64_t *out, lo
 }
 
 cudaError_t launch_limbs(const int64_t *x, long long n_rows, long long K, int8_t *planes, int *flags, cudaStream_t s,
-                         int *nl_out) {
+                         int *nl_out, int *clear0, int *clear1, int64_t *zero, long long zero_n) {
+    const LimbClears clears = {clear0, clear1, zero, zero ? zero_n : 0};
     if (K % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(planes) & 7) == 0)
-        launch_behind(limbs8_kernel, grid_for(n_rows * (K >> 3), 256), 256, 0, s, x, n_rows, K, planes, flags, nl_out);
+        launch_behind(limbs8_kernel, grid_for(n_rows * (K >> 3), 256), 256, 0, s, x, n_rows, K, planes, flags, nl_out, clears);
     else
-        launch_behind(limbs_kernel, grid_for(n_rows * K, 256), 256, 0, s, x, n_rows, K, planes, flags, nl_out);
+        launch_behind(limbs_kernel, grid_for(n_rows * K, 256), 256, 0, s, x, n_rows, K, planes, flags, nl_out, clears);
     note_launch();
     return cudaGetLastError();
 }

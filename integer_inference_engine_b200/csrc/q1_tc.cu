@@ -127,7 +127,6 @@ __device__ __forceinline__ int qc_planes(int nl, bool narrow) { return nl <= 3 &
 
 template <int NT, typename DT>
 __global__ void __launch_bounds__(qc_threads(NT), 1) q1_tc_kernel(const Q1TcArgs a, const __grid_constant__ CUtensorMap xmap) {
-    pdl_enter();
     constexpr int US = 256 + 16 * (int)sizeof(DT);
     constexpr int RAW_BYTES = 8 * QC_CHUNK * US;                   // eight 16-row sub-tiles x eight blocks
     constexpr int QC_READ = qc_read_warps(NT), QC_MMA_WARP = QC_READ + QC_EXPAND, QC_PLANE_WARP = QC_MMA_WARP + 1;
@@ -141,6 +140,18 @@ __global__ void __launch_bounds__(qc_threads(NT), 1) q1_tc_kernel(const Q1TcArgs
     __shared__ int s_abort;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nb = a.nb;
+    if (tid == 0) {
+        s_abort = 0;
+        for (int s = 0; s < QC_MAX_STAGES; s++) { qc_init(full_bar + 8 * s, QC_EXPAND + 1); qc_init(empty_bar + 8 * s, 1); }
+        for (int s = 0; s < 4; s++) { qc_init(acc_bar + 8 * s, 1); qc_init(free_bar + 8 * s, QC_READ); }
+        for (int s = 0; s < QC_RAW_SLOTS; s++) { qc_init(raw_full + 8 * s, 1); qc_init(raw_empty + 8 * s, QC_READ); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == QC_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(qc_u32(&s_tmem)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    pdl_enter();                                                   // what stands above needs nothing of the kernel before
     const int np = qc_planes(max(1, min(8, *a.nl_dev)), a.narrow);           // uniform over the grid
     const int cols = np * NT;                                      // TMEM columns of one buffer
     const int nbuf = cols <= 128 ? 4 : cols <= 256 ? 2 : 1, buf_cols = 512 / nbuf;
@@ -157,17 +168,6 @@ __global__ void __launch_bounds__(qc_threads(NT), 1) q1_tc_kernel(const Q1TcArgs
     } else {
         u0 = 0; u1 = blockIdx.x < a.n_tiles ? (a.n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x * nb : 0;
         t0 = blockIdx.x; tstep = gridDim.x;
-    }
-    if (tid == 0) {
-        s_abort = 0;
-        for (int s = 0; s < QC_MAX_STAGES; s++) { qc_init(full_bar + 8 * s, QC_EXPAND + 1); qc_init(empty_bar + 8 * s, 1); }
-        for (int s = 0; s < 4; s++) { qc_init(acc_bar + 8 * s, 1); qc_init(free_bar + 8 * s, QC_READ); }
-        for (int s = 0; s < QC_RAW_SLOTS; s++) { qc_init(raw_full + 8 * s, 1); qc_init(raw_empty + 8 * s, QC_READ); }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == QC_MMA_WARP) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(qc_u32(&s_tmem)), "r"(512));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -131,7 +131,6 @@ struct TileMaps { CUtensorMap x16, x32, s16, s32; };               // planes and
 
 template <int QT, int MODE>
 __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArgs a, const __grid_constant__ TileMaps maps) {
-    pdl_enter();
     constexpr bool Q4 = QT == QT_Q4K;
     constexpr int HTB = Q4 ? HTB_Q4K : HTB_Q6K, RAW_BYTES = 16 * HTB;
     constexpr int NROW = MODE == MODE_GATEUP ? 64 : 128;           // output rows of a tile
@@ -145,6 +144,17 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
                    raw_full = free_bar + 8 * 4, raw_empty = raw_full + 8 * TL_MAX_RAW, y_full = raw_empty + 8 * TL_MAX_RAW, y_free = y_full + 8;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int nb = a.nb;
+    if (warp == TL_X_WARP && lane == 0) {                          // the tensor maps' first use would wait for them
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x16)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x32)) : "memory");
+        if (Q4) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.s16)) : "memory");
+        if (Q4) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.s32)) : "memory");
+    }
+    if (warp == TL_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tl_u32(&s_tmem)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    pdl_enter();                                                   // what stands above needs nothing of the kernel before
     const int np = tl_planes(a.x_nl ? max(1, min(8, *a.x_nl)) : 8), ns = np + 1;        // uniform over the grid
     const bool wide = np == 3 && a.wide;
     const int bn = wide ? 32 : 16;
@@ -166,7 +176,8 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         int base = 0;
         for (int g0 = 0; g0 < a.n_groups; g0 += 32) {
             const int g = g0 + lane;
-            const int at = g < a.n_groups ? a.grp_off[g] : 0, rows = g < a.n_groups ? a.grp_off[g + 1] - at : 0;
+            const int at = g < a.n_groups && a.grp_off ? a.grp_off[g] : 0;
+            const int rows = g < a.n_groups ? (a.grp_off ? a.grp_off[g + 1] - at : (int)a.n_rows) : 0;
             const int nt = (rows + bn - 1) / bn * n_rt;
             int incl = nt;
 #pragma unroll
@@ -188,14 +199,6 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
                               : Q4 && MODE == MODE_DOWN ? (np <= 5 ? 4 : 7) : Q4 && MODE == MODE_LINEAR ? (np == 3 ? 5 : np <= 5 ? 6 : 7) : 7;
             atomicAdd(&d_tile_launches[shape], 1ULL);
         }
-    }
-    if (warp == TL_X_WARP && lane == 0) {                          // the tensor maps' first use would wait for them
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(wide ? &maps.x32 : &maps.x16)) : "memory");
-        if (Q4) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(wide ? &maps.s32 : &maps.s16)) : "memory");
-    }
-    if (warp == TL_MMA_WARP) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tl_u32(&s_tmem)), "r"(512));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -605,7 +608,7 @@ __global__ void __launch_bounds__(256) tile_rows_kernel(const int8_t *xl, const 
     const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
     const int j = (int)(idx % stride);
     const long long row = idx / stride;
-    if (row >= n_rows || row >= *n_live) return;
+    if (row >= n_rows || (n_live && row >= *n_live)) return;
     const int np = tl_planes(x_nl ? max(1, min(8, *x_nl)) : 8);
     const long long K = (long long)nb * 256;
     int8_t *to = xs ? xs + row * 9 * stride + j : nullptr;
@@ -676,7 +679,7 @@ size_t tile_sums_bytes(long long rows, long long n_blocks) { return (size_t)rows
 
 cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t s) {
     TileArgs a = args;
-    if (a.nb <= 0 || a.nb > 64 || a.n_groups <= 0 || a.n_groups > TL_MAX_GROUPS || a.out_f <= 0 || a.n_rows <= 0 || a.n_rows > (1 << 28) ||
+    if (a.nb <= 0 || a.nb > 64 || a.n_groups <= 0 || a.n_groups > TL_MAX_GROUPS || a.out_f <= 0 || a.n_rows <= 0 || a.n_rows > (1 << 28) || (!a.grp_off && a.n_groups != 1) ||
         (reinterpret_cast<uintptr_t>(a.xl) & 15) || (a.xidx && !a.xg) || !tl_encode()) return cudaErrorNotSupported;
     if (qtype != QT_Q4K && !(qtype == QT_Q6K && mode != MODE_GATEUP)) return cudaErrorNotSupported;
     if (qtype == QT_Q4K && !a.xs) return cudaErrorInvalidValue;
@@ -687,7 +690,7 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
     const bool q4 = qtype == QT_Q4K;
     if (q4 || a.xidx) {
         const long long n = a.n_rows * stride;
-        launch_behind(tile_rows_kernel, (unsigned)((n + 255) / 256), 256, 0, s, a.xl, a.xidx, a.grp_off + a.n_groups, a.x_nl, a.n_rows, a.nb, stride, a.xg, q4 ? a.xs : nullptr);
+        launch_behind(tile_rows_kernel, (unsigned)((n + 255) / 256), 256, 0, s, a.xl, a.xidx, a.grp_off ? a.grp_off + a.n_groups : nullptr, a.x_nl, a.n_rows, a.nb, stride, a.xg, q4 ? a.xs : nullptr);
         note_launch();
     }
     const int8_t *x = a.xidx ? a.xg : a.xl;
