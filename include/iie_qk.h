@@ -210,6 +210,12 @@ int iie_attn_decode_batch_dev(const int64_t *q_dev, const int64_t *k_dev, const 
                               int32_t *vcache_dev, long long pos, long long n_seqs, long long seq_stride, long long window,
                               const int64_t *cos_dev, const int64_t *sin_dev, int rope, int n_heads, int n_kv, int head_dim,
                               long long cache_rows, int fa, long long inv_sqrt, int64_t *out_dev, void *stream);
+/* The same with rows that lie apart (column slices of one [q | k | v] matrix): q_ld, kv_ld = distance of the rows of q and of k and v.
+ * 3: a shape that the one-launch form does not carry; use dense rows. */
+int iie_attn_decode_batch_rows_dev(const int64_t *q_dev, const int64_t *k_dev, const int64_t *v_dev, int32_t *kcache_dev,
+                                   int32_t *vcache_dev, long long q_ld, long long kv_ld, long long pos, long long n_seqs, long long seq_stride,
+                                   long long window, const int64_t *cos_dev, const int64_t *sin_dev, int rope, int n_heads, int n_kv,
+                                   int head_dim, long long cache_rows, int fa, long long inv_sqrt, int64_t *out_dev, void *stream);
 /* The attention half of a decoder block for ONE token, accumulated into the residual row:
  *   x_dev [d_model] += (attention(q, cache) Wo^T), with [q | k | v] = h Wqkv^T,
  * where h is the normalised row whose digit planes the LAST single-token iie_moe_block_dev / iie_moe_forward_dev

@@ -1055,8 +1055,9 @@ extern "C" int iie_attn_prefill_dev(const int64_t *q_dev, const int64_t *k_dev, 
     return 0;
 }
 
-extern "C" int iie_attn_decode_batch_dev(const int64_t *q_dev, const int64_t *k_dev, const int64_t *v_dev, int32_t *kcache_dev,
-                                         int32_t *vcache_dev, long long pos, long long n_seqs, long long seq_stride, long long window,
+// q_ld / kv_ld: distance of the rows of q and of k, v, 0 for dense rows; others go with the cluster form only (3 where the shape is not its)
+static int decode_batch(const int64_t *q_dev, const int64_t *k_dev, const int64_t *v_dev, int32_t *kcache_dev,
+                                         int32_t *vcache_dev, long long q_ld, long long kv_ld, long long pos, long long n_seqs, long long seq_stride, long long window,
                                          const int64_t *cos_dev, const int64_t *sin_dev, int rope, int n_heads, int n_kv, int head_dim,
                                          long long cache_rows, int fa, long long inv_sqrt, int64_t *out_dev, void *stream) {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
@@ -1070,12 +1071,14 @@ extern "C" int iie_attn_decode_batch_dev(const int64_t *q_dev, const int64_t *k_
     a.q = q_dev; a.k = k_dev; a.v = v_dev; a.kcache = kcache_dev; a.vcache = vcache_dev; a.pos = pos; a.window = window;
     a.Lmax = cache_rows; a.Ls = Ls; a.cos = cos_dev; a.sin = sin_dev; a.rope = rope; a.H = n_heads; a.Hkv = n_kv; a.hd = head_dim;
     attn_consts(a, fa, inv_sqrt);
+    a.q_ld = q_ld; a.kv_ld = kv_ld;
     a.out = out_dev; a.flags = g_flags;
     int n_c = 0, tiles = 0;
     if (g_attn_fused == 1 && attn_shape_ok(a.H, a.Hkv, a.hd) && attn_cluster_plan(a, n_c, tiles)) {      // needs no scratch
         if (launch_attn_prefill(a, s) != cudaSuccess) { cudaGetLastError(); return 1; }
         return 0;
     }
+    if (q_ld || kv_ld) return 3;
     // scratch roles of their own (a captured single-token step keeps the addresses of the single-token buffers)
     int64_t *scores = (int64_t *)ensure(R_BSCORES, (size_t)n_seqs * n_heads * Ls * 8);
     int32_t *e = (int32_t *)ensure(R_BEXP, (size_t)n_seqs * n_heads * Ls * 4);
@@ -1092,6 +1095,23 @@ extern "C" int iie_attn_decode_batch_dev(const int64_t *q_dev, const int64_t *k_
     }
     if (launch_attn_prefill(a, s) != cudaSuccess) { cudaGetLastError(); return 1; }
     return 0;
+}
+
+extern "C" int iie_attn_decode_batch_dev(const int64_t *q_dev, const int64_t *k_dev, const int64_t *v_dev, int32_t *kcache_dev,
+                                         int32_t *vcache_dev, long long pos, long long n_seqs, long long seq_stride, long long window,
+                                         const int64_t *cos_dev, const int64_t *sin_dev, int rope, int n_heads, int n_kv, int head_dim,
+                                         long long cache_rows, int fa, long long inv_sqrt, int64_t *out_dev, void *stream) {
+    return decode_batch(q_dev, k_dev, v_dev, kcache_dev, vcache_dev, 0, 0, pos, n_seqs, seq_stride, window, cos_dev, sin_dev, rope, n_heads, n_kv, head_dim, cache_rows,
+                        fa, inv_sqrt, out_dev, stream);
+}
+
+extern "C" int iie_attn_decode_batch_rows_dev(const int64_t *q_dev, const int64_t *k_dev, const int64_t *v_dev, int32_t *kcache_dev,
+                                         int32_t *vcache_dev, long long q_ld, long long kv_ld, long long pos, long long n_seqs, long long seq_stride, long long window,
+                                         const int64_t *cos_dev, const int64_t *sin_dev, int rope, int n_heads, int n_kv, int head_dim,
+                                         long long cache_rows, int fa, long long inv_sqrt, int64_t *out_dev, void *stream) {
+    if (q_ld < (long long)n_heads * head_dim || kv_ld < (long long)n_kv * head_dim) return 1;
+    return decode_batch(q_dev, k_dev, v_dev, kcache_dev, vcache_dev, q_ld, kv_ld, pos, n_seqs, seq_stride, window, cos_dev, sin_dev, rope, n_heads, n_kv, head_dim, cache_rows,
+                        fa, inv_sqrt, out_dev, stream);
 }
 
 // ---- attention bank (north-mini-code/tools/nmc_qk_cuda.cu:877-1551): request-scoped K/V rows on the device and the

@@ -1230,27 +1230,32 @@ __global__ void embed_row_kernel(const uint8_t *w, int qtype, long long nb, cons
     out[i] = val;
 }
 
-// arg-max of each of grid.x rows of n values, lowest index on ties: one CTA per row
+// arg-max of each of grid.x rows of n values, lowest index on ties: the grid.y CTAs of a cluster share a row and hand their candidates to
+// the first.  Bounded by the load latency of a CTA (7 rows of 151936: 21 us with one CTA a row).
+constexpr int AR_PARTS = 8;
+
 __global__ void __launch_bounds__(1024) argmax_rows_kernel(const int64_t *x, long long n, int *out) {
     __shared__ long long s_v[32];
     __shared__ long long s_i[32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ long long s_part[2][AR_PARTS];                       // the first CTA's: every CTA's candidate
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, parts = (int)gridDim.y;
     const int64_t *row = x + (long long)blockIdx.x * n;
+    const long long share = ((n + parts - 1) / parts + 1) & ~1LL, from = min(n, share * blockIdx.y), to = min(n, from + share);
     long long bv = INT64_MIN, bi = n;
     auto better = [](long long ov, long long oi, long long v, long long i) { return ov > v || (ov == v && oi < i); };
-    long long i = tid * 2LL;
+    long long i = from + tid * 2LL;
     if ((reinterpret_cast<uintptr_t>(row) & 15) == 0)
-        for (; i + 1 < n; i += 2048) {                              // two values per load
+        for (; i + 1 < to; i += 2048) {                              // two values per load
             const longlong2 v = *reinterpret_cast<const longlong2 *>(row + i);
             if (better(v.x, i, bv, bi)) { bv = v.x; bi = i; }
             if (better(v.y, i + 1, bv, bi)) { bv = v.y; bi = i + 1; }
         }
     else
-        for (; i + 1 < n; i += 2048) {
+        for (; i + 1 < to; i += 2048) {
             if (better(row[i], i, bv, bi)) { bv = row[i]; bi = i; }
             if (better(row[i + 1], i + 1, bv, bi)) { bv = row[i + 1]; bi = i + 1; }
         }
-    if (i < n && better(row[i], i, bv, bi)) { bv = row[i]; bi = i; }
+    if (i < to && better(row[i], i, bv, bi)) { bv = row[i]; bi = i; }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) {
         const long long ov = __shfl_xor_sync(0xffffffffu, bv, s), oi = __shfl_xor_sync(0xffffffffu, bi, s);
@@ -1265,7 +1270,20 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const int64_t *x, lon
             const long long ov = __shfl_xor_sync(0xffffffffu, bv, s), oi = __shfl_xor_sync(0xffffffffu, bi, s);
             if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
         }
-        if (lane == 0) out[blockIdx.x] = (int)bi;
+        if (lane == 0 && parts == 1) out[blockIdx.x] = (int)bi;
+        if (lane == 0 && parts > 1) {
+            cg::cluster_group cluster = cg::this_cluster();
+            *cluster.map_shared_rank(&s_part[0][blockIdx.y], 0) = bv;
+            *cluster.map_shared_rank(&s_part[1][blockIdx.y], 0) = bi;
+        }
+    }
+    if (parts > 1) {
+        cg::this_cluster().sync();
+        if (blockIdx.y == 0 && tid == 0) {
+            for (int p = 1; p < parts; p++)
+                if (better(s_part[0][p], s_part[1][p], bv, bi)) { bv = s_part[0][p]; bi = s_part[1][p]; }
+            out[blockIdx.x] = (int)bi;
+        }
     }
 }
 
@@ -1497,7 +1515,15 @@ cudaError_t launch_embed_rows(const uint8_t *w, int qtype, long long nb, const i
 
 cudaError_t launch_argmax_rows(const int64_t *x, long long rows, long long n, int *out, cudaStream_t s) {
     if (n <= 0 || rows <= 0 || rows > 0x7fffffffLL) return cudaErrorInvalidValue;
-    argmax_rows_kernel<<<(unsigned)rows, 1024, 0, s>>>(x, n, out);
+    const int parts = rows <= 128 && n >= 32768 ? AR_PARTS : 1;       // (a share of a short row is less than a CTA's start; many rows fill the SMs)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)rows, (unsigned)parts); cfg.blockDim = dim3(1024); cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = (unsigned)parts; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_rows_kernel, x, n, out);
+    if (e != cudaSuccess) return e;
     note_launch();
     return cudaGetLastError();
 }

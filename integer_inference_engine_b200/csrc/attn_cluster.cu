@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
     if (tid == 0) s_wide = 0;
     if (lane < AC_HEADS) s_base[warp][lane] = 0;                            // (no tile: never used)
     // ---- per-head norms where the caller wants them here, rotation, bytes of the queries; the new row into the cache ----------------
-    const int64_t *q_in = a.q + (long long)seq * a.H * HD + (long long)kv * rep * HD, *k_in = a.k + ((long long)seq * a.Hkv + kv) * HD;
-    const int64_t *v_in = a.v + ((long long)seq * a.Hkv + kv) * HD;
+    const long long kv_row = (long long)seq * (a.kv_ld ? a.kv_ld : (long long)a.Hkv * HD) + (long long)kv * HD;
+    const int64_t *q_in = a.q + (long long)seq * (a.q_ld ? a.q_ld : (long long)a.H * HD) + (long long)kv * rep * HD, *k_in = a.k + kv_row, *v_in = a.v + kv_row;
     if (a.qgain) {
         for (int r = warp; r < rep + (own ? 1 : 0); r += AC_WARPS) {
             const int64_t *src = r == rep ? k_in : q_in + r * HD, *gain = r == rep ? a.kgain : a.qgain;

@@ -257,6 +257,7 @@ cudaError_t launch_dispatch(const int *ids, const int64_t *gates, long long T, i
 struct AttnArgs {
     const int64_t *q;              // [H*hd] projected query (rotated on the fly, not modified)
     const int64_t *k, *v;          // [Hkv*hd] projected key / value of the new token
+    long long q_ld, kv_ld;         // cluster form: distance of the sequences' rows of q and of k, v (0: dense)
     int32_t *kcache, *vcache;      // [Hkv][Lmax][hd]
     long long pos, lo, Lmax;       // position of the new token (an upper bound when pos_dev is set), first visible key
                                    // (computed on the device), cache rows

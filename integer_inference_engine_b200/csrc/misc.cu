@@ -219,23 +219,29 @@ __global__ void topk_kernel(const int64_t *logits, long long rows, int n_experts
     if (row >= rows) return;
     const int64_t *lr = logits + row * n_experts;
     unsigned taken = 0;                                   // bit i: element lane + 32*i already selected
-    for (int r = 0; r < k; r++) {
-        int64_t best = INT64_MIN; int best_id = 0x7fffffff;
-        for (int i = 0, e = lane; e < n_experts; i++, e += 32) {
-            if (taken & (1u << i)) continue;
-            const int64_t v = lr[e];
-            if (best_id == 0x7fffffff || v > best) { best = v; best_id = e; }   // ascending e: ties keep the lower id
+    // a round finds the largest high word, among those the largest low word, among those the lowest id (three warp reductions); the gates of 32
+    // rounds are computed side by side
+    for (int r0 = 0; r0 < k; r0 += 32) {
+        int64_t mine = 0; int mine_id = -1;               // of round r0 + lane
+        for (int r = r0; r < min(k, r0 + 32); r++) {
+            int64_t best = INT64_MIN; int best_id = 0x7fffffff;
+            for (int i = 0, e = lane; e < n_experts; i++, e += 32) {
+                if (taken & (1u << i)) continue;
+                const int64_t v = lr[e];
+                if (best_id == 0x7fffffff || v > best) { best = v; best_id = e; }   // ascending e: ties keep the lower id
+            }
+            const unsigned open = __ballot_sync(0xffffffffu, best_id != 0x7fffffff);
+            const bool have = best_id != 0x7fffffff;
+            const int hi = __reduce_max_sync(0xffffffffu, have ? (int)(best >> 32) : INT32_MIN);
+            const bool at_hi = have && (int)(best >> 32) == hi;
+            const unsigned lo = __reduce_max_sync(0xffffffffu, at_hi ? (unsigned)best : 0u);
+            const int id = (int)__reduce_min_sync(0xffffffffu, at_hi && (unsigned)best == lo ? (unsigned)best_id : 0x7fffffffu);
+            if (open && (id & 31) == lane) taken |= 1u << (id >> 5);
+            if (lane == r - r0) { mine = (int64_t)(((uint64_t)(uint32_t)hi << 32) | lo); mine_id = open ? id : -1; }
         }
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1) {
-            const int64_t ov = __shfl_xor_sync(0xffffffffu, best, s);
-            const int oi = __shfl_xor_sync(0xffffffffu, best_id, s);
-            if (oi != 0x7fffffff && (best_id == 0x7fffffff || ov > best || (ov == best && oi < best_id))) { best = ov; best_id = oi; }
-        }
-        if (best_id != 0x7fffffff && (best_id & 31) == lane) taken |= 1u << (best_id >> 5);
-        if (lane == 0) {
-            ids[row * k + r] = best_id == 0x7fffffff ? -1 : best_id;
-            gates[row * k + r] = best_id == 0x7fffffff ? 0 : sigmoid_fixed(best, fa);
+        if (r0 + lane < k) {
+            ids[row * k + r0 + lane] = mine_id;
+            gates[row * k + r0 + lane] = mine_id < 0 ? 0 : sigmoid_fixed(mine, fa);
         }
     }
 }

@@ -91,17 +91,17 @@ class ExpertParallelDecoder:
             a, full = self.attn[li], self.layer_is_full(li)
             h = device.rmsnorm(x, self.stack.gains[li], fa, 1)
             qkv = device.apply(a["wqkv"], h, qd + 2 * kd, fw)
-            att = device.attention_decode_batch(qkv[:, :qd].contiguous(), qkv[:, qd:qd + kd].contiguous(), qkv[:, qd + kd:].contiguous(),
+            att = device.attention_decode_batch(qkv[:, :qd], qkv[:, qd:qd + kd], qkv[:, qd + kd:],
                                                 a["k"], a["v"], self.position, self.H, self.Hkv, self.hd, fa, 0 if full else self.window,
                                                 self.cos, self.sin, 0 if full else 1)
             ao = device.apply(a["wo"], att, self.d, fw)
             if self.blocks[li] is None:
-                moe, _, _ = self.stack.layers[li].forward(h, fa, fw)
+                self.stack.layers[li].forward(h, fa, fw, out=ao, accumulate=True, want_routes=False)      # both halves into one row
             else:
                 moe, _, _ = self.blocks[li].forward(h)
                 self.a2a_bytes_per_block = self.blocks[li].bytes_sent_last
+                x += moe
             x += ao
-            x += moe
         return x
 
     def step(self) -> None:

@@ -1,5 +1,5 @@
 """Attention by clusters against the three-launch form: edges of tiles, warps and clusters, windows, head shapes, scores beyond 32 bits (their
-base moves), queries beyond int32, probabilities of three bytes."""
+base moves), queries beyond int32, probabilities of three bytes; and the other small kernels of a step of several rows."""
 import numpy as np
 import pytest
 
@@ -43,3 +43,51 @@ def test_cluster_form_gives_the_same_bytes(pos, H, Hkv, hd, window, rope, bits, 
     assert flags & ~4 == 0                                             # (a rotated key of 2^30 and more may not fit the cache)
     for a, b in zip(*results):
         assert np.array_equal(a, b)
+
+
+def test_column_slices_as_rows():
+    import torch
+
+    from integer_inference_engine_b200 import device
+    B, H, Hkv, hd, pos = 3, 8, 2, 128, 77
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    qkv = torch.randint(-(1 << 18), 1 << 18, (B, (H + 2 * Hkv) * hd), generator=gen, device="cuda", dtype=torch.int64)
+    kc = torch.randint(-(1 << 18), 1 << 18, (B, Hkv, pos + 1, hd), generator=gen, device="cuda", dtype=torch.int32)
+    parts = qkv[:, :H * hd], qkv[:, H * hd:(H + Hkv) * hd], qkv[:, (H + Hkv) * hd:]
+    caches = [(kc.clone(), kc.flip(0).contiguous()) for _ in range(2)]
+    a = device.attention_decode_batch(*parts, *caches[0], pos, H, Hkv, hd)
+    b = device.attention_decode_batch(*(p.contiguous() for p in parts), *caches[1], pos, H, Hkv, hd)
+    assert torch.equal(a, b) and all(torch.equal(x, y) for x, y in zip(*caches))
+
+
+@pytest.mark.parametrize(("rows", "n"), [(1, 32768), (7, 151936), (3, 100001), (128, 32769), (129, 40000)])
+def test_argmax_rows_shared_by_a_cluster(rows, n):
+    import torch
+
+    from integer_inference_engine_b200 import device
+    x = torch.randint(-50, 50, (rows, n), generator=torch.Generator(device="cuda").manual_seed(n), device="cuda", dtype=torch.int64)
+    x[:, n - 1] = 50
+    x[0, n // 2] = 50                                                   # ties: the lower index
+    assert device.argmax_rows(x).cpu().tolist() == np.argmax(x.cpu().numpy(), axis=1).tolist()
+
+
+@pytest.mark.parametrize(("experts", "k"), [(5, 5), (128, 8), (300, 40), (1024, 64)])
+def test_topk_order_ties_and_gates(experts, k):
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    from oracle import qk_oracle as o
+    rng = np.random.default_rng(experts + k)
+    rows, d = 9, 256
+    h = rng.integers(-(1 << 20), 1 << 20, size=(rows, d), dtype=np.int64)
+    router = rng.integers(-(1 << 14), 1 << 14, size=(experts, d), dtype=np.int64)
+    router[experts // 2:] = router[:experts - experts // 2]             # equal logits
+    handle = qk_cuda.register_i64(router)
+    device.read_flags()
+    ids, gates = device.route(handle, k, torch.from_numpy(h).cuda(), 16, 24)
+    logits = o.linear(h, router, 24)
+    want = np.stack([o.topk_lowidx(r, k) for r in logits])
+    assert np.array_equal(ids.cpu().numpy(), want)
+    assert np.array_equal(gates.cpu().numpy(), np.stack([o.sigmoid_fixed(logits[t][want[t]].astype(np.int64), 16) for t in range(rows)]))
+    assert device.read_flags() == 0
+    qk_cuda.free_all()
