@@ -288,13 +288,13 @@ int iie_rmsnorm_dev(long long gain_h, const int64_t *x_dev, long long rows, long
 void iie_profile_stage_mask(int mask);
 /* Switch programmatic dependent launch between the three single-token kernels on (default) or off. */
 void iie_set_pdl(int enabled);
-/* Token count from which iie_moe_forward_dev uses the tcgen05 grouped GEMMs instead of the streamed
- * kernels (default 32; a very large value disables the tensor-core path). */
+/* Row count from which products use the tcgen05 tiles instead of the streamed kernels (default 2; a very large
+ * value disables the tensor-core path). */
 void iie_set_tc_min_tokens(long long tokens);
 unsigned long long iie_launch_count(void);
 /* Launches of each tensor-core (tcgen05) tile shape since load, so a test can tell which shape served a call:
  * out[0..6] = Q4_K gate/up with 3 / 4 activation digits, Q6_K down with 5 / 6, Q4_K down with 5, Q4_K linear with
- * 3 / 5.  Returns 7, or -1 when capacity < 7. */
+ * 3 / 5; out[7] every other.  Returns the number of entries, or -1 when capacity is too small. */
 int iie_prefill_launch_counts(unsigned long long *out, int capacity);
 /* Workspace generation: changes whenever a scratch buffer of the library is freed (to grow, by
  * qk_moe_workspace_release or qk_free_all).  A CUDA graph captured over iie_*_dev calls holds the scratch addresses of
