@@ -830,13 +830,13 @@ def run_prefill(args):
         nl_gu = 3 if shapes[0] else 4
         nl_dn = 5 if shapes[2] else 6
         algorithmic = 2.0 * 3 * pair_macs
-        issued = 2.0 * pair_macs * (2 * nl_gu * 4 + nl_dn * 5)
+        issued = 2.0 * pair_macs * (2 * nl_gu * 2 + nl_dn * 2)
         blk_s = ms_step / args.layers * 1e-3
-        roofline = {"bound": "tensor", "kernel": "prefill_kernel gate/up + down of one MoE block (router, sort and digit planes included in the time)",
+        roofline = {"bound": "tensor", "kernel": "tile_kernel gate/up + down of one MoE block (router, sort and digit planes included in the time)",
                     "unit": "TOP/s", "peak": i8["sustained_tops"], "peak_kind": "int8 GEMM measured in this run (torch._int_mm, sustained)",
                     "achieved": algorithmic / blk_s / 1e12, "frac": algorithmic / blk_s / 1e12 / i8["sustained_tops"],
                     "issued_achieved": issued / blk_s / 1e12, "issued_frac": issued / blk_s / 1e12 / i8["sustained_tops"],
-                    "digits": {"gate_up": {"activation": nl_gu, "weight": 4}, "down": {"activation": nl_dn, "weight": 5}},
+                    "digits": {"gate_up": {"activation": nl_gu, "weight": 2}, "down": {"activation": nl_dn, "weight": 2}},
                     "tile_launches": shapes, "traffic": None}
         cpu = {"value": len(rows) / cpu_s / args.layers, "unit": "tok/s", "cores": host_cores(), "kind": "port",
                "sample": f"{len(rows)} rows through router, top-{TOP_K} and their {TOP_K} experts of one block on the CPU oracle, scaled to {args.layers} blocks (rows are independent)"}

@@ -679,7 +679,9 @@ __device__ __forceinline__ bool af_group_barrier(unsigned *counter, unsigned tar
 }
 
 // NORM: the per-head norms of queries and key first (a form of its own: their code costs the others about 1 us a launch)
-template <bool NORM>
+// CLUSTER: the chunks of a KV head are one cluster (short spans); maximum, normaliser and sums pass through distributed shared memory in
+// place of global atomics, group barriers and a last arrival, about MEASURED us of a launch.
+template <bool NORM, bool CLUSTER>
 __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs a_in) {
     AttnArgs a = a_in;
     if (!at_span(a_in, a.pos, a.lo)) { at_refuse(a_in); return; }          // uniform over the grid
@@ -888,12 +890,20 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
     mloc = max(mloc, __shfl_xor_sync(0xffffffffu, mloc, 16));
     if (lane < 8 && mloc != INT64_MIN) atomicMax(&s_max[head], mloc);
     __syncthreads();
-    if (tid < rep && s_max[tid] != INT64_MIN) atomicMax(a.hmax + kv * rep + tid, s_max[tid]);
-    if (!af_group_barrier(a.ticket + 1 + kv, gridDim.x)) s_timeout = 1;
+    long long hm = 0;
+    if (CLUSTER) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        hm = INT64_MIN;
+        for (unsigned r = 0; r < gridDim.x; r++) hm = max(hm, *cluster.map_shared_rank(&s_max[head], r));
+    } else {
+        if (tid < rep && s_max[tid] != INT64_MIN) atomicMax(a.hmax + kv * rep + tid, s_max[tid]);
+        if (!af_group_barrier(a.ticket + 1 + kv, gridDim.x)) s_timeout = 1;
+        hm = head < rep ? __ldcg(a.hmax + kv * rep + head) : 0;
+    }
     // ---- pass 2: exponentials into shared memory and their sums ------------------------------------------------------------
     const SoftmaxExp exp2(a.fa, a.log2e, a.clip);
     unsigned long long zloc = 0ULL;
-    const long long hm = head < rep ? __ldcg(a.hmax + kv * rep + head) : 0;
 #pragma unroll
     for (int u = 0; u < 4; u++) {
         const int i = tid + u * AF_THREADS;
@@ -909,14 +919,22 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
     zloc += __shfl_xor_sync(0xffffffffu, zloc, 16);
     if (lane < 8 && zloc) atomicAdd(&s_z[head], zloc);
     __syncthreads();
-    if (tid < rep && s_z[tid]) atomicAdd(a.Z + kv * rep + tid, s_z[tid]);
-    if (!af_group_barrier(a.ticket + 1 + kv, 2u * gridDim.x)) s_timeout = 1;
+    unsigned long long z_all = 0;
+    if (CLUSTER) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        for (unsigned r = 0; r < gridDim.x; r++) z_all += *cluster.map_shared_rank(&s_z[head], r);
+    } else {
+        if (tid < rep && s_z[tid]) atomicAdd(a.Z + kv * rep + tid, s_z[tid]);
+        if (!af_group_barrier(a.ticket + 1 + kv, 2u * gridDim.x)) s_timeout = 1;
+        z_all = head < rep ? __ldcg(a.Z + kv * rep + head) : 0ULL;
+    }
     // ---- pass 3: probabilities as byte planes, then probabilities x values on the tensor cores ---------------------------
     //      out[head][dim] = sum over keys p[key][head] v[key][dim]: A = bytes of p (heads x keys; p <= 2^fa has three unsigned
     //      bytes), B = bytes of v gathered from four key rows (keys x dims), a warp owns eight dimensions for all keys
     const int nk32 = (nk + 31) & ~31;
     // a thread's pairs all belong to head tid % 8: one reciprocal of that head's normaliser
-    const SoftmaxQuotient quotient(head < rep ? __ldcg(a.Z + kv * rep + head) : 0ULL, a.fa);
+    const SoftmaxQuotient quotient(head < rep ? z_all : 0ULL, a.fa);
     for (int idx = tid; idx < nk32 * AF_HEADS; idx += AF_THREADS) {
         const int key = idx >> 3, h = idx & (AF_HEADS - 1);
         const unsigned p = key < nk ? quotient(s_e[idx]) : 0u;
@@ -959,7 +977,8 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
                 long long sum = 0;
 #pragma unroll
                 for (int w = 5; w >= 0; w--) sum = sum * 256 + (long long)acc[w][i];
-                if (g < rep) atomicAdd(reinterpret_cast<unsigned long long *>(accum + g * hd + nt * 8 + 2 * t + i), (unsigned long long)sum);
+                if (CLUSTER) red[g * hd + nt * 8 + 2 * t + i] = sum;
+                else if (g < rep) atomicAdd(reinterpret_cast<unsigned long long *>(accum + g * hd + nt * 8 + 2 * t + i), (unsigned long long)sum);
             }
         }
     }
@@ -967,25 +986,42 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
     //      that arrives last (a counter, no waiting) shifts its heads' sums, writes them and their digit planes, leaves the
     //      digit count of its part in out_nl[kv] and returns the statistics and counters of the head to their initial state.
     //      That spares a third barrier and a reduction over the chunks, and the four read-outs run side by side.
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-        const bool last = atomicAdd(a.ticket + 1 + gridDim.y + kv, 1u) == gridDim.x - 1;
-        if (last) __threadfence();
-        s_last = last ? 1 : 0; s_nl_out = 1;
+    int q_from = 0, q_to = rep * hd;                                        // the outputs this CTA reads out
+    if (CLUSTER) {
+        if (tid == 0) s_nl_out = 1;
+        if (s_timeout && tid == 0) atomicOr(a.flags, 8);
+        cg::this_cluster().sync();
+        const int share = ((rep * hd / 4 + (int)gridDim.x - 1) / (int)gridDim.x) * 4;
+        q_from = min(q_to, (int)blockIdx.x * share); q_to = min(q_to, q_from + share);
+    } else {
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            const bool last = atomicAdd(a.ticket + 1 + gridDim.y + kv, 1u) == gridDim.x - 1;
+            if (last) __threadfence();
+            s_last = last ? 1 : 0; s_nl_out = 1;
+        }
+        __syncthreads();
+        if (s_timeout && tid == 0) atomicOr(a.flags, 8);
+        if (!s_last) return;
     }
-    __syncthreads();
-    if (s_timeout && tid == 0) atomicOr(a.flags, 8);
-    if (!s_last) return;
     const long long n = (long long)a.H * hd, base = (long long)kv * rep * hd;      // plane stride; this head's first output
-    const int cnt = rep * hd;                                               // a multiple of 32
     int nl = 1;
     bool over = false;
     const bool word_planes = (reinterpret_cast<uintptr_t>(a.out_limbs) & 3) == 0;
-    for (int q = tid * 4; q < cnt; q += AF_THREADS * 4) {                   // four consecutive outputs per thread and turn
+    for (int q = q_from + tid * 4; q < q_to; q += AF_THREADS * 4) {                   // four consecutive outputs per thread and turn
         const long long i = base + q;
-        const longlong2 v0 = __ldcg(reinterpret_cast<const longlong2 *>(a.acc + i));
-        const longlong2 v1 = __ldcg(reinterpret_cast<const longlong2 *>(a.acc + i + 2));
+        longlong2 v0 = make_longlong2(0, 0), v1 = v0;
+        if (CLUSTER) {
+            cg::cluster_group cluster = cg::this_cluster();
+            for (unsigned r = 0; r < gridDim.x; r++) {
+                const longlong2 *src = reinterpret_cast<const longlong2 *>(cluster.map_shared_rank(red + q, r));
+                const longlong2 p0 = src[0], p1 = src[1];
+                v0.x += p0.x; v0.y += p0.y; v1.x += p1.x; v1.y += p1.y;
+            }
+        } else {
+            v0 = __ldcg(reinterpret_cast<const longlong2 *>(a.acc + i)); v1 = __ldcg(reinterpret_cast<const longlong2 *>(a.acc + i + 2));
+        }
         const long long y[4] = {v0.x >> a.fa, v0.y >> a.fa, v1.x >> a.fa, v1.y >> a.fa};
         if (a.out) { a.out[i] = y[0]; a.out[i + 1] = y[1]; a.out[i + 2] = y[2]; a.out[i + 3] = y[3]; }
         if (a.out_limbs) {
@@ -1016,10 +1052,22 @@ __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs 
                     for (int e = 0; e < 4; e++) a.out_limbs[l * n + i + e] = (int8_t)(pw[l] >> (8 * e));
             }
         }
-        *reinterpret_cast<longlong2 *>(a.acc + i) = make_longlong2(0, 0);
-        *reinterpret_cast<longlong2 *>(a.acc + i + 2) = make_longlong2(0, 0);
+        if (!CLUSTER) {
+            *reinterpret_cast<longlong2 *>(a.acc + i) = make_longlong2(0, 0);
+            *reinterpret_cast<longlong2 *>(a.acc + i + 2) = make_longlong2(0, 0);
+        }
     }
     if (over) atomicOr(a.flags, 1);
+    if (CLUSTER) {
+        cg::cluster_group cluster = cg::this_cluster();
+        if (a.out_limbs) {
+            nl = __reduce_max_sync(0xffffffffu, nl);
+            if (lane == 0 && nl > 1) atomicMax(cluster.map_shared_rank(&s_nl_out, 0), nl);
+        }
+        cluster.sync();                                                     // nobody leaves while its sums are read
+        if (blockIdx.x == 0 && tid == 0 && a.out_nl) a.out_nl[kv] = s_nl_out;
+        return;
+    }
     if (a.out_limbs) atomicMax(&s_nl_out, nl);
     if (tid < rep) { a.hmax[kv * rep + tid] = INT64_MIN; a.Z[kv * rep + tid] = 0ULL; }
     __syncthreads();
@@ -1376,30 +1424,41 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s) {
         a.fa <= 23 && a.Hkv <= 120) {                                       // probabilities (at most 2^fa) as three bytes
         static bool fat_configured = false;
         if (!fat_configured) {
-            if (cudaFuncSetAttribute(attn_fat_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess ||
-                cudaFuncSetAttribute(attn_fat_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess ||
-                cudaFuncSetAttribute(attn_fat_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) return cudaGetLastError();
+            for (const auto kernel : {attn_fat_kernel<false, false>, attn_fat_kernel<true, false>, attn_fat_kernel<false, true>, attn_fat_kernel<true, true>})
+                if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess ||
+                    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) return cudaGetLastError();
             fat_configured = true;
         }
+        auto smem_of = [&](int C) {
+            return ((size_t)2 * C * a.hd + (size_t)C / 8 * 24) * 4 + (size_t)AF_HEADS * a.hd * 12 + (size_t)C * AF_HEADS * 4 +
+                   (size_t)AF_THREADS / a.hd * AF_HEADS * a.hd * 8 + (size_t)4 * AF_HEADS * (a.hd + 16) + (size_t)3 * AF_HEADS * (C + 16);
+        };
+        // up to 1024 keys: clusters of at most eight CTAs, 128 keys each (as many as the warps take in one turn of the scores)
+        const int Cc = std::max(32, (int)((n_keys + 7) / 8 + 31) / 32 * 32);
+        const bool cluster = Cc <= 128 && smem_of(Cc) <= 208 * 1024;
         const int per_head = std::max(1, std::min(n_sms, 192) / a.Hkv);      // the partial-sum scratch holds 192 chunks
-        int C = (int)((n_keys + per_head - 1) / per_head);
-        C = std::max(32, (C + 31) / 32 * 32);                      // whole 32-key steps of the tensor-core passes
+        // whole 32-key steps of the tensor-core passes
+        const int C = cluster ? Cc : std::max(32, (int)((n_keys + per_head - 1) / per_head + 31) / 32 * 32);
         const unsigned fat_chunks = (unsigned)((n_keys + C - 1) / C);
-        const size_t fat_smem = ((size_t)2 * C * a.hd + (size_t)C / 8 * 24) * 4 + (size_t)AF_HEADS * a.hd * 12 + (size_t)C * AF_HEADS * 4 +
-                                (size_t)AF_THREADS / a.hd * AF_HEADS * a.hd * 8 + (size_t)4 * AF_HEADS * (a.hd + 16) + (size_t)3 * AF_HEADS * (C + 16);
+        const size_t fat_smem = smem_of(C);
+        const auto kernel = cluster ? (a.qgain ? attn_fat_kernel<true, true> : attn_fat_kernel<false, true>)
+                                    : (a.qgain ? attn_fat_kernel<true, false> : attn_fat_kernel<false, false>);
         int per_sm = 0;
         if (C <= 2 * 8 * (AF_THREADS / 32) && fat_smem <= 208 * 1024 &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, a.qgain ? attn_fat_kernel<true> : attn_fat_kernel<false>, AF_THREADS, fat_smem) == cudaSuccess &&
-            (long long)fat_chunks * a.Hkv <= (long long)per_sm * n_sms) {
+            (cluster || (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, AF_THREADS, fat_smem) == cudaSuccess &&
+                         (long long)fat_chunks * a.Hkv <= (long long)per_sm * n_sms))) {
             AttnArgs f = a;
             f.chunk = C;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(fat_chunks, a.Hkv); cfg.blockDim = dim3(AF_THREADS); cfg.dynamicSmemBytes = fat_smem; cfg.stream = s;
             cudaLaunchAttribute attr[2];
-            attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1;
+            if (cluster) {
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = fat_chunks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+            } else { attr[0].id = cudaLaunchAttributeCooperative; attr[0].val.cooperative = 1; }
             attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr; cfg.numAttrs = a.pdl ? 2 : 1;
-            const cudaError_t e = cudaLaunchKernelEx(&cfg, a.qgain ? attn_fat_kernel<true> : attn_fat_kernel<false>, f);
+            const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, f);
             note_launch(1);
             return e != cudaSuccess ? e : cudaGetLastError();
         }
