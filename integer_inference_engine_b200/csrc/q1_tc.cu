@@ -16,7 +16,8 @@
 // What bounds it: the integer instructions of the read-out (about 8 per row, token and block) and the hand-overs of a block,
 // about 1600 clocks per block of a 128 x 64 tile of which the MMAs (4 x N = 192) take 480.  12288 x 4096 at 512 tokens: 162 us
 // (546 us with one MMA per plane, 0 / 1 operands, 64-bit sums for every digit count and one accumulator buffer); at 6 tokens
-// 14 us (370 us with warp-level MMAs), 4096 x 4096 at 6 tokens 8.6 us (123).
+// 14 us (370 us with warp-level MMAs), 4096 x 4096 at 6 tokens 8.6 us (123).  Up to eight tokens a tile of eight halves the read-out:
+// a step of six sequences 1504 -> 1465 us (the hand-overs of a block stay).
 //
 // Split of the work: with at least four tiles per SM each CTA walks whole tiles.  With fewer, the (tile, block) pairs of all
 // tiles are dealt out evenly (a CTA then owns a contiguous run of blocks that may begin and end inside a tile) and the shares
@@ -153,7 +154,8 @@ __global__ void __launch_bounds__(qc_threads(NT), 1) q1_tc_kernel(const Q1TcArgs
     }
     pdl_enter();                                                   // what stands above needs nothing of the kernel before
     const int np = qc_planes(max(1, min(8, *a.nl_dev)), a.narrow);           // uniform over the grid
-    const int cols = np * NT;                                      // TMEM columns of one buffer
+    const int mp = NT == 8 && np == 3 ? 4 : np;                    // planes multiplied: an instruction takes whole sixteens of columns (the fourth plane is zero)
+    const int cols = mp * NT;                                      // TMEM columns of one buffer
     const int nbuf = cols <= 128 ? 4 : cols <= 256 ? 2 : 1, buf_cols = 512 / nbuf;
     const int stage_bytes = QC_A_BYTES + cols * 128;
     const int stages = min(QC_MAX_STAGES, (QC_SMEM - 1024 - QC_RAW_SLOTS * RAW_BYTES) / stage_bytes);
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(qc_threads(NT), 1) q1_tc_kernel(const Q1TcArgs
                     if (st.lapped && !(ok = qc_wait(empty_bar + 8 * st.slot, st.pass ^ 1, &s_abort))) break;
                     const uint32_t dst = qc_u32(smem + st.slot * stage_bytes + QC_A_BYTES);
                     qc_expect(full_bar + 8 * st.slot, cols * 128);
-                    for (int l = 0; l < np; l++)
+                    for (int l = 0; l < mp; l++)
                         asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                                      ::"r"(dst + l * NT * 128), "l"(reinterpret_cast<uint64_t>(&xmap)), "r"(b * 128), "r"(l), "r"(tt * NT),
                                        "r"(full_bar + 8 * st.slot) : "memory");
@@ -457,7 +459,7 @@ QcEncode qc_encode() {
 }
 
 // token tile: the read-out and the planes grow with it, the expansion of the signs does not
-int qc_tile_tokens(long long T) { return T <= 16 ? 16 : T <= 32 ? 32 : 64; }
+int qc_tile_tokens(long long T) { return T <= 8 ? 8 : T <= 16 ? 16 : T <= 32 ? 32 : 64; }
 
 template <int NT, typename DT>
 cudaError_t launch_tc(Q1TcArgs a, const int8_t *planes, cudaStream_t s) {
@@ -510,6 +512,7 @@ cudaError_t launch_q1_tc(const Q1Part *parts, int n_parts, bool sc32, long long 
     // three digit planes: |sum over a block| <= 128 * 8355711 < 2^30; the products of a tile have to add up inside 63 bits
     a.narrow = sh < 32 && max_scale < (1ULL << 32) && max_scale * (unsigned long long)nb < (1ULL << 33);
     const int nt = qc_tile_tokens(T);
+    if (nt == 8) return sc32 ? launch_tc<8, int>(a, planes, s) : launch_tc<8, long long>(a, planes, s);
     if (nt == 16) return sc32 ? launch_tc<16, int>(a, planes, s) : launch_tc<16, long long>(a, planes, s);
     if (nt == 32) return sc32 ? launch_tc<32, int>(a, planes, s) : launch_tc<32, long long>(a, planes, s);
     return sc32 ? launch_tc<64, int>(a, planes, s) : launch_tc<64, long long>(a, planes, s);

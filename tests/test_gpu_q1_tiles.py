@@ -13,7 +13,7 @@ FRAC = 16
 
 @pytest.mark.parametrize("out_f,nb,T,magbits,scale_bits", [
     (1, 1, 2, 20, 12), (127, 9, 16, 22, 12), (129, 8, 17, 22, 12), (640, 33, 32, 22, 14), (300, 7, 33, 30, 12), (4096, 3, 64, 22, 12),
-    (200, 130, 65, 38, 12), (384, 16, 130, 47, 20), (150, 5, 19, 62, 40), (96, 12, 6, 22, 31), (2400, 1, 2047, 22, 12)])
+    (200, 130, 65, 38, 12), (384, 16, 130, 47, 20), (150, 5, 19, 62, 40), (96, 12, 6, 22, 31), (2400, 1, 2047, 22, 12), (130, 4, 8, 22, 12), (257, 9, 2, 62, 40), (64, 35, 7, 30, 12)])
 def test_tiles_match_the_oracle(out_f, nb, T, magbits, scale_bits):
     import torch
 
