@@ -8,7 +8,7 @@
 //       N = np * NT columns per K step, so the expanded signs are read once per K step and not once per plane;
 //   D = np accumulators of NT columns, in two or four TMEM buffers.
 // The floor is per block, so every block's accumulators are read out: acc = sum_l 256^l D_l, acc * scale, shift, add.  With
-// three planes (|x| <= 8355711, what a normalised row has) acc stays below 128 * 8355711 < 2^31 and the read-out is one
+// three planes (-8421504 <= x <= 8355711, what a normalised row has) |acc| stays below 128 * 8421504 < 2^31 and the read-out is one
 // 32 x 32 -> 64 multiplication; more planes take 64-bit sums.
 //
 // Roles: eight or sixteen read-out warps (lane = row, a share of the tokens each), four expanding warps, one warp each for the
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(qc_threads(NT), 1) q1_tc_kernel(const Q1TcArgs
                             const auto &x = r[AHEAD ? ro & 1 : 0];
                             long long v;
                             if (NP == 3) {
-                                // |acc| < 2^31, and the launcher has seen to it that no sum of products leaves 64 bits: the bits
+                                // |acc| <= 1077952512, and the launcher has seen to it that no sum of products leaves 64 bits: the bits
                                 // below the shift are dropped here (the floor), the shift itself is taken once per tile
                                 const int acc = x[0][j] + x[1][j] * 256 + x[2][j] * 65536;
                                 if (sizeof(DT) == 4) { qc_mul_add(slo[ro * RT + j], shi[ro * RT + j], acc, (int)sc, keep); continue; }
@@ -509,8 +509,9 @@ cudaError_t launch_q1_tc(const Q1Part *parts, int n_parts, bool sc32, long long 
         a.part[p] = parts[p];
         a.tile_end[p] = (p ? a.tile_end[p - 1] : 0) + (int)((parts[p].out_f + 127) / 128);
     }
-    // three digit planes: |sum over a block| <= 128 * 8355711 < 2^30; the products of a tile have to add up inside 63 bits
-    a.narrow = sh < 32 && max_scale < (1ULL << 32) && max_scale * (unsigned long long)nb < (1ULL << 33);
+    // three digit planes: |sum over a block| <= 128 * 8421504 (all digits -128), so that the products of a tile, taken down to the shift
+    // (less than 2^32 a block), add up to less than 1077952512 * (2^33 - 2^26) + 2^52 < 2^63
+    a.narrow = sh < 32 && max_scale < (1ULL << 32) && max_scale * (unsigned long long)nb < (1ULL << 33) - (1ULL << 26);
     const int nt = qc_tile_tokens(T);
     if (nt == 8) return sc32 ? launch_tc<8, int>(a, planes, s) : launch_tc<8, long long>(a, planes, s);
     if (nt == 16) return sc32 ? launch_tc<16, int>(a, planes, s) : launch_tc<16, long long>(a, planes, s);

@@ -41,3 +41,24 @@ def test_tiles_match_the_oracle(out_f, nb, T, magbits, scale_bits):
         q1_gpu.apply_dev(h, xd, FRAC, out=xd.view(-1)[:out_f * T].view(T, out_f))
         assert np.array_equal(xd.view(-1)[:out_f * T].view(T, out_f).cpu().numpy(), want)
     assert device.read_flags() == 0
+
+
+@pytest.mark.parametrize(("nb", "scale"), [(4, (1 << 31) - 1), (4, 2130706431), (4, 2130706432), (2, (1 << 32) - 1), (5, 1717986918), (1, (1 << 32) - 1)])
+@pytest.mark.parametrize("T", [2, 16, 70])
+def test_largest_sums_of_three_planes(nb, scale, T):
+    """Every value at an end of three balanced digits, every sign the same, scales around the point (2^33 - 2^26 over the blocks) where
+    the products of a tile still fit 64 bits without a shift in between."""
+    import torch
+
+    from integer_inference_engine_b200 import device, q1_gpu
+    out_f = 40
+    bits = np.zeros((out_f, nb, 16), np.uint8)
+    bits[::2] = 0xFF
+    scales = np.full((out_f, nb), scale, np.int64)
+    scales[::4] *= -1
+    x = np.full((T, nb * 128), -8421504, np.int64)
+    x[1] = 8355711
+    h = q1_gpu.q1_register_weight(bits, scales.astype(np.int32) if scale < 1 << 31 else scales)
+    device.read_flags()
+    assert np.array_equal(q1_gpu.apply_dev(h, torch.from_numpy(x).cuda(), FRAC).cpu().numpy(), onat.q1_linear(x, bits, scales, FRAC))
+    assert device.read_flags() == 0
