@@ -1287,6 +1287,8 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const int64_t *x, lon
     __shared__ long long s_i[32];
     __shared__ long long s_part[2][AR_PARTS];                       // the first CTA's: every CTA's candidate
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, parts = (int)gridDim.y;
+    // the first CTA's shared memory may be written once that CTA runs: arrive here, wait in front of the write, behind the loads
+    if (parts > 1) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
     const int64_t *row = x + (long long)blockIdx.x * n;
     const long long share = ((n + parts - 1) / parts + 1) & ~1LL, from = min(n, share * blockIdx.y), to = min(n, from + share);
     long long bv = INT64_MIN, bi = n;
@@ -1311,6 +1313,7 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const int64_t *x, lon
     }
     if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
     __syncthreads();
+    if (parts > 1) asm volatile("barrier.cluster.wait;" ::: "memory");
     if (warp == 0) {
         bv = s_v[lane]; bi = s_i[lane];
 #pragma unroll

@@ -71,6 +71,17 @@ def test_argmax_rows_shared_by_a_cluster(rows, n):
     assert device.argmax_rows(x).cpu().tolist() == np.argmax(x.cpu().numpy(), axis=1).tolist()
 
 
+def test_argmax_rows_back_to_back():
+    """Clusters of one call start while those of the call before still exchange their candidates."""
+    import torch
+
+    from integer_inference_engine_b200 import device
+    xs = [torch.randint(-(1 << 40), 1 << 40, (128, 32768), generator=torch.Generator(device="cuda").manual_seed(i), device="cuda") for i in range(4)]
+    got = [device.argmax_rows(xs[i % 4]) for i in range(64)]
+    want = [np.argmax(x.cpu().numpy(), axis=1) for x in xs]
+    assert all(np.array_equal(g.cpu().numpy(), want[i % 4]) for i, g in enumerate(got))
+
+
 @pytest.mark.parametrize(("experts", "k"), [(5, 5), (128, 8), (300, 40), (1024, 64)])
 def test_topk_order_ties_and_gates(experts, k):
     import torch
