@@ -313,7 +313,9 @@ unsigned long long iie_workspace_generation(void);
 int iie_apply_dev_static(long long h, const int64_t *x_dev, long long T, int fw, int64_t *out_dev, void *stream);
 
 /* Read and clear the device flag word (synchronises the library stream and `stream`):
- * bit 0 an activation left the 8-limb envelope, bit 1 RMSNorm envelope, bit 2 dense router sum. */
+ * bit 0 an activation left the 8-limb envelope, bit 1 RMSNorm envelope, bit 2 dense router sum or a K/V value beyond int32,
+ * bit 3 a kernel's bounded wait ran out and outputs were left out (a host-array call fails with it: status 1), bit 4 a position
+ * outside the cache. */
 int iie_flags_read_clear(void *stream);
 
 #ifdef __cplusplus

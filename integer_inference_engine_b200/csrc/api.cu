@@ -302,7 +302,7 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
     }
     if (check_flags) {
         const int f = read_flags_clear();
-        if (f < 0) return false;
+        if (f < 0 || (f & FLAG_GAVE_UP)) return false;
         if (f & 1) return launch_exact_linear((const uint8_t *)w.d, w.qtype, w.out_f, w.nb, x, T, fw, out, s) == cudaSuccess;
     }
     return true;
@@ -523,7 +523,7 @@ int moe_host_entry(const long long *gate_h, const long long *up_h, const long lo
                              g_cells, mg, mgm, md, mdm);
         if (!ok) { cudaGetLastError(); return 1; }
         const int f = read_flags_clear();
-        if (f < 0) return 1;
+        if (f < 0 || (f & FLAG_GAVE_UP)) return 1;
         done = (f & 1) == 0;                      // an envelope miss re-runs the exact composition below
     }
     if (!done && !moe_exact_pairs(gw, uw, dw, h_dev, tok_of, gates_dev, m, k, d_model, e_ffn, fa, fw, out_dev)) {
@@ -698,7 +698,7 @@ extern "C" int qk_apply_resident_grouped(const long long *handles, const int *ph
             off += T * w.out_f;
         }
         const int f = download({{out, od, (size_t)total * 8}});
-        if (f < 0) { cudaGetLastError(); return 1; }
+        if (f < 0 || (f & FLAG_GAVE_UP)) { cudaGetLastError(); return 1; }
         if (exact || !(f & 1)) break;
     }
     return 0;
@@ -1816,7 +1816,7 @@ extern "C" int iie_moe_block_host(long long layer, long long gain_h, const int64
     const int rc = iie_moe_block_dev(layer, gain_h, xd, T, fa, fw, eps, od, idd, gd, g_stream);
     if (rc != 0) { cudaGetLastError(); return rc; }
     const int f = download({{out, od, n * 8}, {ids_out, idd, ids_out ? P * sizeof(int) : 0}, {gates_out, gd, gates_out ? P * 8 : 0}});
-    if (f < 0) { cudaGetLastError(); return 1; }
+    if (f < 0 || (f & FLAG_GAVE_UP)) { cudaGetLastError(); return 1; }
     return f ? 3 : 0;
 }
 

@@ -34,6 +34,7 @@ std::vector<Q1Weight> q_w;
 unsigned long long q_weight_bytes = 0;
 cudaStream_t q_stream = nullptr;
 int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [8..15] digits in use (a ring, see next_digits)
+int *q_host_flags = nullptr;            // page-locked: the flag word behind a host-array product
 int q_ready = -1;
 
 enum QRole { QR_X, QR_PLANES, QR_WORK, QR_KEYS, QR_VALUES, QR_LOGITS, QR_OUT, QR_GAIN, QR_COUNT };
@@ -60,7 +61,8 @@ bool q_init() {
     int n = 0;
     if (cudaGetDeviceCount(&n) != cudaSuccess || n <= 0 ||
         cudaStreamCreateWithFlags(&q_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&q_cells, 64) != cudaSuccess || cudaMemset(q_cells, 0, 64) != cudaSuccess) {
+        cudaMalloc(&q_cells, 64) != cudaSuccess || cudaMemset(q_cells, 0, 64) != cudaSuccess ||
+        cudaHostAlloc(&q_host_flags, 64, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError(); q_ready = 1; return false;
     }
     q_ready = 0;
@@ -197,8 +199,14 @@ int apply_host(const Q1Weight &w, const long long *x, long long T, long long fra
     if (cudaMemcpyAsync(xd, x, xsz, cudaMemcpyHostToDevice, q_stream) != cudaSuccess) return 2;
     const int rc = apply_device(w, xd, T, frac, od, max_digits, q_stream);
     if (rc != 0) { cudaStreamSynchronize(q_stream); return rc; }
-    if (cudaMemcpyAsync(out, od, osz, cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
-        cudaStreamSynchronize(q_stream) != cudaSuccess) return 2;
+    const int *flags = shared_flag_word();
+    if (!flags || cudaMemcpyAsync(q_host_flags, flags, sizeof(int), cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
+        cudaMemcpyAsync(out, od, osz, cudaMemcpyDeviceToHost, q_stream) != cudaSuccess || cudaStreamSynchronize(q_stream) != cudaSuccess) return 2;
+    if (*q_host_flags & FLAG_GAVE_UP) {                // goes with the call that reports it; the other bits are device-pointer callers'
+        const int f = iie_flags_read_clear(q_stream);
+        restore_flag_bits(f & ~FLAG_GAVE_UP);
+        return 2;
+    }
     return 0;
 }
 
@@ -771,7 +779,7 @@ extern "C" int bonsai_attention_prefill_gpu(const long long *q, const long long 
         ok = scope.ok && iie_attn_prefill_dev(dq, dk, dv, dkc, dvc, start, M, 0, nullptr, nullptr, 0, (int)H, (int)Hkv, (int)hp, L, (int)frac,
                                               inv_sqrt_fp, dout, q_stream) == 0;
         flags = scope.finish();
-        ok = ok && flags >= 0;
+        ok = ok && flags >= 0 && !(flags & FLAG_GAVE_UP);
     }
     if (ok && flags == 0) {
         ok = cudaMemcpy(qt.data(), dout, qt.size() * 8, cudaMemcpyDeviceToHost) == cudaSuccess;
@@ -835,7 +843,7 @@ extern "C" int bonsai_attention_decode_batched_gpu(const long long *q, const lon
                                      lengths[b] - 1, nullptr, 0, nullptr, nullptr, 0, (int)H, (int)Hkv, (int)hp, cap, (int)frac, inv_sqrt_fp,
                                      dout + (size_t)b * qd, q_stream) == 0;
         flags = scope.finish();
-        ok = ok && flags >= 0;
+        ok = ok && flags >= 0 && !(flags & FLAG_GAVE_UP);
     }
     if (ok && flags == 0) {
         ok = cudaMemcpy(qp.data(), dout, qp.size() * 8, cudaMemcpyDeviceToHost) == cudaSuccess;
@@ -901,7 +909,7 @@ extern "C" int bonsai_prefill_forward_gpu(const long long *x_embed, long long T,
         }
         ok = ok && head_rows(m, w.x + (size_t)(T - 1) * d, 1, logits, fw);
         flags = scope.finish();
-        ok = ok && flags >= 0;
+        ok = ok && flags >= 0 && !(flags & FLAG_GAVE_UP);
     }
     if (ok && flags == 0) ok = cudaMemcpy(out_logits, logits, (size_t)vocab * 8, cudaMemcpyDeviceToHost) == cudaSuccess;
     if (!ok) { cudaStreamSynchronize(q_stream); return fail(1, "prefill forward: CUDA failure"); }
@@ -1002,7 +1010,7 @@ extern "C" int bonsai_decode_step(long long ctx_h, const long long *x_in, const 
         }
         ok = ok && head_rows(m, c.w.x, c.B, c.logits, fw);
         flags = scope.finish();
-        ok = ok && flags >= 0;
+        ok = ok && flags >= 0 && !(flags & FLAG_GAVE_UP);
     }
     if (ok && flags == 0) ok = cudaMemcpy(out_logits, c.logits, (size_t)c.B * c.vocab * 8, cudaMemcpyDeviceToHost) == cudaSuccess;
     if (!ok) return fail(1, "decode step: CUDA failure");

@@ -54,3 +54,42 @@ def test_results_share_no_memory():
     for i, m in enumerate(many):
         m[:] = i
     assert all((m == i).all() for i, m in enumerate(many))
+
+
+def _raise_time_out_bit(lib):
+    getattr(lib, "_ZN3iie17restore_flag_bitsEi")(8)                     # from the host: what a kernel whose wait gave up leaves
+
+
+def test_a_wait_that_gave_up_fails_the_call():
+    """Bit 3 of the flag word says that outputs were left out: no host-array entry reports success with it."""
+    from integer_inference_engine_b200 import device, q1_gpu, qk_cuda
+    rng = np.random.default_rng(5)
+    d, eff, w = 256, 256, 512
+    raw = o.synth_q4k(rng, w, 1)
+    h = qk_cuda.register_weight(raw, w, 1, o.Q4_K)
+    gate, up = (qk_cuda.register_weight(o.synth_q4k(rng, eff, 1), eff, 1, o.Q4_K) for _ in range(2))
+    down = qk_cuda.register_weight(o.synth_q6k(rng, d, 1), d, 1, o.Q6_K)
+    bits, scale = o.synth_q1(rng, 64, 2)
+    q1 = q1_gpu.q1_register_weight(bits, scale.astype(np.int32))
+    x = rng.integers(-(1 << 20), 1 << 20, size=(3, d), dtype=np.int64)
+    wide = x.copy()
+    wide[0, 0] = np.iinfo(np.int64).max                                 # repeats with the exact kernel
+    gates = np.full((3, 1), 1 << 16, np.int64)
+    calls = [lambda: qk_cuda.apply_resident(h, x, w, FW), lambda: qk_cuda.apply_resident(h, wide, w, FW),
+             lambda: qk_cuda.apply_resident_grouped((h, gate), x, (w, eff), FW), lambda: qk_cuda.apply_resident_grouped((h, gate), wide, (w, eff), FW),
+             lambda: qk_cuda.apply_resident_grouped((h, gate), x[:1], (w, eff), FW),
+             lambda: qk_cuda.moe_ffn_batched([gate] * 3, [up] * 3, [down] * 3, 3, 1, x, gates, d, eff, 16, FW),
+             lambda: q1_gpu.q1_apply_resident(q1, x, 64, 2, 16), lambda: q1_gpu.q1_apply_resident(q1, x[:1], 64, 2, 16),
+             lambda: q1_gpu.q1_apply_gpu(x, bits, scale, 16), lambda: q1_gpu.q1_apply_dp4a_gpu(x, bits, scale, 16)]
+    device.read_flags()
+    for i, call in enumerate(calls):
+        good = call()
+        assert good is not None, i
+        _raise_time_out_bit(qk_cuda.load_library())
+        assert call() is None, i
+        again = call()                                                  # the bit went with the call that reported it
+        for a, b in zip(good, again):
+            assert np.array_equal(a, b), i
+        assert device.read_flags() == 0, i
+    qk_cuda.free_all()
+    q1_gpu.q1_free_weights()
