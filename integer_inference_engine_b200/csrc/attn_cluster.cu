@@ -194,8 +194,9 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
     //      above moves it and the distances so far, one more than 2^31 below is beyond every exponential's reach and stays at the edge ---
     const int last = n_keys - 1;                                            // rows past it are read as it
     long long best[2] = {INT64_MIN, INT64_MIN};                            // heads 2t, 2t + 1
-    // this warp's scores of head h so far move to another base
+    // this warp's scores of head h so far, which its lanes stored in another order, move to another base
     auto rebase = [&](int h, long long to, int tiles_done) {
+        __syncwarp();
         const long long by = to - s_base[warp][h];
         for (int j = 0; j <= tiles_done; j++) {
             int32_t *e = off + h * stride + (warp + AC_WARPS * j) * AC_TILE + lane;

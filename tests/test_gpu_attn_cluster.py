@@ -45,6 +45,37 @@ def test_cluster_form_gives_the_same_bytes(pos, H, Hkv, hd, window, rope, bits, 
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_scores_that_move_the_base_count_as_before(hd, wide):
+    """Twelve tiles per CTA, three per warp: scores of the second lie just below the reach of the first one's base, those of the third just
+    above it, so that the base moves while the second tile's scores still have weight.  Against the checker."""
+    import torch
+
+    from integer_inference_engine_b200 import device
+    from oracle import qk_oracle as o
+    H, pos, fa = 8, 3071, 16
+    rng = np.random.default_rng(hd)
+    inv_sqrt = 1 << 13
+    q = np.zeros((1, H, hd), np.int64)
+    q[0, :, 0] = 1 << 22                                                # score = 8 k[0] + what k[1] adds
+    q[0, :, 1] = rng.integers(-(1 << 15), 1 << 15, size=H)
+    if wide:
+        q[0, 0, 2] = 1 << 33                                            # beyond int32 (over a zero key column): the 64-bit products
+    level = (np.arange(pos + 1) // 128) % 3
+    k = np.zeros((1, pos + 1, hd), np.int64)
+    k[0, :, 0] = np.array([0, (1 << 28) - 3, (1 << 28) + 5])[level] + rng.integers(-2, 3, size=pos + 1)
+    k[0, :, 1] = rng.integers(-64, 64, size=pos + 1)
+    v = rng.integers(-(1 << 20), 1 << 20, size=(1, pos + 1, hd), dtype=np.int64)
+    want = o.attention_cached(q, k, v, pos, H, 1, fa, None, inv_sqrt)
+    dev = lambda a, t=torch.int64: torch.from_numpy(np.ascontiguousarray(a)).to("cuda", t)
+    device.read_flags()
+    got = device.attention_decode_batch(dev(q.reshape(1, -1)), dev(k[:, pos]), dev(v[:, pos]), dev(k.reshape(1, *k.shape), torch.int32), dev(v.reshape(1, *v.shape), torch.int32), pos, H, 1,
+                                        hd, fa, inv_sqrt=inv_sqrt)
+    assert device.read_flags() == 0
+    assert np.array_equal(got.cpu().numpy(), want)
+
+
 def test_column_slices_as_rows():
     import torch
 

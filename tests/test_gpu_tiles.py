@@ -67,3 +67,43 @@ def test_expert_tiles_match_the_oracle(down_q, d, eff, E, k, T, mult):
     assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
     assert np.array_equal(out.cpu().numpy(), out_ref)
     layer.close()
+
+
+def test_replays_of_a_short_graph_find_their_digit_count_cleared():
+    """One product captured on its own: a replay over wide rows leaves the replays after it the digit planes that their rows need."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(8)
+    raw = o.synth_q4k(rng, 256, 1)
+    h = qk_cuda.register_weight(raw, 256, 1, o.Q4_K)
+    x, out = torch.zeros((4, 256), dtype=torch.int64, device="cuda"), torch.empty((4, 256), dtype=torch.int64, device="cuda")
+    device.read_flags()
+    for _ in range(9):                                                  # eager calls between: every cell has been used
+        device.apply(h, x, 256, 24, out=out)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        device.apply(h, x, 256, 24, out=out)
+    for bits in (16, 50, 16, 16, 50, 50, 16):
+        rows = rng.integers(-(1 << bits), 1 << bits, size=(4, 256), dtype=np.int64)
+        x.copy_(torch.from_numpy(rows))
+        before = device.prefill_launch_counts()
+        graph.replay()
+        torch.cuda.synchronize()
+        ran = [b - a for a, b in zip(before, device.prefill_launch_counts())]
+        assert ran[5 if bits == 16 else 7] == 1 and sum(ran) == 1, (bits, ran)
+        assert np.array_equal(out.cpu().numpy(), onat.qk_linear(raw, rows, 256, 1, 24, o.Q4_K))
+    assert device.read_flags() == 0
+    del graph
+    qk_cuda.free_all()
+
+
+def test_launch_counts_fit_the_room_of_earlier_callers():
+    import ctypes
+
+    from integer_inference_engine_b200 import qk_cuda
+    lib = qk_cuda.load_library()
+    buf = (ctypes.c_uint64 * 8)(*[77] * 8)
+    assert lib.iie_prefill_launch_counts(buf, 6) == -1
+    assert lib.iie_prefill_launch_counts(buf, 7) == 7 and buf[7] == 77
+    assert lib.iie_prefill_launch_counts(buf, 8) == 8 and buf[7] != 77
