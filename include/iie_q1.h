@@ -143,6 +143,12 @@ int iie_q1_decode_layer_dev(long long wqkv, long long wo, long long w1u, long lo
                             const int64_t *qn, const int64_t *kn, int64_t *x, int64_t *qkv, int64_t *qkvn, int64_t *att, int64_t *h,
                             int32_t *kcache, int32_t *vcache, long long pos, const int *pos_dev, const int64_t *cos, const int64_t *sin,
                             int n_heads, int n_kv, int head_dim, long long cache_rows, long long frac, long long inv_sqrt, void *stream);
+/* The same directly behind another kernel of this library (the embedding row, another layer) on the stream, which does not write n1: the
+ * gain is read before that kernel ends. */
+int iie_q1_decode_layer_behind_dev(long long wqkv, long long wo, long long w1u, long long w2, const int64_t *n1, const int64_t *n2,
+                                   const int64_t *qn, const int64_t *kn, int64_t *x, int64_t *qkv, int64_t *qkvn, int64_t *att, int64_t *h,
+                                   int32_t *kcache, int32_t *vcache, long long pos, const int *pos_dev, const int64_t *cos, const int64_t *sin,
+                                   int n_heads, int n_kv, int head_dim, long long cache_rows, long long frac, long long inv_sqrt, void *stream);
 /* One row of a registered weight as int64 (sign * block scale, reference_bonsai.py:138-146 q1_rows_fp): the row index
  * is read from the device cell `row_dev` when that is not NULL, else `row`. */
 int iie_q1_embed_dev(long long handle, const int *row_dev, long long row, int64_t *out_dev, void *stream);

@@ -387,6 +387,7 @@ struct Q1RowInput {
     bool norm;                     // RMS-normalise the row first, with an optional gain
     const int64_t *gain;
     unsigned long long eps;
+    bool gain_ahead = false;       // the kernel in front on the stream does not write the gain: it is read before that kernel's end
 };
 cudaError_t launch_q1_row(const Q1Part *mats, int n, bool sc32, long long nb, const Q1RowInput &in, bool swiglu, long long frac, cudaStream_t s);
 constexpr int Q1_TC_CTAS = 148;    // one CTA per SM

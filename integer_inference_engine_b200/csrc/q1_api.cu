@@ -370,7 +370,7 @@ extern "C" int iie_q1_apply_fused_dev(long long handle, int mode, const int64_t 
 // One layer of a decode token: norm + Q/K/V product; attention with the per-head norms; O product with the residual; norm + gate/up
 // products + SwiGLU; down product with the residual.  Five launches, each started while the one before it runs and waiting for it
 // behind the requests for its weights.
-extern "C" int iie_q1_decode_layer_dev(long long wqkv, long long wo, long long w1u, long long w2, const int64_t *n1, const int64_t *n2,
+static int decode_layer(bool behind, long long wqkv, long long wo, long long w1u, long long w2, const int64_t *n1, const int64_t *n2,
                                        const int64_t *qn, const int64_t *kn, int64_t *x, int64_t *qkv, int64_t *qkvn, int64_t *att, int64_t *h,
                                        int32_t *kcache, int32_t *vcache, long long pos, const int *pos_dev, const int64_t *cos, const int64_t *sin,
                                        int n_heads, int n_kv, int head_dim, long long cache_rows, long long frac, long long inv_sqrt, void *stream) {
@@ -385,7 +385,7 @@ extern "C" int iie_q1_decode_layer_dev(long long wqkv, long long wo, long long w
     int *flags = iie::shared_flag_word();
     if (!flags) return 2;
     const Q1Part pa = {a.units, a.out_f, qkv, nullptr, a.max_scale}, po = {o.units, o.out_f, x, x, o.max_scale}, pd = {dn.units, dn.out_f, x, x, dn.max_scale};
-    if (!row_products(&pa, 1, a.sc32, a.nb, {x, true, n1, 1ULL}, false, frac, s)) return 2;
+    if (!row_products(&pa, 1, a.sc32, a.nb, {x, true, n1, 1ULL, behind}, false, frac, s)) return 2;
     int rc = attn_decode_normed(qkv, qkv + qd, qkv + qd + kd, kcache, vcache, pos, pos_dev, cos, sin, 2, n_heads, n_kv, head_dim, cache_rows, f,
                                 inv_sqrt, qn, kn, 1ULL, att, s);
     if (rc == 3)                                       // contexts and head shapes beyond the one-launch form
@@ -397,13 +397,28 @@ extern "C" int iie_q1_decode_layer_dev(long long wqkv, long long wo, long long w
     const size_t up_at = (size_t)(ffn / 16) * g.nb * q1_unit_bytes(g.sc32);          // the rows of the up matrix follow the gate's
     const Q1Part gu[2] = {{g.units, ffn, h, nullptr, g.max_scale}, {g.units + up_at, ffn, h, nullptr, g.max_scale}};
     if (g.nb <= 32) {
-        if (!row_products(gu, 2, g.sc32, g.nb, {x, true, n2, 1ULL}, true, frac, s)) return 2;
+        if (!row_products(gu, 2, g.sc32, g.nb, {x, true, n2, 1ULL, true}, true, frac, s)) return 2;
     } else {
         const Q1Part both = {g.units, g.out_f, h, nullptr, g.max_scale};
-        if (!row_products(&both, 1, g.sc32, g.nb, {x, true, n2, 1ULL}, false, frac, s) ||
+        if (!row_products(&both, 1, g.sc32, g.nb, {x, true, n2, 1ULL, true}, false, frac, s) ||
             launch_q1_silu_mul(h, h + ffn, ffn, f, h, s) != cudaSuccess) return 2;
     }
     return row_products(&pd, 1, dn.sc32, dn.nb, {h, false, nullptr, 0}, false, frac, s) ? 0 : 2;
+}
+
+extern "C" int iie_q1_decode_layer_dev(long long wqkv, long long wo, long long w1u, long long w2, const int64_t *n1, const int64_t *n2,
+                                       const int64_t *qn, const int64_t *kn, int64_t *x, int64_t *qkv, int64_t *qkvn, int64_t *att, int64_t *h,
+                                       int32_t *kcache, int32_t *vcache, long long pos, const int *pos_dev, const int64_t *cos, const int64_t *sin,
+                                       int n_heads, int n_kv, int head_dim, long long cache_rows, long long frac, long long inv_sqrt, void *stream) {
+    return decode_layer(false, wqkv, wo, w1u, w2, n1, n2, qn, kn, x, qkv, qkvn, att, h, kcache, vcache, pos, pos_dev, cos, sin, n_heads, n_kv, head_dim,
+                        cache_rows, frac, inv_sqrt, stream);
+}
+extern "C" int iie_q1_decode_layer_behind_dev(long long wqkv, long long wo, long long w1u, long long w2, const int64_t *n1, const int64_t *n2,
+                                              const int64_t *qn, const int64_t *kn, int64_t *x, int64_t *qkv, int64_t *qkvn, int64_t *att, int64_t *h,
+                                              int32_t *kcache, int32_t *vcache, long long pos, const int *pos_dev, const int64_t *cos, const int64_t *sin,
+                                              int n_heads, int n_kv, int head_dim, long long cache_rows, long long frac, long long inv_sqrt, void *stream) {
+    return decode_layer(true, wqkv, wo, w1u, w2, n1, n2, qn, kn, x, qkv, qkvn, att, h, kcache, vcache, pos, pos_dev, cos, sin, n_heads, n_kv, head_dim,
+                        cache_rows, frac, inv_sqrt, stream);
 }
 
 extern "C" int iie_q1_head_norm_dev(const int64_t *x_dev, long long rows_a, long long rows_b, long long width, const int64_t *gain_a_dev,
@@ -606,12 +621,12 @@ bool layer_rows(const Q1Stack &m, long long li, Work &w, long long T, int *flags
     auto norm = [&](long long h) {
         return [&, h](const PlaneDuties &d) { return launch_rmsnorm_planes(w.x, T, m.d, gain(h), f, m.eps, nullptr, planes, flags, d, q_stream); };
     };
-    bool ok = (T == 1 ? products_of_row({w.x, true, gain(m.n1g[i]), m.eps}, {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, false, m.frac)
+    bool ok = (T == 1 ? products_of_row({w.x, true, gain(m.n1g[i]), m.eps, true}, {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, false, m.frac)
                       : products(norm(m.n1g[i]), {{m.wq[i], w.q}, {m.wk[i], w.k}, {m.wv[i], w.v}}, planes, T, m.frac, w.x, T * m.d)) &&
               attend(i);
     if (T == 1)
         return ok && products_of_row({w.att, false, nullptr, 0}, {{m.wo[i], w.x, w.x}}, false, m.frac) &&
-               products_of_row({w.x, true, gain(m.n2g[i]), m.eps}, {{m.w1[i], w.g}, {m.wu[i], w.u}}, true, m.frac) &&
+               products_of_row({w.x, true, gain(m.n2g[i]), m.eps, true}, {{m.w1[i], w.g}, {m.wu[i], w.u}}, true, m.frac) &&
                products_of_row({w.g, false, nullptr, 0}, {{m.w2[i], w.x, w.x}}, false, m.frac);
     return ok && products([&](const PlaneDuties &d) { return launch_q1_prep(w.att, T, qd / 128, planes, d, q_stream); },
                           {{m.wo[i], w.x, w.x}}, planes, T, m.frac, w.att, T * qd) &&
@@ -623,7 +638,7 @@ bool layer_rows(const Q1Stack &m, long long li, Work &w, long long T, int *flags
 // logits of `rows` rows starting at x: final norm, output matrix
 bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logits, int *flags) {
     const int64_t *gain = q_bufs[(size_t)m.finalg].p;
-    if (rows == 1) return products_of_row({x, true, gain, m.eps}, {{m.out_head, logits}}, false, m.frac);
+    if (rows == 1) return products_of_row({x, true, gain, m.eps, true}, {{m.out_head, logits}}, false, m.frac);
     int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)rows * 8 * (size_t)m.d);
     if (!planes) return false;
     return products([&](const PlaneDuties &d) { return launch_rmsnorm_planes(x, rows, m.d, gain, (int)m.frac, m.eps, nullptr, planes, flags, d, q_stream); },

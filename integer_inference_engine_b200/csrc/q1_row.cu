@@ -110,7 +110,7 @@ __device__ __forceinline__ uint64_t rw_unit_sums(const uint2 (&w)[2], const uint
 }
 
 // SWIGLU: two matrices of the same rows, groups of their tiles taken alternately; out[0] = ((silu(product 0)) * product 1) >> frac
-template <typename DT, bool SWIGLU>
+template <typename DT, bool SWIGLU, bool LATE>
 __global__ void __launch_bounds__(RW_THREADS, 2) q1_row_kernel(const Q1RowArgs a) {
     constexpr int US = 256 + 16 * (int)sizeof(DT);
     extern __shared__ __align__(128) uint8_t rw_sm[];
@@ -159,23 +159,31 @@ __global__ void __launch_bounds__(RW_THREADS, 2) q1_row_kernel(const Q1RowArgs a
         __syncwarp();
         for (int q = 0; q < min(a.depth, groups); q++) request(q, q);
     }
-    // the gain is constant, too: asked for before the wait
+    // The gain is read ahead of the wait where the kernel in front does not write it, else (LATE) brought to the cache here and read behind
+    // the wait.  Forms of their own: one form for both, or the late one alone, cost 0.4 us of a product (q1 decode 1600 against 1632 us).
     const int K = a.nb * 128, pk = blocks * 128;
     int64_t gv[2][4];
     uint64_t gm = 1;
-    if (a.norm && a.gain) {
-        gm = 0;
+    auto read_gain = [&]() {
+        if (a.norm && a.gain) {
+            gm = 0;
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const int i = 4 * (tid + q * RW_THREADS);
+            for (int q = 0; q < 2; q++) {
+                const int i = 4 * (tid + q * RW_THREADS);
 #pragma unroll
-            for (int e = 0; e < 4; e++) { gv[q][e] = i < pk ? __ldg(a.gain + b0 * 128 + i + e) : 0; gm |= uabs64(gv[q][e]); }
+                for (int e = 0; e < 4; e++) {
+                    gv[q][e] = i < pk ? (LATE ? a.gain[b0 * 128 + i + e] : __ldg(a.gain + b0 * 128 + i + e)) : 0;
+                    gm |= uabs64(gv[q][e]);
+                }
+            }
+            if (a.parts > 1) for (int i = tid; i < K; i += RW_THREADS) gm |= uabs64(LATE ? a.gain[i] : __ldg(a.gain + i));
+        } else {
+#pragma unroll
+            for (int q = 0; q < 2; q++) { gv[q][0] = gv[q][1] = gv[q][2] = gv[q][3] = 1; }
         }
-        if (a.parts > 1) for (int i = tid; i < K; i += RW_THREADS) gm |= uabs64(__ldg(a.gain + i));
-    } else {
-#pragma unroll
-        for (int q = 0; q < 2; q++) { gv[q][0] = gv[q][1] = gv[q][2] = gv[q][3] = 1; }
-    }
+    };
+    if (!LATE) read_gain();
+    else if (a.norm && a.gain) for (int i = 16 * tid; i < pk; i += 16 * RW_THREADS) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.gain + b0 * 128 + i));
     // behind this wait everything before the preceding kernel has finished, too: each kernel starts its dependents behind its own wait
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
@@ -193,6 +201,7 @@ __global__ void __launch_bounds__(RW_THREADS, 2) q1_row_kernel(const Q1RowArgs a
         }
         x[q][0] = v0.x; x[q][1] = v0.y; x[q][2] = v1.x; x[q][3] = v1.y;
     }
+    if (LATE) read_gain();
 #pragma unroll
     for (int q = 0; q < 2; q++) all |= uabs64(x[q][0]) | uabs64(x[q][1]) | uabs64(x[q][2]) | uabs64(x[q][3]);
     bool bad = false, narrow = (all >> 30) == 0;                          // four digits hold every value
@@ -367,7 +376,7 @@ __global__ void q1_row_init_kernel(int64_t *out, const int64_t *add, long long n
     if (i < n) out[i] = add ? add[i] : 0;
 }
 
-template <typename DT, bool SWIGLU>
+template <typename DT, bool SWIGLU, bool LATE>
 cudaError_t launch_row(const Q1RowArgs &a, cudaStream_t s) {
     const int run = (a.tiles / (SWIGLU ? 2 : 1) + a.per_part - 1) / a.per_part, groups = (run + RW_GROUP - 1) / RW_GROUP * (SWIGLU ? 2 : 1);
     Q1RowArgs b = a;
@@ -378,10 +387,10 @@ cudaError_t launch_row(const Q1RowArgs &a, cudaStream_t s) {
     const size_t slots = groups <= b.depth ? (size_t)(b.depth - 1) * RW_GROUP + (SWIGLU ? std::min(run, RW_GROUP) : run - (groups - 1) * RW_GROUP) : (size_t)b.depth * RW_GROUP;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(q1_row_kernel<DT, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(q1_row_kernel<DT, SWIGLU, LATE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)(RW_HEAD_BYTES + (size_t)RW_RING * RW_GROUP * RW_BLOCKS * (256 + 16 * sizeof(DT))));
         // all of the SM's memory as shared memory: otherwise the next kernel's CTAs do not fit beside these and start behind them, two to an SM
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(q1_row_kernel<DT, SWIGLU>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(q1_row_kernel<DT, SWIGLU, LATE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
         configured = true;
     }
@@ -392,7 +401,7 @@ cudaError_t launch_row(const Q1RowArgs &a, cudaStream_t s) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, q1_row_kernel<DT, SWIGLU>, b);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, q1_row_kernel<DT, SWIGLU, LATE>, b);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -428,8 +437,11 @@ cudaError_t launch_q1_row(const Q1Part *mats, int n, bool sc32, long long nb, co
             q1_row_init_kernel<<<(unsigned)((mats[i].out_f + 255) / 256), 256, 0, s>>>(mats[i].out, mats[i].add, mats[i].out_f);
             note_launch();
         }
-    if (swiglu) return sc32 ? launch_row<int, true>(a, s) : launch_row<long long, true>(a, s);
-    return sc32 ? launch_row<int, false>(a, s) : launch_row<long long, false>(a, s);
+    const bool late = in.norm && in.gain && !in.gain_ahead;
+    if (swiglu && late) return cudaErrorNotSupported;                    // (no caller has that)
+    if (swiglu) return sc32 ? launch_row<int, true, false>(a, s) : launch_row<long long, true, false>(a, s);
+    if (late) return sc32 ? launch_row<int, false, true>(a, s) : launch_row<long long, false, true>(a, s);
+    return sc32 ? launch_row<int, false, false>(a, s) : launch_row<long long, false, false>(a, s);
 }
 
 }  // namespace iie

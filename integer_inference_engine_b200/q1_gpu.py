@@ -28,7 +28,7 @@ EXPORTED_SYMBOLS = (
     "bonsai_q1_register_weight_i32_bmma", "bonsai_q1_apply_resident", "bonsai_q1_free_weights", "bonsai_rmsnorm_gpu",
     "bonsai_buf_upload_i64", "bonsai_attention_prefill_gpu", "bonsai_attention_decode_batched_gpu", "bonsai_prefill_forward_gpu",
     "bonsai_decode_ctx_create", "bonsai_decode_ctx_seed_seq", "bonsai_decode_step", "bonsai_decode_ctx_free",
-    "iie_q1_apply_dev", "iie_q1_apply_fused_dev", "iie_q1_head_norm_dev", "iie_q1_silu_mul_dev", "iie_q1_embed_dev", "iie_q1_decode_layer_dev", "iie_q1_set_stream", "iie_host_take", "iie_host_give", "iie_q1_weight_shape", "iie_q1_workspace_generation",
+    "iie_q1_apply_dev", "iie_q1_apply_fused_dev", "iie_q1_head_norm_dev", "iie_q1_silu_mul_dev", "iie_q1_embed_dev", "iie_q1_decode_layer_dev", "iie_q1_decode_layer_behind_dev", "iie_q1_set_stream", "iie_host_take", "iie_host_give", "iie_q1_weight_shape", "iie_q1_workspace_generation",
 )
 from .qk_cuda import CudaContextError      # noqa: E402  (same error type as the MoE bridge)
 
@@ -83,6 +83,7 @@ def load_library():
         "iie_q1_silu_mul_dev": ([vp, vp, i64, i64, vp, vp], c_int),
         "iie_q1_embed_dev": ([i64, vp, i64, vp, vp], c_int),
         "iie_q1_decode_layer_dev": ([i64] * 4 + [vp] * 11 + [i64, vp, vp, vp] + [c_int] * 3 + [i64] * 3 + [vp], c_int),
+        "iie_q1_decode_layer_behind_dev": ([i64] * 4 + [vp] * 11 + [i64, vp, vp, vp] + [c_int] * 3 + [i64] * 3 + [vp], c_int),
         "iie_host_take": ([u64], vp), "iie_host_give": ([vp], None),
         "iie_q1_set_stream": ([c_int], None), "iie_q1_workspace_generation": ([], ctypes.c_uint64),
         "iie_q1_weight_shape": ([i64, ctypes.POINTER(i64), ctypes.POINTER(i64), ctypes.POINTER(c_int)], c_int),
@@ -416,18 +417,19 @@ def head_norm_dev(x, rows_a: int, rows_b: int, width: int, gain_a, gain_b, frac:
     return out
 
 
-def decode_layer_dev(w: dict, x, qkv, qkvn, att, h, pos: int, pos_dev, cos, sin, n_heads: int, n_kv: int, head_dim: int, frac: int) -> None:
+def decode_layer_dev(w: dict, x, qkv, qkvn, att, h, pos: int, pos_dev, cos, sin, n_heads: int, n_kv: int, head_dim: int, frac: int,
+                     behind: bool = False) -> None:
     """One decoder layer of a decode token in place on ``x``: ``w`` holds the weight handles wqkv, wo, w1u, w2, the CUDA int64
-    gains n1, n2, qn, kn and the int32 caches k, v [n_kv, rows, head_dim]; ``pos_dev`` the position's device cell, ``pos`` its bound."""
+    gains n1, n2, qn, kn and the int32 caches k, v [n_kv, rows, head_dim]; ``pos_dev`` the position's device cell, ``pos`` its bound.
+    ``behind``: the kernel in front on the stream is :func:`embed_dev`'s or another layer's, so that n1 may be read before it ends."""
     import torch
 
     inv_sqrt = int(round((1.0 / head_dim ** 0.5) * (1 << frac)))
     with _CUDA_LOCK:
-        rc = _lib().iie_q1_decode_layer_dev(w["wqkv"], w["wo"], w["w1u"], w["w2"], w["n1"].data_ptr(), w["n2"].data_ptr(), w["qn"].data_ptr(),
-                                            w["kn"].data_ptr(), x.data_ptr(), qkv.data_ptr(), qkvn.data_ptr(), att.data_ptr(), h.data_ptr(),
-                                            w["k"].data_ptr(), w["v"].data_ptr(), int(pos), pos_dev.data_ptr(), cos.data_ptr(), sin.data_ptr(),
-                                            n_heads, n_kv, head_dim, int(w["k"].shape[1]), int(frac), inv_sqrt,
-                                            torch.cuda.current_stream().cuda_stream)
+        entry = _lib().iie_q1_decode_layer_behind_dev if behind else _lib().iie_q1_decode_layer_dev
+        rc = entry(w["wqkv"], w["wo"], w["w1u"], w["w2"], w["n1"].data_ptr(), w["n2"].data_ptr(), w["qn"].data_ptr(), w["kn"].data_ptr(), x.data_ptr(),
+                   qkv.data_ptr(), qkvn.data_ptr(), att.data_ptr(), h.data_ptr(), w["k"].data_ptr(), w["v"].data_ptr(), int(pos), pos_dev.data_ptr(),
+                   cos.data_ptr(), sin.data_ptr(), n_heads, n_kv, head_dim, int(w["k"].shape[1]), int(frac), inv_sqrt, torch.cuda.current_stream().cuda_stream)
     if rc != 0:
         raise CudaContextError(f"decode layer failed with status {rc}")
 

@@ -89,7 +89,7 @@ class Q1Decoder:
         q1_gpu.embed_dev(self.embed, self.token, self.x)
         for L in self.layers:
             q1_gpu.decode_layer_dev(L, self.x, self.qkv, self.qkvn, self.att, self.gu, pos_bound, self.pos, self.cos, self.sin,
-                                    self.H, self.Hkv, self.hd, self.frac)
+                                    self.H, self.Hkv, self.hd, self.frac, behind=True)
         q1_gpu.apply_fused_dev(self.head, self.x, self.frac, self.logits, norm=True, gain=self.out_gain)
         device.argmax(self.logits.view(-1), out=self.token)
         self.pos += 1

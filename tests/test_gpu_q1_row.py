@@ -49,6 +49,30 @@ def test_products(out_f, nb, magnitude):
     assert device.read_flags() == 0
 
 
+def test_gain_written_by_the_kernel_in_front():
+    """Gain and row come from the kernel launched just before the product, whose start overlaps that kernel's end."""
+    import torch
+
+    from integer_inference_engine_b200 import device, q1_gpu
+    rng = np.random.default_rng(77)
+    K, out_f = 4096, 600
+    bits, scale = o.synth_q1(rng, out_f, K // 128)
+    h = q1_gpu.q1_register_weight(bits, scale.astype(np.int32))
+    xs = rng.integers(-(1 << 20), 1 << 20, size=(8, 1, K), dtype=np.int64)
+    gains = rng.integers(-(1 << 17), 1 << 17, size=(8, K), dtype=np.int64)
+    xd, gd = torch.from_numpy(xs).cuda(), torch.from_numpy(gains).cuda()
+    x, gain = torch.zeros((1, K), dtype=torch.int64, device="cuda"), torch.zeros(K + 1, dtype=torch.int64, device="cuda")[1:]
+    device.read_flags()
+    outs = []
+    for i in range(64):
+        x.copy_(xd[i % 8])
+        gain.copy_(gd[i % 8])
+        outs.append(q1_gpu.apply_fused_dev(h, x, FRAC, torch.empty((1, out_f), dtype=torch.int64, device="cuda"), norm=True, gain=gain))
+    want = [onat.q1_linear(o.rmsnorm_fixed(xs[i], FRAC, 1, gains[i]), bits, scale, FRAC) for i in range(8)]
+    assert all(np.array_equal(out.cpu().numpy(), want[i % 8]) for i, out in enumerate(outs))
+    assert device.read_flags() == 0
+
+
 @pytest.mark.parametrize(("d", "H", "Hkv", "hd", "ffn", "context"), [(256, 4, 2, 64, 384, 70), (4224, 4, 1, 128, 256, 33), (512, 8, 8, 32, 128, 40),
                                                                      (384, 48, 3, 64, 256, 20)])
 def test_decoder_steps(d, H, Hkv, hd, ffn, context):
