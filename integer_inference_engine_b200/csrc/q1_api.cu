@@ -10,11 +10,11 @@
 #include <atomic>
 #include <initializer_list>
 #include <mutex>
-#include <thread>
 #include <vector>
 
 #include "../../include/iie_q1.h"
 #include "../../include/iie_qk.h"
+#include "host_threads.h"
 #include "kernels.h"
 
 using namespace iie;
@@ -452,6 +452,7 @@ extern "C" void *iie_host_take(unsigned long long bytes) {
         h_pool.erase(h_pool.begin() + (long)i);
     }
     void *p = nullptr;
+    try { h_pool.reserve(h_pool.size() + 1); } catch (...) { return nullptr; }
     if (total + bytes > HOST_POOL || cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     h_pool.push_back({p, (size_t)bytes, true});
     return p;
@@ -677,10 +678,7 @@ bool upload_rows(int64_t *dst, const long long *src, size_t bytes) {
                 if (cudaMemcpyAsync((uint8_t *)dst + part + at, pin + at, len, cudaMemcpyHostToDevice, q_stream) != cudaSuccess) good = false;
             }
         };
-        std::thread helpers[THREADS - 1];
-        for (auto &t : helpers) t = std::thread(copy);
-        copy();
-        for (auto &t : helpers) t.join();
+        run_with_helpers<THREADS - 1>(copy);
         if (!good) return false;
     }
     return true;
@@ -731,6 +729,7 @@ struct DecodeCtx {
     int32_t *K = nullptr, *V = nullptr;            // [n_layers][B][Hkv][cap][hd]
     int64_t *logits = nullptr;
     int *pos = nullptr;                            // [B]: where the sequences stand in the step under way
+    std::vector<int> at;                           // the same on the host
     Work w;
     std::vector<char> wide;                        // per sequence: a seeded value did not fit the int32 rows
 };
@@ -948,7 +947,7 @@ extern "C" long long bonsai_decode_ctx_create(long long B, long long n_layers, l
     m.inv_sqrt = inv_sqrt; m.finalg = finalg; m.out_head = out_head; m.cos_h = cos_h; m.sin_h = sin_h;
     fill_stack(m, wq, wk, wv, wo, w1, wu, w2, n1g, n2g, qng, kng);
     if (!stack_ok(m, cap) || q_w[(size_t)out_head].out_f != vocab) { fail(1, "decode context: a handle or a dimension does not fit the model"); return -1; }
-    c.B = B; c.cap = cap; c.vocab = vocab; c.wide.assign((size_t)B, 0);
+    c.B = B; c.cap = cap; c.vocab = vocab; c.wide.assign((size_t)B, 0); c.at.assign((size_t)B, 0);
     const size_t kv = (size_t)n_layers * B * Hkv * cap * hd * 4;
     if (cudaMalloc(&c.K, kv) != cudaSuccess || cudaMalloc(&c.V, kv) != cudaSuccess || cudaMemset(c.K, 0, kv) != cudaSuccess ||
         cudaMemset(c.V, 0, kv) != cudaSuccess || cudaMalloc(&c.logits, (size_t)B * vocab * 8) != cudaSuccess || cudaMalloc(&c.pos, (size_t)B * 4) != cudaSuccess || !alloc_work(c.w, m, B, false)) {
@@ -994,10 +993,10 @@ extern "C" int bonsai_decode_step(long long ctx_h, const long long *x_in, const 
     for (char wide : c.wide) if (wide) return fail(4, "decode step: a seeded K/V value is beyond int32");
     const long long qd = m.H * m.hd, kd = m.Hkv * m.hd;
     const size_t per_seq = (size_t)m.Hkv * c.cap * m.hd;
-    std::vector<int> at(pos, pos + c.B);
+    std::copy(pos, pos + c.B, c.at.begin());
     const long long longest = *std::max_element(pos, pos + c.B);
     bool ok = cudaMemcpyAsync(c.w.x, x_in, (size_t)c.B * m.d * 8, cudaMemcpyHostToDevice, q_stream) == cudaSuccess &&
-              cudaMemcpyAsync(c.pos, at.data(), (size_t)c.B * 4, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
+              cudaMemcpyAsync(c.pos, c.at.data(), (size_t)c.B * 4, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
     int flags = -1;
     {
         FlagScope scope;

@@ -93,3 +93,27 @@ def test_a_wait_that_gave_up_fails_the_call():
         assert device.read_flags() == 0, i
     qk_cuda.free_all()
     q1_gpu.q1_free_weights()
+
+
+@pytest.mark.parametrize("T", [16, 77, 620])
+def test_prompt_rows_arrive_whole(T):
+    """Rows below, inside and beyond the page-locked buffer they travel through (1 MB, 32 MB): the exported values of every row against the
+    checker's product of the normalised row."""
+    from integer_inference_engine_b200 import q1_gpu
+    rng = np.random.default_rng(T)
+    d, H, Hkv, hd, dff, vocab = 8192, 2, 1, 64, 128, 40
+    shapes = {"wq": (H * hd, d), "wk": (Hkv * hd, d), "wv": (Hkv * hd, d), "wo": (d, H * hd), "w1": (dff, d), "wu": (dff, d), "w2": (d, dff)}
+    raw = {name: o.synth_q1(rng, out_f, in_f // 128) for name, (out_f, in_f) in shapes.items()}
+    w = {name: [q1_gpu.q1_register_weight(b, s.astype(np.int32))] for name, (b, s) in raw.items()}
+    head_bits, head_scale = o.synth_q1(rng, vocab, d // 128)
+    w["out_head"], w["out_head_vocab"] = q1_gpu.q1_register_weight(head_bits, head_scale.astype(np.int32)), vocab
+    gains = {name: rng.integers(1 << 15, 1 << 17, size=n, dtype=np.int64) for name, n in (("n1g", d), ("n2g", d), ("qng", hd), ("kng", hd))}
+    gh = {name: [q1_gpu.buf_upload_i64(g)] for name, g in gains.items()}
+    cos, sin = o.build_rope_tables(T, hd, frac=16)
+    gh["finalg"], gh["cos_h"], gh["sin_h"] = q1_gpu.buf_upload_i64(gains["n1g"]), q1_gpu.buf_upload_i64(cos), q1_gpu.buf_upload_i64(sin)
+    x = rng.integers(-(1 << 14), 1 << 14, size=(T, d), dtype=np.int64)
+    got = q1_gpu.prefill_forward_gpu(x, (T, d, 1, H, Hkv, hd, dff), w, gh, 16, 1, round((1 << 16) / 8), export_kv=True)
+    assert got is not None
+    want = onat.q1_linear(o.rmsnorm_fixed(x, 16, 1, gains["n1g"]), *raw["wv"], 16)
+    assert np.array_equal(got[2][0, 0], want)
+    q1_gpu.q1_free_weights()
