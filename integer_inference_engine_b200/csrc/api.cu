@@ -243,13 +243,12 @@ bool tiles(int qtype, int mode, TileArgs a, cudaStream_t s) {
     return e == cudaSuccess;
 }
 
-// The cell that receives the digits in use of the next rows' planes, and one for that kernel to clear: a ring of eight, each cleared
-// four planes ahead of its use (one that was not, as in a short replayed graph, is only too large, which costs time and changes no result).
+// The cell that receives the digits in use of the next rows' planes, and the one that their kernel clears (null: not to be had).
 struct DigitCell { int *nl, *clear; };
-DigitCell next_cell() {
-    static unsigned turn = 0;
-    turn++;
-    return {g_cells + 4 + (turn & 7), g_cells + 4 + ((turn + 4) & 7)};
+DigitCell next_cell(cudaStream_t s) {
+    static DigitRing ring;
+    DigitCell c = {nullptr, nullptr};
+    return ring.next(g_cells + 4, s, c.nl, c.clear) ? c : DigitCell{nullptr, nullptr};
 }
 
 // y[T,out_f] on device from x[T,K] on device.  check_flags: synchronise and re-run the exact kernel
@@ -265,8 +264,8 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
         int8_t *buf = (int8_t *)ensure(R_XL, (size_t)T * 8 * K);
         if (!buf) return false;
         if (T >= 2) {
-            const DigitCell c = next_cell();
-            if (launch_limbs(x, T, K, buf, g_flags, s, c.nl, c.clear) != cudaSuccess) return false;
+            const DigitCell c = next_cell(s);
+            if (!c.nl || launch_limbs(x, T, K, buf, g_flags, s, c.nl, c.clear) != cudaSuccess) return false;
             x_nl = c.nl;
         } else if (launch_limbs(x, T, K, buf, g_flags, s) != cudaSuccess) return false;
         xl = buf;
@@ -680,7 +679,7 @@ extern "C" int qk_apply_resident_grouped(const long long *handles, const int *ph
     const long long K = nb * 256;
     int64_t *xd = (int64_t *)ensure(R_X, (size_t)T * K * 8), *od = (int64_t *)ensure(R_OUT, (size_t)total * 8);
     int8_t *xl = (int8_t *)ensure(R_XL, (size_t)T * 8 * K);
-    const DigitCell cell = T > 1 ? next_cell() : DigitCell{nullptr, nullptr};
+    const DigitCell cell = T > 1 ? next_cell(g_stream) : DigitCell{nullptr, nullptr};
     int *nl = cell.nl;
     if (!xd || !od || !xl || !upload(xd, x, (size_t)T * K * 8) ||
         launch_limbs(xd, T, K, xl, g_flags, g_stream, nl, cell.clear) != cudaSuccess) { cudaGetLastError(); return 1; }
@@ -853,7 +852,8 @@ extern "C" int iie_moe_forward_dev(long long layer, const int64_t *h_dev, long l
     int64_t *lg = (int64_t *)ensure(R_LOGITS, (size_t)T * E * 8);
     if (!hl || !lg) return 1;
     // the kernel that splits the rows clears what the experts' kernels add to, too, unless that lies over the rows
-    const DigitCell cell = next_cell();
+    const DigitCell cell = next_cell(s);
+    if (!cell.nl) return 1;
     const long long n_out = T * L.d_model;
     const bool apart = out_dev + n_out <= h_dev || h_dev + n_out <= out_dev, zero_here = !accumulate && stage_on(ST_LIMBS) && apart;
     if (stage_on(ST_LIMBS) && launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, cell.nl, cell.clear, g_cells + 1, zero_here ? out_dev : nullptr, n_out) != cudaSuccess) return 1;
@@ -918,7 +918,8 @@ extern "C" int iie_moe_experts_dev(long long layer, const int64_t *h_dev, long l
     const long long P = T * slots;
     int8_t *hl = (int8_t *)ensure(R_XL, (size_t)T * 8 * L.d_model);
     if (!hl) return 1;
-    const DigitCell cell = next_cell();
+    const DigitCell cell = next_cell(s);
+    if (!cell.nl) return 1;
     const long long n_out = T * L.d_model;
     const bool zero_here = !accumulate && (out_dev + n_out <= h_dev || h_dev + n_out <= out_dev);
     if (launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, cell.nl, cell.clear, g_cells + 1, zero_here ? out_dev : nullptr, n_out) != cudaSuccess) return 1;

@@ -24,6 +24,27 @@ cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
 extern unsigned long long g_launches;
 inline void note_launch(unsigned long long n = 1) { __atomic_fetch_add(&g_launches, n, __ATOMIC_RELAXED); }
 
+// Digits in use of the planes written last, by the kernel that writes them for the products behind it: a ring of eight cells, each cleared
+// four planes ahead of its use by that kernel (one that was not, as behind a replayed graph, is only too large, which costs time and
+// changes no result).  A captured graph with fewer planes than cells would never clear some of its own: its first planes clear the ring.
+struct DigitRing {
+    unsigned turn = 0;
+    unsigned long long capture = 0;            // graph being captured that has its clear
+    // cell to write and cell to clear; false when the clear could not be queued
+    bool next(int *cells, cudaStream_t s, int *&nl, int *&clear) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        if (cudaStreamGetCaptureInfo(s, &status, &id) != cudaSuccess) { cudaGetLastError(); status = cudaStreamCaptureStatusNone; }
+        if (status == cudaStreamCaptureStatusActive && id != capture) {
+            if (cudaMemsetAsync(cells, 0, 8 * sizeof(int), s) != cudaSuccess) return false;
+            capture = id;
+        }
+        turn++;
+        nl = cells + (turn & 7); clear = cells + ((turn + 4) & 7);
+        return true;
+    }
+};
+
 // What a kernel that writes digit planes does beside them for the product behind it (Q1_0)
 struct PlaneDuties {
     int *nl = nullptr;             // receives the digits in use (raised, never lowered)

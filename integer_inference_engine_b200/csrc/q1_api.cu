@@ -33,7 +33,7 @@ std::recursive_mutex q_mu;
 std::vector<Q1Weight> q_w;
 unsigned long long q_weight_bytes = 0;
 cudaStream_t q_stream = nullptr;
-int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [8..15] digits in use (a ring, see next_digits)
+int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [8..15] digits in use (a DigitRing)
 int *q_host_flags = nullptr;            // page-locked: the flag word behind a host-array product
 int q_ready = -1;
 
@@ -80,14 +80,11 @@ void *q_ensure(int role, size_t bytes) {
     return b.p;
 }
 
-// The cell that receives the digits in use of the next digit planes, and the one to clear for later: a ring of eight, each
-// cleared four planes ahead of its use by the kernel that writes the planes (a cell that was not, as in a short replayed
-// graph, is only too large, which costs time and changes no result).
-PlaneDuties next_digits() {
-    static unsigned turn = 0;
-    turn++;
+// The cell that receives the digits in use of the next digit planes, and the one that their kernel clears (null: not to be had).
+PlaneDuties next_digits(cudaStream_t s) {
+    static DigitRing ring;
     PlaneDuties d;
-    d.nl = q_cells + 8 + (turn & 7); d.nl_clear = q_cells + 8 + ((turn + 4) & 7);
+    if (!ring.next(q_cells + 8, s, d.nl, d.nl_clear)) d.nl = nullptr;
     return d;
 }
 
@@ -97,7 +94,8 @@ PlaneDuties next_digits() {
 template <typename Write>
 bool planes_and_products(Write write, const Q1Part *parts, int n, bool sc32, long long nb, const int8_t *planes, long long T, long long frac,
                          const int64_t *in, const int64_t *in2, long long in_n, cudaStream_t s) {
-    PlaneDuties d = next_digits();
+    PlaneDuties d = next_digits(s);
+    if (!d.nl) return false;
     bool fused = true;
     long long row_tiles = 0;
     for (int i = 0; i < n; i++) row_tiles += (parts[i].out_f + 127) / 128;
