@@ -294,7 +294,8 @@ void iie_set_tc_min_tokens(long long tokens);
 unsigned long long iie_launch_count(void);
 /* Launches of each tensor-core (tcgen05) tile shape since load, so a test can tell which shape served a call:
  * out[0..6] = Q4_K gate/up with 3 / 4 activation digits, Q6_K down with 5 / 6, Q4_K down with 5, Q4_K linear with
- * 3 / 5; out[7] every other.  Returns the number of entries, or -1 when capacity is too small. */
+ * 3 / up to 5; out[7] every other.  Counted on the device: synchronises, and a replayed launch counts.  Returns the number of entries
+ * written (capacity, eight at most), or -1 when capacity is below seven. */
 int iie_prefill_launch_counts(unsigned long long *out, int capacity);
 /* Workspace generation: changes whenever a scratch buffer of the library is freed (to grow, by
  * qk_moe_workspace_release or qk_free_all).  A CUDA graph captured over iie_*_dev calls holds the scratch addresses of

@@ -1762,9 +1762,12 @@ extern "C" unsigned long long iie_workspace_generation(void) {
 }
 
 extern "C" int iie_prefill_launch_counts(unsigned long long *out, int capacity) {
-    if (!out || capacity < iie::TILE_SHAPES) return -1;
-    iie::tile_launch_counts(out);
-    return iie::TILE_SHAPES;
+    if (!out || capacity < 7) return -1;                  // (seven entries are as old as the call)
+    unsigned long long counts[iie::TILE_SHAPES];
+    iie::tile_launch_counts(counts);
+    const int n = std::min(capacity, iie::TILE_SHAPES);
+    std::copy(counts, counts + n, out);
+    return n;
 }
 
 extern "C" unsigned long long iie_launch_count(void) { return __atomic_load_n(&iie::g_launches, __ATOMIC_RELAXED); }

@@ -96,3 +96,14 @@ def test_replays_of_a_short_graph_find_their_digit_count_cleared():
     assert device.read_flags() == 0
     del graph
     qk_cuda.free_all()
+
+
+def test_launch_counts_fit_the_room_of_earlier_callers():
+    import ctypes
+
+    from integer_inference_engine_b200 import qk_cuda
+    lib = qk_cuda.load_library()
+    buf = (ctypes.c_uint64 * 8)(*[77] * 8)
+    assert lib.iie_prefill_launch_counts(buf, 6) == -1
+    assert lib.iie_prefill_launch_counts(buf, 7) == 7 and buf[7] == 77
+    assert lib.iie_prefill_launch_counts(buf, 8) == 8 and buf[7] != 77
