@@ -88,7 +88,9 @@ int bonsai_attention_decode_batched_gpu(const long long *q, const long long *Kc,
 /* bonsai_q1_gpu.cu:3694 - the whole prefill on the device: x_embed [T][d] -> every layer -> final norm and output matrix
  * on the last row -> out_logits [vocab].  wq .. w2: per-layer weight handles; n1g .. kng: per-layer buffer handles of the
  * gains; finalg, cos_h, sin_h buffer handles; out_head a weight handle.  out_k / out_v (nullable): the K (after head
- * norm and rotation) and V rows of every layer, [n_layers][Hkv][T][hd].  0 ok, 1 bad arguments / CUDA, 4 overflow. */
+ * norm and rotation) and V rows of every layer, [n_layers][Hkv][T][hd].  0 ok, 1 bad arguments / CUDA, 4 overflow.
+ * The call keeps its device buffers for the next prompt up to 512 MB (those of a longer prompt are freed with it), besides the
+ * digit planes that all products share, and up to 32 MB of page-locked host memory; bonsai_q1_free_weights gives all of it back. */
 int bonsai_prefill_forward_gpu(const long long *x_embed, long long T, long long d, long long n_layers, long long H, long long Hkv,
                                long long hd, long long dff, long long frac, long long eps, long long inv_sqrt_fp,
                                const long long *wq, const long long *wk, const long long *wv, const long long *wo,
@@ -155,7 +157,8 @@ int iie_q1_embed_dev(long long handle, const int *row_dev, long long row, int64_
 /* Kept for its callers: the single-token product has one launch form, whose weights come by bulk copies. */
 void iie_q1_set_stream(int on);
 /* Page-locked host memory for results, from a pool of at most 64 MB (NULL when that is in use or nothing can be locked: use
- * pageable memory then); give it back when nobody reads it any more.  Safe with several threads. */
+ * pageable memory then); give it back when nobody reads it any more.  Safe with several threads.  bonsai_q1_free_weights unlocks
+ * what is not in use. */
 void *iie_host_take(unsigned long long bytes);
 void iie_host_give(void *p);
 /* Changes whenever a scratch buffer of the Q1_0 entries is freed (to grow, or by bonsai_q1_free_weights): a CUDA graph

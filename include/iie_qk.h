@@ -38,7 +38,7 @@ long long qk_register_weight(const uint8_t *W, long long out_f, long long n_bloc
 long long qk_register_i64(const int64_t *W, long long rows, long long cols);
 long long qk_resident_count(void);                   /* nmc_qk_cuda.cu:1805 */
 long long qk_resident_capacity(void);                /* nmc_qk_cuda.cu:1806 */
-void qk_free_all(void);                              /* nmc_qk_cuda.cu:1783 */
+void qk_free_all(void);                              /* nmc_qk_cuda.cu:1783; also the 5 MB of page-locked staging */
 
 /* nmc_qk_cuda.cu:1252 */
 int qk_apply_resident(long long h, const int64_t *x, long long T, int fw, int64_t *out);

@@ -125,9 +125,10 @@ bool sync() { return cudaStreamSynchronize(g_stream) == cudaSuccess; }
 // staging and a wait.  One upload and one download per call (the entries hold the lock and end synchronised); larger arrays go direct.
 constexpr size_t PIN_IN = 1 << 20, PIN_OUT = 4 << 20;
 uint8_t *g_pin = nullptr;
+bool g_pin_tried = false;
+void free_pin() { if (g_pin) cudaFreeHost(g_pin); g_pin = nullptr; g_pin_tried = false; }
 bool pinned() {
-    static bool tried = false;
-    if (!tried) { tried = true; if (cudaHostAlloc(&g_pin, PIN_IN + PIN_OUT, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); g_pin = nullptr; } }
+    if (!g_pin_tried) { g_pin_tried = true; if (cudaHostAlloc(&g_pin, PIN_IN + PIN_OUT, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); g_pin = nullptr; } }
     return g_pin != nullptr;
 }
 bool upload(void *dst, const void *src, size_t n) {
@@ -648,6 +649,7 @@ extern "C" void qk_free_all(void) {
     for (auto &w : g_w) if (w.live && w.d) { cudaFree(w.d); prof(PM_FREE_CALLS); }
     std::vector<Weight>().swap(g_w);                  // capacity returns to zero
     release_workspace();
+    free_pin();
 }
 
 extern "C" int qk_apply_resident(long long h, const int64_t *x, long long T, int fw, int64_t *out) {

@@ -80,6 +80,18 @@ void *q_ensure(int role, size_t bytes) {
     return b.p;
 }
 
+// The prompt call's buffers stay for the next prompt (allocating and freeing them takes a millisecond) up to this many bytes in all, 1400
+// rows of the 8B model; those of a longer prompt go with its call.
+constexpr size_t PROMPT_KEEP = 512 << 20;
+struct PromptBuffers {
+    ~PromptBuffers() {
+        size_t total = 0;
+        for (int role = QR_WORK; role <= QR_LOGITS; role++) total += q_buf[role].cap;
+        for (int role = QR_WORK; total > PROMPT_KEEP && role <= QR_LOGITS; role++)
+            if (q_buf[role].p) { cudaFree(q_buf[role].p); q_buf[role].p = nullptr; q_buf[role].cap = 0; }
+    }
+};
+
 // The cell that receives the digits in use of the next digit planes, and the one that their kernel clears (null: not to be had).
 PlaneDuties next_digits(cudaStream_t s) {
     static DigitRing ring;
@@ -291,6 +303,7 @@ extern "C" int bonsai_q1_apply_resident(long long handle, const long long *x, lo
 }
 
 static void q1_release_model_state();
+static void free_host_pool();
 
 extern "C" void bonsai_q1_free_weights(void) {
     std::lock_guard<std::recursive_mutex> lk(q_mu);
@@ -299,6 +312,7 @@ extern "C" void bonsai_q1_free_weights(void) {
     q_w.clear();
     q_weight_bytes = 0;
     for (auto &b : q_buf) if (b.p) { cudaFree(b.p); b.p = nullptr; b.cap = 0; q_generation++; }
+    free_host_pool();
     q1_release_model_state();                      // uploaded gain / table buffers and decode contexts name these weights
 }
 
@@ -454,6 +468,14 @@ extern "C" void *iie_host_take(unsigned long long bytes) {
     if (total + bytes > HOST_POOL || cudaHostAlloc(&p, bytes, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     h_pool.push_back({p, (size_t)bytes, true});
     return p;
+}
+static void free_host_pool() {                           // but for the arrays in use
+    std::lock_guard<std::mutex> lk(h_mu);
+    for (size_t i = 0; i < h_pool.size();) {
+        if (h_pool[i].used) { i++; continue; }
+        cudaFreeHost(h_pool[i].p);
+        h_pool.erase(h_pool.begin() + (long)i);
+    }
 }
 extern "C" void iie_host_give(void *p) {
     std::lock_guard<std::mutex> lk(h_mu);
@@ -645,16 +667,20 @@ bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logi
 }
 
 // Rows from pageable host memory: four threads copy pieces into a page-locked buffer and send each on its way (one thread, or the
-// driver's own staging, copies 11 GB/s: 1.4 ms for 512 rows of 4096).  A single buffer of at most 32 MB, kept.
+// driver's own staging, copies 11 GB/s: 1.4 ms for 512 rows of 4096).  A single buffer of at most 32 MB, kept until the
+// weights are freed.
+uint8_t *q_pin = nullptr;
+size_t q_pin_cap = 0;
+void free_pin() { if (q_pin) cudaFreeHost(q_pin); q_pin = nullptr; q_pin_cap = 0; }
 bool upload_rows(int64_t *dst, const long long *src, size_t bytes) {
     constexpr size_t LEAST = 1 << 20, MOST = 32 << 20, PIECE = 512 << 10;
     constexpr int THREADS = 4;
-    static uint8_t *pin = nullptr;
-    static size_t cap = 0;
+    uint8_t *&pin = q_pin;
+    size_t &cap = q_pin_cap;
     if (bytes < LEAST) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
     const size_t want = std::min(bytes, MOST);
     if (cap < want) {
-        if (pin) { cudaStreamSynchronize(q_stream); cudaFreeHost(pin); pin = nullptr; cap = 0; }
+        if (pin) { cudaStreamSynchronize(q_stream); free_pin(); }
         if (cudaHostAlloc(&pin, want, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError(); pin = nullptr;
             return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, q_stream) == cudaSuccess;
@@ -888,7 +914,7 @@ extern "C" int bonsai_prefill_forward_gpu(const long long *x_embed, long long T,
     const long long vocab = q_w[(size_t)out_head].out_f;
     const size_t kv_elems = (size_t)Hkv * T * hd;
     Work w;
-    // buffers kept between calls: allocating and freeing them took a millisecond of every prompt
+    PromptBuffers buffers;
     int32_t *kc = (int32_t *)q_ensure(QR_KEYS, kv_elems * 4), *vc = (int32_t *)q_ensure(QR_VALUES, kv_elems * 4);
     int64_t *logits = (int64_t *)q_ensure(QR_LOGITS, (size_t)vocab * 8);
     bool ok = kc && vc && logits && alloc_work(w, m, T, true);
@@ -1038,6 +1064,7 @@ extern "C" void bonsai_decode_ctx_free(long long ctx_h) {
 }
 
 static void q1_release_model_state() {
+    free_pin();
     for (auto &c : q_ctx) if (c.alive) free_ctx(c);
     q_ctx.clear();
     for (auto &b : q_bufs) if (b.p) cudaFree(b.p);

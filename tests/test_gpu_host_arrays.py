@@ -117,3 +117,36 @@ def test_prompt_rows_arrive_whole(T):
     want = onat.q1_linear(o.rmsnorm_fixed(x, 16, 1, gains["n1g"]), *raw["wv"], 16)
     assert np.array_equal(got[2][0, 0], want)
     q1_gpu.q1_free_weights()
+
+
+def test_buffers_of_a_long_prompt_go_with_the_call():
+    """600 rows with a feed-forward width of 65536 need 632 MB of activation rows, beyond what a call keeps; all of it is given back with
+    the weights."""
+    import torch
+
+    from integer_inference_engine_b200 import q1_gpu
+    rng = np.random.default_rng(1)
+    d, H, Hkv, hd, dff, vocab, T = 128, 2, 1, 64, 65536, 40, 600
+    shapes = {"wq": (H * hd, d), "wk": (Hkv * hd, d), "wv": (Hkv * hd, d), "wo": (d, H * hd), "w1": (dff, d), "wu": (dff, d), "w2": (d, dff)}
+    x = rng.integers(-(1 << 14), 1 << 14, size=(T, d), dtype=np.int64)
+
+    def prompt(rows):
+        w = {}
+        for name, (out_f, in_f) in shapes.items():
+            bits, scale = o.synth_q1(np.random.default_rng(len(name)), out_f, in_f // 128)
+            w[name] = [q1_gpu.q1_register_weight(bits, scale.astype(np.int32))]
+        bits, scale = o.synth_q1(rng, vocab, 1)
+        w["out_head"], w["out_head_vocab"] = q1_gpu.q1_register_weight(bits, scale.astype(np.int32)), vocab
+        gh = {name: [q1_gpu.buf_upload_i64(np.full(n, 1 << 16, np.int64))] for name, n in (("n1g", d), ("n2g", d), ("qng", hd), ("kng", hd))}
+        cos, sin = o.build_rope_tables(T, hd, frac=16)
+        gh["finalg"], gh["cos_h"], gh["sin_h"] = q1_gpu.buf_upload_i64(np.full(d, 1 << 16, np.int64)), q1_gpu.buf_upload_i64(cos), q1_gpu.buf_upload_i64(sin)
+        assert q1_gpu.prefill_forward_gpu(x[:rows], (rows, d, 1, H, Hkv, hd, dff), w, gh, 16, 1, 1 << 13) is not None
+
+    q1_gpu.q1_free_weights()
+    prompt(8)
+    before = torch.cuda.mem_get_info()[0]
+    prompt(T)
+    kept = before - torch.cuda.mem_get_info()[0]
+    assert kept < 450 << 20, kept                                       # the shared digit planes (315 MB) and attention scratch
+    q1_gpu.q1_free_weights()
+    assert before - torch.cuda.mem_get_info()[0] < 64 << 20
