@@ -63,8 +63,14 @@ __global__ void q1_repack_kernel(const uint8_t *bits, const ST *scale, long long
 
 // ---- activations: digit planes [tok][8][K], digits in use ---------------------------
 // With `up` the activation is the SwiGLU of two rows of width K: ((x * sigmoid(x)) >> frac) * up >> frac, wrapping products;
-// x and up then advance by `ld` per token.
-__global__ void q1_prep_kernel(const int64_t *x, const int64_t *up, long long ld, int frac, int64_t log2e, int64_t clip, long long T,
+// x and up then advance by `ld` per token.  `wide`: every row starts on 16 bytes.
+__device__ __forceinline__ void q1_four(const int64_t *src, bool wide, int64_t (&v)[4]) {
+    longlong2 a, b;
+    if (wide) { a = *reinterpret_cast<const longlong2 *>(src); b = *reinterpret_cast<const longlong2 *>(src + 2); }
+    else { a = make_longlong2(src[0], src[1]); b = make_longlong2(src[2], src[3]); }
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__global__ void q1_prep_kernel(const int64_t *x, const int64_t *up, long long ld, bool wide, int frac, int64_t log2e, int64_t clip, long long T,
                                long long nb, int8_t *planes, const PlaneDuties duties) {
     pdl_enter();
     int *nl_out = duties.nl;
@@ -75,12 +81,12 @@ __global__ void q1_prep_kernel(const int64_t *x, const int64_t *up, long long ld
     if (wid >= T * nb) return;
     const long long tok = wid / nb, b = wid - tok * nb, K = nb * 128;
     const int64_t *src = x + tok * (up ? ld : K) + b * 128 + lane * 4;
-    const longlong2 v0 = *reinterpret_cast<const longlong2 *>(src), v1 = *reinterpret_cast<const longlong2 *>(src + 2);
-    int64_t v[4] = {v0.x, v0.y, v1.x, v1.y};
+    int64_t v[4];
+    q1_four(src, wide, v);
     if (up) {
         const int64_t *us = up + tok * ld + b * 128 + lane * 4;
-        const longlong2 u0 = *reinterpret_cast<const longlong2 *>(us), u1 = *reinterpret_cast<const longlong2 *>(us + 2);
-        const int64_t u[4] = {u0.x, u0.y, u1.x, u1.y};
+        int64_t u[4];
+        q1_four(us, wide, u);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int64_t sg = sigmoid_fixed_c(v[i], frac, log2e, clip);
@@ -151,7 +157,7 @@ cudaError_t launch_q1_repack(const uint8_t *bits, const void *scale, int src_bit
 cudaError_t launch_q1_prep(const int64_t *x, long long T, long long nb, int8_t *planes, const PlaneDuties &duties,
                            cudaStream_t s) {
     const long long warps = T * nb;
-    launch_behind(q1_prep_kernel, (unsigned)((warps * 32 + 255) / 256), 256, 0, s, x, nullptr, 0, 0, 0, 0, T, nb, planes, duties);
+    launch_behind(q1_prep_kernel, (unsigned)((warps * 32 + 255) / 256), 256, 0, s, x, nullptr, 0, (reinterpret_cast<uintptr_t>(x) & 15) == 0, 0, 0, 0, T, nb, planes, duties);
     note_launch();
     return cudaGetLastError();
 }
@@ -160,7 +166,8 @@ cudaError_t launch_q1_prep_swiglu(const int64_t *gate, const int64_t *up, long l
                                   int8_t *planes, const PlaneDuties &duties, cudaStream_t s) {
     if (!gate || !up || frac < 1 || frac > 29) return cudaErrorInvalidValue;
     const long long warps = T * nb;
-    launch_behind(q1_prep_kernel, (unsigned)((warps * 32 + 255) / 256), 256, 0, s, gate, up, ld, frac, sigmoid_log2e(frac), sigmoid_clip(frac), T, nb,
+    const bool wide = ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | (uintptr_t)(ld * 8)) & 15) == 0;
+    launch_behind(q1_prep_kernel, (unsigned)((warps * 32 + 255) / 256), 256, 0, s, gate, up, ld, wide, frac, sigmoid_log2e(frac), sigmoid_clip(frac), T, nb,
                                                                         planes, duties);
     note_launch();
     return cudaGetLastError();

@@ -62,3 +62,31 @@ def test_largest_sums_of_three_planes(nb, scale, T):
     device.read_flags()
     assert np.array_equal(q1_gpu.apply_dev(h, torch.from_numpy(x).cuda(), FRAC).cpu().numpy(), onat.q1_linear(x, bits, scales, FRAC))
     assert device.read_flags() == 0
+
+
+@pytest.mark.parametrize("T", [1, 2, 9])
+def test_rows_that_start_on_eight_bytes(T):
+    """Activations, gain, gate and up at odd element offsets and an odd row distance."""
+    import torch
+
+    from integer_inference_engine_b200 import device, q1_gpu
+    rng = np.random.default_rng(T)
+    out_f, nb = 70, 3
+    K = nb * 128
+    bits, scale = o.synth_q1(rng, out_f, nb)
+    h = q1_gpu.q1_register_weight(bits, scale.astype(np.int32))
+    odd = lambda a: torch.cat([torch.zeros(1, dtype=torch.int64), torch.from_numpy(a.reshape(-1))]).cuda()[1:].view(a.shape)
+    x, gain = rng.integers(-(1 << 20), 1 << 20, size=(T, K), dtype=np.int64), rng.integers(-(1 << 17), 1 << 17, size=K, dtype=np.int64)
+    gu = rng.integers(-(1 << 18), 1 << 18, size=(T, 2 * K + 1), dtype=np.int64)
+    new = lambda: torch.empty((T, out_f), dtype=torch.int64, device="cuda")
+    device.read_flags()
+    assert np.array_equal(q1_gpu.apply_dev(h, odd(x), FRAC).cpu().numpy(), onat.q1_linear(x, bits, scale, FRAC))
+    got = q1_gpu.apply_fused_dev(h, odd(x), FRAC, new(), norm=True, gain=odd(gain)).cpu().numpy()
+    assert np.array_equal(got, onat.q1_linear(o.rmsnorm_fixed(x, FRAC, 1, gain), bits, scale, FRAC))
+    g, u = gu[:, :K], gu[:, K + 1:]
+    act = ((g * o.sigmoid_fixed(g, FRAC) >> FRAC) * u) >> FRAC
+    gud = odd(gu)
+    for gd, ud in ((gud[:, :K], gud[:, K + 1:]), (torch.from_numpy(gu).cuda()[:, :K], torch.from_numpy(gu).cuda()[:, K + 1:])):
+        got = q1_gpu.apply_fused_dev(h, gd, FRAC, new(), up=ud).cpu().numpy()
+        assert np.array_equal(got, onat.q1_linear(act, bits, scale, FRAC))
+    assert device.read_flags() == 0
