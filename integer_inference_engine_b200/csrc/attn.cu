@@ -680,7 +680,7 @@ __device__ __forceinline__ bool af_group_barrier(unsigned *counter, unsigned tar
 
 // NORM: the per-head norms of queries and key first (a form of its own: their code costs the others about 1 us a launch)
 // CLUSTER: the chunks of a KV head are one cluster (short spans); maximum, normaliser and sums pass through distributed shared memory in
-// place of global atomics, group barriers and a last arrival: 0.4 to 0.7 us of a launch.
+// place of global atomics, group barriers and a last arrival (figures and border: launch_attn_decode).
 template <bool NORM, bool CLUSTER>
 __global__ void __launch_bounds__(AF_THREADS, 1) attn_fat_kernel(const AttnArgs a_in) {
     AttnArgs a = a_in;
@@ -1425,21 +1425,31 @@ cudaError_t launch_attn_decode(const AttnArgs &a, cudaStream_t s) {
     // one CTA per SM where a KV head's keys, cut into n_sms / Hkv chunks, fit the shared memory of a CTA
     if (g_attn_fused == 1 && a.partial && n_sms > 0 && !a.batch && rep <= AF_HEADS && AF_THREADS % a.hd == 0 && a.hd % 32 == 0 &&
         a.fa <= 23 && a.Hkv <= 120) {                                       // probabilities (at most 2^fa) as three bytes
-        static bool fat_configured = false;
+        static bool fat_configured = false, clusters_run = false;          // eight CTAs of the largest size, as the device at hand schedules them
         if (!fat_configured) {
             for (const auto kernel : {attn_fat_kernel<false, false>, attn_fat_kernel<true, false>, attn_fat_kernel<false, true>, attn_fat_kernel<true, true>})
                 if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 208 * 1024) != cudaSuccess ||
                     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess) return cudaGetLastError();
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 8; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3(8, 1); cfg.blockDim = dim3(AF_THREADS); cfg.dynamicSmemBytes = 208 * 1024; cfg.attrs = attr; cfg.numAttrs = 1;
+            int at_once = 0;
+            clusters_run = cudaOccupancyMaxActiveClusters(&at_once, attn_fat_kernel<true, true>, &cfg) == cudaSuccess && at_once > 0;
+            cudaGetLastError();
             fat_configured = true;
         }
         auto smem_of = [&](int C) {
             return ((size_t)2 * C * a.hd + (size_t)C / 8 * 24) * 4 + (size_t)AF_HEADS * a.hd * 12 + (size_t)C * AF_HEADS * 4 +
                    (size_t)AF_THREADS / a.hd * AF_HEADS * a.hd * 8 + (size_t)4 * AF_HEADS * (a.hd + 16) + (size_t)3 * AF_HEADS * (C + 16);
         };
-        // up to 768 keys: clusters of at most eight CTAs, 96 keys each (at 1000 keys, 128 each, the wider split is 0.5 % quicker again; clusters
-        // of sixteen are no quicker)
+        // Up to 768 keys: clusters of at most eight CTAs, 96 keys each.  A launch at 64 / 256 / 512 / 768 keys, 32 query and 8 KV heads of 128:
+        // 9.9 / 10.8 / 12.0 / 13.1 us against 12.6 / 13.0 / 13.5 / 14.7 of the cooperative form (4 KV heads 10.3 / 11.0 / 12.2 / 13.1 against
+        // 12.8 / 13.1 / 13.4 / 13.8); a whole token at 300 keys 2043 against 2067, of the 1-bit model at 512 keys 1617 against 1648, runs within
+        // 0.2 %.  Beyond, at 128 keys a CTA, the two disagree: 820 keys over 4 KV heads 2099 against 2057 a token, over 8 KV heads 1667 against 1682.
         const int Cc = std::max(32, (int)((n_keys + 7) / 8 + 31) / 32 * 32);
-        const bool cluster = Cc <= 96 && smem_of(Cc) <= 208 * 1024;
+        const bool cluster = Cc <= 96 && smem_of(Cc) <= 208 * 1024 && clusters_run;
         const int per_head = std::max(1, std::min(n_sms, 192) / a.Hkv);      // the partial-sum scratch holds 192 chunks
         // whole 32-key steps of the tensor-core passes
         const int C = cluster ? Cc : std::max(32, (int)((n_keys + per_head - 1) / per_head + 31) / 32 * 32);
