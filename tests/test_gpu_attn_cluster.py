@@ -1,4 +1,4 @@
-"""Attention by clusters against the three-launch form: edges of tiles, warps and clusters, windows, head shapes, scores beyond 32 bits (their
+"""Attention by clusters against the three-launch form and the checker: edges of tiles, warps and clusters, windows, head shapes, scores beyond 32 bits (their
 base moves), queries beyond int32, probabilities of three bytes; and the other small kernels of a step of several rows."""
 import numpy as np
 import pytest
@@ -74,6 +74,29 @@ def test_scores_that_move_the_base_count_as_before(hd, wide):
                                         hd, fa, inv_sqrt=inv_sqrt)
     assert device.read_flags() == 0
     assert np.array_equal(got.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize(("pos", "H", "Hkv", "hd", "window", "rope", "fa"), [(0, 8, 1, 64, 0, 1, 16), (95, 6, 2, 128, 0, 2, 16), (517, 8, 2, 64, 300, 1, 16),
+                                                                            (1025, 4, 1, 128, 0, 0, 22), (640, 16, 2, 64, 641, 2, 12)])
+def test_cluster_form_against_the_checker(pos, H, Hkv, hd, window, rope, fa):
+    import torch
+
+    from integer_inference_engine_b200 import device
+    from integer_inference_engine_b200.model import rope_tables
+    from oracle import qk_oracle as o
+    B, rng = 3, np.random.default_rng(pos + hd)
+    q, k, v = (rng.integers(-(1 << 18), 1 << 18, size=(B, n * hd), dtype=np.int64) for n in (H, Hkv, Hkv))
+    kc, vc = (rng.integers(-(1 << 18), 1 << 18, size=(B, Hkv, pos + 2, hd), dtype=np.int64) for _ in range(2))
+    cos, sin = (np.ascontiguousarray(t, np.int64) for t in rope_tables(pos + 1, hd, 50000.0, fa))
+    dev = lambda a, t=torch.int64: torch.from_numpy(np.ascontiguousarray(a)).to("cuda", t)
+    device.read_flags()
+    got = device.attention_decode_batch(dev(q), dev(k), dev(v), dev(kc, torch.int32), dev(vc, torch.int32), pos, H, Hkv, hd, fa, window, dev(cos), dev(sin), rope)
+    for b in range(B):
+        turn = lambda a, n: o.rope_fixed(a.reshape(n, 1, hd), cos[pos:pos + 1], sin[pos:pos + 1], fa, neox=rope == 2) if rope else a.reshape(n, 1, hd)
+        kc[b, :, pos], vc[b, :, pos] = turn(k[b], Hkv)[:, 0], v[b].reshape(Hkv, hd)
+        want = o.attention_cached(turn(q[b], H).transpose(1, 0, 2), kc[b][:, :pos + 1], vc[b][:, :pos + 1], pos, H, Hkv, fa, window or None)
+        assert np.array_equal(got[b:b + 1].cpu().numpy(), want), b
+    assert device.read_flags() == 0
 
 
 def test_column_slices_as_rows():

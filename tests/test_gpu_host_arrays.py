@@ -150,3 +150,43 @@ def test_buffers_of_a_long_prompt_go_with_the_call():
     assert kept < 450 << 20, kept                                       # the shared digit planes (315 MB) and attention scratch
     q1_gpu.q1_free_weights()
     assert before - torch.cuda.mem_get_info()[0] < 64 << 20
+
+
+@pytest.mark.parametrize(("H", "Hkv", "positions"), [(8, 1, (0, 31, 32, 1000, 2300)), (4, 2, (127, 128, 129, 5)), (8, 1, (16384, 3, 700)), (32, 2, (70, 0, 40))])
+def test_sequences_at_their_own_positions(H, Hkv, positions):
+    """One decode step of sequences of very different lengths (in the one launch for all of them the shorter ones leave warps and CTAs of their
+    clusters without keys), beyond the keys that launch takes, and with more query heads per KV head than it takes; against the checker."""
+    from integer_inference_engine_b200 import q1_gpu
+    from integer_inference_engine_b200.model import rope_tables
+    from oracle import model_oracle
+    rng = np.random.default_rng(sum(positions))
+    d, hd, dff, vocab, B, cap = 256, 64, 128, 96, len(positions), max(positions) + 2
+    qd, kd, inv_sqrt = H * hd, Hkv * hd, 1 << 13
+    q1 = lambda out_f, in_f: o.synth_q1(rng, out_f, in_f // 128)
+    raw = {"wqkv": q1(qd + 2 * kd, d), "wo": q1(d, qd), "w1u": q1(2 * dff, d), "w2": q1(d, dff)}
+    top = {"embed": q1(vocab, d), "head": q1(vocab, d), "out_gain": rng.integers(1 << 15, 1 << 17, size=d, dtype=np.int64)}
+    gains = {n: rng.integers(1 << 15, 1 << 17, size=s, dtype=np.int64) for n, s in (("n1", d), ("n2", d), ("qn", hd), ("kn", hd))}
+    cos, sin = (np.ascontiguousarray(t, np.int64) for t in rope_tables(cap, hd, 1e6, 16))
+    rows = {"wq": ("wqkv", 0, qd), "wk": ("wqkv", qd, qd + kd), "wv": ("wqkv", qd + kd, qd + 2 * kd), "wo": ("wo", 0, d), "w1": ("w1u", 0, dff),
+            "wu": ("w1u", dff, 2 * dff), "w2": ("w2", 0, d)}
+    w = {n: [q1_gpu.q1_register_weight(raw[m][0][a:b], raw[m][1][a:b].astype(np.int32))] for n, (m, a, b) in rows.items()}
+    w["out_head"], w["out_head_vocab"] = q1_gpu.q1_register_weight(top["head"][0], top["head"][1].astype(np.int32)), vocab
+    gh = {n: [q1_gpu.buf_upload_i64(gains[m])] for n, m in (("n1g", "n1"), ("n2g", "n2"), ("qng", "qn"), ("kng", "kn"))}
+    gh["finalg"], gh["cos_h"], gh["sin_h"] = (q1_gpu.buf_upload_i64(a) for a in (top["out_gain"], cos, sin))
+    ctx = q1_gpu.decode_ctx_create((B, 1, H, Hkv, hd, d, dff, vocab), w, gh, 16, 1, inv_sqrt, cap)
+    assert ctx is not None
+    caches = [[rng.integers(-(1 << 17), 1 << 17, size=(Hkv, cap, hd), dtype=np.int64) for _ in range(2)] for _ in range(B)]
+    for b, pos in enumerate(positions):
+        assert q1_gpu.decode_ctx_seed_seq(ctx, b, caches[b][0][None, :, :pos], caches[b][1][None, :, :pos])
+    tokens = rng.integers(0, vocab, size=(2, B))
+    cfg = dict(d=d, H=H, Hkv=Hkv, hd=hd, ffn=dff, frac=16)
+    for step in range(2):
+        x = np.concatenate([model_oracle.q1_rows(*top["embed"], int(t)) for t in tokens[step]])
+        logits = q1_gpu.decode_step(ctx, x, [p + step for p in positions], vocab)
+        assert logits is not None
+        for b, pos in enumerate(positions):
+            layer = dict(raw, **gains, k=caches[b][0], v=caches[b][1])
+            _, _, want = model_oracle.q1_decode_token(int(tokens[step][b]), pos + step, [layer], top, cfg, cos, sin)
+            assert np.array_equal(logits[b], want), (step, b)
+    q1_gpu.decode_ctx_free(ctx)
+    q1_gpu.q1_free_weights()

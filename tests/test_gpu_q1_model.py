@@ -187,8 +187,9 @@ def test_rmsnorm_long_rows(rows, width):
 
 
 @pytest.mark.parametrize(("out_f", "nb"), [(48, 1), (200, 4), (4096, 32), (1000, 96), (33, 128)])
-def test_single_token_launch_forms_agree(out_f, nb):
-    """The bulk-copy kernel and the per-lane-load kernel against the checker, int32 and int64 scales."""
+def test_single_row_products_with_scales_of_both_widths(out_f, nb):
+    """The single-row kernel against the checker: int32 and int64 scales, rows of more than four digits, and rows within four digits at their
+    ends with scales on both sides of 2^20, where the product of factor, sum and scale still fits 64 bits and where it does not."""
     import torch
 
     from integer_inference_engine_b200 import device, q1_gpu
@@ -196,15 +197,14 @@ def test_single_token_launch_forms_agree(out_f, nb):
     rng = np.random.default_rng(70 + out_f + nb)
     bits, scale = o.synth_q1(rng, out_f, nb)
     x = rng.integers(-(1 << 40), 1 << 40, size=(1, nb * 128), dtype=np.int64)
-    xd = torch.from_numpy(x).cuda()
+    ends = np.where(rng.integers(0, 2, size=x.shape) == 1, (1 << 30) - 1, -(1 << 30) + 1)
+    one_sign = bits.copy()
+    one_sign[::2], one_sign[1::4] = 0xFF, 0
     device.read_flags()
-    try:
-        for sc in (scale.astype(np.int32), rng.integers(-(1 << 40), 1 << 40, size=scale.shape, dtype=np.int64)):
-            h = q1_gpu.q1_register_weight(bits, sc)
-            want = onat.q1_linear(x, bits, sc.astype(np.int64), FRAC)
-            for form in (True, False):
-                q1_gpu.set_stream_form(form)
-                assert np.array_equal(q1_gpu.apply_dev(h, xd, FRAC).cpu().numpy(), want), (form, sc.dtype)
-    finally:
-        q1_gpu.set_stream_form(False)
+    limit = lambda top: np.where(rng.integers(0, 2, size=scale.shape) == 1, top, -top)
+    for b, sc, row in ((bits, scale.astype(np.int32), x), (bits, rng.integers(-(1 << 40), 1 << 40, size=scale.shape, dtype=np.int64), x),
+                       (one_sign, limit((1 << 20) - 1).astype(np.int32), ends), (one_sign, limit((1 << 20) - 1).astype(np.int32), np.full_like(x, -(1 << 30) + 1)),
+                       (one_sign, limit(1 << 20).astype(np.int32), np.full_like(x, -(1 << 30) + 1)), (one_sign, limit((1 << 31) - 1), ends)):
+        h = q1_gpu.q1_register_weight(b, sc)
+        assert np.array_equal(q1_gpu.apply_dev(h, torch.from_numpy(row).cuda(), FRAC).cpu().numpy(), onat.q1_linear(row, b, sc.astype(np.int64), FRAC)), sc.dtype
     assert device.read_flags() == 0

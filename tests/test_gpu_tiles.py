@@ -107,3 +107,59 @@ def test_launch_counts_fit_the_room_of_earlier_callers():
     assert lib.iie_prefill_launch_counts(buf, 6) == -1
     assert lib.iie_prefill_launch_counts(buf, 7) == 7 and buf[7] == 77
     assert lib.iie_prefill_launch_counts(buf, 8) == 8 and buf[7] != 77
+
+
+@pytest.mark.parametrize("qtype", [o.Q4_K, o.Q6_K])
+@pytest.mark.parametrize("T", [2, 33])
+def test_largest_sums_of_a_row(qtype, T):
+    """64 super-blocks of the largest scales, minima and codes at the largest block scales the tiles take, every value at one end of its digits."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    out_f, nb = 16, 64
+    raw = np.zeros((out_f, nb, 144 if qtype == o.Q4_K else 210), np.uint8)
+    raw[:, :, slice(4, 144) if qtype == o.Q4_K else slice(0, 208)] = 0xFF
+    raw[1::4, :, 16 if qtype == o.Q4_K else 0:144 if qtype == o.Q4_K else 192] = 0            # the smallest codes
+    if qtype == o.Q6_K:
+        raw[::2, :, 192:208] = 0x80                                            # scales of -128
+    half = lambda v: np.frombuffer(np.float16(v).tobytes(), np.uint8)
+    if qtype == o.Q4_K:
+        raw[:, :, 0:2], raw[:, :, 2:4] = half(0.49975586), half(3.9980469)     # d below 2^23, dmin below 2^26 at 2^24
+    else:
+        raw[:, :, 208:210] = half(0.49975586)
+    buf = raw.tobytes()
+    h = qk_cuda.register_weight(buf, out_f, nb, qtype)
+    device.read_flags()
+    for top, bottom in ((8355711, -8421504), (0x7F7F7F7F, -0x80808080), (0x7F7F7F7F7F7F, -0x808080808080), (0x7F7F7F7F7F7F7F7F, -0x7F7F7F7F7F7F7F7F)):
+        x = np.full((T, nb * 256), bottom, np.int64)
+        x[1::2] = top
+        before = device.prefill_launch_counts()
+        got = device.apply(h, torch.from_numpy(x).cuda(), out_f, FW).cpu().numpy()
+        assert sum(device.prefill_launch_counts()) == sum(before) + 1, "the product did not run on the tiles"
+        assert np.array_equal(got, onat.qk_linear(buf, x, out_f, nb, FW, qtype))
+    assert device.read_flags() == 0
+
+
+@pytest.mark.parametrize("fa", [1, 5, 12, 20, 24, 25])
+def test_expert_tiles_at_other_activation_scales(fa):
+    """The epilogue's 32-bit SiLU up to a scale of 2^24, the general one beyond; gates of all magnitudes around the sigmoid's clip."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(fa)
+    d, eff, E, k, T = 256, 256, 2, 2, 40
+    q4 = lambda r, c: o.synth_q4k(rng, r, c // 256)
+    router, gate, up, down = q4(E, d), [q4(eff, d) for _ in range(E)], [q4(eff, d) for _ in range(E)], [q4(d, eff) for _ in range(E)]
+    h = np.rint(rng.standard_normal((T, d)) * np.exp2(rng.uniform(-3, 9, size=(T, 1))) * (1 << fa)).astype(np.int64)
+    reg = lambda w, r, c: qk_cuda.register_weight(w, r, c // 256, o.Q4_K)
+    layer = device.MoELayer(reg(router, E, d), [reg(w, eff, d) for w in gate], [reg(w, eff, d) for w in up], [reg(w, d, eff) for w in down], k, d, eff)
+    device.read_flags()
+    before = device.prefill_launch_counts()
+    out, ids, gates = layer.forward(torch.from_numpy(h).cuda(), fa, FW)
+    torch.cuda.synchronize()
+    assert sum(device.prefill_launch_counts()) - sum(before) == 3
+    ids_ref, gates_ref, out_ref = onat.moe_block(router, o.Q4_K, gate, up, down, o.Q4_K, o.Q4_K, k, h, d, eff, fa, FW)
+    assert device.read_flags() == 0
+    assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
+    assert np.array_equal(out.cpu().numpy(), out_ref)
+    layer.close()
