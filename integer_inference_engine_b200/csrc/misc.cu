@@ -381,7 +381,16 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const NormArgs a) {
     }
     const bool fast = nr.fast;
     const uint64_t inv = !fast && nr.rms < (1ULL << 62) ? recip_below(nr.rms) : 0;
-    const uint64_t gm = !fast && gain ? warp_gain_max(gain, a.width) : 0;      // the general form refuses against the row's largest |gain|
+    uint64_t gm = 0;                                               // the general form refuses against the row's largest |gain|
+    if (!fast && gain) {
+        gm = warp_max64(gmx);
+        if (wpr > 1) {                                             // (every warp of the CTA is here: a row has one form)
+            __shared__ uint64_t s_gm[32];
+            if (lane == 0) s_gm[warp] = gm;
+            __syncthreads();
+            gm = warp_max64(lane < wpr ? s_gm[lane] : 0);
+        }
+    }
     bool bad = false;
     int nl = 0;
 #pragma unroll
@@ -453,16 +462,11 @@ __global__ void __launch_bounds__(256) rmsnorm_any_kernel(const NormArgs a) {
         ssq += (u128)m * m;
         mx = m > mx ? m : mx; gm = gv > gm ? gv : gm;
     }
-    auto top = [&](uint64_t v) {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) { const uint64_t o = __shfl_xor_sync(0xffffffffu, v, off); v = o > v ? o : v; }
-        return v;
-    };
-    ssq = warp_sum128(ssq); mx = top(mx); gm = top(gm);
+    ssq = warp_sum128(ssq); mx = warp_max64(mx); gm = warp_max64(gm);
     if (lane == 0) { s_lo[warp] = (uint64_t)ssq; s_hi[warp] = (uint64_t)(ssq >> 64); s_max[warp] = mx; s_gmax[warp] = gm; }
     __syncthreads();
     ssq = warp_sum128(lane < 8 ? ((u128)s_hi[lane] << 64) | s_lo[lane] : (u128)0);
-    mx = top(lane < 8 ? s_max[lane] : 0); gm = top(lane < 8 ? s_gmax[lane] : 0);
+    mx = warp_max64(lane < 8 ? s_max[lane] : 0); gm = warp_max64(lane < 8 ? s_gmax[lane] : 0);
     const u128 root = isqrt128(ssq / (u128)(unsigned)a.width + a.eps);
     if (mx > (1ULL << 57) || a.width > 8192 || root == 0 || (root >> 64) != 0) { if (tid == 0) atomicOr(a.flags, 2); return; }
     const uint64_t rms = (uint64_t)root, inv = rms < (1ULL << 62) ? recip_below(rms) : 0;

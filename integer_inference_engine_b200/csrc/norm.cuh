@@ -127,13 +127,16 @@ struct NormRow {
         return (int)(((int64_t)q * g) >> sh);
     }
 };
+__device__ __forceinline__ uint64_t warp_max64(uint64_t v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) { const uint64_t o = __shfl_xor_sync(0xffffffffu, v, off); v = o > v ? o : v; }
+    return v;
+}
 // largest |gain| of a row, for the values that take the general form: the whole warp
 __device__ __forceinline__ uint64_t warp_gain_max(const int64_t *gain, int width) {
     uint64_t gm = 0;
     for (int k = 0; k < width; k += 32) { const int i = k + (threadIdx.x & 31); const uint64_t v = i < width ? uabs64(gain[i]) : 0; gm = v > gm ? v : gm; }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) { const uint64_t o = __shfl_xor_sync(0xffffffffu, gm, off); gm = o > gm ? o : gm; }
-    return gm;
+    return warp_max64(gm);
 }
 
 }  // namespace iie
