@@ -1279,7 +1279,7 @@ __global__ void embed_row_kernel(const uint8_t *w, int qtype, long long nb, cons
 }
 
 // arg-max of each of grid.x rows of n values, lowest index on ties: the grid.y CTAs of a cluster share a row and hand their candidates to
-// the first.  Bounded by the load latency of a CTA (7 rows of 151936: 21 us with one CTA a row).
+// the first.  Bounded by the load latency of a CTA (7 rows of 151936: 21 us with one CTA a row, 7 with eight).
 constexpr int AR_PARTS = 8;
 
 __global__ void __launch_bounds__(1024) argmax_rows_kernel(const int64_t *x, long long n, int *out) {
@@ -1588,7 +1588,10 @@ cudaError_t launch_embed_rows(const uint8_t *w, int qtype, long long nb, const i
 
 cudaError_t launch_argmax_rows(const int64_t *x, long long rows, long long n, int *out, cudaStream_t s) {
     if (n <= 0 || rows <= 0 || rows > 0x7fffffffLL) return cudaErrorInvalidValue;
-    const int parts = rows <= 128 && n >= 32768 ? AR_PARTS : 1;       // (a share of a short row is less than a CTA's start; many rows fill the SMs)
+    // Of eight, four or two CTAs a row the most that make 256 CTAs at most, what the SMs hold in whole clusters at two CTAs each: 151936 values,
+    // 32 / 64 / 128 rows 11.6 / 17.5 / 29.5 us (one CTA a row 35.2 / 36.3 / 39.9; eight for all of them 11.6 / 21.4 / 40.7); 32768 values, 128 rows
+    // 10.1 (11.2; 19.7).  A share of a row below 32768 values is less than a CTA's start; more rows fill the SMs.
+    const int parts = n < 32768 ? 1 : rows <= 32 ? AR_PARTS : rows <= 64 ? AR_PARTS / 2 : rows <= 128 ? AR_PARTS / 4 : 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)rows, (unsigned)parts); cfg.blockDim = dim3(1024); cfg.stream = s;
     cudaLaunchAttribute attr[1];

@@ -114,7 +114,7 @@ def test_column_slices_as_rows():
     assert torch.equal(a, b) and all(torch.equal(x, y) for x, y in zip(*caches))
 
 
-@pytest.mark.parametrize(("rows", "n"), [(1, 32768), (7, 151936), (3, 100001), (128, 32769), (129, 40000)])
+@pytest.mark.parametrize(("rows", "n"), [(1, 32768), (7, 151936), (3, 100001), (32, 32771), (33, 40001), (64, 65536), (65, 33333), (128, 32769), (129, 40000)])
 def test_argmax_rows_shared_by_a_cluster(rows, n):
     import torch
 
