@@ -288,8 +288,8 @@ int iie_rmsnorm_dev(long long gain_h, const int64_t *x_dev, long long rows, long
 void iie_profile_stage_mask(int mask);
 /* Switch programmatic dependent launch between the three single-token kernels on (default) or off. */
 void iie_set_pdl(int enabled);
-/* Row count from which products use the tcgen05 tiles instead of the streamed kernels (default 2; a very large
- * value disables the tensor-core path). */
+/* Row count from which products use the tcgen05 tiles instead of the streamed kernels (default 0: by rows and sizes, always from
+ * 192 rows on; a very large value disables the tensor-core path). */
 void iie_set_tc_min_tokens(long long tokens);
 unsigned long long iie_launch_count(void);
 /* Launches of each tensor-core (tcgen05) tile shape since load, so a test can tell which shape served a call:

@@ -62,7 +62,8 @@ int g_pdl = 1;                        // programmatic dependent launch between t
 long long g_hl_d = 0;                 // width of the digit planes the last single-token routing left in the R_XL scratch
 int64_t *g_pow2 = nullptr;            // device: 2^i for i = 0..31 (unit gates at any activation scale)
 int g_attn_parity = 0;                // which of the two attention digit-count cells the next block call uses
-long long g_tc_min_tokens = 2;        // from this many rows on, products run on the tcgen05 tiles
+long long g_tc_min_tokens = 0;        // from this many rows on, products run on the tcgen05 tiles (0: by size, see linear_dev and moe_fused)
+constexpr long long TILES_FROM = 192; // rows from which every product takes the tiles
 int g_ready = -1;                     // -1 unknown, 0 usable, 1 unusable
 int g_stage_mask = 0;                 // profiling: when non-zero, iie_moe_forward_dev runs only these stages
 enum Stage { ST_LIMBS = 1, ST_ROUTER = 2, ST_TOPK = 4, ST_GATEUP = 8, ST_DOWN = 16 };
@@ -271,8 +272,23 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
         } else if (launch_limbs(x, T, K, buf, g_flags, s) != cudaSuccess) return false;
         xl = buf;
     }
-    bool done = false;
-    if (T >= 2 && T >= g_tc_min_tokens && T < (1 << 24) && g_stage_mask == 0 && tile_scales(w.qtype, w.nb, w.maxd, w.maxdmin, fw)) {
+    auto batch = [&]() {
+        // a few rows: one group that owns all of them, every tile streamed once
+        int *off = (int *)ensure(R_META, 64);
+        if (!off || launch_set2(off, 0, (int)T, s) != cudaSuccess) return false;
+        BatchArgs ba = {};
+        ba.wa = w.cell; ba.wb = w.cell; ba.grp_off = off; ba.n_groups = 1; ba.out_f = w.out_f; ba.n_blocks = w.nb; ba.fw = fw; ba.fa = 16;
+        ba.fast = small_scales(w.maxd, w.maxdmin, fw); ba.xl = xl; ba.x_nl = x_nl; ba.out = out; ba.flags = g_flags;
+        if (launch_batch(w.qtype, MODE_LINEAR, ba, s) == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+    };
+    // Two and three rows of a matrix that the streaming kernel has read in a wave or two: a tile walks its super-blocks one behind the other
+    // (1.3 us each), whatever the rows.  Q4_K, three rows, 512 x 2048 11 us (tiles 20), 5120 x 2048 13 (20), 40960 x 2048 41 (44), 81920 x
+    // 2048 75 (68); Q6_K 2048 x 2048 12 (17), 5120 x 2048 17 (18), 10240 x 2048 24 (18).  Four rows 20 (20) and 23 (17).
+    const bool few = g_tc_min_tokens == 0 && T >= 2 && T <= 3 && (w.qtype == QT_Q4K ? w.out_f <= 40960 : w.out_f * w.nb <= 40960);
+    bool done = few && g_stage_mask == 0 && batch();
+    if (!done && T >= 2 && T >= g_tc_min_tokens && T < (1 << 24) && g_stage_mask == 0 && tile_scales(w.qtype, w.nb, w.maxd, w.maxdmin, fw)) {
         TileArgs ta = {};
         ta.wa = w.cell; ta.wb = w.cell; ta.grp_off = nullptr; ta.n_groups = 1; ta.nb = (int)w.nb; ta.n_rows = T; ta.out_f = w.out_f; ta.fw = fw;
         ta.fa = 16; ta.xl = xl; ta.x_nl = x_nl; ta.out = out;
@@ -287,13 +303,7 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
         sa.fast = small_scales(w.maxd, w.maxdmin, fw); sa.pdl = sa.early_weights = early && g_pdl ? 1 : 0;      // early: weights asked for while the kernel before runs
         if (launch_stream(w.qtype, MODE_LINEAR, sa, s) != cudaSuccess) return false;
     } else if (T >= 2 && T < (1 << 20) && g_stage_mask == 0) {
-        // a few rows: one group that owns all of them, every tile streamed once
-        int *off = (int *)ensure(R_META, 64);
-        if (!off || launch_set2(off, 0, (int)T, s) != cudaSuccess) return false;
-        BatchArgs ba = {};
-        ba.wa = w.cell; ba.wb = w.cell; ba.grp_off = off; ba.n_groups = 1; ba.out_f = w.out_f; ba.n_blocks = w.nb; ba.fw = fw; ba.fa = 16;
-        ba.fast = small_scales(w.maxd, w.maxdmin, fw); ba.xl = xl; ba.x_nl = x_nl; ba.out = out; ba.flags = g_flags;
-        if (launch_batch(w.qtype, MODE_LINEAR, ba, s) != cudaSuccess) return false;
+        if (few || !batch()) return false;
     } else {
         SkinnyArgs a = {};
         a.wa = w.cell; a.wb = w.cell; a.pairs_per_group = (int)T; a.out_f = w.out_f; a.n_blocks = w.nb; a.fw = fw; a.fa = 16;
@@ -349,11 +359,21 @@ bool moe_fused(const MoePlan &p, const int8_t *hl, long long rows, const int *xi
             td.wa = p.down; td.wb = p.down; td.grp_off = grp_off; td.n_groups = n_groups; td.nb = (int)(p.e_ffn / 256); td.n_rows = n_pairs;
             td.out_f = p.d_model; td.fw = fw; td.fa = fa; td.xl = gul; td.x_nl = g_cells + 1; td.out = out; td.gates = pair_gate; td.pair_tok = pair_tok;
             // gate / up below three rows per expert on average: the warp-level kernel, which multiplies one row at a time without a
-            // tile's padding, is the faster one (16 tokens over 128 experts 81 against 88 us, 45 tokens 139 / 141, 64 tokens 163 / 135);
-            // down takes the tiles from two rows on (16 tokens 55 against 78 us)
-            const bool first = n_pairs >= 3LL * n_groups && tiles(p.gate_q, MODE_GATEUP, tg, s);
-            if (first || launch_batch(p.gate_q, MODE_GATEUP, gateup_batch(), s) == cudaSuccess)
-                return tiles(p.down_q, MODE_DOWN, td, s) || launch_batch(p.down_q, MODE_DOWN, down_batch(), s) == cudaSuccess;
+            // tile's padding, is the faster one (16 tokens over 128 experts 81 against 88 us, 45 tokens 139 / 141, 64 tokens 163 / 135), and
+            // where all tiles together are a fraction of a wave, so that one tile's walk and its epilogue are the launch (gate / up of 768 x
+            // 2048: 4 experts, 16 pairs 8 us less than the tiles, 64 pairs 1 to 9, 128 pairs 4 to 16 more; 16 experts 64 pairs 5 less, 128 pairs 2
+            // to 10 more; of 256 x 256 10 us less throughout).  Down takes the tiles (16 tokens over 128 experts 55 against 78 us) from eight
+            // pairs on: below them the warp-level kernel takes row by row and is up to 5 us quicker.
+            const bool by_size = g_tc_min_tokens == 0 && rows < TILES_FROM;
+            const bool gate_tiles = n_pairs >= 3LL * n_groups && (!by_size || n_pairs * (p.e_ffn / 64) * (p.d_model / 256) >= 8192);
+            const bool down_tiles = !by_size || n_pairs >= 8;
+            auto either = [&](bool first, int q, int mode, const TileArgs &t, const BatchArgs &b) {
+                if (first && tiles(q, mode, t, s)) return true;
+                if (launch_batch(q, mode, b, s) == cudaSuccess) return true;
+                cudaGetLastError();
+                return !first && tiles(q, mode, t, s);
+            };
+            if (either(gate_tiles, p.gate_q, MODE_GATEUP, tg, gateup_batch())) return either(down_tiles, p.down_q, MODE_DOWN, td, down_batch());
             cudaGetLastError();
         }
         const BatchArgs ga = gateup_batch();
@@ -1735,7 +1755,7 @@ extern "C" int iie_rmsnorm_dev(long long gain_h, const int64_t *x_dev, long long
 
 extern "C" void iie_set_tc_min_tokens(long long tokens) {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
-    g_tc_min_tokens = tokens < 2 ? 2 : tokens;
+    g_tc_min_tokens = tokens <= 0 ? 0 : tokens < 2 ? 2 : tokens;
 }
 
 extern "C" void iie_set_attn_fused(int enabled) {

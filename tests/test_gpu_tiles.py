@@ -163,3 +163,50 @@ def test_expert_tiles_at_other_activation_scales(fa):
     assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
     assert np.array_equal(out.cpu().numpy(), out_ref)
     layer.close()
+
+
+@pytest.mark.parametrize(("qtype", "out_f", "nb", "T", "tiles"), [(o.Q4_K, 40960, 1, 3, 0), (o.Q4_K, 40961, 1, 3, 1), (o.Q4_K, 300, 9, 2, 0), (o.Q4_K, 300, 9, 4, 1),
+                                                                  (o.Q6_K, 5120, 8, 3, 0), (o.Q6_K, 5121, 8, 2, 1), (o.Q6_K, 64, 3, 4, 1), (o.Q4_K, 24, 48, 3, 1)])
+def test_dense_products_by_size(qtype, out_f, nb, T, tiles):
+    """Both sides of the border between the streaming kernel and the tiles, and a row length that only the tiles take."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    qk_cuda.load_library().iie_set_tc_min_tokens(0)
+    rng = np.random.default_rng(out_f + T)
+    raw = (o.synth_q4k if qtype == o.Q4_K else o.synth_q6k)(rng, out_f, nb)
+    h = qk_cuda.register_weight(raw, out_f, nb, qtype)
+    x = rng.integers(-(1 << 22), 1 << 22, size=(T, nb * 256), dtype=np.int64)
+    device.read_flags()
+    before = device.prefill_launch_counts()
+    got = device.apply(h, torch.from_numpy(x).cuda(), out_f, FW).cpu().numpy()
+    assert sum(device.prefill_launch_counts()) - sum(before) == tiles
+    assert device.read_flags() == 0
+    assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, qtype))
+
+
+@pytest.mark.parametrize(("d", "eff", "E", "k", "T", "tiles"), [(256, 256, 4, 2, 3, 0), (256, 256, 4, 2, 4, 2), (256, 256, 4, 2, 191, 2), (256, 256, 4, 2, 192, 3),
+                                                                (1024, 512, 2, 2, 127, 2), (1024, 512, 2, 2, 128, 3), (512, 256, 200, 1, 40, 2)])
+def test_expert_blocks_by_size(d, eff, E, k, T, tiles):
+    """The kernels of router, gate / up and down change one by one with the rows; the block's bytes do not."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    qk_cuda.load_library().iie_set_tc_min_tokens(0)
+    rng = np.random.default_rng(d + E + T)
+    q4 = lambda r, c: o.synth_q4k(rng, r, c // 256)
+    router, gate, up = q4(E, d), [q4(eff, d) for _ in range(E)], [q4(eff, d) for _ in range(E)]
+    down = [o.synth_q6k(rng, d, eff // 256) for _ in range(E)]
+    h = o.to_fixed(rng.standard_normal((T, d)), FA)
+    reg = lambda w, r, c, q=o.Q4_K: qk_cuda.register_weight(w, r, c // 256, q)
+    layer = device.MoELayer(reg(router, E, d), [reg(w, eff, d) for w in gate], [reg(w, eff, d) for w in up], [reg(w, d, eff, o.Q6_K) for w in down], k, d, eff)
+    device.read_flags()
+    before = device.prefill_launch_counts()
+    out, ids, gates = layer.forward(torch.from_numpy(h).cuda(), FA, FW)
+    torch.cuda.synchronize()
+    assert sum(device.prefill_launch_counts()) - sum(before) == tiles
+    assert device.read_flags() == 0
+    ids_ref, gates_ref, out_ref = onat.moe_block(router, o.Q4_K, gate, up, down, o.Q4_K, o.Q6_K, k, h, d, eff, FA, FW)
+    assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
+    assert np.array_equal(out.cpu().numpy(), out_ref)
+    layer.close()
