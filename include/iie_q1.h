@@ -56,7 +56,8 @@ long long bonsai_q1_register_weight_i32_gpu_layout(const unsigned char *bits, co
                                                    long long n_blocks);
 long long bonsai_q1_register_weight_i32_bmma(const unsigned char *bits, const int *scale, long long out_f,
                                              long long n_blocks);
-/* bonsai_q1_gpu.cu:2388 - product with a registered weight. */
+/* bonsai_q1_gpu.cu:2388 - product with a registered weight (results of up to 256 KB travel through page-locked memory, kept until
+ * bonsai_q1_free_weights). */
 int bonsai_q1_apply_resident(long long handle, const long long *x, long long tokens, long long frac, long long *out);
 /* bonsai_q1_gpu.cu:3659 - drop every registered weight; handles start again at 0. */
 void bonsai_q1_free_weights(void);

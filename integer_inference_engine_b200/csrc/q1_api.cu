@@ -34,7 +34,6 @@ std::vector<Q1Weight> q_w;
 unsigned long long q_weight_bytes = 0;
 cudaStream_t q_stream = nullptr;
 int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [8..15] digits in use (a DigitRing)
-int *q_host_flags = nullptr;            // page-locked: the flag word behind a host-array product
 int q_ready = -1;
 
 enum QRole { QR_X, QR_PLANES, QR_WORK, QR_KEYS, QR_VALUES, QR_LOGITS, QR_OUT, QR_GAIN, QR_COUNT };
@@ -61,8 +60,7 @@ bool q_init() {
     int n = 0;
     if (cudaGetDeviceCount(&n) != cudaSuccess || n <= 0 ||
         cudaStreamCreateWithFlags(&q_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&q_cells, 64) != cudaSuccess || cudaMemset(q_cells, 0, 64) != cudaSuccess ||
-        cudaHostAlloc(&q_host_flags, 64, cudaHostAllocDefault) != cudaSuccess) {
+        cudaMalloc(&q_cells, 64) != cudaSuccess || cudaMemset(q_cells, 0, 64) != cudaSuccess) {
         cudaGetLastError(); q_ready = 1; return false;
     }
     q_ready = 0;
@@ -202,6 +200,32 @@ int apply_device(const Q1Weight &w, const int64_t *xd, long long T, long long fr
     return used > max_digits ? 4 : 2;
 }
 
+// Result and flag word to the host behind one wait, results of up to 256 KB through page-locked memory (a copy to pageable memory and
+// one more for the flag word take 3 to 8 us longer).  False on a CUDA failure and where a kernel's wait gave up.
+constexpr size_t STAGE = 256 << 10;
+uint8_t *q_stage = nullptr;
+bool q_stage_tried = false;
+bool download_checked(void *dst, const void *src, size_t n) {
+    if (!q_stage_tried) {
+        q_stage_tried = true;
+        if (cudaHostAlloc(&q_stage, STAGE + 64, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); q_stage = nullptr; }
+    }
+    const bool staged = q_stage && n <= STAGE;
+    int pageable = 0;
+    int *seen = q_stage ? reinterpret_cast<int *>(q_stage) : &pageable;
+    const int *flags = shared_flag_word();
+    if (!flags || cudaMemcpyAsync(seen, flags, sizeof(int), cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
+        cudaMemcpyAsync(staged ? q_stage + 64 : dst, src, n, cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
+        cudaStreamSynchronize(q_stream) != cudaSuccess) return false;
+    if (*seen & FLAG_GAVE_UP) {                        // goes with the call that reports it; the other bits are device-pointer callers'
+        const int f = iie_flags_read_clear(q_stream);
+        restore_flag_bits(f & ~FLAG_GAVE_UP);
+        return false;
+    }
+    if (staged) memcpy(dst, q_stage + 64, n);
+    return true;
+}
+
 int apply_host(const Q1Weight &w, const long long *x, long long T, long long frac, long long *out, int max_digits) {
     const size_t xsz = (size_t)T * w.nb * 128 * 8, osz = (size_t)T * w.out_f * 8;
     int64_t *xd = (int64_t *)q_ensure(QR_X, xsz), *od = (int64_t *)q_ensure(QR_OUT, osz);
@@ -209,15 +233,7 @@ int apply_host(const Q1Weight &w, const long long *x, long long T, long long fra
     if (cudaMemcpyAsync(xd, x, xsz, cudaMemcpyHostToDevice, q_stream) != cudaSuccess) return 2;
     const int rc = apply_device(w, xd, T, frac, od, max_digits, q_stream);
     if (rc != 0) { cudaStreamSynchronize(q_stream); return rc; }
-    const int *flags = shared_flag_word();
-    if (!flags || cudaMemcpyAsync(q_host_flags, flags, sizeof(int), cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
-        cudaMemcpyAsync(out, od, osz, cudaMemcpyDeviceToHost, q_stream) != cudaSuccess || cudaStreamSynchronize(q_stream) != cudaSuccess) return 2;
-    if (*q_host_flags & FLAG_GAVE_UP) {                // goes with the call that reports it; the other bits are device-pointer callers'
-        const int f = iie_flags_read_clear(q_stream);
-        restore_flag_bits(f & ~FLAG_GAVE_UP);
-        return 2;
-    }
-    return 0;
+    return download_checked(out, od, osz) ? 0 : 2;
 }
 
 int one_shot(const long long *x, const unsigned char *bits, const long long *scale, long long tokens, long long out_f,
@@ -671,7 +687,12 @@ bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logi
 // weights are freed.
 uint8_t *q_pin = nullptr;
 size_t q_pin_cap = 0;
-void free_pin() { if (q_pin) cudaFreeHost(q_pin); q_pin = nullptr; q_pin_cap = 0; }
+void free_pin() {
+    if (q_pin) cudaFreeHost(q_pin);
+    if (q_stage) cudaFreeHost(q_stage);
+    q_pin = q_stage = nullptr;
+    q_pin_cap = 0; q_stage_tried = false;
+}
 bool upload_rows(int64_t *dst, const long long *src, size_t bytes) {
     constexpr size_t LEAST = 1 << 20, MOST = 32 << 20, PIECE = 512 << 10;
     constexpr int THREADS = 4;
