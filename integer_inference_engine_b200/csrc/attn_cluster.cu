@@ -12,8 +12,8 @@
 //
 // What bounds it: 64 sequences of 4096 keys, 4 KV heads of 128 (1.07 GB): 258 us; the copies alone take 164, the rest is the latency of
 // eight warps per SM (their registers hold the loads under way: with twelve warps and less of it 330), about 1800 instructions per
-// tile.  Three kernels with the scores in memory took 540.  One sequence does not come here: its chain of one warp per tile is longer
-// than that of attn_fat_kernel (16 against 12 us at 513 keys).
+// tile.  Three kernels with the scores in memory took 540.  A call for one sequence goes to attn_fat_kernel, whose chain is shorter than
+// one warp's over a tile (12 against 16 us at 513 keys); a batched call comes here whatever its number of sequences.
 #include <cooperative_groups.h>
 
 #include <algorithm>

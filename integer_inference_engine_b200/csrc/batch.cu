@@ -1,4 +1,5 @@
-// Grouped expert products for small batches (2 .. ~190 rows): every touched expert tile is streamed ONCE.
+// Grouped expert products for small batches: two and three rows of a matrix, experts of few rows (which calls: api.cu), and what the
+// tcgen05 tiles do not take.  Every touched expert tile is streamed ONCE.
 //
 // The reference's batched entries (north-mini-code/tools/nmc_qk_cuda.cu:2184-2346 matmul_multi_tok and the host
 // loop around it) stream a whole expert per (token, expert) pair.  With a few rows per expert the step is still

@@ -24,8 +24,11 @@
 // warp each for the MMAs, the TMA loads of planes and sums, and the bulk copies of packed weights (one super-block of 128 rows per copy slot); for gate / up four
 // epilogue warps.  CTAs are
 // persistent, one per SM, and walk the tiles of all groups, the column tiles of one weight slab next to each other.
-// What bounds it: the instructions of all roles together (about 6600 warp instructions per 128 x 256 weights at sixteen columns, a third
-// of them the hand-overs, at 2.4 per clock and SM); tensor pipe 12 - 15 % active, shared memory and HBM far from their limits.
+// What bounds it: the instructions of all roles together, 6750 warp instructions per 128 x 256 weights at sixteen columns, a good part
+// of them the hand-overs, at 2.3 to 2.7 per clock and SM; tensor pipe 12 % active at four rows an expert, 14 to 24 % at 2048 rows, HBM a
+// quarter of its rate at most.  The forms of several digit counts share one allocation of registers: gate / up (64) and the dense product (72)
+// spill, 1 % of the instructions.  One tile walks its super-blocks one behind the other, 1.3 us each: calls of few tiles are dispatched
+// elsewhere (api.cu).
 // Per block at 2048 tokens: gate / up 840 us, down 670, 5120 x 2048 dense 240 (fully dequantised weights in four or five digits: 940, 1140,
 // 280); at 64 tokens 130, 80, 21 (warp-level MMAs: 165, 190, 45).
 // Every wait is bounded; on a time-out the CTA raises flag bit 3, leaves its loops, frees TMEM and exits.
