@@ -6,8 +6,8 @@
 // tile, nothing is recycled so no barrier is ever re-armed), and its warps unpack and multiply the
 // tiles as they land.  The arithmetic is the limb-MMA scheme of skinny.cu: the activation's eight
 // balanced base-256 digits are the N=8 columns of a warp MMA; sub-block scales and minimums are
-// applied in int32, the block scale in int64, the columns are recombined in 128 bits and shifted
-// once.  Epilogues fuse the integer SiLU * up product (gate/up pair) and the gate-weighted combine
+// applied in int32, the block scale in int64, the warps' sums of a tile meet in shared memory, the columns are recombined in
+// 128 bits and shifted once.  Epilogues fuse the integer SiLU * up product (gate/up pair) and the gate-weighted combine
 // (down), replacing north-mini-code/tools/nmc_qk_cuda.cu:208-237 (silu_k, mul_shift_k,
 // matmul_multi_k, combine_k).
 //
@@ -74,10 +74,8 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
     const int tile_bytes = 2 * nb * HTB;
     const int tpc = a.tiles_per_cta;
     uint8_t *wbuf = smem;
-    unsigned long long *red = reinterpret_cast<unsigned long long *>(smem + (size_t)tpc * tile_bytes);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(red + (size_t)tpc * 128);
-    int *done = reinterpret_cast<int *>(bars + tpc);             // blocks of each tile already accumulated
-    int *t_sel = done + tpc, *t_pos = t_sel + tpc;               // tile -> (selected matrix slot, tile inside it)
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + (size_t)tpc * tile_bytes);
+    int *t_sel = reinterpret_cast<int *>(bars + tpc), *t_pos = t_sel + tpc;      // tile -> (selected matrix slot, tile inside it)
     // MODE_FRONT only: digit planes of the normalised row [8][K + pad], the staged row and gain
     const int pstride = (int)K + FR_PAD;
     int8_t *planes = reinterpret_cast<int8_t *>((reinterpret_cast<uintptr_t>(t_pos + tpc) + 15) & ~(uintptr_t)15);
@@ -98,9 +96,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
     const int n_ht = (int)((a.out_f + 7) >> 3), n_ht_b = (int)((a.out_f_b + 7) >> 3);
     const bool topk = MODE != MODE_FRONT && MODE != MODE_LINEAR && a.logits != nullptr;
 
-    for (int i = threadIdx.x; i < my_tiles * 128; i += blockDim.x) red[i] = 0ULL;
     for (int i = threadIdx.x; i < my_tiles; i += blockDim.x) {
-        done[i] = 0;
         const int tau = tile0 + i;
         int sl, ps;
         if (MODE == MODE_FRONT) { sl = tau < a.tiles_per_expert ? 0 : 1; ps = tau - sl * a.tiles_per_expert; }
@@ -369,7 +365,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
             else load_bfrag<QT, true>(xp + xoff + (long long)b * 256, t, bf);
             xcur = xp; bcur = b;
         }
-        const uint8_t *ua = wbuf + (size_t)ti * tile_bytes + (size_t)b * HTB;
+        uint8_t *ua = wbuf + (size_t)ti * tile_bytes + (size_t)b * HTB;
         const uint8_t *ub;
         if (MODE == MODE_GATEUP) ub = ua + (size_t)nb * HTB;
         else ub = (2 * p + 1 < ((MODE == MODE_FRONT && s == 1) ? n_ht_b : n_ht)) ? ua + (size_t)nb * HTB : ua;
@@ -379,49 +375,42 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
         if (!mbar_wait(&bars[ti_now], 0)) { s_timeout = 1; continue; }
         int64_t acc[4] = {0, 0, 0, 0};
         run_item<QT, FAST>(ua, ub, lane, a.fw, bf, half, acc);
-        unsigned long long *r = red + (size_t)ti_now * 128;
-        atomicAdd(&r[g * 8 + 2 * t], (unsigned long long)acc[0]);
-        atomicAdd(&r[(g + 8) * 8 + 2 * t], (unsigned long long)acc[2]);
-        if (!half) {
-            atomicAdd(&r[g * 8 + 2 * t + 1], (unsigned long long)acc[1]);
-            atomicAdd(&r[(g + 8) * 8 + 2 * t + 1], (unsigned long long)acc[3]);
-        }
-        if (MODE == MODE_GATEUP) continue;                    // its epilogue is long: all rows run it in parallel below
-        // the warp that completes a tile (all nb blocks added) runs its epilogue; nobody waits
-        __threadfence_block();
-        int prior = 0;
-        if (lane == 0) prior = atomicAdd(&done[ti_now], 1);
-        prior = __shfl_sync(0xffffffffu, prior, 0);
-        if (prior != nb - 1) continue;
-        __threadfence_block();
-        const volatile unsigned long long *rv = r;
-        if (lane < 16) {
-            const long long row = (long long)p * 16 + lane;
-            if (row < ((MODE == MODE_FRONT && s == 1) ? a.out_f_b : a.out_f)) {
-                unsigned long long cc[8];
-#pragma unroll
-                for (int c = 0; c < 8; c++) cc[c] = rv[lane * 8 + c];
-                const int64_t y = recombine_cols(cc, a.fw);
-                if (MODE == MODE_FRONT) (s == 0 ? a.out : a.out_b)[row] = y;
-                else if (MODE == MODE_LINEAR) a.out[(long long)s * a.out_f + row] = y;
-                else atomicAdd(reinterpret_cast<unsigned long long *>(a.out + row),
-                               (unsigned long long)mul_shift(y, topk ? s_gates[s] : a.gates[s], a.fa));
-            }
-        }
+        // The item's sums take the place of its weights, which nobody reads again: entry 4 row + digit, the digits from four on behind
+        // the others.  (Shared 64-bit atomics on one set of sums per tile are compare-and-swap loops: 115 clocks each alone, 700 with
+        // sixteen warps at the same tile.)
+        __syncwarp();
+        unsigned long long *part = reinterpret_cast<unsigned long long *>(ua);
+        part[lane] = (unsigned long long)acc[0]; part[32 + lane] = (unsigned long long)acc[2];
+        if (!half) { part[64 + lane] = (unsigned long long)acc[1]; part[96 + lane] = (unsigned long long)acc[3]; }
     }
-    if (MODE == MODE_GATEUP) {
-        // rows 0..7 of a tile are the gate projection, rows 8..15 the up projection of the same output index
-        __syncthreads();
-        int nl = 0;
-        for (int idx = threadIdx.x; idx < my_tiles * 8; idx += blockDim.x) {
-            const int tq = idx >> 3, r8 = idx & 7;
-            const int s = t_sel[tq], p = t_pos[tq];
-            const long long row = (long long)p * 8 + r8;
-            if (row >= a.out_f) continue;
-            const unsigned long long *rr = red + (size_t)tq * 128;
-            const int64_t yg = recombine_cols(rr + r8 * 8, a.fw), yu = recombine_cols(rr + (r8 + 8) * 8, a.fw);
-            const int64_t sg = mul_shift(yg, sigmoid_fixed_c(yg, a.fa, a.sig_log2e, a.sig_clip), a.fa);
-            const int64_t gu = mul_shift(sg, yu, a.fa);
+    __syncthreads();
+    int nl = 0;
+    for (int tq = s_timeout ? my_tiles : warp; tq < my_tiles; tq += NWARPS) {      // a tile per warp (a wait that gave up: nothing is stored)
+        const int s = t_sel[tq], p = t_pos[tq];
+        const unsigned long long *part = reinterpret_cast<const unsigned long long *>(wbuf + (size_t)tq * tile_bytes) + lane;
+        int64_t y[2];                                             // rows g and g + 8 of the tile, in all four lanes of g
+        {
+            unsigned long long c0 = 0, c1 = 0, c2 = 0, c3 = 0;
+            for (int k = 0; k < nb; k++, part += HTB / 8) {
+                c0 += part[0]; c1 += part[32];
+                if (!half) { c2 += part[64]; c3 += part[96]; }
+            }
+            i128 v0 = (i128)(int64_t)c0, v1 = (i128)(int64_t)c1;
+            if (!half) { v0 += (i128)(int64_t)c2 << 32; v1 += (i128)(int64_t)c3 << 32; }
+            v0 <<= 8 * t; v1 <<= 8 * t;
+#pragma unroll
+            for (int off = 1; off <= 2; off <<= 1) {
+                v0 += (i128)(((u128)__shfl_xor_sync(0xffffffffu, (unsigned long long)((u128)v0 >> 64), off) << 64) | __shfl_xor_sync(0xffffffffu, (unsigned long long)v0, off));
+                v1 += (i128)(((u128)__shfl_xor_sync(0xffffffffu, (unsigned long long)((u128)v1 >> 64), off) << 64) | __shfl_xor_sync(0xffffffffu, (unsigned long long)v1, off));
+            }
+            y[0] = (int64_t)(v0 >> a.fw); y[1] = (int64_t)(v1 >> a.fw);
+        }
+        if (MODE == MODE_GATEUP) {
+            // rows 0..7 of a tile are the gate projection, rows 8..15 the up projection of the same output index
+            const long long row = (long long)p * 8 + g;
+            if (t != 0 || row >= a.out_f) continue;
+            const int64_t sg = mul_shift(y[0], sigmoid_fixed_c(y[0], a.fa, a.sig_log2e, a.sig_clip), a.fa);
+            const int64_t gu = mul_shift(sg, y[1], a.fa);
             if (a.out) a.out[(long long)s * a.out_f + row] = gu;
             bool ok;
             const uint64_t d = balanced_digits8(gu, ok);
@@ -429,13 +418,20 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
             nl = max(nl, digits_used(d));
 #pragma unroll
             for (int l = 0; l < 8; l++) a.out_limbs[((long long)s * 8 + l) * a.out_f + row] = (int8_t)(d >> (8 * l));
+        } else {
+            const long long row = (long long)p * 16 + g + 8 * t;
+            if (t >= 2 || row >= ((MODE == MODE_FRONT && s == 1) ? a.out_f_b : a.out_f)) continue;
+            const int64_t v = t ? y[1] : y[0];
+            if (MODE == MODE_FRONT) (s == 0 ? a.out : a.out_b)[row] = v;
+            else if (MODE == MODE_LINEAR) a.out[(long long)s * a.out_f + row] = v;
+            else atomicAdd(reinterpret_cast<unsigned long long *>(a.out + row),
+                           (unsigned long long)mul_shift(v, topk ? s_gates[s] : a.gates[s], a.fa));
         }
-        nl = max(nl, __shfl_xor_sync(0xffffffffu, nl, 16)); nl = max(nl, __shfl_xor_sync(0xffffffffu, nl, 8));
-        nl = max(nl, __shfl_xor_sync(0xffffffffu, nl, 4));  nl = max(nl, __shfl_xor_sync(0xffffffffu, nl, 2));
-        nl = max(nl, __shfl_xor_sync(0xffffffffu, nl, 1));
+    }
+    if (MODE == MODE_GATEUP) {
+        nl = __reduce_max_sync(0xffffffffu, nl);
         if (lane == 0 && nl > 0 && a.out_nl) atomicMax(a.out_nl, nl);
     }
-    __syncthreads();
     if (s_timeout && threadIdx.x == 0) atomicOr(a.flags, 8);
 }
 
@@ -447,7 +443,7 @@ cudaError_t launch_stream_t(const StreamArgs &a_in, cudaStream_t s) {
     a.tiles_per_expert = (int)(MODE == MODE_GATEUP ? n_ht : (n_ht + 1) / 2);
     a.tiles_b = MODE == MODE_FRONT ? (int)((((a.out_f_b + 7) >> 3) + 1) / 2) : 0;
     const long long n_tiles = MODE == MODE_FRONT ? (long long)a.tiles_per_expert + a.tiles_b : (long long)a.n_sel * a.tiles_per_expert;
-    const size_t tile_bytes = (size_t)2 * a.n_blocks * HTB, per_tile = tile_bytes + 128 * 8 + 8 + 12;
+    const size_t tile_bytes = (size_t)2 * a.n_blocks * HTB, per_tile = tile_bytes + 8 + 8;
     const size_t front_bytes = MODE == MODE_FRONT ? (size_t)8 * (a.n_blocks * 256 + FR_PAD) + (size_t)16 * a.n_blocks * 256 + 16 : 0;
     if (MODE == MODE_FRONT && (!a.x || !a.out || !a.out_b || a.out_f_b <= 0 || a.n_blocks * 256 > 8192)) return cudaErrorInvalidValue;
     if (MODE != MODE_FRONT && a.logits && (a.n_experts <= 0 || a.n_experts > SK_MAXE || a.n_sel > SK_MAXK || a.n_sel > a.n_experts)) return cudaErrorInvalidValue;
