@@ -211,7 +211,7 @@ struct TileArgs {
     const int64_t *gates;          // DOWN: per pair
     const int *pair_tok;           // DOWN: pair -> token row, or nullptr (identity)
     int *flags;                    // bit 0 digit envelope, bit 3 a wait gave up
-    int wide;                      // filled in by the launcher
+    int wide, split;               // filled in by the launcher
     long long sig_log2e, sig_clip;
 };
 cudaError_t launch_tiles(int qtype, int mode, const TileArgs &a, cudaStream_t s);

@@ -27,8 +27,9 @@
 // What bounds it: the instructions of all roles together, 6750 warp instructions per 128 x 256 weights at sixteen columns, a good part
 // of them the hand-overs, at 2.3 to 2.7 per clock and SM; tensor pipe 12 % active at four rows an expert, 14 to 24 % at 2048 rows, HBM a
 // quarter of its rate at most.  The forms of several digit counts share one allocation of registers: gate / up (64) and the dense product (72)
-// spill, 1 % of the instructions.  One tile walks its super-blocks one behind the other, 1.3 us each: calls of few tiles are dispatched
-// elsewhere (api.cu).
+// spill, 1 % of the instructions.  One tile walks its super-blocks one behind the other, 1.3 us each: of a dense product with few tiles
+// the CTAs of a cluster take a share of them each and join their sums through distributed shared memory (launch_tiles), calls of two and
+// three rows are dispatched elsewhere (api.cu).
 // Per block at 2048 tokens: gate / up 840 us, down 670, 5120 x 2048 dense 240 (fully dequantised weights in four or five digits: 940, 1140,
 // 280); at 64 tokens 130, 80, 21 (warp-level MMAs: 165, 190, 45).
 // Every wait is bounded; on a time-out the CTA raises flag bit 3, leaves its loops, frees TMEM and exits.
@@ -92,6 +93,28 @@ __device__ __forceinline__ uint32_t tl_elect() {
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
     return r;
 }
+// split tiles: the same shared-memory address in another CTA of the cluster, and what goes there
+__device__ __forceinline__ uint32_t tl_remote(uint32_t a, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void tl_remote_store(uint32_t a, long long v) { asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }
+__device__ __forceinline__ void tl_remote_arrive(uint32_t b) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(b) : "memory"); }
+__device__ __noinline__ bool tl_wait_cluster(uint32_t b, uint32_t parity, volatile int *abort_flag) {       // bounded; the whole warp, one answer
+    bool done = false;
+    for (unsigned it = 0; it < TL_WAIT_LIMIT && !done && !*abort_flag; it++) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok) : "r"(b), "r"(parity), "r"(20000u) : "memory");
+        done = ok != 0;
+    }
+    if (!done) *abort_flag = 1;
+    return __all_sync(0xffffffffu, done);
+}
+__device__ __forceinline__ void tl_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
 // a position in a ring of slots, stepped (a division by a run-time slot count in every role's loop costs hundreds of clocks)
 struct TlRing {
     int slot = 0;
@@ -139,14 +162,19 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     constexpr int NROW = MODE == MODE_GATEUP ? 64 : 128;           // output rows of a tile
     extern __shared__ __align__(1024) unsigned char tl_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tl_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t bars[2 * TL_MAX_STAGES + 8 + 2 * TL_MAX_RAW + 2];
+    constexpr bool CAN_SPLIT = MODE == MODE_LINEAR;
+    const int split = CAN_SPLIT ? a.split : 1;                     // CTAs of a cluster that share a tile's super-blocks
+    __shared__ __align__(8) uint64_t bars[2 * TL_MAX_STAGES + 8 + 2 * TL_MAX_RAW + 4];
     __shared__ int s_first[TL_MAX_GROUPS + 1], s_off[TL_MAX_GROUPS + 1];       // first tile and first row of each group
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const uint32_t full_bar = tl_u32(bars), empty_bar = full_bar + 8 * TL_MAX_STAGES, acc_bar = empty_bar + 8 * TL_MAX_STAGES, free_bar = acc_bar + 8 * 4,
-                   raw_full = free_bar + 8 * 4, raw_empty = raw_full + 8 * TL_MAX_RAW, y_full = raw_empty + 8 * TL_MAX_RAW, y_free = y_full + 8;
+                   raw_full = free_bar + 8 * 4, raw_empty = raw_full + 8 * TL_MAX_RAW, y_full = raw_empty + 8 * TL_MAX_RAW, y_free = y_full + 8,
+                   x_full = y_free + 8, x_free = x_full + 8;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int nb = a.nb;
+    const int nb = a.nb, rank = split > 1 ? (int)(blockIdx.x & (split - 1)) : 0;
+    const int b_lo = nb * rank / split, b_hi = nb * (rank + 1) / split;        // super-blocks of this CTA
+    const int first_tile = CAN_SPLIT ? blockIdx.x / split : blockIdx.x, tile_step = CAN_SPLIT ? gridDim.x / split : gridDim.x;
     if (warp == TL_X_WARP && lane == 0) {                          // the tensor maps' first use would wait for them
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x16)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x32)) : "memory");
@@ -170,9 +198,10 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     const int x_bytes = np * bn * 128, s_bytes = Q4 ? ns * bn * 32 : 0;
     const int stage_bytes = (TL_A_BYTES + x_bytes + s_bytes + 1023) & ~1023;
     constexpr int FIXED = 1024 + (Q4 ? TL_MINS : 0) + (MODE == MODE_GATEUP ? TL_EXCH : 0);
-    const int raw_slots = FIXED + 3 * stage_bytes + TL_MAX_RAW * RAW_BYTES <= TL_SMEM ? TL_MAX_RAW : 2;
-    const int stages = min(TL_MAX_STAGES, (TL_SMEM - FIXED - raw_slots * RAW_BYTES) / stage_bytes);
-    unsigned char *mins = smem + stages * stage_bytes, *exch = mins + (Q4 ? TL_MINS : 0), *raw = exch + (MODE == MODE_GATEUP ? TL_EXCH : 0);
+    const int xch_bytes = split > 1 ? 128 * bn * ((np + 2) / 2) * 8 : 0;       // split tiles: sums of this CTA's share of the columns
+    const int raw_slots = FIXED + xch_bytes + 3 * stage_bytes + TL_MAX_RAW * RAW_BYTES <= TL_SMEM ? TL_MAX_RAW : 2;
+    const int stages = min(TL_MAX_STAGES, (TL_SMEM - FIXED - xch_bytes - raw_slots * RAW_BYTES) / stage_bytes);
+    unsigned char *mins = smem + stages * stage_bytes, *exch = mins + (Q4 ? TL_MINS : 0), *raw = exch + (MODE == MODE_GATEUP ? TL_EXCH : xch_bytes);
 
     const int n_rt = (int)((a.out_f + NROW - 1) / NROW);
     if (warp == 0) {                                               // first tile of every group
@@ -195,6 +224,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         for (int s = 0; s < TL_MAX_STAGES; s++) { tl_init(full_bar + 8 * s, n_expand + 1); tl_init(empty_bar + 8 * s, 1); }
         for (int s = 0; s < 4; s++) { tl_init(acc_bar + 8 * s, 1); tl_init(free_bar + 8 * s, n_read); }
         tl_init(y_full, n_read); tl_init(y_free, TL_EPI);
+        tl_init(x_full, split * n_read); tl_init(x_free, split * n_read);
         for (int s = 0; s < TL_MAX_RAW; s++) { tl_init(raw_full + 8 * s, 1); tl_init(raw_empty + 8 * s, TL_WORK); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (blockIdx.x == 0) {                                     // which tile shape ran (launch statistics)
@@ -205,6 +235,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (split > 1) tl_cluster_sync();                              // the other CTAs' barriers stand
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
     const int n_tiles = s_first[a.n_groups];
@@ -241,7 +272,9 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
             TlRing rs, buf;
             uint32_t y_pass = 0;
             bool y_used = false;
-            for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            uint32_t x_pass = 0;
+            bool x_used = false;
+            for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
                 const Where w = locate(tile);
                 long long L[NLV][TPW];
 #pragma unroll
@@ -249,7 +282,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
 #pragma unroll
                     for (int j = 0; j < TPW; j++) L[i][j] = 0;
                 bool ok = true;
-                for (int b = 0; b < nb; b++) {
+                for (int b = b_lo; b < b_hi; b++) {
                     if (!(ok = tl_wait(raw_full + 8 * rs.slot, rs.pass, &s_abort))) break;
                     const unsigned char *meta = raw + rs.slot * RAW_BYTES + meta_off;
                     int d, dm = 0;
@@ -309,6 +342,43 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
                 if (!ok) break;
                 // ---- y = floor(V / 2^fw), then what the product is for ---------------------------------------
                 const int sh = a.fw + (Q4 && !THIRDS ? 4 : 0);
+                if (CAN_SPLIT && split > 1) {
+                    // column c of the tile belongs to CTA c mod split, as its column c / split there: everybody's sums go to the owner,
+                    // which adds them up, joins the digits and stores
+                    const int cols = BN / split;                   // of this CTA
+                    const uint32_t here = tl_u32(exch);
+                    if (x_used && !(ok = tl_wait_cluster(x_free, x_pass ^ 1, &s_abort))) break;
+#pragma unroll
+                    for (int j = 0; j < TPW; j++) {
+                        const int c = cg * TPW + j, slot = c / split;
+                        const uint32_t to = tl_remote(here + (uint32_t)((((rank * cols + slot) * NLV) * 128 + rowt) * 8), c & (split - 1));
+#pragma unroll
+                        for (int i = 0; i < NLV; i++) tl_remote_store(to + i * 1024, L[i][j]);
+                    }
+                    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+                    __syncwarp();
+                    if (lane < split) tl_remote_arrive(tl_remote(x_full, lane));
+                    if (!(ok = tl_wait_cluster(x_full, x_pass, &s_abort))) break;
+                    const long long row = (long long)w.rt * 128 + rowt;
+                    for (int slot = cg; slot < cols; slot += n_read / 4) {
+                        long long S[NLV];
+#pragma unroll
+                        for (int i = 0; i < NLV; i++) S[i] = 0;
+                        const long long *from = reinterpret_cast<const long long *>(exch) + slot * NLV * 128 + rowt;
+                        for (int k = 0; k < split; k++, from += cols * NLV * 128)
+#pragma unroll
+                            for (int i = 0; i < NLV; i++) S[i] += from[i * 128];
+                        i128 v = S[NLV - 1];
+#pragma unroll
+                        for (int i = NLV - 2; i >= 0; i--) v = (v << 16) + (i128)S[i];
+                        const int colx = w.m0 + slot * split + rank;
+                        if (row < a.out_f && colx < w.m_end) a.out[(long long)colx * a.out_f + row] = (long long)(v >> sh);
+                    }
+                    __syncwarp();
+                    if (lane < split) tl_remote_arrive(tl_remote(x_free, lane));
+                    x_used = true; x_pass ^= 1;
+                    continue;
+                }
                 long long y[TPW];
 #pragma unroll
                 for (int j = 0; j < TPW; j++) {
@@ -373,8 +443,8 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         TlRing rs, st;
         int n_mins = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            for (int b = 0; b < nb && ok; b++) {
+        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
+            for (int b = b_lo; b < b_hi && ok; b++) {
                 if (!(ok = tl_wait(raw_full + 8 * rs.slot, rs.pass, &s_abort))) break;
                 const unsigned char *slot = raw + rs.slot * RAW_BYTES;
 #pragma unroll
@@ -477,8 +547,8 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         TlRing st, buf;
         int n_mins = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x)
-            for (int b = 0; b < nb && ok; b++) {
+        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step)
+            for (int b = b_lo; b < b_hi && ok; b++) {
                 if (buf.lapped && !(ok = tl_wait(free_bar + 8 * buf.slot, buf.pass ^ 1, &s_abort))) break;
                 const uint32_t d = tmem + buf.slot * buf_cols;
                 for (int p = 0; p < 2; p++) {
@@ -518,9 +588,9 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
             const CUtensorMap *xm = wide ? &maps.x32 : &maps.x16, *sm = wide ? &maps.s32 : &maps.s16;
             TlRing st;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
                 const Where w = locate(tile);
-                for (int c = 0; c < 2 * nb; c++) {
+                for (int c = 2 * b_lo; c < 2 * b_hi; c++) {
                     const uint32_t eb = empty_bar + 8 * st.slot, fb = full_bar + 8 * st.slot;
                     if (st.lapped && !(ok = tl_try(eb, st.pass ^ 1) || tl_wait_slow(eb, st.pass ^ 1, &s_abort))) break;
                     const uint32_t dst = tl_u32(smem + st.slot * stage_bytes + TL_A_BYTES);
@@ -539,12 +609,12 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         // ================= packed weights: one super-block of the tile's 16 half-tiles per slot ===============
         TlRing rs;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
             const Where w = locate(tile);
             const uint8_t *src = nullptr;
             const bool live = lane < 16 && unit_of(w, lane, src);
             const int n_live = __popc(__ballot_sync(0xffffffffu, live));
-            for (int b = 0; b < nb; b++) {
+            for (int b = b_lo; b < b_hi; b++) {
                 const uint32_t eb = raw_empty + 8 * rs.slot, fb = raw_full + 8 * rs.slot;
                 if (rs.lapped && !(ok = tl_wait(eb, rs.pass ^ 1, &s_abort))) break;
                 if (lane == 0) tl_expect(fb, n_live * HTB);
@@ -562,7 +632,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         int nl_max = 0;
         uint32_t pass = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
             const Where w = locate(tile);
             const long long row = (long long)w.rt * 64 + r;
             for (int q = 0; q < bn / 4; q += 4) {                  // wide: columns 8 g + q + (0..3) of column group g = 0..3
@@ -596,6 +666,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         }
     }
     __syncthreads();
+    if (split > 1) tl_cluster_sync();                              // nobody leaves while another CTA stores or arrives here
     if (warp == TL_MMA_WARP) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -671,6 +742,18 @@ cudaError_t launch_tile(const TileArgs &a, const TileMaps &maps, cudaStream_t s)
     // an upper bound on the tiles: every group may end in a partial one
     const long long n_rt = (a.out_f + (MODE == MODE_GATEUP ? 63 : 127)) / (MODE == MODE_GATEUP ? 64 : 128);
     const long long most = (a.n_rows / 16 + std::min<long long>(a.n_groups, a.n_rows)) * n_rt;
+    if (a.split > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(a.split * ((a.n_rows + (a.wide ? 31 : 15)) / (a.wide ? 32 : 16)) * n_rt));
+        cfg.blockDim = dim3(tl_threads(MODE)); cfg.dynamicSmemBytes = TL_SMEM; cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)a.split; attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 2;
+        cudaLaunchKernelEx(&cfg, tile_kernel<QT, MODE>, a, maps);
+    } else
     launch_behind(tile_kernel<QT, MODE>, (unsigned)std::max<long long>(1, std::min<long long>(148, most)), tl_threads(MODE), TL_SMEM, s, a, maps);
     note_launch();
     return cudaGetLastError();
@@ -689,6 +772,13 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
     a.sig_log2e = sigmoid_log2e(a.fa); a.sig_clip = sigmoid_clip(a.fa);
     // sixteen columns while a group has few rows: a 32-column tile would multiply mostly padding
     a.wide = a.n_rows > 12LL * a.n_groups && a.n_rows > 16;
+    // A matrix of few tiles: clusters of CTAs share a tile's super-blocks, as long as all clusters fit on the device at once (one CTA per
+    // SM; 33 clusters of four, 15 of eight).  A super-block is 1.3 to 1.7 us of a tile's walk, the exchange of the sums 3: a call of 7 rows
+    // 128 x 2048 19.8 -> 14.7 us, 5120 x 2048 20.6 -> 19.1, 2048 x 4096 31.3 -> 19.4; of 64 rows 24.7 -> 17.1, 28.0 (not split), 39.4 -> 25.6.
+    // (16 clusters of eight for the last but one: two waves, 28.4.)
+    a.split = 1;
+    const long long whole = ((a.n_rows + (a.wide ? 31 : 15)) / (a.wide ? 32 : 16)) * ((a.out_f + 127) / 128);
+    while (mode == MODE_LINEAR && a.split < 8 && 2 * a.split <= a.nb && whole <= (a.split == 1 ? 74 : a.split == 2 ? 33 : 15)) a.split *= 2;
     const int stride = (a.nb * 8 + 31) / 32 * 32;
     const bool q4 = qtype == QT_Q4K;
     if (q4 || a.xidx) {

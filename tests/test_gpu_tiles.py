@@ -46,6 +46,24 @@ def test_dense_tiles_match_the_oracle(qtype, out_f, nb, T, xbits):
     assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, qtype))
 
 
+@pytest.mark.parametrize("qtype", [o.Q4_K, o.Q6_K])
+@pytest.mark.parametrize("out_f,nb,T,xbits", [(128, 2, 2, 20), (1928, 8, 16, 22), (1900, 9, 5, 22), (264, 16, 64, 22), (264, 16, 64, 30), (520, 7, 100, 62), (9400, 3, 9, 22)])
+def test_tiles_shared_by_clusters_match_the_oracle(qtype, out_f, nb, T, xbits):
+    """Few tiles: two, four or eight CTAs share a tile's super-blocks (even and odd numbers of them), also where more digits than expected
+    make the tiles narrower and a cluster walks several."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(out_f + nb * 7 + T)
+    raw = np.frombuffer((o.synth_q4k if qtype == o.Q4_K else o.synth_q6k)(rng, out_f, nb), np.uint8).tobytes()
+    x = rng.integers(-(1 << xbits), 1 << xbits, size=(T, nb * 256), dtype=np.int64)
+    device.read_flags()
+    h = qk_cuda.register_weight(raw, out_f, nb, qtype)
+    got = device.apply(h, torch.from_numpy(x).cuda(), out_f, FW).cpu().numpy()
+    assert device.read_flags() == 0
+    assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, qtype))
+
+
 @pytest.mark.parametrize("down_q", [o.Q4_K, o.Q6_K])
 @pytest.mark.parametrize("d,eff,E,k,T,mult", [(256, 256, 5, 2, 3, 1), (512, 256, 40, 1, 2, 1), (768, 512, 6, 3, 70, 1), (256, 768, 3, 3, 33, 200)])
 def test_expert_tiles_match_the_oracle(down_q, d, eff, E, k, T, mult):
