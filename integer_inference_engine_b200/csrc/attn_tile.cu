@@ -278,37 +278,49 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_tile_scores_kernel(const A
 // ---- pass 2: exponentials, their sum and the probabilities, one warp per (token, head) row ----------------------------------
 // e_l = 2^-((min(max - score_l, clip) * log2e) >> fa) for the visible keys of the row, in place of the scores, four keys per lane and
 // step; the row belongs to this warp, so its normaliser Z needs no atomics and the same lanes turn their e_l into p_l = (e_l << fa) / Z.
-// Bounded by instructions (about 30 per key) and the eight bytes per key in and out: 2048 tokens x 32 heads 189 us, with 64-bit
-// scores and 64-bit exponentials and quotients 300.
+// Bounded by instructions and the eight bytes per key in and out: 2048 tokens x 32 heads 205 -> 165 us with the 32-bit products of
+// softmax.cuh where fa <= 16 (333 tokens over 3233 keys 146 -> 125).  A row's keys kept in registers between the two passes: 193 (64 keys a
+// thread), 244 (32 keys, four warps a row).
+template <bool SHORT>                                              // fa <= 16
 __global__ void __launch_bounds__(256) attn_tile_exp_kernel(const AttnArgs a) {
     pdl_enter();
+    using Exp = std::conditional_t<SHORT, SoftmaxExp16, SoftmaxExp>;
+    using Quotient = std::conditional_t<SHORT, SoftmaxQuotient16, SoftmaxQuotient>;
+    using Below = std::conditional_t<SHORT, uint32_t, long long>;
     const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5), n_rows = (long long)a.batch * a.H;
     if (row >= n_rows) return;
     const int lane = threadIdx.x & 31;
     const long long tok = row / a.H, pos = a.pos + tok, lo = pt_lo(a, pos), Ls = a.Ls ? a.Ls : a.Lmax;
     const int64_t *far = a.scores + row * Ls;
     int32_t *e = a.e + row * Ls;
-    const long long m = a.hmax[row];
-    const SoftmaxExp exp2(a.fa, a.log2e, a.clip);
+    const long long m = a.hmax[row], first = lo & ~3LL;
+    const int skip = (int)(lo - first), n = (int)(pos - first);   // keys first + skip .. first + n are visible
+    const bool near = m >= INT32_MIN && m <= INT32_MAX;            // scores in 32 bits are then less than 2^32 below the maximum
+    const Exp exp2(a.fa, a.log2e, a.clip);
+    e += first; far += first;
     unsigned long long sum = 0;
-    for (long long l = (lo & ~3LL) + 4 * lane; l <= pos; l += 128) {
+#pragma unroll 2
+    for (int l = 4 * lane; l <= n; l += 128) {
         const int4 s4 = *reinterpret_cast<const int4 *>(e + l);
         int v[4] = {s4.x, s4.y, s4.z, s4.w};
+        uint32_t part = 0;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const bool seen = l + k >= lo && l + k <= pos;
-            long long d = m - v[k];
-            if (v[k] == INT32_MIN && seen) d = m - far[l + k];
-            v[k] = seen ? exp2(d) : 0;
-            sum += (unsigned)v[k];
+            const bool seen = l + k >= skip && l + k <= n;
+            Below below = SHORT ? (Below)((uint32_t)m - (uint32_t)v[k]) : (Below)(m - v[k]);
+            if (seen && (v[k] == INT32_MIN || (SHORT && !near))) below = (Below)min(m - (v[k] == INT32_MIN ? (long long)far[l + k] : (long long)v[k]), a.clip);
+            v[k] = seen ? (int)exp2(below) : 0;
+            part += (uint32_t)v[k];
         }
+        sum += part;
         *reinterpret_cast<int4 *>(e + l) = make_int4(v[0], v[1], v[2], v[3]);
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, s);
     if (lane == 0) a.Z[row] = sum;
-    const SoftmaxQuotient quotient(sum, a.fa);
-    for (long long l = (lo & ~3LL) + 4 * lane; l <= pos; l += 128) {
+    const Quotient quotient(sum, a.fa);
+#pragma unroll 2
+    for (int l = 4 * lane; l <= n; l += 128) {
         int4 *at = reinterpret_cast<int4 *>(e + l);                // this lane's own stores
         const int4 v = *at;
         *at = make_int4((int)quotient((uint32_t)v.x), (int)quotient((uint32_t)v.y), (int)quotient((uint32_t)v.z), (int)quotient((uint32_t)v.w));
@@ -990,7 +1002,9 @@ cudaError_t launch_attn_tile_scores(const AttnArgs &a, cudaStream_t s) {
 cudaError_t launch_attn_tile_exp(const AttnArgs &a, cudaStream_t s) {
     if (!attn_tiles_ok(a)) return cudaErrorInvalidValue;
     const long long rows = (long long)a.batch * a.H;
-    launch_behind(attn_tile_exp_kernel, (unsigned)((rows + 7) / 8), 256, 0, s, a);
+    // (the short form's quotients take normalisers up to 2^31)
+    if (a.fa <= 16 && (a.pos + a.batch) << a.fa <= 1LL << 31) launch_behind(attn_tile_exp_kernel<true>, (unsigned)((rows + 7) / 8), 256, 0, s, a);
+    else launch_behind(attn_tile_exp_kernel<false>, (unsigned)((rows + 7) / 8), 256, 0, s, a);
     note_launch();
     return cudaGetLastError();
 }

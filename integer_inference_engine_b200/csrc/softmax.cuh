@@ -37,4 +37,37 @@ struct SoftmaxQuotient {
     __device__ __forceinline__ uint32_t operator()(uint32_t e) const { return (uint32_t)(((uint64_t)e * mh + (((uint64_t)e * ml) >> 31)) >> post); }
 };
 
+// The same two where fa <= 16, in fewer and narrower multiplications (a 32-bit product is half the price of a 64-bit one).
+// Every operand of the polynomial is at most 2^16 and none of its products both factors, so that they fit 32 bits.
+struct SoftmaxExp16 {
+    uint32_t c0, c1, c2, c3, log2e, clip;
+    int fa;
+    __device__ __forceinline__ SoftmaxExp16(int fa_, long long log2e_, long long clip_)
+        : c0(65536u >> (16 - fa_)), c1(45426u >> (16 - fa_)), c2(15743u >> (16 - fa_)), c3(3638u >> (16 - fa_)), log2e((uint32_t)log2e_), clip((uint32_t)clip_), fa(fa_) {}
+    __device__ __forceinline__ uint32_t operator()(uint32_t below) const {
+        const uint32_t u = (uint32_t)(((uint64_t)min(below, clip) * log2e) >> fa), f = u & ((1u << fa) - 1), f2 = (f * f) >> fa, f3 = (f2 * f) >> fa;
+        const int p = (int)(c0 - ((c1 * f) >> fa) + ((c2 * f2) >> fa) - ((c3 * f3) >> fa));
+        return (uint32_t)(max(p, 0) >> (u >> fa));
+    }
+};
+// For 2^l < z <= 2^(l + 1) <= 2^31, M = floor(2^(33 + l) / z) + 1 lies in (2^32, 2^33) and floor((e << fa) / z) = (e M) >> (33 + l - fa) for
+// e <= 2^fa <= z: with d = M z - 2^(33 + l) <= z the right side's quotient is e d / (z 2^(33 + l - fa)) above the left one's, less than 1 / z
+// (or 1 / z with e = 2^fa and z a power of two, where the quotient is whole).  e = 0 for every key where z = 0.
+struct SoftmaxQuotient16 {
+    uint32_t m = 0;                                                // M - 2^32
+    int post = 0;
+    __device__ __forceinline__ SoftmaxQuotient16(unsigned long long z, int fa) {
+        if (z == 0) return;
+        const int l = 63 - __clzll((long long)(z - 1));
+        const unsigned long long n = 1ULL << (33 + l);
+        unsigned long long q = (unsigned long long)((double)n / (double)z);
+        long long r = (long long)(n - q * z);
+        while (r < 0) { q--; r += (long long)z; }
+        while (r >= (long long)z) { q++; r -= (long long)z; }
+        m = (uint32_t)(q + 1);
+        post = 1 + l - fa;
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t e) const { return (__umulhi(e, m) + e) >> post; }
+};
+
 }  // namespace iie

@@ -202,6 +202,29 @@ def test_prefill_attention_matches_the_checker(H, Hkv, hd, start, m, window, rop
     assert np.array_equal(got1.cpu().numpy().reshape(1, -1), want1)
 
 
+@pytest.mark.parametrize("fa", [6, 12, 16, 17, 21])
+def test_prefill_softmax_at_other_activation_scales(fa):
+    """Exponentials and probabilities on either side of the scale up to which they take 32-bit products; a few dominant keys give
+    probabilities near one, the rest near zero."""
+    import torch
+
+    from integer_inference_engine_b200 import device
+    H, Hkv, hd, start, m = 8, 2, 64, 150, 21
+    rng = np.random.default_rng(300 + fa)
+    one = 1 << fa
+    draw = lambda *s: rng.integers(-3 * one, 3 * one, size=s, dtype=np.int64)
+    ck, cv, q, k, v = draw(Hkv, start + m, hd), draw(Hkv, start + m, hd), draw(m, H, hd) // 4, draw(m, Hkv, hd), draw(m, Hkv, hd)
+    want_k, want_v = ck.copy(), cv.copy()
+    want_k[:, start:], want_v[:, start:] = np.transpose(k, (1, 0, 2)), np.transpose(v, (1, 0, 2))
+    want = o.attention_cached(q, want_k, want_v, start, H, Hkv, fa, None)
+    cuda = lambda a, dt=torch.int64: torch.from_numpy(np.ascontiguousarray(a)).to(dt).cuda()
+    device.read_flags()
+    got = device.attention_prefill(cuda(q.reshape(m, -1)), cuda(k.reshape(m, -1)), cuda(v.reshape(m, -1)), cuda(ck, torch.int32), cuda(cv, torch.int32),
+                                   start, H, Hkv, hd, fa, 0, None, None, 0)
+    assert device.read_flags() == 0
+    assert np.array_equal(got.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("qbits", [19, 40])
 def test_prefill_tiles_equal_the_per_token_kernels(qbits):
     """A longer prefill (several key chunks, a window that cuts through them, a ragged last tile) through the sixteen-token
