@@ -213,7 +213,10 @@ struct TileArgs {
     int *flags;                    // bit 0 digit envelope, bit 3 a wait gave up
     int wide, split;               // filled in by the launcher
     long long sig_log2e, sig_clip;
+    unsigned long long *counts;    // launches by tile shape (device)
+    int few;                       // GATEUP of Q4_K: the tiles of eight rows (tiles_few.cu)
 };
+cudaError_t launch_tiles_few(const TileArgs &a, const int8_t *x, cudaStream_t s);
 cudaError_t launch_tiles(int qtype, int mode, const TileArgs &a, cudaStream_t s);
 size_t tile_sums_bytes(long long rows, long long n_blocks);
 // launches by tile shape since the library was loaded: Q4_K gate/up with 3 / 4 activation digits, Q6_K down with up to 5 / 6,

@@ -33,14 +33,13 @@
 // Per block at 2048 tokens: gate / up 840 us, down 670, 5120 x 2048 dense 240 (fully dequantised weights in four or five digits: 940, 1140,
 // 280); at 64 tokens 130, 80, 21 (warp-level MMAs: 165, 190, 45).
 // Every wait is bounded; on a time-out the CTA raises flag bit 3, leaves its loops, frees TMEM and exits.
-#include <cuda.h>
-
 #include <algorithm>
 #include <type_traits>
 
 #include "kernels.h"
 #include "layout.cuh"
 #include "mma_items.cuh"
+#include "tile_ops.cuh"
 
 namespace iie {
 
@@ -59,99 +58,8 @@ constexpr int TL_MINS = TL_MIN_SLOTS * 128 * 32;                   // are at mos
 constexpr int TL_EXCH = 16 * 128 * 8;                              // gate / up: sixteen columns of y on their way to the epilogue warps
 constexpr int TL_SMEM = 217 * 1024;
 constexpr int TL_MAX_GROUPS = 1024;
-constexpr unsigned TL_WAIT_LIMIT = 1u << 17;
-
-__device__ __forceinline__ uint32_t tl_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void tl_init(uint32_t b, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b), "r"(n)); }
-__device__ __forceinline__ void tl_arrive(uint32_t b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b) : "memory"); }
-__device__ __forceinline__ void tl_expect(uint32_t b, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool tl_try(uint32_t b, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(b), "r"(parity) : "memory");
-    return ok != 0;
-}
-__device__ __noinline__ bool tl_wait_slow(uint32_t b, uint32_t parity, volatile int *abort_flag) {      // bounded
-    for (unsigned it = 0; it < TL_WAIT_LIMIT; it++) {
-        uint32_t ok;                                               // asleep for up to 20 us at a time
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok) : "r"(b), "r"(parity), "r"(20000u) : "memory");
-        if (ok) return true;
-        if (*abort_flag) return false;
-    }
-    *abort_flag = 1;
-    return false;
-}
-__device__ __forceinline__ bool tl_wait(uint32_t b, uint32_t parity, volatile int *abort_flag) {        // the whole warp, one answer
-    if (__all_sync(0xffffffffu, tl_try(b, parity))) return true;
-    return __all_sync(0xffffffffu, tl_wait_slow(b, parity, abort_flag));
-}
-__device__ __forceinline__ uint32_t tl_elect() {
-    uint32_t r;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-    return r;
-}
-// split tiles: the same shared-memory address in another CTA of the cluster, and what goes there
-__device__ __forceinline__ uint32_t tl_remote(uint32_t a, int rank) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void tl_remote_store(uint32_t a, long long v) { asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }
-__device__ __forceinline__ void tl_remote_arrive(uint32_t b) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(b) : "memory"); }
-__device__ __noinline__ bool tl_wait_cluster(uint32_t b, uint32_t parity, volatile int *abort_flag) {       // bounded; the whole warp, one answer
-    bool done = false;
-    for (unsigned it = 0; it < TL_WAIT_LIMIT && !done && !*abort_flag; it++) {
-        uint32_t ok;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok) : "r"(b), "r"(parity), "r"(20000u) : "memory");
-        done = ok != 0;
-    }
-    if (!done) *abort_flag = 1;
-    return __all_sync(0xffffffffu, done);
-}
-__device__ __forceinline__ void tl_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
-}
-// a position in a ring of slots, stepped (a division by a run-time slot count in every role's loop costs hundreds of clocks)
-struct TlRing {
-    int slot = 0;
-    uint32_t pass = 0;
-    bool lapped = false;
-    __device__ __forceinline__ void step(int n) { if (++slot == n) { slot = 0; pass ^= 1; lapped = true; } }
-};
-// K-major operands: rows of 128 bytes with the 128-byte swizzle, rows of 32 bytes with the 32-byte swizzle
-__device__ __forceinline__ uint64_t tl_desc128(uint32_t a) {
-    return (uint64_t)((a >> 4) & 0x3FFF) | (1ULL << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ULL << 46) | (2ULL << 61);
-}
-__device__ __forceinline__ uint64_t tl_desc32(uint32_t a) {
-    return (uint64_t)((a >> 4) & 0x3FFF) | (1ULL << 16) | ((uint64_t)(256 >> 4) << 32) | (1ULL << 46) | (6ULL << 61);
-}
-__device__ __forceinline__ uint32_t tl_idesc(int n, bool a_signed) {     // u8 / s8 x s8 -> s32, M = 128
-    return (2u << 4) | (a_signed ? 1u << 7 : 0u) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-__device__ __forceinline__ void tl_mma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}"
-                 ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
-}
-__device__ __forceinline__ void tl_commit(uint32_t b) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(b) : "memory");
-}
-__device__ __forceinline__ void tl_ld4(uint32_t addr, int (&r)[4]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void tl_tma(uint32_t dst, const CUtensorMap *map, int col, int plane, int row, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(col), "r"(plane), "r"(row), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void tl_sts64(uint32_t a, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y)); }
-__device__ __forceinline__ void tl_sts32(uint32_t a, uint32_t x) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(x)); }
-
 // digit planes carried for `nl` digits in use, and columns of a tile: 32 only where the accumulators of three planes leave two
 // TMEM buffers and the registers of the read-out hold sixteen columns
-__device__ __forceinline__ int tl_planes(int nl) { return nl <= 3 ? 3 : nl <= 6 ? nl : 8; }
 
 struct TileMaps { CUtensorMap x16, x32, s16, s32; };               // planes and sums, boxes of 16 and of 32 rows
 
@@ -710,27 +618,6 @@ __global__ void __launch_bounds__(256) tile_rows_kernel(const int8_t *xl, const 
     }
 }
 
-using TlEncode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                              const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                              CUtensorMapFloatOOBfill);
-TlEncode tl_encode() {
-    static TlEncode fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
-        return reinterpret_cast<TlEncode>(p);
-    }();
-    return fn;
-}
-// [rows][planes][width] bytes, boxes of `cols` columns x one plane x `rows_box` rows
-bool tl_map(CUtensorMap *map, const int8_t *p, long long width, long long planes, long long rows, int cols, int rows_box, CUtensorMapSwizzle swizzle) {
-    const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)planes, (cuuint64_t)rows};
-    const cuuint64_t strides[2] = {(cuuint64_t)width, (cuuint64_t)(planes * width)};
-    const cuuint32_t box[3] = {(cuuint32_t)cols, 1, (cuuint32_t)rows_box}, estr[3] = {1, 1, 1};
-    return tl_encode()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                       swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int QT, int MODE>
 cudaError_t launch_tile(const TileArgs &a, const TileMaps &maps, cudaStream_t s) {
     static bool configured = false;
@@ -787,6 +674,12 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
         note_launch();
     }
     const int8_t *x = a.xidx ? a.xg : a.xl;
+    if (a.few && q4 && mode == MODE_GATEUP && a.grp_off) {
+        void *counts = nullptr;
+        if (cudaGetSymbolAddress(&counts, d_tile_launches) != cudaSuccess) return cudaErrorInvalidValue;
+        a.counts = static_cast<unsigned long long *>(counts);
+        return launch_tiles_few(a, x, s);
+    }
     TileMaps maps;
     const long long K = (long long)a.nb * 256;
     bool ok = tl_map(&maps.x16, x, K, 8, a.n_rows, 128, 16, CU_TENSOR_MAP_SWIZZLE_128B) && tl_map(&maps.x32, x, K, 8, a.n_rows, 128, 32, CU_TENSOR_MAP_SWIZZLE_128B);

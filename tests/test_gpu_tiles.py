@@ -65,7 +65,8 @@ def test_tiles_shared_by_clusters_match_the_oracle(qtype, out_f, nb, T, xbits):
 
 
 @pytest.mark.parametrize("down_q", [o.Q4_K, o.Q6_K])
-@pytest.mark.parametrize("d,eff,E,k,T,mult", [(256, 256, 5, 2, 3, 1), (512, 256, 40, 1, 2, 1), (768, 512, 6, 3, 70, 1), (256, 768, 3, 3, 33, 200)])
+@pytest.mark.parametrize("d,eff,E,k,T,mult", [(256, 256, 5, 2, 3, 1), (512, 256, 40, 1, 2, 1), (768, 512, 6, 3, 70, 1), (256, 768, 3, 3, 33, 200), (2304, 256, 24, 4, 48, 1),
+                                                 (768, 512, 40, 2, 90, 200), (512, 256, 17, 2, 9, 20000)])
 def test_expert_tiles_match_the_oracle(down_q, d, eff, E, k, T, mult):
     import torch
 
