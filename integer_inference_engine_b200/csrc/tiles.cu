@@ -63,15 +63,16 @@ constexpr int TL_MAX_GROUPS = 1024;
 
 struct TileMaps { CUtensorMap x16, x32, s16, s32; };               // planes and sums, boxes of 16 and of 32 rows
 
-template <int QT, int MODE>
+// SPLIT: the CTAs of a cluster share the super-blocks of a tile (LINEAR; a form of its own: in one with the others it cost 2048 rows of a
+// dense product 4 %)
+template <int QT, int MODE, bool SPLIT>
 __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArgs a, const __grid_constant__ TileMaps maps) {
     constexpr bool Q4 = QT == QT_Q4K;
     constexpr int HTB = Q4 ? HTB_Q4K : HTB_Q6K, RAW_BYTES = 16 * HTB;
     constexpr int NROW = MODE == MODE_GATEUP ? 64 : 128;           // output rows of a tile
     extern __shared__ __align__(1024) unsigned char tl_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tl_raw) + 1023) & ~(uintptr_t)1023);
-    constexpr bool CAN_SPLIT = MODE == MODE_LINEAR;
-    const int split = CAN_SPLIT ? a.split : 1;                     // CTAs of a cluster that share a tile's super-blocks
+    const int split = SPLIT ? a.split : 1;                         // CTAs of a cluster that share a tile's super-blocks
     __shared__ __align__(8) uint64_t bars[2 * TL_MAX_STAGES + 8 + 2 * TL_MAX_RAW + 4];
     __shared__ int s_first[TL_MAX_GROUPS + 1], s_off[TL_MAX_GROUPS + 1];       // first tile and first row of each group
     __shared__ uint32_t s_tmem;
@@ -80,9 +81,9 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
                    raw_full = free_bar + 8 * 4, raw_empty = raw_full + 8 * TL_MAX_RAW, y_full = raw_empty + 8 * TL_MAX_RAW, y_free = y_full + 8,
                    x_full = y_free + 8, x_free = x_full + 8;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int nb = a.nb, rank = split > 1 ? (int)(blockIdx.x & (split - 1)) : 0;
+    const int nb = a.nb, rank = SPLIT ? (int)(blockIdx.x & (split - 1)) : 0;
     const int b_lo = nb * rank / split, b_hi = nb * (rank + 1) / split;        // super-blocks of this CTA
-    const int first_tile = CAN_SPLIT ? blockIdx.x / split : blockIdx.x, tile_step = CAN_SPLIT ? gridDim.x / split : gridDim.x;
+    const int first_tile = SPLIT ? blockIdx.x / split : blockIdx.x, tile_step = SPLIT ? gridDim.x / split : gridDim.x;
     if (warp == TL_X_WARP && lane == 0) {                          // the tensor maps' first use would wait for them
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x16)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x32)) : "memory");
@@ -106,7 +107,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     const int x_bytes = np * bn * 128, s_bytes = Q4 ? ns * bn * 32 : 0;
     const int stage_bytes = (TL_A_BYTES + x_bytes + s_bytes + 1023) & ~1023;
     constexpr int FIXED = 1024 + (Q4 ? TL_MINS : 0) + (MODE == MODE_GATEUP ? TL_EXCH : 0);
-    const int xch_bytes = split > 1 ? 128 * bn * ((np + 2) / 2) * 8 : 0;       // split tiles: sums of this CTA's share of the columns
+    const int xch_bytes = SPLIT ? 128 * bn * ((np + 2) / 2) * 8 : 0;       // split tiles: sums of this CTA's share of the columns
     const int raw_slots = FIXED + xch_bytes + 3 * stage_bytes + TL_MAX_RAW * RAW_BYTES <= TL_SMEM ? TL_MAX_RAW : 2;
     const int stages = min(TL_MAX_STAGES, (TL_SMEM - FIXED - xch_bytes - raw_slots * RAW_BYTES) / stage_bytes);
     unsigned char *mins = smem + stages * stage_bytes, *exch = mins + (Q4 ? TL_MINS : 0), *raw = exch + (MODE == MODE_GATEUP ? TL_EXCH : xch_bytes);
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (split > 1) tl_cluster_sync();                              // the other CTAs' barriers stand
+    if (SPLIT) tl_cluster_sync();                              // the other CTAs' barriers stand
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
     const int n_tiles = s_first[a.n_groups];
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
                 if (!ok) break;
                 // ---- y = floor(V / 2^fw), then what the product is for ---------------------------------------
                 const int sh = a.fw + (Q4 && !THIRDS ? 4 : 0);
-                if (CAN_SPLIT && split > 1) {
+                if (SPLIT) {
                     // column c of the tile belongs to CTA c mod split, as its column c / split there: everybody's sums go to the owner,
                     // which adds them up, joins the digits and stores
                     const int cols = BN / split;                   // of this CTA
@@ -574,7 +575,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         }
     }
     __syncthreads();
-    if (split > 1) tl_cluster_sync();                              // nobody leaves while another CTA stores or arrives here
+    if (SPLIT) tl_cluster_sync();                              // nobody leaves while another CTA stores or arrives here
     if (warp == TL_MMA_WARP) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -618,18 +619,16 @@ __global__ void __launch_bounds__(256) tile_rows_kernel(const int8_t *xl, const 
     }
 }
 
-template <int QT, int MODE>
+template <int QT, int MODE, bool SPLIT>
 cudaError_t launch_tile(const TileArgs &a, const TileMaps &maps, cudaStream_t s) {
     static bool configured = false;
     if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(tile_kernel<QT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM);
+        const cudaError_t e = cudaFuncSetAttribute(tile_kernel<QT, MODE, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TL_SMEM);
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    // an upper bound on the tiles: every group may end in a partial one
     const long long n_rt = (a.out_f + (MODE == MODE_GATEUP ? 63 : 127)) / (MODE == MODE_GATEUP ? 64 : 128);
-    const long long most = (a.n_rows / 16 + std::min<long long>(a.n_groups, a.n_rows)) * n_rt;
-    if (a.split > 1) {
+    if (SPLIT) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(a.split * ((a.n_rows + (a.wide ? 31 : 15)) / (a.wide ? 32 : 16)) * n_rt));
         cfg.blockDim = dim3(tl_threads(MODE)); cfg.dynamicSmemBytes = TL_SMEM; cfg.stream = s;
@@ -639,9 +638,13 @@ cudaError_t launch_tile(const TileArgs &a, const TileMaps &maps, cudaStream_t s)
         attr[1].id = cudaLaunchAttributeClusterDimension;
         attr[1].val.clusterDim.x = (unsigned)a.split; attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
         cfg.attrs = attr; cfg.numAttrs = 2;
-        cudaLaunchKernelEx(&cfg, tile_kernel<QT, MODE>, a, maps);
-    } else
-    launch_behind(tile_kernel<QT, MODE>, (unsigned)std::max<long long>(1, std::min<long long>(148, most)), tl_threads(MODE), TL_SMEM, s, a, maps);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, tile_kernel<QT, MODE, SPLIT>, a, maps);
+        note_launch();
+        return e != cudaSuccess ? e : cudaGetLastError();
+    }
+    // an upper bound on the tiles: every group may end in a partial one
+    const long long most = (a.n_rows / 16 + std::min<long long>(a.n_groups, a.n_rows)) * n_rt;
+    launch_behind(tile_kernel<QT, MODE, SPLIT>, (unsigned)std::max<long long>(1, std::min<long long>(148, most)), tl_threads(MODE), TL_SMEM, s, a, maps);
     note_launch();
     return cudaGetLastError();
 }
@@ -686,11 +689,12 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
     if (q4) ok = ok && tl_map(&maps.s16, a.xs, stride, 9, a.n_rows, 32, 16, CU_TENSOR_MAP_SWIZZLE_32B) && tl_map(&maps.s32, a.xs, stride, 9, a.n_rows, 32, 32, CU_TENSOR_MAP_SWIZZLE_32B);
     else maps.s16 = maps.s32 = maps.x16;
     if (!ok) return cudaErrorInvalidValue;
-    if (q4 && mode == MODE_LINEAR) return launch_tile<QT_Q4K, MODE_LINEAR>(a, maps, s);
-    if (q4 && mode == MODE_GATEUP) return launch_tile<QT_Q4K, MODE_GATEUP>(a, maps, s);
-    if (q4) return launch_tile<QT_Q4K, MODE_DOWN>(a, maps, s);
-    if (mode == MODE_LINEAR) return launch_tile<QT_Q6K, MODE_LINEAR>(a, maps, s);
-    return launch_tile<QT_Q6K, MODE_DOWN>(a, maps, s);
+    if (a.split > 1) return q4 ? launch_tile<QT_Q4K, MODE_LINEAR, true>(a, maps, s) : launch_tile<QT_Q6K, MODE_LINEAR, true>(a, maps, s);
+    if (q4 && mode == MODE_LINEAR) return launch_tile<QT_Q4K, MODE_LINEAR, false>(a, maps, s);
+    if (q4 && mode == MODE_GATEUP) return launch_tile<QT_Q4K, MODE_GATEUP, false>(a, maps, s);
+    if (q4) return launch_tile<QT_Q4K, MODE_DOWN, false>(a, maps, s);
+    if (mode == MODE_LINEAR) return launch_tile<QT_Q6K, MODE_LINEAR, false>(a, maps, s);
+    return launch_tile<QT_Q6K, MODE_DOWN, false>(a, maps, s);
 }
 
 void tile_launch_counts(unsigned long long *out) {
