@@ -253,10 +253,24 @@ DigitCell next_cell(cudaStream_t s) {
     return ring.next(g_cells + 4, s, c.nl, c.clear) ? c : DigitCell{nullptr, nullptr};
 }
 
+// which products of several rows the warp-level kernel takes first (measurements: linear_dev), and which the tiles can take
+bool few_rows(const Weight &w, long long T) {
+    return g_tc_min_tokens == 0 && T >= 2 && T <= 3 && (w.qtype == QT_Q4K ? w.out_f <= 40960 : w.out_f * w.nb <= 40960);
+}
+bool tiles_can(const Weight &w, long long T, int fw) {
+    return T >= 2 && T >= g_tc_min_tokens && T < (1 << 24) && g_stage_mask == 0 && tile_scales(w.qtype, w.nb, w.maxd, w.maxdmin, fw);
+}
+bool takes_tiles(const Weight &w, long long T, int fw) { return !few_rows(w, T) && tiles_can(w, T, fw); }
+// where the kernel that splits rows for the tiles of a Q4_K matrix leaves their sums, too: a launch less (null: the tiles' own kernel does it)
+int8_t *tile_sums(int qtype, const int64_t *x, long long T, long long nb) {
+    if (qtype != QT_Q4K || (reinterpret_cast<uintptr_t>(x) & 15)) return nullptr;
+    return (int8_t *)ensure(R_XS, tile_sums_bytes(T, nb));
+}
+
 // y[T,out_f] on device from x[T,K] on device.  check_flags: synchronise and re-run the exact kernel
 // if an activation left the limb envelope (host-pointer entries); otherwise flags stay raised.
 bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t *out, bool check_flags, cudaStream_t s,
-                const int8_t *xl_ready = nullptr, const int *nl_ready = nullptr, bool early = false) {
+                const int8_t *xl_ready = nullptr, const int *nl_ready = nullptr, bool early = false, bool sums_ready = false) {
     const long long K = w.nb * 256;
     if (!fast_envelope(w.qtype, w.nb, w.maxd, w.maxdmin, fw))
         return launch_exact_linear((const uint8_t *)w.d, w.qtype, w.out_f, w.nb, x, T, fw, out, s) == cudaSuccess;
@@ -267,8 +281,9 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
         if (!buf) return false;
         if (T >= 2) {
             const DigitCell c = next_cell(s);
-            if (!c.nl || launch_limbs(x, T, K, buf, g_flags, s, c.nl, c.clear) != cudaSuccess) return false;
-            x_nl = c.nl;
+            int8_t *sums = takes_tiles(w, T, fw) ? tile_sums(w.qtype, x, T, w.nb) : nullptr;
+            if (!c.nl || launch_limbs(x, T, K, buf, g_flags, s, c.nl, c.clear, nullptr, nullptr, 0, sums) != cudaSuccess) return false;
+            x_nl = c.nl; sums_ready = sums != nullptr;
         } else if (launch_limbs(x, T, K, buf, g_flags, s) != cudaSuccess) return false;
         xl = buf;
     }
@@ -283,13 +298,14 @@ bool linear_dev(const Weight &w, const int64_t *x, long long T, int fw, int64_t 
         cudaGetLastError();
         return false;
     };
-    // Two and three rows of a matrix that the streaming kernel has read in a wave or two: a tile walks its super-blocks one behind the other
+    // (few_rows) Two and three rows of a matrix that the streaming kernel has read in a wave or two: a tile walks its super-blocks one behind the other
     // (1.3 us each), whatever the rows.  Q4_K, three rows, 512 x 2048 11 us (tiles 20), 5120 x 2048 13 (20), 40960 x 2048 41 (44), 81920 x
     // 2048 75 (68); Q6_K 2048 x 2048 12 (17), 5120 x 2048 17 (18), 10240 x 2048 24 (18).  Four rows 20 (20) and 23 (17).
-    const bool few = g_tc_min_tokens == 0 && T >= 2 && T <= 3 && (w.qtype == QT_Q4K ? w.out_f <= 40960 : w.out_f * w.nb <= 40960);
+    const bool few = few_rows(w, T);
     bool done = few && g_stage_mask == 0 && batch();
-    if (!done && T >= 2 && T >= g_tc_min_tokens && T < (1 << 24) && g_stage_mask == 0 && tile_scales(w.qtype, w.nb, w.maxd, w.maxdmin, fw)) {
+    if (!done && tiles_can(w, T, fw)) {
         TileArgs ta = {};
+        ta.xs_ready = sums_ready;
         ta.wa = w.cell; ta.wb = w.cell; ta.grp_off = nullptr; ta.n_groups = 1; ta.nb = (int)w.nb; ta.n_rows = T; ta.out_f = w.out_f; ta.fw = fw;
         ta.fa = 16; ta.xl = xl; ta.x_nl = x_nl; ta.out = out;
         done = tiles(w.qtype, MODE_LINEAR, ta, s);
@@ -709,8 +725,10 @@ extern "C" int qk_apply_resident_grouped(const long long *handles, const int *ph
     int8_t *xl = (int8_t *)ensure(R_XL, (size_t)T * 8 * K);
     const DigitCell cell = T > 1 ? next_cell(g_stream) : DigitCell{nullptr, nullptr};
     int *nl = cell.nl;
+    int8_t *sums = nullptr;                                // for all matrices, where one takes the tiles
+    for (int i = 0; i < count && T > 1 && !sums; i++) if (takes_tiles(g_w[handles[i]], T, fw)) sums = tile_sums(g_w[handles[i]].qtype, xd, T, nb);
     if (!xd || !od || !xl || !upload(xd, x, (size_t)T * K * 8) ||
-        launch_limbs(xd, T, K, xl, g_flags, g_stream, nl, cell.clear) != cudaSuccess) { cudaGetLastError(); return 1; }
+        launch_limbs(xd, T, K, xl, g_flags, g_stream, nl, cell.clear, nullptr, nullptr, 0, sums) != cudaSuccess) { cudaGetLastError(); return 1; }
     // the products do not wait for the verdict on the digits: an activation beyond them repeats the call with the exact kernel
     for (int exact = 0; exact < 2; exact++) {
         long long off = 0;
@@ -720,7 +738,7 @@ extern "C" int qk_apply_resident_grouped(const long long *handles, const int *ph
             static const int calls[5] = {PM_OTHER_CALLS, PM_Q_CALLS, PM_K_CALLS, PM_V_CALLS, PM_O_CALLS};
             if (!exact) prof(calls[phase >= 0 && phase <= 4 ? phase : 0]);
             const bool ok = exact ? launch_exact_linear((const uint8_t *)w.d, w.qtype, w.out_f, w.nb, xd, T, fw, od + off, g_stream) == cudaSuccess
-                                  : linear_dev(w, xd, T, fw, od + off, false, g_stream, xl, nl, true);
+                                  : linear_dev(w, xd, T, fw, od + off, false, g_stream, xl, nl, true, sums != nullptr);
             if (!ok) { cudaGetLastError(); return 1; }
             off += T * w.out_f;
         }
@@ -884,11 +902,12 @@ extern "C" int iie_moe_forward_dev(long long layer, const int64_t *h_dev, long l
     if (!cell.nl) return 1;
     const long long n_out = T * L.d_model;
     const bool apart = out_dev + n_out <= h_dev || h_dev + n_out <= out_dev, zero_here = !accumulate && stage_on(ST_LIMBS) && apart;
-    if (stage_on(ST_LIMBS) && launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, cell.nl, cell.clear, g_cells + 1, zero_here ? out_dev : nullptr, n_out) != cudaSuccess) return 1;
+    int8_t *sums = r.qtype != QT_I64 && T >= 2 && takes_tiles(r, T, fw) ? tile_sums(r.qtype, h_dev, T, r.nb) : nullptr;
+    if (stage_on(ST_LIMBS) && launch_limbs(h_dev, T, L.d_model, hl, g_flags, s, cell.nl, cell.clear, g_cells + 1, zero_here ? out_dev : nullptr, n_out, sums) != cudaSuccess) return 1;
     if (stage_on(ST_ROUTER)) {
         if (r.qtype == QT_I64) {
             if (launch_exact_dense((const int64_t *)r.d, E, L.d_model, h_dev, T, fw, lg, g_flags, s) != cudaSuccess) return 1;
-        } else if (!linear_dev(r, h_dev, T, fw, lg, false, s, hl, cell.nl)) return 1;
+        } else if (!linear_dev(r, h_dev, T, fw, lg, false, s, hl, cell.nl, false, sums != nullptr)) return 1;
     }
     if (stage_on(ST_TOPK) && launch_topk(lg, T, E, k, fa, ids, gates, s) != cudaSuccess) return 1;
     if (!accumulate && !zero_here && cudaMemsetAsync(out_dev, 0, (size_t)T * L.d_model * 8, s) != cudaSuccess) return 1;

@@ -214,6 +214,7 @@ struct TileArgs {
     int wide, split;               // filled in by the launcher
     long long sig_log2e, sig_clip;
     unsigned long long *counts;    // launches by tile shape (device)
+    int xs_ready;                  // xs holds the sums (without xidx)
     int few;                       // GATEUP of Q4_K: the tiles of eight rows (tiles_few.cu)
 };
 cudaError_t launch_tiles_few(const TileArgs &a, const int8_t *x, cudaStream_t s);
@@ -235,7 +236,10 @@ cudaError_t launch_unpack(const uint8_t *src, uint8_t *raw, long long out_f, lon
 // int64 rows -> balanced base-256 limb planes [row][8][K]; sets flags bit 0 on overflow.
 cudaError_t launch_limbs(const int64_t *x, long long n_rows, long long K, int8_t *planes, int *flags, cudaStream_t s,
                          int *nl_out = nullptr,    // nl_out: atomicMax of the limbs in use (zero before)
-                         int *clear0 = nullptr, int *clear1 = nullptr, int64_t *zero = nullptr, long long zero_n = 0);   // words that later kernels find zeroed
+                         int *clear0 = nullptr, int *clear1 = nullptr, int64_t *zero = nullptr, long long zero_n = 0,    // words that later kernels find zeroed
+                         // the sums of every 32 columns as nine balanced digits [row][9][K / 32 rounded up to 32], what the Q4_K tiles multiply with the
+                         // minima (K a multiple of 256, x on 16 bytes)
+                         int8_t *sums = nullptr);
 
 // p[0] = a, p[1] = b on the stream (kernel arguments travel by value, so a captured launch replays correctly where a
 // copy from a host stack variable would not)

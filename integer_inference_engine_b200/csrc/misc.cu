@@ -47,7 +47,7 @@ __global__ void repack_kernel(const uint8_t *src, uint8_t *dst, long long out_f,
 // ---------------------------------------------------------------------------------------------------
 // activation limb planes
 // ---------------------------------------------------------------------------------------------------
-struct LimbClears { int *a, *b; int64_t *zero; long long zero_n; };
+struct LimbClears { int *a, *b; int64_t *zero; long long zero_n; int8_t *sums; int stride; };      // and sums of 32 columns, see launch_limbs
 __device__ __forceinline__ void limb_clears(const LimbClears &c) {
     if (blockIdx.x == 0 && threadIdx.x == 0) { if (c.a) *c.a = 0; if (c.b) *c.b = 0; }
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < c.zero_n; i += (long long)gridDim.x * blockDim.x) c.zero[i] = 0;
@@ -87,9 +87,12 @@ __global__ void __launch_bounds__(256) limbs8_kernel(const int64_t *x, long long
         const long long row = g / per_row, col = (g - row * per_row) << 3;
         const ulonglong2 *src = reinterpret_cast<const ulonglong2 *>(x + row * K + col);
         uint32_t lo[8], hi[8];
+        uint64_t sum_lo = 0;                               // of the low words, and of the signed high words
+        int64_t sum_hi = 0;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const ulonglong2 v = __ldcg(src + i);
+            sum_lo += (uint64_t)(uint32_t)v.x + (uint32_t)v.y; sum_hi += (int64_t)(int32_t)(v.x >> 32) + (int32_t)(v.y >> 32);
             bool ok0, ok1;
             const uint64_t d0 = balanced_digits8((int64_t)v.x, ok0), d1 = balanced_digits8((int64_t)v.y, ok1);
             bad |= !ok0 | !ok1;
@@ -116,6 +119,17 @@ __global__ void __launch_bounds__(256) limbs8_kernel(const int64_t *x, long long
             }
 #pragma unroll
             for (int l = 0; l < 4; l++) *reinterpret_cast<uint2 *>(dst + (half * 4 + l) * K) = make_uint2(a[l], b[l]);
+        }
+        if (clears.sums) {                                 // (K is a multiple of 256: four lanes hold the 32 columns of a sub-block)
+            for (int off = 1; off <= 2; off <<= 1) { sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, off); sum_hi += __shfl_xor_sync(0xffffffffu, sum_hi, off); }
+            // balanced digits of hi 2^32 + lo: bytes of the sum with 128 added to each of the nine
+            const u128 biased = (u128)((i128)sum_hi * ((i128)1 << 32) + (i128)sum_lo) + (((u128)0x80 << 64) | 0x8080808080808080ULL);
+            const int t = threadIdx.x & 3;
+            const long long j = col >> 5;
+            int8_t *to = clears.sums + row * 9 * clears.stride + j;
+            for (int l = t; l < 9; l += 4) to[l * clears.stride] = (int8_t)((uint8_t)(biased >> (8 * l)) ^ 0x80);
+            for (long long pad = (K >> 5) + t; j == (K >> 5) - 1 && pad < clears.stride; pad += 4)
+                for (int l = 0; l < 9; l++) to[l * clears.stride + pad - j] = 0;
         }
     }
     if (bad) atomicOr(flags, 1);
@@ -557,8 +571,9 @@ cudaError_t launch_add_rows(const int64_t *a, const int64_t *b, int64_t *out, lo
 }
 
 cudaError_t launch_limbs(const int64_t *x, long long n_rows, long long K, int8_t *planes, int *flags, cudaStream_t s,
-                         int *nl_out, int *clear0, int *clear1, int64_t *zero, long long zero_n) {
-    const LimbClears clears = {clear0, clear1, zero, zero ? zero_n : 0};
+                         int *nl_out, int *clear0, int *clear1, int64_t *zero, long long zero_n, int8_t *sums) {
+    const LimbClears clears = {clear0, clear1, zero, zero ? zero_n : 0, sums, (int)((K / 32 + 31) / 32 * 32)};
+    if (sums && (K % 256 || (reinterpret_cast<uintptr_t>(x) & 15))) return cudaErrorInvalidValue;
     if (K % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(planes) & 7) == 0)
         launch_behind(limbs8_kernel, grid_for(n_rows * (K >> 3), 256), 256, 0, s, x, n_rows, K, planes, flags, nl_out, clears);
     else

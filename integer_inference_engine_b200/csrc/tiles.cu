@@ -671,7 +671,7 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
     while (mode == MODE_LINEAR && a.split < 8 && 2 * a.split <= a.nb && whole <= (a.split == 1 ? 74 : a.split == 2 ? 33 : 15)) a.split *= 2;
     const int stride = (a.nb * 8 + 31) / 32 * 32;
     const bool q4 = qtype == QT_Q4K;
-    if (q4 || a.xidx) {
+    if ((q4 && !a.xs_ready) || a.xidx) {
         const long long n = a.n_rows * stride;
         launch_behind(tile_rows_kernel, (unsigned)((n + 255) / 256), 256, 0, s, a.xl, a.xidx, a.grp_off ? a.grp_off + a.n_groups : nullptr, a.x_nl, a.n_rows, a.nb, stride, a.xg, q4 ? a.xs : nullptr);
         note_launch();
