@@ -128,12 +128,10 @@ __host__ __device__ __forceinline__ int64_t mul_shift(int64_t a, int64_t b, int 
 
 __host__ __device__ __forceinline__ int64_t silu_fixed(int64_t x, int fa) { return mul_shift(x, sigmoid_fixed(x, fa), fa); }
 
-// ((g * sigmoid(g)) >> fa) * u >> fa, the gated product of an expert.  For 1 <= fa <= 24 every operand of the sigmoid fits 32 bits:
-// 32 x 32 -> 64 products, single funnel shifts, a division without a loop; no branch, so that several evaluations interleave in one
-// thread (the general form's 64- and 128-bit shifts by a run-time amount and its fix-up loops took 3100 clocks each in the epilogue
-// of the tiles, where a warp has no other work to hide them under).  The same values.
-__host__ __device__ __forceinline__ int64_t silu_up_fixed(int64_t g, int64_t u, int fa, int64_t log2e, int64_t clip) {
-    if (fa > 24 || fa < 1) return mul_shift(mul_shift(g, sigmoid_fixed_c(g, fa, log2e, clip), fa), u, fa);
+// The same for 1 <= fa <= 24, where every operand fits 32 bits: 32 x 32 -> 64 products, single funnel shifts, a division without a loop; no
+// branch, so that several evaluations interleave in one thread (the general form's 64- and 128-bit shifts by a run-time amount and its
+// fix-up loops took 3100 clocks each in the epilogue of the tiles, where a warp has no other work to hide them under).
+__host__ __device__ __forceinline__ uint32_t sigmoid_short(int64_t g, int fa, int64_t log2e, int64_t clip) {
     const bool neg = g < 0;
     const uint64_t mag = neg ? 0ULL - (uint64_t)g : (uint64_t)g;
     const uint32_t d = mag > (uint64_t)clip ? (uint32_t)clip : (uint32_t)mag;                   // clip < 2^(fa + 5)
@@ -155,9 +153,16 @@ __host__ __device__ __forceinline__ int64_t silu_up_fixed(int64_t g, int64_t u, 
     const int q2 = __float2int_rn((float)r * rz);
     r -= q2 * (int)z;
     sg += (uint32_t)q2 - (r < 0 ? 1u : 0u);
+    return sg;
 #else
-    const uint32_t sg = (uint32_t)(((uint64_t)num << fa) / z);
+    return (uint32_t)(((uint64_t)num << fa) / z);
 #endif
+}
+
+// ((g * sigmoid(g)) >> fa) * u >> fa, the gated product of an expert.
+__host__ __device__ __forceinline__ int64_t silu_up_fixed(int64_t g, int64_t u, int fa, int64_t log2e, int64_t clip) {
+    if (fa > 24 || fa < 1) return mul_shift(mul_shift(g, sigmoid_fixed_c(g, fa, log2e, clip), fa), u, fa);
+    const uint32_t sg = sigmoid_short(g, fa, log2e, clip);
     // g * sg = (high word) * sg * 2^32 + (low word) * sg: only the second part is floored
     const uint64_t lo = (uint64_t)(uint32_t)g * sg;
     const int64_t hi = (int64_t)(int32_t)(g >> 32) * (int64_t)sg;
@@ -167,6 +172,17 @@ __host__ __device__ __forceinline__ int64_t silu_up_fixed(int64_t g, int64_t u, 
 #else
     return mul_shift(silu, u, fa);
 #endif
+}
+// The same for every g: the distance of INT64_MIN wraps as in the general form.
+__host__ __device__ __forceinline__ int64_t silu_up_any(int64_t g, int64_t u, int fa, int64_t log2e, int64_t clip) {
+    if (g == INT64_MIN) return mul_shift(mul_shift(g, sigmoid_fixed_c(g, fa, log2e, clip), fa), u, fa);
+    return silu_up_fixed(g, u, fa, log2e, clip);
+}
+// The gated product of the 1-bit decoder: both products wrap at 64 bits.
+__host__ __device__ __forceinline__ int64_t silu_up_wrapped(int64_t g, int64_t u, int fa, int64_t log2e, int64_t clip) {
+    const uint64_t sg = fa > 24 || fa < 1 || g == INT64_MIN ? (uint64_t)sigmoid_fixed_c(g, fa, log2e, clip) : sigmoid_short(g, fa, log2e, clip);
+    const int64_t silu = (int64_t)((uint64_t)g * sg) >> fa;
+    return (int64_t)((uint64_t)silu * (uint64_t)u) >> fa;
 }
 
 // ---- balanced base-256 digits: x = sum_l d_l * 256^l, d_l in [-128,127] --------------------------------

@@ -88,11 +88,7 @@ __global__ void q1_prep_kernel(const int64_t *x, const int64_t *up, long long ld
         int64_t u[4];
         q1_four(us, wide, u);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int64_t sg = sigmoid_fixed_c(v[i], frac, log2e, clip);
-            const int64_t silu = (int64_t)((unsigned long long)v[i] * (unsigned long long)sg) >> frac;
-            v[i] = (int64_t)((unsigned long long)silu * (unsigned long long)u[i]) >> frac;
-        }
+        for (int i = 0; i < 4; i++) v[i] = silu_up_wrapped(v[i], u[i], frac, log2e, clip);
     }
     uint32_t pl[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int nl = 0;
@@ -116,10 +112,7 @@ __global__ void q1_silu_mul_kernel(const int64_t *gate, const int64_t *up, long 
                                    int64_t *out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t g = gate[i];
-    const int64_t sg = sigmoid_fixed_c(g, frac, log2e, clip);
-    const int64_t silu = (int64_t)((unsigned long long)g * (unsigned long long)sg) >> frac;
-    out[i] = (int64_t)((unsigned long long)silu * (unsigned long long)up[i]) >> frac;
+    out[i] = silu_up_wrapped(gate[i], up[i], frac, log2e, clip);
 }
 
 // one row of a registered Q1_0 matrix as int64: sign * block scale (reference_bonsai.py:138-146 q1_rows_fp)
