@@ -205,11 +205,15 @@ int apply_device(const Q1Weight &w, const int64_t *xd, long long T, long long fr
 constexpr size_t STAGE = 256 << 10;
 uint8_t *q_stage = nullptr;
 bool q_stage_tried = false;
-bool download_checked(void *dst, const void *src, size_t n) {
+uint8_t *staging() {
     if (!q_stage_tried) {
         q_stage_tried = true;
         if (cudaHostAlloc(&q_stage, STAGE + 64, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); q_stage = nullptr; }
     }
+    return q_stage;
+}
+bool download_checked(void *dst, const void *src, size_t n) {
+    staging();
     const bool staged = q_stage && n <= STAGE;
     int pageable = 0;
     int *seen = q_stage ? reinterpret_cast<int *>(q_stage) : &pageable;
@@ -682,6 +686,34 @@ bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logi
                     {{m.out_head, logits}}, planes, rows, m.frac, x, rows * m.d);
 }
 
+// The same for a step's rows, the output matrix in two halves of whole waves where it is large: the first half's logits are on their way to
+// the host while the second is multiplied (7 MB take 130 us, the product of six rows 120).  `first`: rows of the first half, 0 for one piece;
+// its logits [rows][first] lie in front of the others'.
+cudaStream_t q_copy = nullptr;
+cudaEvent_t q_half = nullptr;
+long long head_first(const Q1Stack &m, long long rows) {
+    const Q1Weight &w = q_w[(size_t)m.out_head];
+    const long long tiles = (w.out_f + 127) / 128, first = tiles / 2 / Q1_TC_CTAS * Q1_TC_CTAS;
+    if (rows < 2 || first <= 0 || q1_tc_split(first, rows) || q1_tc_split(tiles - first, rows)) return 0;
+    if (!q_copy && cudaStreamCreateWithFlags(&q_copy, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); q_copy = nullptr; return 0; }
+    if (!q_half && cudaEventCreateWithFlags(&q_half, cudaEventDisableTiming) != cudaSuccess) { cudaGetLastError(); q_half = nullptr; return 0; }
+    return first * 128;
+}
+bool head_halves(const Q1Stack &m, const int64_t *x, long long rows, long long first, int64_t *logits, int *flags) {
+    const Q1Weight &w = q_w[(size_t)m.out_head];
+    int8_t *planes = (int8_t *)q_ensure(QR_PLANES, (size_t)rows * 8 * (size_t)m.d);
+    const PlaneDuties d = next_digits(q_stream);
+    const Q1Part a = {w.units, first, logits, nullptr, w.max_scale},
+                 b = {w.units + (size_t)(first / 16) * w.nb * q1_unit_bytes(w.sc32), w.out_f - first, logits + rows * first, nullptr, w.max_scale};
+    return planes && d.nl &&
+           launch_rmsnorm_planes(x, rows, m.d, q_bufs[(size_t)m.finalg].p, (int)m.frac, m.eps, nullptr, planes, flags, d, q_stream) == cudaSuccess &&
+           launch_q1_apply(&a, 1, w.sc32, w.nb, planes, rows, m.frac, d.nl, q_stream) == cudaSuccess && cudaEventRecord(q_half, q_stream) == cudaSuccess &&
+           launch_q1_apply(&b, 1, w.sc32, w.nb, planes, rows, m.frac, d.nl, q_stream) == cudaSuccess;
+}
+bool copy_half(long long *out, const int64_t *logits, long long rows, long long vocab, long long from, long long n, cudaStream_t s) {
+    return cudaMemcpy2DAsync(out + from, (size_t)vocab * 8, logits + rows * from, (size_t)n * 8, (size_t)n * 8, (size_t)rows, cudaMemcpyDeviceToHost, s) == cudaSuccess;
+}
+
 // Rows from pageable host memory: four threads copy pieces into a page-locked buffer and send each on its way (one thread, or the
 // driver's own staging, copies 11 GB/s: 1.4 ms for 512 rows of 4096).  A single buffer of at most 32 MB, kept until the
 // weights are freed.
@@ -760,11 +792,24 @@ long long padded_head_dim(long long hd) {
 }
 
 // Flags other callers left in the shared word are set aside while one of these entries runs and put back afterwards.
+// (Both ends on the stream, one wait at the second: the word as it was is kept in a cell meanwhile.)
 struct FlagScope {
-    int earlier = 0;
     bool ok = false;
-    FlagScope() { earlier = iie_flags_read_clear(q_stream); ok = earlier >= 0; }
-    int finish() { const int f = iie_flags_read_clear(q_stream); if (earlier > 0) iie::restore_flag_bits(earlier); return f; }
+    FlagScope() {
+        int *word = shared_flag_word();
+        ok = word && cudaMemcpyAsync(q_cells + 4, word, sizeof(int), cudaMemcpyDeviceToDevice, q_stream) == cudaSuccess &&
+             cudaMemsetAsync(word, 0, sizeof(int), q_stream) == cudaSuccess;
+    }
+    int finish() {
+        int pageable[2] = {0, 0};
+        int *seen = staging() ? reinterpret_cast<int *>(q_stage) : pageable, *word = shared_flag_word();
+        if (!ok || cudaMemcpyAsync(seen, word, sizeof(int), cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
+            cudaMemcpyAsync(seen + 1, q_cells + 4, sizeof(int), cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
+            cudaMemsetAsync(word, 0, sizeof(int), q_stream) != cudaSuccess || cudaStreamSynchronize(q_stream) != cudaSuccess) return -1;
+        const int f = seen[0], earlier = seen[1];
+        if (earlier > 0) iie::restore_flag_bits(earlier);
+        return f;
+    }
 };
 
 struct DecodeCtx {
@@ -1067,11 +1112,19 @@ extern "C" int bonsai_decode_step(long long ctx_h, const long long *x_in, const 
                 return true;
             });
         }
-        ok = ok && head_rows(m, c.w.x, c.B, c.logits, fw);
+        const long long first = ok ? head_first(m, c.B) : 0;
+        if (first) {
+            ok = ok && head_halves(m, c.w.x, c.B, first, c.logits, fw) && cudaStreamWaitEvent(q_copy, q_half, 0) == cudaSuccess &&
+                 copy_half(out_logits, c.logits, c.B, c.vocab, 0, first, q_copy);
+        } else ok = ok && head_rows(m, c.w.x, c.B, c.logits, fw);
         flags = scope.finish();
         ok = ok && flags >= 0 && !(flags & FLAG_GAVE_UP);
+        if (ok && flags == 0)
+            ok = first ? copy_half(out_logits, c.logits, c.B, c.vocab, first, c.vocab - first, q_copy)
+                       : cudaMemcpyAsync(out_logits, c.logits, (size_t)c.B * c.vocab * 8, cudaMemcpyDeviceToHost, q_stream) == cudaSuccess;
+        // (nothing is on its way into the caller's array when the call ends, whatever it returns)
+        if (cudaStreamSynchronize(first ? q_copy : q_stream) != cudaSuccess) ok = false;
     }
-    if (ok && flags == 0) ok = cudaMemcpy(out_logits, c.logits, (size_t)c.B * c.vocab * 8, cudaMemcpyDeviceToHost) == cudaSuccess;
     if (!ok) return fail(1, "decode step: CUDA failure");
     if (flags) return fail(4, "decode step: a value left the exact envelope");
     return 0;

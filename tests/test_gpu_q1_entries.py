@@ -87,6 +87,29 @@ def test_decode_context_steps_sequences_at_their_own_positions(model):
     assert q1_gpu.decode_step(ctx, x, [5, 3], s["vocab"]) is None
 
 
+@pytest.mark.parametrize("vocab", (152597, 151680))
+def test_logits_of_a_large_vocabulary_leave_in_two_halves(model, golden_dir, vocab):
+    """The recorded output matrix repeated: the halves meet where they should, and a refused step leaves the context usable."""
+    from integer_inference_engine_b200 import q1_gpu
+    g, w, gh, s, inv_sqrt = model
+    rows = np.arange(vocab) % s["vocab"]
+    head = q1_gpu.q1_register_weight(np.ascontiguousarray(g["output_bits"][rows]), np.ascontiguousarray(g["output_scale_fp"][rows]))
+    dims = (2, s["layers"], s["H"], s["Hkv"], s["hd"], s["d"], s["dff"], vocab)
+    ctx = q1_gpu.decode_ctx_create(dims, {**w, "out_head": head, "out_head_vocab": vocab}, gh, FRAC, 1, inv_sqrt, 8)
+    assert ctx is not None
+    full_k = np.stack([g["k0"], g["k1"]]); full_v = np.stack([g["v0"], g["v1"]])
+    for b in range(2):
+        assert q1_gpu.decode_ctx_seed_seq(ctx, b, full_k, full_v)
+    x0 = model_oracle.q1_rows(g["embed_bits"], g["embed_scale_fp"], int(g["token"]))
+    bad = np.concatenate([x0, x0])
+    bad[1, :2] = np.iinfo(np.int64).min
+    assert q1_gpu.decode_step(ctx, bad, [5, 5], vocab) is None
+    logits = q1_gpu.decode_step(ctx, np.concatenate([x0, x0]), [5, 5], vocab)
+    for b in range(2):
+        assert np.array_equal(logits[b], g["logits"][0][rows])
+    q1_gpu.decode_ctx_free(ctx)
+
+
 def _host_attention(q, k, v, start, frac, inv_sqrt):
     """q (H, M, hd), k / v (Hkv, L, hd) -> (H, M, hd) with the checker's cached attention (token-major layout)."""
     H, M, hd = q.shape
