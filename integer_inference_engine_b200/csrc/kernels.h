@@ -53,7 +53,7 @@ struct PlaneDuties {
     long long zero_n = 0;
 };
 
-enum SkinnyMode { MODE_LINEAR = 0, MODE_GATEUP = 1, MODE_DOWN = 2, MODE_FRONT = 3 };
+enum SkinnyMode { MODE_LINEAR = 0, MODE_GATEUP = 1, MODE_DOWN = 2, MODE_FRONT = 3, MODE_SEVERAL = 4 };
 
 // Arguments of the streamed ("skinny") fused-dequant product.  Work is organised in groups: group g
 // uses weight matrix `expert = grp_expert ? grp_expert[g] : g` and owns the activation rows
@@ -139,6 +139,11 @@ struct StreamArgs {
     const uint8_t *const *rank_tabs;
     const uint8_t **rank_ptrs;
     int tiles_b;                   // filled in by the launcher
+    // MODE_SEVERAL: the row with up to four matrices of one block format and length in one launch, out = their products one behind the other
+    const uint8_t *mat[4];
+    long long mat_rows[4];
+    int n_mats;
+    int mat_end[4];                // filled in by the launcher: tiles up to and with that matrix
 };
 cudaError_t launch_stream(int qtype, int mode, const StreamArgs &a, cudaStream_t s);
 

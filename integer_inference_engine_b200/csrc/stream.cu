@@ -89,18 +89,25 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
     __shared__ unsigned long long s_rms, s_inv, s_gm;
     __shared__ int s_bad, s_nl, s_fast;
 
-    const int n_tiles = MODE == MODE_FRONT ? a.tiles_per_expert + a.tiles_b : a.n_sel * a.tiles_per_expert;
+    const int n_tiles = MODE == MODE_FRONT ? a.tiles_per_expert + a.tiles_b : MODE == MODE_SEVERAL ? a.mat_end[3] : a.n_sel * a.tiles_per_expert;
+    auto rows_of = [&](int s) {                                  // rows of matrix s
+        if (MODE == MODE_SEVERAL) return s == 0 ? a.mat_rows[0] : s == 1 ? a.mat_rows[1] : s == 2 ? a.mat_rows[2] : a.mat_rows[3];
+        return MODE == MODE_FRONT && s == 1 ? a.out_f_b : a.out_f;
+    };
+    auto half_tiles_of = [&](int s) { return (int)((rows_of(s) + 7) >> 3); };
     const int tile0 = (int)blockIdx.x * tpc;
     const int my_tiles = min(tpc, n_tiles - tile0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n_ht = (int)((a.out_f + 7) >> 3), n_ht_b = (int)((a.out_f_b + 7) >> 3);
-    const bool topk = MODE != MODE_FRONT && MODE != MODE_LINEAR && a.logits != nullptr;
+    const bool topk = (MODE == MODE_GATEUP || MODE == MODE_DOWN) && a.logits != nullptr;
 
     for (int i = threadIdx.x; i < my_tiles; i += blockDim.x) {
         const int tau = tile0 + i;
         int sl, ps;
         if (MODE == MODE_FRONT) { sl = tau < a.tiles_per_expert ? 0 : 1; ps = tau - sl * a.tiles_per_expert; }
-        else { sl = tau / a.tiles_per_expert; ps = tau - sl * a.tiles_per_expert; }
+        else if (MODE == MODE_SEVERAL) {
+            sl = (tau >= a.mat_end[0]) + (tau >= a.mat_end[1]) + (tau >= a.mat_end[2]);
+            ps = tau - (sl == 0 ? 0 : sl == 1 ? a.mat_end[0] : sl == 2 ? a.mat_end[1] : a.mat_end[2]);
+        } else { sl = tau / a.tiles_per_expert; ps = tau - sl * a.tiles_per_expert; }
         t_sel[i] = sl; t_pos[i] = ps;
         mbar_init(&bars[i], 1);
     }
@@ -159,6 +166,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
         const int s = t_sel[i], p = t_pos[i];
         const uint8_t *pa, *pb = nullptr;
         if (MODE == MODE_FRONT) pa = s == 0 ? a.wa[0] : a.wb[0];
+        else if (MODE == MODE_SEVERAL) pa = s == 0 ? a.mat[0] : s == 1 ? a.mat[1] : s == 2 ? a.mat[2] : a.mat[3];
         else if (topk) { const int e = s_ids[s]; pa = a.wa[e]; if (MODE == MODE_GATEUP) pb = a.wb[e]; }
         else if (a.sel_wa) { pa = a.sel_wa[s]; if (MODE == MODE_GATEUP) pb = a.sel_wb[s]; }
         else { const int e = a.sel ? a.sel[s] : s; pa = a.wa[e]; if (MODE == MODE_GATEUP) pb = a.wb[e]; }
@@ -168,7 +176,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
             bulk_g2s(dst, pa + (size_t)p * nb * HTB, (uint32_t)(nb * HTB), &bars[i]);
             bulk_g2s(dst + nb * HTB, pb + (size_t)p * nb * HTB, (uint32_t)(nb * HTB), &bars[i]);
         } else {
-            const int units = (2 * p + 1 < ((MODE == MODE_FRONT && s == 1) ? n_ht_b : n_ht)) ? 2 : 1;   // an odd last half-tile stands alone
+            const int units = 2 * p + 1 < half_tiles_of(s) ? 2 : 1;   // an odd last half-tile stands alone
             mbar_expect_tx(&bars[i], (uint32_t)(units * nb * HTB));
             bulk_g2s(dst, pa + (size_t)(2 * p) * nb * HTB, (uint32_t)(units * nb * HTB), &bars[i]);
         }
@@ -368,7 +376,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
         uint8_t *ua = wbuf + (size_t)ti * tile_bytes + (size_t)b * HTB;
         const uint8_t *ub;
         if (MODE == MODE_GATEUP) ub = ua + (size_t)nb * HTB;
-        else ub = (2 * p + 1 < ((MODE == MODE_FRONT && s == 1) ? n_ht_b : n_ht)) ? ua + (size_t)nb * HTB : ua;
+        else ub = 2 * p + 1 < half_tiles_of(s) ? ua + (size_t)nb * HTB : ua;
         const int ti_now = ti;
         b += step_b; ti += step_t;
         if (b >= nb) { b -= nb; ti++; }
@@ -420,10 +428,11 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const StreamArgs
             for (int l = 0; l < 8; l++) a.out_limbs[((long long)s * 8 + l) * a.out_f + row] = (int8_t)(d >> (8 * l));
         } else {
             const long long row = (long long)p * 16 + g + 8 * t;
-            if (t >= 2 || row >= ((MODE == MODE_FRONT && s == 1) ? a.out_f_b : a.out_f)) continue;
+            if (t >= 2 || row >= rows_of(s)) continue;
             const int64_t v = t ? y[1] : y[0];
             if (MODE == MODE_FRONT) (s == 0 ? a.out : a.out_b)[row] = v;
             else if (MODE == MODE_LINEAR) a.out[(long long)s * a.out_f + row] = v;
+            else if (MODE == MODE_SEVERAL) a.out[(s > 0 ? a.mat_rows[0] : 0) + (s > 1 ? a.mat_rows[1] : 0) + (s > 2 ? a.mat_rows[2] : 0) + row] = v;
             else atomicAdd(reinterpret_cast<unsigned long long *>(a.out + row),
                            (unsigned long long)mul_shift(v, topk ? s_gates[s] : a.gates[s], a.fa));
         }
@@ -442,7 +451,17 @@ cudaError_t launch_stream_t(const StreamArgs &a_in, cudaStream_t s) {
     const long long n_ht = (a.out_f + 7) >> 3;
     a.tiles_per_expert = (int)(MODE == MODE_GATEUP ? n_ht : (n_ht + 1) / 2);
     a.tiles_b = MODE == MODE_FRONT ? (int)((((a.out_f_b + 7) >> 3) + 1) / 2) : 0;
-    const long long n_tiles = MODE == MODE_FRONT ? (long long)a.tiles_per_expert + a.tiles_b : (long long)a.n_sel * a.tiles_per_expert;
+    if (MODE == MODE_SEVERAL) {
+        if (a.n_mats < 1 || a.n_mats > 4) return cudaErrorInvalidValue;
+        long long tiles = 0;
+        for (int i = 0; i < 4; i++) {
+            if (i >= a.n_mats) a.mat_rows[i] = 0;
+            tiles += (((a.mat_rows[i] + 7) >> 3) + 1) / 2;
+            if (tiles > (1 << 28) || (i < a.n_mats && (!a.mat[i] || a.mat_rows[i] <= 0))) return cudaErrorInvalidValue;
+            a.mat_end[i] = (int)tiles;
+        }
+    }
+    const long long n_tiles = MODE == MODE_SEVERAL ? a.mat_end[3] : MODE == MODE_FRONT ? (long long)a.tiles_per_expert + a.tiles_b : (long long)a.n_sel * a.tiles_per_expert;
     const size_t tile_bytes = (size_t)2 * a.n_blocks * HTB, per_tile = tile_bytes + 8 + 8;
     const size_t front_bytes = MODE == MODE_FRONT ? (size_t)8 * (a.n_blocks * 256 + FR_PAD) + (size_t)16 * a.n_blocks * 256 + 16 : 0;
     if (MODE == MODE_FRONT && (!a.x || !a.out || !a.out_b || a.out_f_b <= 0 || a.n_blocks * 256 > 8192)) return cudaErrorInvalidValue;
@@ -482,17 +501,19 @@ cudaError_t launch_stream_f(const StreamArgs &a, cudaStream_t s) {
 }  // namespace
 
 cudaError_t launch_stream(int qtype, int mode, const StreamArgs &a, cudaStream_t s) {
-    if (a.n_sel <= 0 || a.out_f <= 0 || a.n_blocks <= 0) return cudaErrorInvalidValue;
+    if (a.n_blocks <= 0 || (mode != MODE_SEVERAL && (a.n_sel <= 0 || a.out_f <= 0))) return cudaErrorInvalidValue;
     if (qtype == QT_Q4K) {
         if (mode == MODE_LINEAR) return launch_stream_f<QT_Q4K, MODE_LINEAR>(a, s);
         if (mode == MODE_GATEUP) return launch_stream_f<QT_Q4K, MODE_GATEUP>(a, s);
         if (mode == MODE_FRONT) return launch_stream_f<QT_Q4K, MODE_FRONT>(a, s);
+        if (mode == MODE_SEVERAL) return launch_stream_f<QT_Q4K, MODE_SEVERAL>(a, s);
         return launch_stream_f<QT_Q4K, MODE_DOWN>(a, s);
     }
     if (qtype == QT_Q6K) {
         if (mode == MODE_LINEAR) return launch_stream_f<QT_Q6K, MODE_LINEAR>(a, s);
         if (mode == MODE_GATEUP) return launch_stream_f<QT_Q6K, MODE_GATEUP>(a, s);
         if (mode == MODE_FRONT) return launch_stream_f<QT_Q6K, MODE_FRONT>(a, s);
+        if (mode == MODE_SEVERAL) return launch_stream_f<QT_Q6K, MODE_SEVERAL>(a, s);
         return launch_stream_f<QT_Q6K, MODE_DOWN>(a, s);
     }
     return cudaErrorInvalidValue;

@@ -34,6 +34,24 @@ def test_grouped_products(rows):
     qk_cuda.free_all()
 
 
+@pytest.mark.parametrize("qtype", [o.Q4_K, o.Q6_K])
+@pytest.mark.parametrize("nb,widths,bits", [(1, (8, 1), 20), (3, (129, 7, 640), 30), (8, (33, 264, 16, 9), 40), (5, (2000, 3000), 62), (2, (100, 5, 77, 16, 40), 20)])
+def test_one_row_with_several_matrices(qtype, nb, widths, bits):
+    """Matrices that end in odd half-tiles, one behind the other in one launch (up to four; five take a launch each)."""
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(nb)
+    synth = o.synth_q4k if qtype == o.Q4_K else o.synth_q6k
+    raw = [synth(np.random.default_rng(i + nb), w, nb) for i, w in enumerate(widths)]
+    hs = [qk_cuda.register_weight(r, w, nb, qtype) for r, w in zip(raw, widths)]
+    device.read_flags()
+    x = rng.integers(-(1 << bits), 1 << bits, size=(1, nb * 256), dtype=np.int64)
+    got = qk_cuda.apply_resident_grouped(hs, x, widths, FW)
+    assert device.read_flags() == 0
+    for a, r, w in zip(got, raw, widths):
+        assert np.array_equal(a, onat.qk_linear(r, x, w, nb, FW, qtype))
+    qk_cuda.free_all()
+
+
 def test_results_share_no_memory():
     import gc
 
