@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.h"
 #include "mma_items.cuh"
@@ -81,8 +82,10 @@ __device__ __forceinline__ void ac_rotate(const AttnArgs &a, long long pos, int 
     x0 = y0; x1 = y1;
 }
 
-template <int HD>
+template <int HD, bool SHORT>                                      // SHORT: fa <= 16, exponentials and probabilities of 32-bit products
 __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnArgs a) {
+    using Exp = std::conditional_t<SHORT, SoftmaxExp16, SoftmaxExp>;
+    using Quotient = std::conditional_t<SHORT, SoftmaxQuotient16, SoftmaxQuotient>;
     pdl_enter();
     constexpr int QLD = HD + 16, HALF = HD / 2;
     extern __shared__ __align__(128) unsigned char ac_sm[];
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
     m_all = max(m_all, __shfl_xor_sync(0xffffffffu, m_all, 16));
     const long long above = __shfl_sync(0xffffffffu, m_all, g) - s_base[warp][g];      // from here on a lane has head g, keys 8t .. 8t + 7 of a tile
     // ---- pass 2: exponentials over the scores, their sum --------------------------------------------------------------------------
-    const SoftmaxExp exp2(a.fa, a.log2e, a.clip);
+    const Exp exp2(a.fa, a.log2e, a.clip);
     unsigned long long z = 0;
     for (int tile = first + warp; tile < end; tile += AC_WARPS) {
         int4 *e4 = reinterpret_cast<int4 *>(off + g * stride + (tile - first) * AC_TILE + 8 * t);
@@ -343,7 +346,7 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
         int e[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const int v = exp2(above - e[i]);
+            const int v = SHORT ? (int)exp2((uint32_t)min(above - e[i], a.clip)) : (int)exp2(above - e[i]);
             e[i] = i < left && g < rep ? v : 0;
             z += (unsigned)e[i];
         }
@@ -358,7 +361,7 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
     z_all += __shfl_xor_sync(0xffffffffu, z_all, 8);
     z_all += __shfl_xor_sync(0xffffffffu, z_all, 16);
     z = __shfl_sync(0xffffffffu, z_all, g);
-    const SoftmaxQuotient quotient(g < rep ? z : 0, a.fa);
+    const Quotient quotient(g < rep ? z : 0, a.fa);
     // ---- pass 3: probabilities floor(e 2^fa / z) as bytes, times the values --------------------------------------------------------
     long long sum[HD / 8][2];
 #pragma unroll
@@ -464,14 +467,14 @@ __global__ void __launch_bounds__(AC_THREADS, 2) attn_cluster_kernel(const AttnA
     cluster.sync();                                                         // nobody leaves while its sums are read
 }
 
-template <int HD>
+template <int HD, bool SHORT>
 cudaError_t launch_cluster(const AttnArgs &a_in, int n_c, int tiles, cudaStream_t s) {
     AttnArgs a = a_in;
     a.chunk = tiles;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_cluster_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ac_smem<HD>(AC_MAX_TILES));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_cluster_kernel<HD>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaError_t e = cudaFuncSetAttribute(attn_cluster_kernel<HD, SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ac_smem<HD>(AC_MAX_TILES));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_cluster_kernel<HD, SHORT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;
         configured = true;
     }
@@ -484,7 +487,7 @@ cudaError_t launch_cluster(const AttnArgs &a_in, int n_c, int tiles, cudaStream_
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)n_c; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_cluster_kernel<HD>, a);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_cluster_kernel<HD, SHORT>, a);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
@@ -514,7 +517,8 @@ bool attn_cluster_plan(const AttnArgs &a, int &n_c, int &tiles) {
 }
 
 cudaError_t launch_attn_cluster(const AttnArgs &a, int n_c, int tiles, cudaStream_t s) {
-    return a.hd == 128 ? launch_cluster<128>(a, n_c, tiles, s) : launch_cluster<64>(a, n_c, tiles, s);
+    if (a.fa <= 16) return a.hd == 128 ? launch_cluster<128, true>(a, n_c, tiles, s) : launch_cluster<64, true>(a, n_c, tiles, s);
+    return a.hd == 128 ? launch_cluster<128, false>(a, n_c, tiles, s) : launch_cluster<64, false>(a, n_c, tiles, s);
 }
 
 }  // namespace iie
