@@ -58,9 +58,9 @@ constexpr int TL_MINS = TL_MIN_SLOTS * 128 * 32;                   // are at mos
 constexpr int TL_EXCH = 16 * 128 * 8;                              // gate / up: sixteen columns of y on their way to the epilogue warps
 constexpr int TL_SMEM = 217 * 1024;
 constexpr int TL_MAX_GROUPS = 1024;
-// digit planes carried for `nl` digits in use, and columns of a tile: 32 only where the accumulators of three planes leave two
-// TMEM buffers and the registers of the read-out hold sixteen columns
-
+// Columns of a tile: 32 where the accumulators leave two TMEM buffers and the read-out's registers hold eight columns' sums: three planes, and up
+// to five of Q6_K, which has no minima (a weight is expanded half as often: a block of 2048 tokens, whose down projection has five digits,
+// 3208 -> 3050 us).
 struct TileMaps { CUtensorMap x16, x32, s16, s32; };               // planes and sums, boxes of 16 and of 32 rows
 
 // SPLIT: the CTAs of a cluster share the super-blocks of a tile (LINEAR; a form of its own: in one with the others it cost 2048 rows of a
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     }
     pdl_enter();                                                   // what stands above needs nothing of the kernel before
     const int np = tl_planes(a.x_nl ? max(1, min(8, *a.x_nl)) : 8), ns = np + 1;        // uniform over the grid
-    const bool wide = np == 3 && a.wide;
+    const bool wide = a.wide && (np == 3 || (!Q4 && np <= 5));
     const int bn = wide ? 32 : 16;
     // The expansion bounds a tile of sixteen columns: sixteen of the warps expand there, as long as eight can hold the sums of the
     // read-out (eight columns a thread) in their registers
@@ -329,7 +329,9 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
             }
         };
         using std::integral_constant;
-        if (np == 3 && wide) read_out(integral_constant<int, 3>{}, integral_constant<int, 32>{}, integral_constant<int, 8>{});
+        if (!Q4 && wide && np == 4) read_out(integral_constant<int, Q4 ? 3 : 4>{}, integral_constant<int, 32>{}, integral_constant<int, 8>{});
+        else if (!Q4 && wide && np == 5) read_out(integral_constant<int, Q4 ? 3 : 5>{}, integral_constant<int, 32>{}, integral_constant<int, 8>{});
+        else if (np == 3 && wide) read_out(integral_constant<int, 3>{}, integral_constant<int, 32>{}, integral_constant<int, 8>{});
         else if (np == 3) read_out(integral_constant<int, 3>{}, integral_constant<int, 16>{}, integral_constant<int, 8>{});
         else if (np == 4) read_out(integral_constant<int, 4>{}, integral_constant<int, 16>{}, integral_constant<int, 8>{});
         else if (np == 5) read_out(integral_constant<int, 5>{}, integral_constant<int, 16>{}, integral_constant<int, 8>{});
