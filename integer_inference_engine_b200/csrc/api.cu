@@ -10,6 +10,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "../../include/iie_qk.h"
@@ -56,6 +57,8 @@ std::vector<Weight> g_w;
 std::vector<MoeLayer> g_layers;
 cudaStream_t g_stream = nullptr;
 int *g_flags = nullptr;               // device flag word
+thread_local int *t_flags = nullptr;  // the word that takes its place for kernels this thread launches (a 1-bit host call's own, see set_flag_word)
+int *flag_word() { return t_flags ? t_flags : g_flags; }
 int *g_cells = nullptr;               // device ints: [0] limbs of h, [1] limbs of gate*up, [2] routing ticket
 const uint8_t **g_selptr = nullptr;   // device: [3][64] pointers of the experts the last routing selected
 int g_pdl = 1;                        // programmatic dependent launch between the decode kernels
@@ -598,8 +601,9 @@ int apply_resident_impl(long long h, const int64_t *x, long long T, int fw, int6
 namespace iie {
 int *shared_flag_word() {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
-    return init() ? g_flags : nullptr;
+    return init() ? flag_word() : nullptr;
 }
+int *set_flag_word(int *word) { return std::exchange(t_flags, word); }
 void restore_flag_bits(int bits) {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
     if (bits <= 0 || !init()) return;
@@ -1042,7 +1046,7 @@ extern "C" int iie_attn_decode_dev(const int64_t *q_dev, const int64_t *k_dev, c
     a.cos = cos_dev; a.sin = sin_dev; a.rope = rope; a.H = n_heads; a.Hkv = n_kv; a.hd = head_dim;
     attn_consts(a, fa, inv_sqrt);
     if (!attn_scratch(a, (cudaStream_t)stream)) return 1;
-    a.out = out_dev; a.flags = g_flags;
+    a.out = out_dev; a.flags = flag_word();
     const cudaError_t e = launch_attn_decode(a, (cudaStream_t)stream);
     if (e != cudaSuccess) { cudaGetLastError(); return 1; }
     return 0;
@@ -1061,7 +1065,7 @@ int iie::attn_decode_normed(const int64_t *q, const int64_t *k, const int64_t *v
     attn_consts(a, fa, inv_sqrt);
     if (!attn_scratch(a, s)) return 1;
     a.qgain = qgain; a.kgain = kgain; a.eps = eps; a.pdl = 1;
-    a.out = out; a.flags = g_flags;
+    a.out = out; a.flags = flag_word();
     const cudaError_t e = launch_attn_decode(a, s);
     if (e == cudaErrorNotSupported) return 3;
     if (e != cudaSuccess) { cudaGetLastError(); return 1; }
@@ -1081,7 +1085,7 @@ int iie::attn_decode_each(const int64_t *q, const int64_t *k, const int64_t *v, 
     a.q = q; a.k = k; a.v = v; a.kcache = kcache; a.vcache = vcache; a.pos = pos_max; a.Lmax = cache_rows;
     a.cos = cos; a.sin = sin; a.rope = rope; a.H = H; a.Hkv = Hkv; a.hd = hd;
     attn_consts(a, fa, inv_sqrt);
-    a.qgain = qgain; a.kgain = kgain; a.eps = eps; a.out = out; a.flags = g_flags;
+    a.qgain = qgain; a.kgain = kgain; a.eps = eps; a.out = out; a.flags = flag_word();
     int n_c = 0, tiles = 0;
     if (g_attn_fused != 1 || n_seqs > 65535 || pos_max >= cache_rows || !attn_shape_ok(H, Hkv, hd) || !attn_cluster_plan(a, n_c, tiles)) return 3;
     if (launch_attn_cluster(a, n_c, tiles, s) != cudaSuccess) { cudaGetLastError(); return 1; }
@@ -1113,7 +1117,7 @@ extern "C" int iie_attn_prefill_dev(const int64_t *q_dev, const int64_t *k_dev, 
         a.cos = cos_dev; a.sin = sin_dev; a.rope = rope; a.H = n_heads; a.Hkv = n_kv; a.hd = head_dim;
         attn_consts(a, fa, inv_sqrt);
         a.scores = scores; a.e = e; a.hmax = (long long *)st; a.Z = (unsigned long long *)(st + (size_t)slab * n_heads * 8);
-        a.out = out_dev + t0 * n_heads * head_dim; a.flags = g_flags;
+        a.out = out_dev + t0 * n_heads * head_dim; a.flags = flag_word();
         if (launch_attn_prefill(a, s) != cudaSuccess) { cudaGetLastError(); return 1; }
     }
     return 0;

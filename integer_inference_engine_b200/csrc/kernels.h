@@ -434,9 +434,12 @@ cudaError_t launch_q1_tc(const Q1Part *parts, int n_parts, bool sc32, long long 
 cudaError_t launch_rmsnorm_pair(const int64_t *x, long long rows_a, long long rows_b, long long width, const int64_t *gain_a,
                                 const int64_t *gain_b, int fa, unsigned long long eps, int64_t *out, int *flags, cudaStream_t s);
 bool attn_shape_ok(int n_heads, int n_kv, int head_dim);      // shapes launch_attn_decode accepts
-int *shared_flag_word();           // the library's device flag word, NULL without a device
+int *shared_flag_word();           // the library's device flag word (or the thread's own, see below), NULL without a device
+// Until the next call kernels that this thread launches through the attention and 1-bit entries raise their flags in `word` (null: in the
+// shared one); returns the word before.
+int *set_flag_word(int *word);
 constexpr int FLAG_GAVE_UP = 8;    // its bit 3: a bounded wait ran out and outputs were left out
-void restore_flag_bits(int bits);  // OR bits back into the flag word (flags an entry set aside while it ran)
+void restore_flag_bits(int bits);  // OR bits back into the shared flag word
 cudaError_t launch_q1_silu_mul(const int64_t *gate, const int64_t *up, long long n, int frac, int64_t *out, cudaStream_t s);
 cudaError_t launch_q1_embed_row(const uint8_t *units, bool sc32, long long nb, const int *row_dev, long long row_host, int64_t *out,
                                 cudaStream_t s);

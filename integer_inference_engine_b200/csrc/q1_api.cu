@@ -33,7 +33,7 @@ std::recursive_mutex q_mu;
 std::vector<Q1Weight> q_w;
 unsigned long long q_weight_bytes = 0;
 cudaStream_t q_stream = nullptr;
-int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [8..15] digits in use (a DigitRing)
+int *q_cells = nullptr;                 // device ints: [0] digits of a row, [1] rmsnorm flags, [2..3] largest scale of a matrix being registered, [4] flags of the host call under way, [8..15] digits in use (a DigitRing)
 int q_ready = -1;
 
 enum QRole { QR_X, QR_PLANES, QR_WORK, QR_KEYS, QR_VALUES, QR_LOGITS, QR_OUT, QR_GAIN, QR_COUNT };
@@ -791,24 +791,20 @@ long long padded_head_dim(long long hd) {
     return 0;
 }
 
-// Flags other callers left in the shared word are set aside while one of these entries runs and put back afterwards.
-// (Both ends on the stream, one wait at the second: the word as it was is kept in a cell meanwhile.)
+// The flags of one of these host calls are a word of its own: the shared word is read and cleared by other threads' calls, whose flags it
+// holds meanwhile.  Cleared and read on the stream, one wait.
 struct FlagScope {
+    int *const word = q_cells + 4, *const before;
     bool ok = false;
-    FlagScope() {
-        int *word = shared_flag_word();
-        ok = word && cudaMemcpyAsync(q_cells + 4, word, sizeof(int), cudaMemcpyDeviceToDevice, q_stream) == cudaSuccess &&
-             cudaMemsetAsync(word, 0, sizeof(int), q_stream) == cudaSuccess;
-    }
+    FlagScope() : before(iie::set_flag_word(word)) { ok = cudaMemsetAsync(word, 0, sizeof(int), q_stream) == cudaSuccess; }
+    ~FlagScope() { iie::set_flag_word(before); }
+    FlagScope(const FlagScope &) = delete;
+    FlagScope &operator=(const FlagScope &) = delete;
     int finish() {
-        int pageable[2] = {0, 0};
-        int *seen = staging() ? reinterpret_cast<int *>(q_stage) : pageable, *word = shared_flag_word();
+        int pageable = 0, *seen = staging() ? reinterpret_cast<int *>(q_stage) : &pageable;
         if (!ok || cudaMemcpyAsync(seen, word, sizeof(int), cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
-            cudaMemcpyAsync(seen + 1, q_cells + 4, sizeof(int), cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
-            cudaMemsetAsync(word, 0, sizeof(int), q_stream) != cudaSuccess || cudaStreamSynchronize(q_stream) != cudaSuccess) return -1;
-        const int f = seen[0], earlier = seen[1];
-        if (earlier > 0) iie::restore_flag_bits(earlier);
-        return f;
+            cudaStreamSynchronize(q_stream) != cudaSuccess) return -1;
+        return *seen;
     }
 };
 
@@ -990,8 +986,7 @@ extern "C" int bonsai_prefill_forward_gpu(const long long *x_embed, long long T,
     if (ok) {
         FlagScope scope;
         ok = scope.ok;
-        int *fw = iie::shared_flag_word();
-        ok = ok && fw;
+        int *const fw = scope.word;
         const int64_t *cosd = q_bufs[(size_t)cos_h].p, *sind = q_bufs[(size_t)sin_h].p;
         for (long long li = 0; ok && li < n_layers; li++) {
             ok = layer_rows(m, li, w, T, fw, [&](size_t layer) {
@@ -1091,8 +1086,7 @@ extern "C" int bonsai_decode_step(long long ctx_h, const long long *x_in, const 
     {
         FlagScope scope;
         ok = ok && scope.ok;
-        int *fw = iie::shared_flag_word();
-        ok = ok && fw;
+        int *const fw = scope.word;
         const int64_t *cosd = q_bufs[(size_t)m.cos_h].p, *sind = q_bufs[(size_t)m.sin_h].p;
         for (long long li = 0; ok && li < m.n_layers; li++) {
             int32_t *Kl = c.K + (size_t)li * c.B * per_seq, *Vl = c.V + (size_t)li * c.B * per_seq;

@@ -87,6 +87,56 @@ def test_decode_context_steps_sequences_at_their_own_positions(model):
     assert q1_gpu.decode_step(ctx, x, [5, 3], s["vocab"]) is None
 
 
+def test_flags_of_a_step_and_of_another_threads_products_stay_apart(model):
+    """Host-array products beyond eight digits find their own flag and are repeated exactly, however many steps of a 1-bit decode context
+    run in another thread, and no step is refused for a value that is not its own.  (Through the C interface: the Python bridges take turns.)"""
+    import threading
+    import time
+
+    from integer_inference_engine_b200 import device, q1_gpu, qk_cuda
+    from oracle import native as onat
+    g, w, gh, s, inv_sqrt = model
+    B, vocab = 8, 600000                                                # the last product runs on for a while after the call has issued it
+    rows = np.arange(vocab) % s["vocab"]
+    head = q1_gpu.q1_register_weight(np.ascontiguousarray(g["output_bits"][rows]), np.ascontiguousarray(g["output_scale_fp"][rows]))
+    dims = (B, s["layers"], s["H"], s["Hkv"], s["hd"], s["d"], s["dff"], vocab)
+    ctx = q1_gpu.decode_ctx_create(dims, {**w, "out_head": head, "out_head_vocab": vocab}, gh, FRAC, 1, inv_sqrt, 8)
+    full_k = np.stack([g["k0"], g["k1"]]); full_v = np.stack([g["v0"], g["v1"]])
+    for b in range(B):
+        assert q1_gpu.decode_ctx_seed_seq(ctx, b, full_k, full_v)
+    x0 = model_oracle.q1_rows(g["embed_bits"], g["embed_scale_fp"], int(g["token"]))
+    xs = np.repeat(x0, B, axis=0)
+    rng = np.random.default_rng(4)
+    raw = o.synth_q4k(rng, 16, 1)
+    h = qk_cuda.register_weight(raw, 16, 1, o.Q4_K)
+    wide = rng.integers(-(1 << 20), 1 << 20, size=(1, 256), dtype=np.int64)
+    wide[:, ::64] = np.iinfo(np.int64).max
+    want = onat.qk_linear(raw, wide, 16, 1, 24, o.Q4_K)
+    assert np.array_equal(qk_cuda.apply_resident(h, wide, 16, 24), want)
+    device.read_flags()
+    lib, y, logits, at = qk_cuda.load_library(), np.empty((1, 16), np.int64), np.empty((B, vocab), np.int64), np.full(B, 5, np.int64)
+    decode, product = q1_gpu.load_library().bonsai_decode_step, lib.qk_apply_resident
+    ends, wrong, steps = time.monotonic() + 3.0, [], []
+
+    def step():
+        while time.monotonic() < ends:
+            steps.append(decode(ctx, xs.ctypes.data, at.ctypes.data, logits.ctypes.data) == 0 and np.array_equal(logits[B - 1], g["logits"][0][rows]))
+
+    thread = threading.Thread(target=step)
+    thread.start()
+    products = 0
+    while time.monotonic() < ends:
+        wrong.append(product(h, wide.ctypes.data, 1, 24, y.ctypes.data) != 0 or not np.array_equal(y, want))
+        products += 1
+    thread.join()
+    assert products > 100 and len(steps) > 20
+    assert not any(wrong), f"{sum(wrong)} of {products} products lost their flag"
+    assert all(steps), f"{steps.count(False)} of {len(steps)} steps took another call's flag for their own"
+    assert device.read_flags() == 0
+    q1_gpu.decode_ctx_free(ctx)
+    qk_cuda.free_all()
+
+
 @pytest.mark.parametrize("vocab", (152597, 151680))
 def test_logits_of_a_large_vocabulary_leave_in_two_halves(model, golden_dir, vocab):
     """The recorded output matrix repeated: the halves meet where they should, and a refused step leaves the context usable."""
