@@ -102,7 +102,9 @@ int bonsai_prefill_forward_gpu(const long long *x_embed, long long T, long long 
 /* bonsai_q1_gpu.cu:3517,3565,3588,3649 - decode context of B sequences with device K/V of `cap` rows each: create
  * (handle >= 0 or -1), seed sequence b with the K/V rows of its prefill, one decode step for all sequences
  * (x_in [B][d] the new tokens' embedded rows, pos [B] each sequence's position = rows cached before the step,
- * out_logits [B][vocab], of which a step that ends with 4 may have written a part; 0 ok, 1 bad arguments / CUDA, 4 overflow), free. */
+ * out_logits [B][vocab], left alone by a step that ends with 4; 0 ok, 1 bad arguments / CUDA, 4 overflow), free.  A step that ends
+ * with 1 because the device failed while logits were on their way, or because a wait of the last product ran out, may have written a
+ * part of them. */
 long long bonsai_decode_ctx_create(long long B, long long n_layers, long long H, long long Hkv, long long hd, long long d,
                                    long long dff, long long cap, long long vocab, long long frac, long long eps,
                                    long long inv_sqrt, const long long *wq, const long long *wk, const long long *wv,

@@ -687,8 +687,9 @@ bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logi
 }
 
 // The same for a step's rows, the output matrix in two halves of whole waves where it is large: the first half's logits are on their way to
-// the host while the second is multiplied (7 MB take 130 us, the product of six rows 120).  `first`: rows of the first half, 0 for one piece;
-// its logits [rows][first] lie in front of the others'.
+// the host while the second is multiplied (7 MB take 130 us, the product of six rows 120), as long as nothing was refused: behind the first
+// half the flags say all that they will but whether a wait of the second product gave up.  `first`: rows of the first half, 0 for one
+// piece; its logits [rows][first] lie in front of the others'.
 cudaStream_t q_copy = nullptr;
 cudaEvent_t q_half = nullptr;
 long long head_first(const Q1Stack &m, long long rows) {
@@ -800,12 +801,12 @@ struct FlagScope {
     ~FlagScope() { iie::set_flag_word(before); }
     FlagScope(const FlagScope &) = delete;
     FlagScope &operator=(const FlagScope &) = delete;
-    int finish() {
+    int read(cudaStream_t s) const {                   // negative on a CUDA failure
         int pageable = 0, *seen = staging() ? reinterpret_cast<int *>(q_stage) : &pageable;
-        if (!ok || cudaMemcpyAsync(seen, word, sizeof(int), cudaMemcpyDeviceToHost, q_stream) != cudaSuccess ||
-            cudaStreamSynchronize(q_stream) != cudaSuccess) return -1;
+        if (!ok || cudaMemcpyAsync(seen, word, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return -1;
         return *seen;
     }
+    int finish() const { return read(q_stream); }
 };
 
 struct DecodeCtx {
@@ -1108,8 +1109,8 @@ extern "C" int bonsai_decode_step(long long ctx_h, const long long *x_in, const 
         }
         const long long first = ok ? head_first(m, c.B) : 0;
         if (first) {
-            ok = ok && head_halves(m, c.w.x, c.B, first, c.logits, fw) && cudaStreamWaitEvent(q_copy, q_half, 0) == cudaSuccess &&
-                 copy_half(out_logits, c.logits, c.B, c.vocab, 0, first, q_copy);
+            ok = head_halves(m, c.w.x, c.B, first, c.logits, fw) && cudaStreamWaitEvent(q_copy, q_half, 0) == cudaSuccess &&
+                 (scope.read(q_copy) != 0 || copy_half(out_logits, c.logits, c.B, c.vocab, 0, first, q_copy));
         } else ok = ok && head_rows(m, c.w.x, c.B, c.logits, fw);
         flags = scope.finish();
         ok = ok && flags >= 0 && !(flags & FLAG_GAVE_UP);

@@ -153,7 +153,9 @@ def test_logits_of_a_large_vocabulary_leave_in_two_halves(model, golden_dir, voc
     x0 = model_oracle.q1_rows(g["embed_bits"], g["embed_scale_fp"], int(g["token"]))
     bad = np.concatenate([x0, x0])
     bad[1, :2] = np.iinfo(np.int64).min
-    assert q1_gpu.decode_step(ctx, bad, [5, 5], vocab) is None
+    untouched, at = np.full((2, vocab), 7, np.int64), np.array([5, 5], np.int64)
+    assert q1_gpu.load_library().bonsai_decode_step(ctx, bad.ctypes.data, at.ctypes.data, untouched.ctypes.data) == 4
+    assert np.all(untouched == 7), "a refused step wrote logits"
     logits = q1_gpu.decode_step(ctx, np.concatenate([x0, x0]), [5, 5], vocab)
     for b in range(2):
         assert np.array_equal(logits[b], g["logits"][0][rows])
