@@ -1830,10 +1830,19 @@ extern "C" unsigned long long iie_workspace_generation(void) {
 
 extern "C" int iie_prefill_launch_counts(unsigned long long *out, int capacity) {
     if (!out || capacity < 7) return -1;                  // (seven entries are as old as the call)
-    unsigned long long counts[iie::TILE_SHAPES];
+    unsigned long long counts[iie::TILE_SHAPES + iie::TILE_FORMS];
     iie::tile_launch_counts(counts);
     const int n = std::min(capacity, iie::TILE_SHAPES);
     std::copy(counts, counts + n, out);
+    return n;
+}
+
+extern "C" int iie_tile_form_counts(unsigned long long *out, int capacity) {
+    if (!out || capacity < 1) return -1;
+    unsigned long long counts[iie::TILE_SHAPES + iie::TILE_FORMS];
+    iie::tile_launch_counts(counts);
+    const int n = std::min(capacity, iie::TILE_FORMS);
+    std::copy(counts + iie::TILE_SHAPES, counts + iie::TILE_SHAPES + n, out);
     return n;
 }
 

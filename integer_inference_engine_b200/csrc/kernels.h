@@ -228,7 +228,9 @@ size_t tile_sums_bytes(long long rows, long long n_blocks);
 // launches by tile shape since the library was loaded: Q4_K gate/up with 3 / 4 activation digits, Q6_K down with up to 5 / 6,
 // Q4_K down with up to 5, Q4_K linear with 3 / up to 5, all others (counted on the device, where the digits are known)
 constexpr int TILE_SHAPES = 8;
-void tile_launch_counts(unsigned long long *out);
+// ... and how many of the linear ones were shared by clusters
+constexpr int TILE_FORMS = 1;
+void tile_launch_counts(unsigned long long *out);      // [TILE_SHAPES + TILE_FORMS]
 
 // Re-order raw GGUF blocks into the half-tile layout; also reduces max |d| and max |dmin| half bit
 // patterns (sign stripped) into maxbits[0..1] (device memory, caller zeroes).

@@ -46,7 +46,9 @@ __device__ __forceinline__ uint32_t tl_remote(uint32_t a, int rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void tl_remote_store(uint32_t a, long long v) { asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }
+__device__ __forceinline__ void tl_remote_store(uint32_t a, i128 v) {
+    asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"((unsigned long long)v), "l"((unsigned long long)((u128)v >> 64)) : "memory");
+}
 __device__ __forceinline__ void tl_remote_arrive(uint32_t b) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(b) : "memory"); }
 static __device__ __noinline__ bool tl_wait_cluster(uint32_t b, uint32_t parity, volatile int *abort_flag) {       // bounded; the whole warp, one answer
     bool done = false;

@@ -43,7 +43,7 @@
 
 namespace iie {
 
-__device__ unsigned long long d_tile_launches[TILE_SHAPES];
+__device__ unsigned long long d_tile_launches[TILE_SHAPES + TILE_FORMS];
 
 namespace {
 
@@ -72,18 +72,15 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     constexpr int NROW = MODE == MODE_GATEUP ? 64 : 128;           // output rows of a tile
     extern __shared__ __align__(1024) unsigned char tl_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tl_raw) + 1023) & ~(uintptr_t)1023);
-    const int split = SPLIT ? a.split : 1;                         // CTAs of a cluster that share a tile's super-blocks
-    __shared__ __align__(8) uint64_t bars[2 * TL_MAX_STAGES + 8 + 2 * TL_MAX_RAW + 4];
+    __shared__ __align__(8) uint64_t bars[2 * TL_MAX_STAGES + 8 + 2 * TL_MAX_RAW + 3];
     __shared__ int s_first[TL_MAX_GROUPS + 1], s_off[TL_MAX_GROUPS + 1];       // first tile and first row of each group
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const uint32_t full_bar = tl_u32(bars), empty_bar = full_bar + 8 * TL_MAX_STAGES, acc_bar = empty_bar + 8 * TL_MAX_STAGES, free_bar = acc_bar + 8 * 4,
                    raw_full = free_bar + 8 * 4, raw_empty = raw_full + 8 * TL_MAX_RAW, y_full = raw_empty + 8 * TL_MAX_RAW, y_free = y_full + 8,
-                   x_full = y_free + 8, x_free = x_full + 8;
+                   x_full = y_free + 8;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int nb = a.nb, rank = SPLIT ? (int)(blockIdx.x & (split - 1)) : 0;
-    const int b_lo = nb * rank / split, b_hi = nb * (rank + 1) / split;        // super-blocks of this CTA
-    const int first_tile = SPLIT ? blockIdx.x / split : blockIdx.x, tile_step = SPLIT ? gridDim.x / split : gridDim.x;
+    const int nb = a.nb;
     if (warp == TL_X_WARP && lane == 0) {                          // the tensor maps' first use would wait for them
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x16)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x32)) : "memory");
@@ -96,8 +93,21 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     }
     pdl_enter();                                                   // what stands above needs nothing of the kernel before
     const int np = tl_planes(a.x_nl ? max(1, min(8, *a.x_nl)) : 8), ns = np + 1;        // uniform over the grid
-    const bool wide = a.wide && (np == 3 || (!Q4 && np <= 5));
+    const bool wide = a.wide && (np == 3 || (!Q4 && np <= (SPLIT ? 4 : 5)));      // (five digits beside the exchange: one stage)
     const int bn = wide ? 32 : 16;
+    const int n_rt = (int)((a.out_f + NROW - 1) / NROW);
+    // CTAs that share a tile's super-blocks: those of a cluster, or of a half of it and so on where more digits than expected make the tiles
+    // narrower and twice as many, so that no CTA walks two
+    int split = SPLIT ? a.split : 1;
+    if (SPLIT) while (split > 1 && (long long)split * ((a.n_rows + bn - 1) / bn) * n_rt > gridDim.x) split >>= 1;
+    const int rank = SPLIT ? (int)(blockIdx.x & (split - 1)) : 0;
+    // kept in shared memory: in registers they would push sums of the read-out out of theirs
+    __shared__ int s_share[5];
+    if (SPLIT && tid == 0) { s_share[0] = __ffs(split) - 1; s_share[1] = rank; s_share[2] = nb * rank / split; s_share[3] = nb * (rank + 1) / split; s_share[4] = (int)(blockIdx.x & (a.split - 1)) - rank; }
+    auto share = [&](int i) { return *const_cast<const volatile int *>(&s_share[i]); };
+    auto b_lo = [&] { return SPLIT ? share(2) : 0; };              // super-blocks of this CTA
+    auto b_hi = [&] { return SPLIT ? share(3) : nb; };
+    auto first_tile = [&] { return SPLIT ? (int)blockIdx.x >> share(0) : (int)blockIdx.x; };
     // The expansion bounds a tile of sixteen columns: sixteen of the warps expand there, as long as eight can hold the sums of the
     // read-out (eight columns a thread) in their registers
     const int n_read = wide || np > 5 ? 16 : 8, n_expand = TL_WORK - n_read;
@@ -107,12 +117,11 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     const int x_bytes = np * bn * 128, s_bytes = Q4 ? ns * bn * 32 : 0;
     const int stage_bytes = (TL_A_BYTES + x_bytes + s_bytes + 1023) & ~1023;
     constexpr int FIXED = 1024 + (Q4 ? TL_MINS : 0) + (MODE == MODE_GATEUP ? TL_EXCH : 0);
-    const int xch_bytes = SPLIT ? 128 * bn * ((np + 2) / 2) * 8 : 0;       // split tiles: sums of this CTA's share of the columns
+    const int xch_bytes = SPLIT && split > 1 ? 128 * bn * 16 : 0;              // split tiles: sums of this CTA's share of the columns
     const int raw_slots = FIXED + xch_bytes + 3 * stage_bytes + TL_MAX_RAW * RAW_BYTES <= TL_SMEM ? TL_MAX_RAW : 2;
     const int stages = min(TL_MAX_STAGES, (TL_SMEM - FIXED - xch_bytes - raw_slots * RAW_BYTES) / stage_bytes);
     unsigned char *mins = smem + stages * stage_bytes, *exch = mins + (Q4 ? TL_MINS : 0), *raw = exch + (MODE == MODE_GATEUP ? TL_EXCH : xch_bytes);
 
-    const int n_rt = (int)((a.out_f + NROW - 1) / NROW);
     if (warp == 0) {                                               // first tile of every group
         int base = 0;
         for (int g0 = 0; g0 < a.n_groups; g0 += 32) {
@@ -133,21 +142,23 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         for (int s = 0; s < TL_MAX_STAGES; s++) { tl_init(full_bar + 8 * s, n_expand + 1); tl_init(empty_bar + 8 * s, 1); }
         for (int s = 0; s < 4; s++) { tl_init(acc_bar + 8 * s, 1); tl_init(free_bar + 8 * s, n_read); }
         tl_init(y_full, n_read); tl_init(y_free, TL_EPI);
-        tl_init(x_full, split * n_read); tl_init(x_free, split * n_read);
+        tl_init(x_full, split * n_read);
         for (int s = 0; s < TL_MAX_RAW; s++) { tl_init(raw_full + 8 * s, 1); tl_init(raw_empty + 8 * s, TL_WORK); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         if (blockIdx.x == 0) {                                     // which tile shape ran (launch statistics)
             const int shape = Q4 && MODE == MODE_GATEUP ? (np == 3 ? 0 : np == 4 ? 1 : 7) : !Q4 && MODE == MODE_DOWN ? (np <= 5 ? 2 : np == 6 ? 3 : 7)
                               : Q4 && MODE == MODE_DOWN ? (np <= 5 ? 4 : 7) : Q4 && MODE == MODE_LINEAR ? (np == 3 ? 5 : np <= 5 ? 6 : 7) : 7;
             atomicAdd(&d_tile_launches[shape], 1ULL);
+            if (SPLIT && split > 1) atomicAdd(&d_tile_launches[TILE_SHAPES], 1ULL);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (SPLIT) tl_cluster_sync();                              // the other CTAs' barriers stand
+    if (SPLIT && split > 1) tl_cluster_sync();                     // the other CTAs' barriers stand
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
     const int n_tiles = s_first[a.n_groups];
+    auto next = [&](int tile) { return SPLIT ? n_tiles : tile + (int)gridDim.x; };       // (shared tiles: one per CTA)
 
     // tile -> group, row tile, first and past-the-last activation row
     struct Where { int g, rt, m0, m_end; };
@@ -181,9 +192,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
             TlRing rs, buf;
             uint32_t y_pass = 0;
             bool y_used = false;
-            uint32_t x_pass = 0;
-            bool x_used = false;
-            for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
+            for (int tile = first_tile(); tile < n_tiles; tile = next(tile)) {
                 const Where w = locate(tile);
                 long long L[NLV][TPW];
 #pragma unroll
@@ -191,7 +200,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
 #pragma unroll
                     for (int j = 0; j < TPW; j++) L[i][j] = 0;
                 bool ok = true;
-                for (int b = b_lo; b < b_hi; b++) {
+                for (int b = b_lo(); b < b_hi(); b++) {
                     if (!(ok = tl_wait(raw_full + 8 * rs.slot, rs.pass, &s_abort))) break;
                     const unsigned char *meta = raw + rs.slot * RAW_BYTES + meta_off;
                     int d, dm = 0;
@@ -251,41 +260,32 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
                 if (!ok) break;
                 // ---- y = floor(V / 2^fw), then what the product is for ---------------------------------------
                 const int sh = a.fw + (Q4 && !THIRDS ? 4 : 0);
-                if (SPLIT) {
-                    // column c of the tile belongs to CTA c mod split, as its column c / split there: everybody's sums go to the owner,
-                    // which adds them up, joins the digits and stores
-                    const int cols = BN / split;                   // of this CTA
-                    const uint32_t here = tl_u32(exch);
-                    if (x_used && !(ok = tl_wait_cluster(x_free, x_pass ^ 1, &s_abort))) break;
+                if (SPLIT && share(0) > 0) {
+                    // column c of the tile belongs to CTA c mod split, as its column c / split there: everybody's sums go to the owner in 128
+                    // bits, which adds them up and stores
 #pragma unroll
                     for (int j = 0; j < TPW; j++) {
-                        const int c = cg * TPW + j, slot = c / split;
-                        const uint32_t to = tl_remote(here + (uint32_t)((((rank * cols + slot) * NLV) * 128 + rowt) * 8), c & (split - 1));
+                        const int c = cg * TPW + j, ls = share(0);
+                        i128 v = L[NLV - 1][j];
 #pragma unroll
-                        for (int i = 0; i < NLV; i++) tl_remote_store(to + i * 1024, L[i][j]);
+                        for (int i = NLV - 2; i >= 0; i--) v = (v << 16) + (i128)L[i][j];
+                        tl_remote_store(tl_remote(tl_u32(exch) + (uint32_t)((share(1) * (BN >> ls) + (c >> ls)) * 128 + rowt) * 16, share(4) + (c & ((1 << ls) - 1))), v);
                     }
                     asm volatile("fence.acq_rel.cluster;" ::: "memory");
                     __syncwarp();
-                    if (lane < split) tl_remote_arrive(tl_remote(x_full, lane));
-                    if (!(ok = tl_wait_cluster(x_full, x_pass, &s_abort))) break;
+                    const int ls = share(0), split = 1 << ls, cols = BN >> ls;   // columns of this CTA
+                    if (lane < split) tl_remote_arrive(tl_remote(x_full, share(4) + lane));
+                    if (!(ok = tl_wait_cluster(x_full, 0, &s_abort))) break;      // (one tile per CTA: the barrier's only phase)
                     const long long row = (long long)w.rt * 128 + rowt;
+#pragma unroll 1                                                   // (unrolled, these two cost the whole read-out registers)
                     for (int slot = cg; slot < cols; slot += n_read / 4) {
-                        long long S[NLV];
-#pragma unroll
-                        for (int i = 0; i < NLV; i++) S[i] = 0;
-                        const long long *from = reinterpret_cast<const long long *>(exch) + slot * NLV * 128 + rowt;
-                        for (int k = 0; k < split; k++, from += cols * NLV * 128)
-#pragma unroll
-                            for (int i = 0; i < NLV; i++) S[i] += from[i * 128];
-                        i128 v = S[NLV - 1];
-#pragma unroll
-                        for (int i = NLV - 2; i >= 0; i--) v = (v << 16) + (i128)S[i];
-                        const int colx = w.m0 + slot * split + rank;
+                        const ulonglong2 *from = reinterpret_cast<const ulonglong2 *>(exch) + slot * 128 + rowt;
+                        i128 v = 0;
+#pragma unroll 1
+                        for (int k = 0; k < split; k++, from += cols * 128) { const ulonglong2 p = *from; v += (i128)(((u128)p.y << 64) | p.x); }
+                        const int colx = w.m0 + slot * split + share(1);
                         if (row < a.out_f && colx < w.m_end) a.out[(long long)colx * a.out_f + row] = (long long)(v >> sh);
                     }
-                    __syncwarp();
-                    if (lane < split) tl_remote_arrive(tl_remote(x_free, lane));
-                    x_used = true; x_pass ^= 1;
                     continue;
                 }
                 long long y[TPW];
@@ -354,8 +354,8 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         TlRing rs, st;
         int n_mins = 0;
         bool ok = true;
-        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
-            for (int b = b_lo; b < b_hi && ok; b++) {
+        for (int tile = first_tile(); tile < n_tiles && ok; tile = next(tile)) {
+            for (int b = b_lo(); b < b_hi() && ok; b++) {
                 if (!(ok = tl_wait(raw_full + 8 * rs.slot, rs.pass, &s_abort))) break;
                 const unsigned char *slot = raw + rs.slot * RAW_BYTES;
 #pragma unroll
@@ -458,8 +458,8 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         TlRing st, buf;
         int n_mins = 0;
         bool ok = true;
-        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step)
-            for (int b = b_lo; b < b_hi && ok; b++) {
+        for (int tile = first_tile(); tile < n_tiles && ok; tile = next(tile))
+            for (int b = b_lo(); b < b_hi() && ok; b++) {
                 if (buf.lapped && !(ok = tl_wait(free_bar + 8 * buf.slot, buf.pass ^ 1, &s_abort))) break;
                 const uint32_t d = tmem + buf.slot * buf_cols;
                 for (int p = 0; p < 2; p++) {
@@ -499,9 +499,9 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
             const CUtensorMap *xm = wide ? &maps.x32 : &maps.x16, *sm = wide ? &maps.s32 : &maps.s16;
             TlRing st;
             bool ok = true;
-            for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
+            for (int tile = first_tile(); tile < n_tiles && ok; tile = next(tile)) {
                 const Where w = locate(tile);
-                for (int c = 2 * b_lo; c < 2 * b_hi; c++) {
+                for (int c = 2 * b_lo(); c < 2 * b_hi(); c++) {
                     const uint32_t eb = empty_bar + 8 * st.slot, fb = full_bar + 8 * st.slot;
                     if (st.lapped && !(ok = tl_try(eb, st.pass ^ 1) || tl_wait_slow(eb, st.pass ^ 1, &s_abort))) break;
                     const uint32_t dst = tl_u32(smem + st.slot * stage_bytes + TL_A_BYTES);
@@ -520,12 +520,12 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         // ================= packed weights: one super-block of the tile's 16 half-tiles per slot ===============
         TlRing rs;
         bool ok = true;
-        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
+        for (int tile = first_tile(); tile < n_tiles && ok; tile = next(tile)) {
             const Where w = locate(tile);
             const uint8_t *src = nullptr;
             const bool live = lane < 16 && unit_of(w, lane, src);
             const int n_live = __popc(__ballot_sync(0xffffffffu, live));
-            for (int b = b_lo; b < b_hi; b++) {
+            for (int b = b_lo(); b < b_hi(); b++) {
                 const uint32_t eb = raw_empty + 8 * rs.slot, fb = raw_full + 8 * rs.slot;
                 if (rs.lapped && !(ok = tl_wait(eb, rs.pass ^ 1, &s_abort))) break;
                 if (lane == 0) tl_expect(fb, n_live * HTB);
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         int nl_max = 0;
         uint32_t pass = 0;
         bool ok = true;
-        for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
+        for (int tile = first_tile(); tile < n_tiles && ok; tile = next(tile)) {
             const Where w = locate(tile);
             const long long row = (long long)w.rt * 64 + r;
             for (int q = 0; q < bn / 4; q += 4) {                  // wide: columns 8 g + q + (0..3) of column group g = 0..3
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         }
     }
     __syncthreads();
-    if (SPLIT) tl_cluster_sync();                              // nobody leaves while another CTA stores or arrives here
+    if (SPLIT && share(0) > 0) tl_cluster_sync();                  // nobody leaves while another CTA stores or arrives here
     if (warp == TL_MMA_WARP) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -665,14 +665,19 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
     // sixteen columns while a group has few rows: a 32-column tile would multiply mostly padding
     a.wide = a.n_rows > 12LL * a.n_groups && a.n_rows > 16;
     // A matrix of few tiles: clusters of CTAs share a tile's super-blocks, as long as all clusters fit on the device at once (one CTA per
-    // SM; 33 clusters of four, 15 of eight).  A super-block is 1.3 to 1.7 us of a tile's walk, the exchange of the sums 3: a call of 7 rows
-    // 128 x 2048 19.8 -> 14.7 us, 5120 x 2048 20.6 -> 19.1, 2048 x 4096 31.3 -> 19.4; of 64 rows 24.7 -> 17.1, 28.0 (not split), 39.4 -> 25.6.
-    // (16 clusters of eight for the last but one: two waves, 28.4.)
+    // SM; 33 clusters of four, 15 of eight) and the walk gets shorter by more than the clusters cost.  A super-block is 1.2 to 1.7 us of a
+    // tile's walk; the launch of clusters and the exchange are 3.5 us (Q4_K) to 5.  Q4_K, 7 rows: 128 x 2048 19.8 -> 13 us, 5120 x 2048 20.2
+    // -> 16.9, 2048 x 4096 30.4 -> 16.9, three super-blocks saved 1024 x 1024 14.8 -> 12.9, one saved 2048 x 768 13.6 -> 14.9; 64 rows: 2048 x
+    // 2048 23.2 -> 19.4, 2048 x 4096 36.2 -> 23.4.  Q6_K, 7 rows: 5120 x 2048 (four saved) 17.9 -> 16.5, 1024 x 1024 (three) 12.6 -> 12.3; 64 rows:
+    // 2048 x 2048 21.3 -> 18.0, 100 rows (four) 22.7 -> 21.5.  With more digits than three the tiles of 17 rows and more are narrower, and half as
+    // many CTAs share one: that is 10 % and more faster, too (Q4_K 2048 x 4096, 64 rows, four digits 35.2 -> 27.9), or as fast but for Q6_K of
+    // five digits and more where nobody shares (4096 x 4096, 40 rows 31.2 -> 33.9 us, and 20.1 -> 22.5 were four saved enough).
     a.split = 1;
+    const bool q4 = qtype == QT_Q4K;
     const long long whole = ((a.n_rows + (a.wide ? 31 : 15)) / (a.wide ? 32 : 16)) * ((a.out_f + 127) / 128);
     while (mode == MODE_LINEAR && a.split < 8 && 2 * a.split <= a.nb && whole <= (a.split == 1 ? 74 : a.split == 2 ? 33 : 15)) a.split *= 2;
+    if (a.nb - (a.nb + a.split - 1) / a.split < (q4 ? 3 : a.wide ? 6 : 4)) a.split = 1;
     const int stride = (a.nb * 8 + 31) / 32 * 32;
-    const bool q4 = qtype == QT_Q4K;
     if ((q4 && !a.xs_ready) || a.xidx) {
         const long long n = a.n_rows * stride;
         launch_behind(tile_rows_kernel, (unsigned)((n + 255) / 256), 256, 0, s, a.xl, a.xidx, a.grp_off ? a.grp_off + a.n_groups : nullptr, a.x_nl, a.n_rows, a.nb, stride, a.xg, q4 ? a.xs : nullptr);
@@ -700,9 +705,9 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
 }
 
 void tile_launch_counts(unsigned long long *out) {
-    if (cudaMemcpyFromSymbol(out, d_tile_launches, sizeof(unsigned long long) * TILE_SHAPES) != cudaSuccess) {
+    if (cudaMemcpyFromSymbol(out, d_tile_launches, sizeof(unsigned long long) * (TILE_SHAPES + TILE_FORMS)) != cudaSuccess) {
         cudaGetLastError();
-        for (int i = 0; i < TILE_SHAPES; i++) out[i] = 0;
+        for (int i = 0; i < TILE_SHAPES + TILE_FORMS; i++) out[i] = 0;
     }
 }
 

@@ -349,6 +349,13 @@ def prefill_launch_counts() -> list:
     return [int(buf[i]) for i in range(n)]
 
 
+def tile_form_counts() -> list:
+    """Of those launches: [linear products whose tiles were shared by clusters]."""
+    buf = (ctypes.c_uint64 * 8)()
+    n = qk_cuda.load_library().iie_tile_form_counts(buf, 8)
+    return [int(buf[i]) for i in range(n)]
+
+
 def launch_count() -> int:
     """Kernels launched by the library since it was loaded."""
     return int(qk_cuda.load_library().iie_launch_count())

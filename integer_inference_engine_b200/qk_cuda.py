@@ -93,7 +93,8 @@ def _signatures():
         "iie_decoder_create": ([c_int, c_int, c_int, c_int, i64, i64, c_int, c_int, u64, i64, vp, vp], i64),
         "iie_decoder_set_layer": ([i64, c_int, i64, i64, i64, i64, vp, vp, c_int], c_int),
         "iie_decoder_step_dev": ([i64, vp, i64, vp, vp, vp, vp], c_int), "iie_decoder_destroy": ([i64], None),
-        "iie_prefill_launch_counts": ([ctypes.POINTER(ctypes.c_uint64), c_int], c_int), "iie_workspace_generation": ([], u64),
+        "iie_prefill_launch_counts": ([ctypes.POINTER(ctypes.c_uint64), c_int], c_int), "iie_tile_form_counts": ([ctypes.POINTER(ctypes.c_uint64), c_int], c_int),
+        "iie_workspace_generation": ([], u64),
         "iie_attn_decode_batch_rows_dev": ([vp, vp, vp, vp, vp, i64, i64, i64, i64, i64, i64, vp, vp, c_int, c_int, c_int, c_int, i64, c_int, i64, vp, vp], c_int),
         "iie_attn_decode_batch_dev": ([vp, vp, vp, vp, vp, i64, i64, i64, i64, vp, vp, c_int, c_int, c_int, c_int, i64, c_int, i64, vp, vp], c_int),
         "iie_attn_block_dev": ([i64, i64, vp, vp, vp, i64, vp, i64, vp, vp, c_int, c_int, c_int, c_int, i64, c_int, c_int, i64, vp], c_int),

@@ -64,6 +64,28 @@ def test_tiles_shared_by_clusters_match_the_oracle(qtype, out_f, nb, T, xbits):
     assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, qtype))
 
 
+@pytest.mark.parametrize("qtype,out_f,nb,T,xbits,shared", [
+    # the border in super-blocks saved, rows up to sixteen and above; the least and the most tiles that clusters share
+    (o.Q4_K, 640, 2, 5, 22, 0), (o.Q4_K, 2048, 3, 5, 22, 0), (o.Q4_K, 1024, 4, 9, 22, 1), (o.Q4_K, 9472, 6, 16, 22, 1), (o.Q4_K, 9473, 6, 16, 22, 0), (o.Q4_K, 300, 3, 33, 22, 0),
+    (o.Q6_K, 640, 2, 5, 22, 0), (o.Q6_K, 1024, 4, 9, 22, 0), (o.Q6_K, 200, 6, 2, 22, 1), (o.Q6_K, 9000, 8, 4, 22, 1), (o.Q6_K, 200, 8, 33, 22, 1), (o.Q6_K, 2048, 8, 100, 22, 0),
+    # more digits than three: half of a cluster to a tile, or nobody shares; the wide Q6_K tiles of four digits, sixteen columns from five on
+    (o.Q4_K, 1100, 8, 40, 30, 1), (o.Q4_K, 1100, 8, 40, 62, 1), (o.Q4_K, 4096, 8, 40, 30, 0), (o.Q6_K, 1100, 8, 40, 30, 1), (o.Q6_K, 1100, 8, 40, 38, 1), (o.Q6_K, 4090, 13, 40, 38, 0)])
+def test_tiles_that_clusters_share(qtype, out_f, nb, T, xbits, shared):
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(out_f + nb * 3 + T)
+    raw = np.frombuffer((o.synth_q4k if qtype == o.Q4_K else o.synth_q6k)(rng, out_f, nb), np.uint8).tobytes()
+    x = rng.integers(-(1 << xbits), 1 << xbits, size=(T, nb * 256), dtype=np.int64)
+    device.read_flags()
+    h = qk_cuda.register_weight(raw, out_f, nb, qtype)
+    before = device.tile_form_counts()
+    got = device.apply(h, torch.from_numpy(x).cuda(), out_f, FW).cpu().numpy()
+    assert device.tile_form_counts()[0] - before[0] == shared
+    assert device.read_flags() == 0
+    assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, qtype))
+
+
 @pytest.mark.parametrize("down_q", [o.Q4_K, o.Q6_K])
 @pytest.mark.parametrize("d,eff,E,k,T,mult", [(256, 256, 5, 2, 3, 1), (512, 256, 40, 1, 2, 1), (768, 512, 6, 3, 70, 1), (256, 768, 3, 3, 33, 200), (2304, 256, 24, 4, 48, 1),
                                                  (768, 512, 40, 2, 90, 200), (512, 256, 17, 2, 9, 20000)])
