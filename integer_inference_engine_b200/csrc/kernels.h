@@ -216,7 +216,7 @@ struct TileArgs {
     const int64_t *gates;          // DOWN: per pair
     const int *pair_tok;           // DOWN: pair -> token row, or nullptr (identity)
     int *flags;                    // bit 0 digit envelope, bit 3 a wait gave up
-    int wide, split;               // filled in by the launcher
+    int wide, split;               // filled in by the launcher: 1 tiles of 32 columns at three digits, 2 also of Q6_K at four and five; CTAs of a cluster
     long long sig_log2e, sig_clip;
     unsigned long long *counts;    // launches by tile shape (device)
     int xs_ready;                  // xs holds the sums (without xidx)
@@ -228,8 +228,8 @@ size_t tile_sums_bytes(long long rows, long long n_blocks);
 // launches by tile shape since the library was loaded: Q4_K gate/up with 3 / 4 activation digits, Q6_K down with up to 5 / 6,
 // Q4_K down with up to 5, Q4_K linear with 3 / up to 5, all others (counted on the device, where the digits are known)
 constexpr int TILE_SHAPES = 8;
-// ... and how many of the linear ones were shared by clusters
-constexpr int TILE_FORMS = 1;
+// ... and how many of the linear ones were shared by clusters, how many had 32 columns at four or five digits
+constexpr int TILE_FORMS = 2;
 void tile_launch_counts(unsigned long long *out);      // [TILE_SHAPES + TILE_FORMS]
 
 // Re-order raw GGUF blocks into the half-tile layout; also reduces max |d| and max |dmin| half bit

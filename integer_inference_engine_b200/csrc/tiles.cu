@@ -58,9 +58,6 @@ constexpr int TL_MINS = TL_MIN_SLOTS * 128 * 32;                   // are at mos
 constexpr int TL_EXCH = 16 * 128 * 8;                              // gate / up: sixteen columns of y on their way to the epilogue warps
 constexpr int TL_SMEM = 217 * 1024;
 constexpr int TL_MAX_GROUPS = 1024;
-// Columns of a tile: 32 where the accumulators leave two TMEM buffers and the read-out's registers hold eight columns' sums: three planes, and up
-// to five of Q6_K, which has no minima (a weight is expanded half as often: a block of 2048 tokens, whose down projection has five digits,
-// 3208 -> 3050 us).
 struct TileMaps { CUtensorMap x16, x32, s16, s32; };               // planes and sums, boxes of 16 and of 32 rows
 
 // SPLIT: the CTAs of a cluster share the super-blocks of a tile (LINEAR; a form of its own: in one with the others it cost 2048 rows of a
@@ -93,7 +90,10 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
     }
     pdl_enter();                                                   // what stands above needs nothing of the kernel before
     const int np = tl_planes(a.x_nl ? max(1, min(8, *a.x_nl)) : 8), ns = np + 1;        // uniform over the grid
-    const bool wide = a.wide && (np == 3 || (!Q4 && np <= (SPLIT ? 4 : 5)));      // (five digits beside the exchange: one stage)
+    const bool wide = a.wide && (np == 3 || (!Q4 && (SPLIT ? np == 4 : a.wide == 2 && np <= 5)));      // (five digits beside the exchange: one stage)
+    // Columns of a tile: 32 where the accumulators leave two TMEM buffers and the read-out's registers hold eight columns' sums: three planes, and
+    // up to five of Q6_K, which has no minima (a weight is expanded half as often: a block of 2048 tokens, whose down projection has five digits,
+    // 3208 -> 3050 us).
     const int bn = wide ? 32 : 16;
     const int n_rt = (int)((a.out_f + NROW - 1) / NROW);
     // CTAs that share a tile's super-blocks: those of a cluster, or of a half of it and so on where more digits than expected make the tiles
@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
                               : Q4 && MODE == MODE_DOWN ? (np <= 5 ? 4 : 7) : Q4 && MODE == MODE_LINEAR ? (np == 3 ? 5 : np <= 5 ? 6 : 7) : 7;
             atomicAdd(&d_tile_launches[shape], 1ULL);
             if (SPLIT && split > 1) atomicAdd(&d_tile_launches[TILE_SHAPES], 1ULL);
+            if (wide && np > 3) atomicAdd(&d_tile_launches[TILE_SHAPES + 1], 1ULL);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -662,8 +663,12 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
     if (qtype != QT_Q4K && !(qtype == QT_Q6K && mode != MODE_GATEUP)) return cudaErrorNotSupported;
     if (qtype == QT_Q4K && !a.xs) return cudaErrorInvalidValue;
     a.sig_log2e = sigmoid_log2e(a.fa); a.sig_clip = sigmoid_clip(a.fa);
-    // sixteen columns while a group has few rows: a 32-column tile would multiply mostly padding
+    // Sixteen columns while a group has few rows: a 32-column tile would multiply mostly padding.  A 32-column tile of four and five digits takes
+    // a fifth longer than one of sixteen, so it also wants more narrow tiles than one wave (Q6_K, five digits: 5120 x 2048, 33 rows, 120 narrow
+    // tiles 19.8 us against 24.0; 64 rows, 160 narrow tiles 33.8 against 25.4; 9216 x 4096, 100 rows 104 against 72.5) and groups that fill more
+    // than one (blocks of 128 experts with 14 / 16 / 20 / 24 / 32 rows each 410 / 427 / 469 / 516 / 620 us narrow, 415 / 434 / 475 / 508 / 605 wide).
     a.wide = a.n_rows > 12LL * a.n_groups && a.n_rows > 16;
+    if (a.wide && a.n_rows > (a.grp_off ? 20LL * a.n_groups : 0) && (a.n_rows + 15) / 16 * ((a.out_f + 127) / 128) > 148) a.wide = 2;
     // A matrix of few tiles: clusters of CTAs share a tile's super-blocks, as long as all clusters fit on the device at once (one CTA per
     // SM; 33 clusters of four, 15 of eight) and the walk gets shorter by more than the clusters cost.  A super-block is 1.2 to 1.7 us of a
     // tile's walk; the launch of clusters and the exchange are 3.5 us (Q4_K) to 5.  Q4_K, 7 rows: 128 x 2048 19.8 -> 13 us, 5120 x 2048 20.2

@@ -64,6 +64,25 @@ def test_tiles_shared_by_clusters_match_the_oracle(qtype, out_f, nb, T, xbits):
     assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, qtype))
 
 
+@pytest.mark.parametrize("out_f,nb,T,xbits", [(4700, 3, 47, 30), (4700, 3, 47, 38), (6200, 3, 49, 30), (6200, 5, 49, 38), (2500, 8, 130, 30), (2500, 9, 130, 38)])
+def test_narrow_and_wide_tiles_of_four_and_five_digits(out_f, nb, T, xbits):
+    """Q6_K rows of four and five digits on either side of a wave of narrow tiles, over several super-blocks."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(out_f + nb + T)
+    raw = o.synth_q6k(rng, out_f, nb)
+    x = rng.integers(-(1 << xbits), 1 << xbits, size=(T, nb * 256), dtype=np.int64)
+    device.read_flags()
+    h = qk_cuda.register_weight(raw, out_f, nb, o.Q6_K)
+    before = device.tile_form_counts()
+    got = device.apply(h, torch.from_numpy(x).cuda(), out_f, FW).cpu().numpy()
+    wide = (T + 15) // 16 * ((out_f + 127) // 128) > 148
+    assert [b - a for a, b in zip(before, device.tile_form_counts())][1] == wide
+    assert device.read_flags() == 0
+    assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, o.Q6_K))
+
+
 @pytest.mark.parametrize("qtype,out_f,nb,T,xbits,shared", [
     # the border in super-blocks saved, rows up to sixteen and above; the least and the most tiles that clusters share
     (o.Q4_K, 640, 2, 5, 22, 0), (o.Q4_K, 2048, 3, 5, 22, 0), (o.Q4_K, 1024, 4, 9, 22, 1), (o.Q4_K, 9472, 6, 16, 22, 1), (o.Q4_K, 9473, 6, 16, 22, 0), (o.Q4_K, 300, 3, 33, 22, 0),
