@@ -298,7 +298,7 @@ unsigned long long iie_launch_count(void);
  * written (capacity, eight at most), or -1 when capacity is below seven. */
 int iie_prefill_launch_counts(unsigned long long *out, int capacity);
 /* Among them, by form: out[0] = linear products whose tiles were shared by clusters, out[1] = Q6_K tiles of 32 columns at four or
- * five digits.  Returns the number of entries written. */
+ * five digits, out[2] = gate/up by tiles of eight rows.  Returns the number of entries written. */
 int iie_tile_form_counts(unsigned long long *out, int capacity);
 /* Workspace generation: changes whenever a scratch buffer of the library is freed (to grow, by
  * qk_moe_workspace_release or qk_free_all).  A CUDA graph captured over iie_*_dev calls holds the scratch addresses of

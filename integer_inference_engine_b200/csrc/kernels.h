@@ -220,7 +220,8 @@ struct TileArgs {
     long long sig_log2e, sig_clip;
     unsigned long long *counts;    // launches by tile shape (device)
     int xs_ready;                  // xs holds the sums (without xidx)
-    int few;                       // GATEUP of Q4_K: the tiles of eight rows (tiles_few.cu)
+    int few;                       // GATEUP of Q4_K: the tiles of eight rows (tiles_few.cu); 2 (the launcher): as the groups have it, beside tiles of sixteen
+    int *form;                     // ... what they have (1 of sixteen), filled in before
 };
 cudaError_t launch_tiles_few(const TileArgs &a, const int8_t *x, cudaStream_t s);
 cudaError_t launch_tiles(int qtype, int mode, const TileArgs &a, cudaStream_t s);
@@ -228,8 +229,9 @@ size_t tile_sums_bytes(long long rows, long long n_blocks);
 // launches by tile shape since the library was loaded: Q4_K gate/up with 3 / 4 activation digits, Q6_K down with up to 5 / 6,
 // Q4_K down with up to 5, Q4_K linear with 3 / up to 5, all others (counted on the device, where the digits are known)
 constexpr int TILE_SHAPES = 8;
-// ... and how many of the linear ones were shared by clusters, how many had 32 columns at four or five digits
-constexpr int TILE_FORMS = 2;
+// ... and how many of the linear ones were shared by clusters, how many had 32 columns at four or five
+// digits, and how many gate / up had tiles of eight rows
+constexpr int TILE_FORMS = 3;
 void tile_launch_counts(unsigned long long *out);      // [TILE_SHAPES + TILE_FORMS]
 
 // Re-order raw GGUF blocks into the half-tile layout; also reduces max |d| and max |dmin| half bit

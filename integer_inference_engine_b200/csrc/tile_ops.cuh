@@ -7,6 +7,7 @@
 namespace iie {
 
 constexpr unsigned TL_WAIT_LIMIT = 1u << 17;
+constexpr int TL_SIXTEEN_FROM = 288;
 
 __device__ __forceinline__ uint32_t tl_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void tl_init(uint32_t b, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b), "r"(n)); }
@@ -97,6 +98,12 @@ __device__ __forceinline__ void tl_tma(uint32_t dst, const CUtensorMap *map, int
 }
 __device__ __forceinline__ void tl_sts64(uint32_t a, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y)); }
 __device__ __forceinline__ void tl_sts32(uint32_t a, uint32_t x) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(x)); }
+
+// Whether gate / up tiles of sixteen rows take a call from those of eight, counted as each would have them: the weights are expanded once per
+// tile, in eight-row tiles at two thirds of the price, so that few experts with many rows each are quicker in the larger ones once they fill the
+// device.  128 experts, top 8, all tokens on the same eight: 64 / 100 / 128 tokens 126 / 172 / 194 us a block by eight rows, 109 / 153 / 169 by
+// sixteen, 48 tokens 101 / 99; spread over all 128 experts 231 / 264 / 291 against 267 / 288 / 307; 32 experts, top 4, 64 tokens on the same four 80 / 87.
+__device__ __forceinline__ bool tl_rows_of_sixteen(long long of8, long long of16) { return 2 * of8 > 3 * of16 + TL_SIXTEEN_FROM; }
 
 // digit planes carried for `nl` digits in use
 __device__ __forceinline__ int tl_planes(int nl) { return nl <= 3 ? 3 : nl <= 6 ? nl : 8; }

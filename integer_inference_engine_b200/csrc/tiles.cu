@@ -44,6 +44,7 @@
 namespace iie {
 
 __device__ unsigned long long d_tile_launches[TILE_SHAPES + TILE_FORMS];
+__device__ int d_tile_form;                                        // gate / up of the call under way (tile_rows_kernel)
 
 namespace {
 
@@ -84,11 +85,15 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
         if (Q4) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.s16)) : "memory");
         if (Q4) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.s32)) : "memory");
     }
+    if (MODE == MODE_GATEUP && a.few) {                            // tiles of eight rows may have the call
+        pdl_enter();
+        if (!*a.form) return;
+    }
     if (warp == TL_MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tl_u32(&s_tmem)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    pdl_enter();                                                   // what stands above needs nothing of the kernel before
+    if (MODE != MODE_GATEUP || !a.few) pdl_enter();                // what stands above needs nothing of the kernel before
     const int np = tl_planes(a.x_nl ? max(1, min(8, *a.x_nl)) : 8), ns = np + 1;        // uniform over the grid
     const bool wide = a.wide && (np == 3 || (!Q4 && (SPLIT ? np == 4 : a.wide == 2 && np <= 5)));      // (five digits beside the exchange: one stage)
     // Columns of a tile: 32 where the accumulators leave two TMEM buffers and the read-out's registers hold eight columns' sums: three planes, and
@@ -588,9 +593,18 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
 
 // Sums of the 32 columns of every sub-block as nine balanced digits, xs[row][9][stride] (columns from nb * 8 on are zero), and with
 // `xidx` the digit planes in use copied into pair order.  One thread per (row, sub-block).
+// With `form` the last block says which tiles of gate / up take the rows: 1 of sixteen, 0 of eight.
 __global__ void __launch_bounds__(256) tile_rows_kernel(const int8_t *xl, const int *xidx, const int *n_live, const int *x_nl,
-                                                        long long n_rows, int nb, int stride, int8_t *xg, int8_t *xs) {
+                                                        long long n_rows, int nb, int stride, int8_t *xg, int8_t *xs, const int *grp_off, int n_groups, int n_rt, int *form) {
     pdl_enter();
+    if (form && blockIdx.x == gridDim.x - 1) {
+        int of8 = 0, of16 = 0;
+        if (threadIdx.x >= 32) return;
+        for (int g = threadIdx.x; g < n_groups; g += 32) { const int rows = grp_off[g + 1] - grp_off[g]; of8 += (rows + 7) / 8; of16 += (rows + 15) / 16; }
+        of8 = __reduce_add_sync(0xffffffffu, of8); of16 = __reduce_add_sync(0xffffffffu, of16);
+        if (threadIdx.x == 0) *form = tl_rows_of_sixteen((long long)of8 * n_rt, (long long)of16 * n_rt) ? 1 : 0;
+        return;
+    }
     const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
     const int j = (int)(idx % stride);
     const long long row = idx / stride;
@@ -683,17 +697,25 @@ cudaError_t launch_tiles(int qtype, int mode, const TileArgs &args, cudaStream_t
     while (mode == MODE_LINEAR && a.split < 8 && 2 * a.split <= a.nb && whole <= (a.split == 1 ? 74 : a.split == 2 ? 33 : 15)) a.split *= 2;
     if (a.nb - (a.nb + a.split - 1) / a.split < (q4 ? 3 : a.wide ? 6 : 4)) a.split = 1;
     const int stride = (a.nb * 8 + 31) / 32 * 32;
+    // Gate / up by tiles of eight rows, and by those of sixteen beside them where the rows may lie on so few experts that these are quicker
+    // (tl_rows_of_sixteen): the kernel in front finds out for both; the launch that has nothing to do costs 1.5 us.
+    a.few = !a.few || !q4 || mode != MODE_GATEUP || !a.grp_off ? 0 : a.n_rows * ((a.out_f + 63) / 64) > 16LL * TL_SIXTEEN_FROM ? 2 : 1;
+    if (a.few) {
+        void *counts = nullptr, *form = nullptr;
+        if (cudaGetSymbolAddress(&counts, d_tile_launches) != cudaSuccess || cudaGetSymbolAddress(&form, d_tile_form) != cudaSuccess) return cudaErrorInvalidValue;
+        a.counts = static_cast<unsigned long long *>(counts); a.form = static_cast<int *>(form);
+        a.wide = 0;
+    }
     if ((q4 && !a.xs_ready) || a.xidx) {
         const long long n = a.n_rows * stride;
-        launch_behind(tile_rows_kernel, (unsigned)((n + 255) / 256), 256, 0, s, a.xl, a.xidx, a.grp_off ? a.grp_off + a.n_groups : nullptr, a.x_nl, a.n_rows, a.nb, stride, a.xg, q4 ? a.xs : nullptr);
+        launch_behind(tile_rows_kernel, (unsigned)((n + 255) / 256 + (a.few == 2)), 256, 0, s, a.xl, a.xidx, a.grp_off ? a.grp_off + a.n_groups : nullptr, a.x_nl, a.n_rows, a.nb, stride, a.xg, q4 ? a.xs : nullptr,
+                      a.grp_off, a.n_groups, (int)((a.out_f + 63) / 64), a.few == 2 ? a.form : nullptr);
         note_launch();
-    }
+    } else if (a.few) a.few = 1;
     const int8_t *x = a.xidx ? a.xg : a.xl;
-    if (a.few && q4 && mode == MODE_GATEUP && a.grp_off) {
-        void *counts = nullptr;
-        if (cudaGetSymbolAddress(&counts, d_tile_launches) != cudaSuccess) return cudaErrorInvalidValue;
-        a.counts = static_cast<unsigned long long *>(counts);
-        return launch_tiles_few(a, x, s);
+    if (a.few) {
+        const cudaError_t e = launch_tiles_few(a, x, s);
+        if (e != cudaSuccess || a.few == 1) return e;
     }
     TileMaps maps;
     const long long K = (long long)a.nb * 256;

@@ -81,14 +81,18 @@ __global__ void __launch_bounds__(TF_THREADS, 1) tile_few_kernel(const TileArgs 
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.x)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.s)) : "memory");
     }
+    if (a.few == 2) {                                              // the kernel before knows which form takes the call
+        pdl_enter();
+        if (*a.form) return;
+    }
     if (warp == TF_MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tl_u32(&s_tmem)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    pdl_enter();                                                   // what stands above needs nothing of the kernel before
+    if (a.few != 2) pdl_enter();                                   // what stands above needs nothing of the kernel before
     const int np = tl_planes(a.x_nl ? max(1, min(8, *a.x_nl)) : 8), walks = np > TF_PLANES ? 2 : 1;       // uniform over the grid
     const int n_rt = (int)((a.out_f + 63) / 64);
-    if (tid == 0 && blockIdx.x == 0) atomicAdd(a.counts + (np == 3 ? 0 : np == 4 ? 1 : 7), 1ULL);      // (as a gate / up tile of tiles.cu)
+    if (tid == 0 && blockIdx.x == 0) { atomicAdd(a.counts + (np == 3 ? 0 : np == 4 ? 1 : 7), 1ULL); atomicAdd(a.counts + TILE_SHAPES + 2, 1ULL); }      // (as a gate / up tile of tiles.cu, too)
     if (warp == 0) {                                               // first tile of every group
         int base = 0;
         for (int g0 = 0; g0 < a.n_groups; g0 += 32) {

@@ -350,7 +350,8 @@ def prefill_launch_counts() -> list:
 
 
 def tile_form_counts() -> list:
-    """Of those launches: [linear products whose tiles were shared by clusters, Q6_K tiles of 32 columns at four or five digits]."""
+    """Of those launches: [linear products whose tiles were shared by clusters, Q6_K tiles of 32 columns at four or five digits,
+    gate/up by tiles of eight rows]."""
     buf = (ctypes.c_uint64 * 8)()
     n = qk_cuda.load_library().iie_tile_form_counts(buf, 8)
     return [int(buf[i]) for i in range(n)]

@@ -129,6 +129,33 @@ def test_expert_tiles_match_the_oracle(down_q, d, eff, E, k, T, mult):
     layer.close()
 
 
+@pytest.mark.parametrize("T,distinct,eight", [(128, 1, 0), (128, 0, 1), (71, 1, 1), (73, 1, 0), (96, 2, 0), (40, 1, 1), (33, 0, 1)])
+def test_gate_up_tiles_follow_the_routing(T, distinct, eight):
+    """Tokens that all choose the same few experts (`distinct` different rows among them, 0: all) give those many rows each: tiles of sixteen rows.  Spread
+    over the experts, or too few to fill the device, they have tiles of eight."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(T + distinct)
+    d, eff, E, k = 256, 768, 128, 8
+    q4 = lambda r, c: o.synth_q4k(rng, r, c // 256)
+    router, gate, up, down = q4(E, d), [q4(eff, d) for _ in range(E)], [q4(eff, d) for _ in range(E)], [q4(d, eff) for _ in range(E)]
+    h = o.to_fixed(rng.standard_normal((T, d)), FA)
+    if distinct:
+        h = h[np.arange(T) % distinct] + rng.integers(-3, 4, size=(T, d))      # the same experts, other values
+    reg = lambda w, r, c: qk_cuda.register_weight(w, r, c // 256, o.Q4_K)
+    layer = device.MoELayer(reg(router, E, d), [reg(w, eff, d) for w in gate], [reg(w, eff, d) for w in up], [reg(w, d, eff) for w in down], k, d, eff)
+    device.read_flags()
+    before, shapes = device.tile_form_counts()[2], sum(device.prefill_launch_counts())
+    out, ids, gates = layer.forward(torch.from_numpy(h).cuda(), FA, FW)
+    assert device.tile_form_counts()[2] - before == eight and sum(device.prefill_launch_counts()) - shapes == 3
+    assert device.read_flags() == 0
+    ids_ref, gates_ref, out_ref = onat.moe_block(router, o.Q4_K, gate, up, down, o.Q4_K, o.Q4_K, k, h, d, eff, FA, FW)
+    assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
+    assert np.array_equal(out.cpu().numpy(), out_ref)
+    layer.close()
+
+
 def test_replays_of_a_short_graph_find_their_digit_count_cleared():
     """One product captured on its own: a replay over wide rows leaves the replays after it the digit planes that their rows need."""
     import torch
