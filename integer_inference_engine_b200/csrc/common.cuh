@@ -159,7 +159,7 @@ __host__ __device__ __forceinline__ uint32_t sigmoid_short(int64_t g, int fa, in
 #endif
 }
 
-// ((g * sigmoid(g)) >> fa) * u >> fa, the gated product of an expert.
+// ((g * sigmoid(g)) >> fa) * u >> fa, the gated product of an expert, for g > INT64_MIN (silu_up_any: for every g).
 __host__ __device__ __forceinline__ int64_t silu_up_fixed(int64_t g, int64_t u, int fa, int64_t log2e, int64_t clip) {
     if (fa > 24 || fa < 1) return mul_shift(mul_shift(g, sigmoid_fixed_c(g, fa, log2e, clip), fa), u, fa);
     const uint32_t sg = sigmoid_short(g, fa, log2e, clip);
@@ -173,7 +173,8 @@ __host__ __device__ __forceinline__ int64_t silu_up_fixed(int64_t g, int64_t u, 
     return mul_shift(silu, u, fa);
 #endif
 }
-// The same for every g: the distance of INT64_MIN wraps as in the general form.
+// The distance of INT64_MIN from zero wraps (at a scale of 2^16 its sigmoid is one half).  The tiles go through this one behind the loop over
+// their values, and only where one is INT64_MIN, so that the loop stays without branches.
 __host__ __device__ __forceinline__ int64_t silu_up_any(int64_t g, int64_t u, int fa, int64_t log2e, int64_t clip) {
     if (g == INT64_MIN) return mul_shift(mul_shift(g, sigmoid_fixed_c(g, fa, log2e, clip), fa), u, fa);
     return silu_up_fixed(g, u, fa, log2e, clip);

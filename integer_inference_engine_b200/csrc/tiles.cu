@@ -556,9 +556,16 @@ __global__ void __launch_bounds__(tl_threads(MODE), 1) tile_kernel(const TileArg
                 if (!(ok = tl_wait(y_full, pass, &s_abort))) break;
                 const long long *from = reinterpret_cast<const long long *>(exch) + half * 128 + r;
                 int64_t gu[8];
+                bool least = false;
 #pragma unroll
-                for (int i = 0; i < 8; i++)                        // every column, live or not: the chains interleave
-                    gu[i] = silu_up_fixed(from[2 * i * 128], from[2 * i * 128 + 64], a.fa, a.sig_log2e, a.sig_clip);
+                for (int i = 0; i < 8; i++) {                      // every column, live or not: the chains interleave
+                    const int64_t g = from[2 * i * 128];
+                    least |= g == INT64_MIN;
+                    gu[i] = silu_up_fixed(g, from[2 * i * 128 + 64], a.fa, a.sig_log2e, a.sig_clip);
+                }
+                if (least)
+#pragma unroll
+                    for (int i = 0; i < 8; i++) gu[i] = silu_up_any(from[2 * i * 128], from[2 * i * 128 + 64], a.fa, a.sig_log2e, a.sig_clip);
                 __syncwarp();
                 if (lane == 0) tl_arrive(y_free);
                 pass ^= 1;

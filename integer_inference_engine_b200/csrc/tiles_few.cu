@@ -370,11 +370,19 @@ __global__ void __launch_bounds__(TF_THREADS, 1) tile_few_kernel(const TileArgs 
             const int n = min(TF_BN, w.m_end - w.m0);
             const long long *from = reinterpret_cast<const long long *>(exch) + part * 128 + r;
             int64_t gu[TF_BN / 2];
+            bool least = false;
 #pragma unroll
             for (int i = 0; i < TF_BN / 2; i++) {
                 gu[i] = 0;
-                if ((i & ~1) * 2 < n) gu[i] = silu_up_fixed(from[2 * i * 128], from[2 * i * 128 + 64], a.fa, a.sig_log2e, a.sig_clip);      // four columns at a time
+                if ((i & ~1) * 2 < n) {                            // four columns at a time
+                    const int64_t g = from[2 * i * 128];
+                    least |= g == INT64_MIN;
+                    gu[i] = silu_up_fixed(g, from[2 * i * 128 + 64], a.fa, a.sig_log2e, a.sig_clip);
+                }
             }
+            if (least)
+#pragma unroll
+                for (int i = 0; i < TF_BN / 2; i++) gu[i] = silu_up_any(from[2 * i * 128], from[2 * i * 128 + 64], a.fa, a.sig_log2e, a.sig_clip);
             __syncwarp();
             if (lane == 0) tl_arrive(y_free);
             pass ^= 1;

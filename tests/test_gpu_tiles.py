@@ -252,6 +252,37 @@ def test_expert_tiles_at_other_activation_scales(fa):
     layer.close()
 
 
+@pytest.mark.parametrize("T", [3, 40])
+def test_gate_values_of_the_least_int64(T):
+    """A gate product of exactly -2^63, whose sigmoid is one half because its distance from zero wraps: both kinds of gate / up tiles."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    d, eff, E, k = 256, 256, 2, 2
+    def one_weight(d_half, col, code):                                         # rows of one block: scale 1, `code` at one of the first 32 columns
+        raw = np.zeros((eff, 144), np.uint8)
+        raw[:, 0:2] = np.frombuffer(np.float16(d_half).tobytes(), np.uint8)
+        raw[:, 4], raw[:, 16 + col] = 1, code
+        return raw.tobytes()
+    rng = np.random.default_rng(T)
+    gate, up = [one_weight(0.25, 0, 8)] * E, [one_weight(0.125, 1, 1)] * E
+    router, down = np.zeros((E, 144), np.uint8).tobytes(), [o.synth_q4k(rng, d, eff // 256) for _ in range(E)]
+    h = o.to_fixed(rng.standard_normal((T, d)), FA)
+    h[1, :2] = -(1 << 62), 1000                                                # gate -2^62 * 8 / 4, up 125
+    reg = lambda w, r, c: qk_cuda.register_weight(w, r, c // 256, o.Q4_K)
+    layer = device.MoELayer(reg(router, E, d), [reg(w, eff, d) for w in gate], [reg(w, eff, d) for w in up], [reg(w, d, eff) for w in down], k, d, eff)
+    device.read_flags()
+    before = device.tile_form_counts()[2]
+    out, ids, gates = layer.forward(torch.from_numpy(h).cuda(), FA, FW)
+    assert device.tile_form_counts()[2] - before == (T == 3)
+    assert device.read_flags() == 0
+    ids_ref, gates_ref, out_ref = onat.moe_block(router, o.Q4_K, gate, up, down, o.Q4_K, o.Q4_K, k, h, d, eff, FA, FW)
+    assert np.any(out_ref[1] != 0)
+    assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
+    assert np.array_equal(out.cpu().numpy(), out_ref)
+    layer.close()
+
+
 @pytest.mark.parametrize(("qtype", "out_f", "nb", "T", "tiles"), [(o.Q4_K, 40960, 1, 3, 0), (o.Q4_K, 40961, 1, 3, 1), (o.Q4_K, 300, 9, 2, 0), (o.Q4_K, 300, 9, 4, 1),
                                                                   (o.Q6_K, 5120, 8, 3, 0), (o.Q6_K, 5121, 8, 2, 1), (o.Q6_K, 64, 3, 4, 1), (o.Q4_K, 24, 48, 3, 1)])
 def test_dense_products_by_size(qtype, out_f, nb, T, tiles):

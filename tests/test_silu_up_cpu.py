@@ -8,6 +8,7 @@ from pathlib import Path
 import numpy as np
 import pytest
 
+from oracle import native as onat
 from oracle import qk_oracle as o
 
 ROOT = Path(__file__).resolve().parents[1]
@@ -39,3 +40,15 @@ def test_gated_product(lib, fa):
     small = np.abs(g) < (1 << 46)
     want = [(int(s) * int(v)) >> fa for s, v in zip(o.silu_int(g[small], fa), u[small])]
     assert [int(v) for v in y[small]] == [((w + (1 << 63)) % (1 << 64)) - (1 << 63) for w in want]
+
+
+@pytest.mark.parametrize("fa", [1, 8, 14, 15, 16, 24, 25])
+def test_gated_product_of_the_least_int64(lib, fa):
+    """The distance of INT64_MIN from zero wraps in the sigmoid, as NumPy's does."""
+    g = np.array([np.iinfo(np.int64).min, np.iinfo(np.int64).min + 1, np.iinfo(np.int64).max], np.int64)
+    u, y = np.full(3, 3, np.int64), np.empty(3, np.int64)
+    p = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
+    lib.h_silu_up_any(p(g), p(u), p(y), ctypes.c_longlong(3), fa)
+    sig = onat.sigmoid(g, fa)
+    wrapped = lambda v: (v + (1 << 63)) % (1 << 64) - (1 << 63)
+    assert list(y) == [wrapped((((int(a) * int(b)) >> fa) * 3) >> fa) for a, b in zip(g, sig)]
