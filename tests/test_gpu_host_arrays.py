@@ -52,6 +52,28 @@ def test_one_row_with_several_matrices(qtype, nb, widths, bits):
     qk_cuda.free_all()
 
 
+@pytest.mark.parametrize("formats,beyond,launches", [((o.Q4_K,) * 3, False, 2), ((o.Q6_K,) * 2, False, 2), ((o.Q4_K, o.Q6_K), False, 3), ((o.Q4_K,) * 5, False, 6),
+                                                      ((o.Q4_K,) * 3, True, 5), ((o.Q6_K,) * 4, True, 6), ((o.Q6_K, o.Q4_K), True, 5)])
+def test_launches_of_one_row_with_several_matrices(formats, beyond, launches):
+    """The digits and one launch for up to four matrices of one format, else a launch per matrix; a row beyond eight digits once more through the
+    exact kernel, matrix by matrix."""
+    from integer_inference_engine_b200 import device, qk_cuda
+    nb, widths = 3, (300, 40, 129, 8, 77)[:len(formats)]
+    raw = [(o.synth_q4k if q == o.Q4_K else o.synth_q6k)(np.random.default_rng(i), w, nb) for i, (q, w) in enumerate(zip(formats, widths))]
+    hs = [qk_cuda.register_weight(r, w, nb, q) for r, w, q in zip(raw, widths, formats)]
+    x = np.random.default_rng(9).integers(-(1 << 20), 1 << 20, size=(1, nb * 256), dtype=np.int64)
+    if beyond:
+        x[0, 300] = np.iinfo(np.int64).max
+    device.read_flags()
+    before = device.launch_count()
+    got = qk_cuda.apply_resident_grouped(hs, x, widths, FW)
+    assert device.launch_count() - before == launches
+    assert device.read_flags() == 0
+    for a, r, w, q in zip(got, raw, widths, formats):
+        assert np.array_equal(a, onat.qk_linear(r, x, w, nb, FW, q))
+    qk_cuda.free_all()
+
+
 def test_results_share_no_memory():
     import gc
 

@@ -328,3 +328,154 @@ def test_expert_blocks_by_size(d, eff, E, k, T, tiles):
     assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
     assert np.array_equal(out.cpu().numpy(), out_ref)
     layer.close()
+
+
+@pytest.mark.parametrize("qtype", [o.Q4_K, o.Q6_K])
+@pytest.mark.parametrize("T,xbits", [(9, 22), (9, 30), (16, 38), (9, 46), (9, 62), (130, 22), (130, 30), (130, 38)])
+def test_dense_tiles_beyond_those_that_clusters_share(qtype, T, xbits):
+    """The usual form over several super-blocks (their rings wrap; the minima of four share a row of sums), three to eight digits, narrow and wide
+    tiles, extreme blocks among the others."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    out_f, nb = (9500, 6) if T <= 16 else (2500, 9)
+    rng = np.random.default_rng(T + xbits)
+    raw = np.frombuffer((o.synth_q4k if qtype == o.Q4_K else o.synth_q6k)(rng, out_f, nb), np.uint8).copy().reshape(out_f * nb, -1)
+    raw[::5, slice(4, 144) if qtype == o.Q4_K else slice(0, 208)] = 0xFF
+    if qtype == o.Q6_K:
+        raw[1::5, 192:208] = 0x80
+    raw = raw.tobytes()
+    x = rng.integers(-(1 << xbits), 1 << xbits, size=(T, nb * 256), dtype=np.int64)
+    device.read_flags()
+    h = qk_cuda.register_weight(raw, out_f, nb, qtype)
+    before, shared = device.prefill_launch_counts(), device.tile_form_counts()[0]
+    got = device.apply(h, torch.from_numpy(x).cuda(), out_f, FW).cpu().numpy()
+    assert sum(device.prefill_launch_counts()) == sum(before) + 1 and device.tile_form_counts()[0] == shared
+    assert device.read_flags() == 0
+    assert np.array_equal(got, onat.qk_linear(raw, x, out_f, nb, FW, qtype))
+
+
+def _largest_blocks(qtype, rows, nb):
+    """The largest scales, minima and codes at the largest block scales the tiles take, with the smallest codes in every fourth row."""
+    raw = np.zeros((rows, nb, 144 if qtype == o.Q4_K else 210), np.uint8)
+    raw[:, :, slice(4, 144) if qtype == o.Q4_K else slice(0, 208)] = 0xFF
+    raw[1::4, :, 16 if qtype == o.Q4_K else 0:144 if qtype == o.Q4_K else 192] = 0
+    half = lambda v: np.frombuffer(np.float16(v).tobytes(), np.uint8)
+    if qtype == o.Q4_K:
+        raw[:, :, 0:2], raw[:, :, 2:4] = half(0.49975586), half(3.9980469)     # d below 2^23, dmin below 2^26 at 2^24
+    else:
+        raw[::2, :, 192:208] = 0x80                                            # scales of -128
+        raw[:, :, 208:210] = half(0.49975586)
+    return raw
+
+
+@pytest.mark.parametrize("qtype", [o.Q4_K, o.Q6_K])
+@pytest.mark.parametrize("T", [2, 33])
+def test_largest_sums_of_a_row_beyond_those_that_clusters_share(qtype, T):
+    """64 super-blocks of the largest blocks in the usual form: sixteen rows of them, repeated over more tiles than clusters take."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    nb, repeat = 64, 600
+    buf = _largest_blocks(qtype, 16, nb).tobytes()
+    h = qk_cuda.register_weight(buf * repeat, 16 * repeat, nb, qtype)
+    device.read_flags()
+    for digits in (3, 4, 5, 6, 8):
+        top = int.from_bytes(b"\x7f" * digits, "little")
+        x = np.full((T, nb * 256), -top, np.int64)
+        x[1::2] = top
+        before, shared = device.prefill_launch_counts(), device.tile_form_counts()[0]
+        got = device.apply(h, torch.from_numpy(x).cuda(), 16 * repeat, FW).cpu().numpy()
+        assert sum(device.prefill_launch_counts()) == sum(before) + 1 and device.tile_form_counts()[0] == shared
+        want = onat.qk_linear(buf, x[:2], 16, nb, FW, qtype)
+        assert np.array_equal(got.reshape(T, repeat, 16), np.broadcast_to(want[np.arange(T) % 2][:, None], (T, repeat, 16)))
+    assert device.read_flags() == 0
+    qk_cuda.free_all()
+
+
+@pytest.mark.parametrize("digits", [3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("T", [3, 8])
+def test_largest_sums_of_the_eight_row_tiles(digits, T):
+    """Gate / up over 64 super-blocks of the largest blocks, every value at one end of its digits: the 32-bit sums of a super-block and both walks at
+    their limits.  Successive super-blocks have opposite signs and the last two ordinary values, so that the products stay in range."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    d, eff, E, k, nb = 64 * 256, 256, 2, 2, 64
+    rng = np.random.default_rng(digits)
+    weights = []
+    for _ in range(2 * E):
+        raw = _largest_blocks(o.Q4_K, eff, nb)
+        raw[:, 62:] = np.frombuffer(o.synth_q4k(rng, eff, 2), np.uint8).reshape(eff, 2, 144)
+        raw[:, 2] = np.frombuffer(o.synth_q4k(rng, eff, 1), np.uint8).reshape(eff, 144)      # and a pair of another scale
+        raw[:, 3] = raw[:, 2]
+        weights.append(raw.tobytes())
+    gate, up, router = weights[:E], weights[E:], np.zeros((E * nb, 144), np.uint8).tobytes()
+    down = [o.synth_q4k(rng, d, eff // 256) for _ in range(E)]
+    top = int.from_bytes(b"\x7f" * digits, "little")
+    h = np.full((T, nb, 256), top, np.int64)
+    h[:, 1::2] = -top
+    h[1::3] = -h[1::3]
+    h[2::3, :, ::2] = 0
+    h[:, 62:] = rng.integers(-(1 << 17), 1 << 17, size=(T, 2, 256))
+    h = h.reshape(T, d)
+    reg = lambda w, r, c: qk_cuda.register_weight(w, r, c // 256, o.Q4_K)
+    layer = device.MoELayer(reg(router, E, d), [reg(w, eff, d) for w in gate], [reg(w, eff, d) for w in up], [reg(w, d, eff) for w in down], k, d, eff)
+    device.read_flags()
+    before = device.tile_form_counts()[2]
+    out, ids, gates = layer.forward(torch.from_numpy(h).cuda(), FA, FW)
+    assert device.tile_form_counts()[2] - before == 1
+    assert device.read_flags() == 0
+    ids_ref, gates_ref, out_ref = onat.moe_block(router, o.Q4_K, gate, up, down, o.Q4_K, o.Q4_K, k, h, d, eff, FA, FW)
+    assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
+    assert np.array_equal(out.cpu().numpy(), out_ref)
+    layer.close()
+
+
+@pytest.mark.parametrize("fa", [1, 5, 12, 20, 24, 25])
+def test_eight_row_tiles_at_other_activation_scales(fa):
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    rng = np.random.default_rng(fa)
+    d, eff, E, k, T = 256, 256, 5, 2, 17
+    q4 = lambda r, c: o.synth_q4k(rng, r, c // 256)
+    router, gate, up, down = q4(E, d), [q4(eff, d) for _ in range(E)], [q4(eff, d) for _ in range(E)], [q4(d, eff) for _ in range(E)]
+    h = np.rint(rng.standard_normal((T, d)) * np.exp2(rng.uniform(-3, 9, size=(T, 1))) * (1 << fa)).astype(np.int64)
+    reg = lambda w, r, c: qk_cuda.register_weight(w, r, c // 256, o.Q4_K)
+    layer = device.MoELayer(reg(router, E, d), [reg(w, eff, d) for w in gate], [reg(w, eff, d) for w in up], [reg(w, d, eff) for w in down], k, d, eff)
+    device.read_flags()
+    before = device.tile_form_counts()[2]
+    out, ids, gates = layer.forward(torch.from_numpy(h).cuda(), fa, FW)
+    assert device.tile_form_counts()[2] - before == 1
+    ids_ref, gates_ref, out_ref = onat.moe_block(router, o.Q4_K, gate, up, down, o.Q4_K, o.Q4_K, k, h, d, eff, fa, FW)
+    assert device.read_flags() == 0
+    assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
+    assert np.array_equal(out.cpu().numpy(), out_ref)
+    layer.close()
+
+
+@pytest.mark.parametrize("T,eight", [(5, 0), (6, 1), (64, 1), (65, 0)])
+def test_eight_row_tiles_by_size(T, eight):
+    """Both borders of the eight-row tiles: the experts that are met have tiles for the device, eight rows per expert."""
+    import torch
+
+    from integer_inference_engine_b200 import device, qk_cuda
+    qk_cuda.load_library().iie_set_tc_min_tokens(0)
+    rng = np.random.default_rng(T)
+    d, eff, E, k = 1024, 768, 32, 4
+    q4 = lambda r, c: o.synth_q4k(rng, r, c // 256)
+    router, gate, up = q4(E, d), [q4(eff, d) for _ in range(E)], [q4(eff, d) for _ in range(E)]
+    down = [o.synth_q6k(rng, d, eff // 256) for _ in range(E)]
+    h = o.to_fixed(rng.standard_normal((T, d)), FA)
+    reg = lambda w, r, c, q=o.Q4_K: qk_cuda.register_weight(w, r, c // 256, q)
+    layer = device.MoELayer(reg(router, E, d), [reg(w, eff, d) for w in gate], [reg(w, eff, d) for w in up], [reg(w, d, eff, o.Q6_K) for w in down], k, d, eff)
+    device.read_flags()
+    before = device.tile_form_counts()[2]
+    out, ids, gates = layer.forward(torch.from_numpy(h).cuda(), FA, FW)
+    assert device.tile_form_counts()[2] - before == eight
+    assert device.read_flags() == 0
+    ids_ref, gates_ref, out_ref = onat.moe_block(router, o.Q4_K, gate, up, down, o.Q4_K, o.Q6_K, k, h, d, eff, FA, FW)
+    assert np.array_equal(ids.cpu().numpy(), ids_ref) and np.array_equal(gates.cpu().numpy(), gates_ref)
+    assert np.array_equal(out.cpu().numpy(), out_ref)
+    layer.close()
