@@ -379,17 +379,19 @@ bool moe_fused(const MoePlan &p, const int8_t *hl, long long rows, const int *xi
             td.out_f = p.d_model; td.fw = fw; td.fa = fa; td.xl = gul; td.x_nl = g_cells + 1; td.out = out; td.gates = pair_gate; td.pair_tok = pair_tok;
             const bool by_size = g_tc_min_tokens == 0 && rows < TILES_FROM;
             // Up to eight rows per expert on average gate / up takes tiles of eight rows and unscaled codes (tiles_few.cu), as long as the
-            // experts that are met have tiles for a good part of the device: 128 experts, top 8, 16 / 32 / 64 / 128 tokens 156 / 196 / 233 / 294 us
-            // for the block (177 / 219 / 263 / 303 without), 160 tokens 323 (313); 32 experts, top 4, 2 / 32 tokens 44 / 96 (46 / 109); 8
-            // experts of 768 x 2048, top 2, 4 / 16 tokens 49 / 54 (44 / 54), 16 of 512 x 1024 3 us slower throughout.
+            // experts that are met (of rows spread evenly) have tiles for a good part of the device; rows on few experts: launch_tiles.  Experts of
+            // 768 x 2048, us for the block: 128 experts, top 8, 16 / 32 / 64 / 96 tokens 159 / 182 / 229 / 259 (without 171 / 210 / 256 / 264), 128
+            // tokens even, 160 325 (322); 32 experts, top 4, 8 / 32 / 64 tokens 68 / 97 / 110 (72 / 111 / 116); 16, top 2, 8 / 64 tokens 50 / 69 (52 /
+            // 78).  At the line, 8 experts, top 2, 16 tokens (614) 51 (50), 32 tokens (683) 55 (60); 32, top 4, 2 tokens (614) 45 (44).  Below it, 4
+            // experts, top 2, 4 tokens 46 (40), 16 of 512 x 1024, 16 tokens 44 (41).
             const double met = (double)n_pairs * n_groups / (n_pairs + n_groups);
-            tg.few = n_pairs <= 8LL * n_groups && (g_tc_min_tokens > 0 || met * (double)(p.e_ffn / 64) * (double)(p.d_model / 256) >= 600.0);
+            tg.few = n_pairs <= 8LL * n_groups && (g_tc_min_tokens > 0 || met * (double)(p.e_ffn / 64) * (double)(p.d_model / 256) >= 650.0);
             // Otherwise, gate / up below three rows per expert on average: the warp-level kernel, which multiplies one row at a time without a
-            // tile's padding, is the faster one (16 tokens over 128 experts 81 against 88 us, 45 tokens 139 / 141, 64 tokens 163 / 135), and
-            // where all tiles together are a fraction of a wave, so that one tile's walk and its epilogue are the launch (gate / up of 768 x
-            // 2048: 4 experts, 16 pairs 8 us less than the tiles, 64 pairs 1 to 9, 128 pairs 4 to 16 more; 16 experts 64 pairs 5 less, 128 pairs 2
-            // to 10 more; of 256 x 256 10 us less throughout).  Down takes the tiles (16 tokens over 128 experts 55 against 78 us) from eight
-            // pairs on: below them the warp-level kernel takes row by row and is up to 5 us quicker.
+            // tile's padding, is the faster one, and where all tiles together are a fraction of a wave, so that one tile's walk and its epilogue
+            // are the launch.  Blocks, warp-level (tiles of sixteen rows): 4 experts of 768 x 2048, top 2, 8 / 16 / 32 tokens 48 / 48 / 53 us (55 /
+            // 55 / 66), 64 tokens 78 (74); 16 of 512 x 1024, 16 / 64 tokens 41 / 50 (50 / 56), 100 tokens 64 (64); 4 of 256 x 256, 8 / 32 / 128 tokens 30 /
+            // 32 / 36 (40 / 47 / 48); 128 of 768 x 2048, 160 tokens 399 (322), 32, 66 tokens 138 (115).  Down takes the tiles (16 tokens over 128 experts
+            // 55 against 78 us) from eight pairs on: below them the warp-level kernel takes row by row and is up to 5 us quicker.
             const bool gate_tiles = tg.few || (n_pairs >= 3LL * n_groups && (!by_size || n_pairs * (p.e_ffn / 64) * (p.d_model / 256) >= 8192));
             const bool down_tiles = !by_size || n_pairs >= 8;
             auto either = [&](bool first, int q, int mode, const TileArgs &t, const BatchArgs &b) {

@@ -102,7 +102,8 @@ __device__ __forceinline__ void tl_sts32(uint32_t a, uint32_t x) { asm volatile(
 // Whether gate / up tiles of sixteen rows take a call from those of eight, counted as each would have them: the weights are expanded once per
 // tile, in eight-row tiles at two thirds of the price, so that few experts with many rows each are quicker in the larger ones once they fill the
 // device.  128 experts, top 8, all tokens on the same eight: 64 / 100 / 128 tokens 126 / 172 / 194 us a block by eight rows, 109 / 153 / 169 by
-// sixteen, 48 tokens 101 / 99; spread over all 128 experts 231 / 264 / 291 against 267 / 288 / 307; 32 experts, top 4, 64 tokens on the same four 80 / 87.
+// sixteen; spread over all 128 experts 221 / 259 (96 tokens) / 280 against 255 / 264 / 284; 32 experts, top 4, 64 tokens on the same four 79 / 79.  (48
+// tokens on the same eight, 99 / 89, stay with eight rows: the second launch would be every call's of 33 tokens and more.)
 __device__ __forceinline__ bool tl_rows_of_sixteen(long long of8, long long of16) { return 2 * of8 > 3 * of16 + TL_SIXTEEN_FROM; }
 
 // digit planes carried for `nl` digits in use

@@ -455,7 +455,7 @@ def test_eight_row_tiles_at_other_activation_scales(fa):
     layer.close()
 
 
-@pytest.mark.parametrize("T,eight", [(5, 0), (6, 1), (64, 1), (65, 0)])
+@pytest.mark.parametrize("T,eight", [(5, 0), (6, 1), (64, 1), (65, 0)])      # 591 and 658 of 650
 def test_eight_row_tiles_by_size(T, eight):
     """Both borders of the eight-row tiles: the experts that are met have tiles for the device, eight rows per expert."""
     import torch
