@@ -688,8 +688,10 @@ bool head_rows(const Q1Stack &m, const int64_t *x, long long rows, int64_t *logi
 
 // The same for a step's rows, the output matrix in two halves of whole waves where it is large: the first half's logits are on their way to
 // the host while the second is multiplied (7 MB take 130 us, the product of six rows 120), as long as nothing was refused: behind the first
-// half the flags say all that they will but whether a wait of the second product gave up.  `first`: rows of the first half, 0 for one
-// piece; its logits [rows][first] lie in front of the others'.
+// half the flags say all that they will but whether a wait of the second product gave up.  No tile of either half is split among CTAs
+// (q1_tc_split), which up to 64 tokens takes four waves of tiles each: a matrix of fewer than 151552 rows is one piece (a step of two layers and
+// six sequences 457 us with 151936 rows in halves, 464 with 128256 in one piece).  `first`: rows of the first half, 0 for one piece; its logits
+// [rows][first] lie in front of the others'.
 cudaStream_t q_copy = nullptr;
 cudaEvent_t q_half = nullptr;
 long long head_first(const Q1Stack &m, long long rows) {

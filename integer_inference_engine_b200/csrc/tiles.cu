@@ -30,8 +30,8 @@
 // spill, 1 % of the instructions.  One tile walks its super-blocks one behind the other, 1.3 us each: of a dense product with few tiles
 // the CTAs of a cluster take a share of them each and join their sums through distributed shared memory (launch_tiles), calls of two and
 // three rows are dispatched elsewhere (api.cu).
-// Per block at 2048 tokens: gate / up 840 us, down 670, 5120 x 2048 dense 240 (fully dequantised weights in four or five digits: 940, 1140,
-// 280); at 64 tokens 130, 80, 21 (warp-level MMAs: 165, 190, 45).
+// Per block at 2048 tokens, in a profile: gate / up 880 us, down 583 (fully dequantised weights in four or five digits: 940, 1140); dense with the
+// digits in front, 5120 x 2048: 2048 rows 277, 64 rows 23.5; at 64 tokens down 80 (warp-level MMAs 190; gate / up: tiles_few.cu).
 // Every wait is bounded; on a time-out the CTA raises flag bit 3, leaves its loops, frees TMEM and exits.
 #include <algorithm>
 #include <type_traits>
